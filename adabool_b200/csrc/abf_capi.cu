@@ -153,17 +153,35 @@ struct abf_workspace {
 struct abf_worker {
     abf_index* ix = nullptr;
     int kind = 0;  // 0 sparse, 1 dense (host bitmaps copied), 2 dense (caller device bitmaps)
-    // sparse
-    uint64_t n_keys = 0;
+    void* arena = nullptr;          // the one allocation behind every pointer below but d_ext
+    // the lists to merge: sparse, the keys as given; dense, the terms of a
+    // window of query bitmaps, extracted when the worker runs
+    uint64_t n_keys = 0;            // sparse
+    uint32_t term_cap = 0;          // room in d_keys
     uint32_t* d_keys = nullptr;
-    uint64_t* d_off1 = nullptr;     // {0, n_keys}: the keys as one query
-    uint64_t* d_offk = nullptr;     // 0..n_keys: every key its own query
+    uint64_t* d_off1 = nullptr;     // sparse: {0, n_keys}, the keys as one query
+    uint64_t* d_off = nullptr;      // offsets of the queries (sparse: runs of keys with one bitmap index)
+    uint32_t* d_slot = nullptr;     // sparse: bitmap index of each run
+    uint32_t* d_n_q = nullptr;      // sparse: number of runs; dense: overflow word of the term lists
+    uint32_t* d_cnt = nullptr;      // dense: terms per query
+    // planning scratch (see PlanArgs); the dense-bitmap lists and saturation
+    // marks cover the first q_cap queries or runs
+    uint32_t q_cap = 0;
     uint32_t* d_heavy = nullptr;
     uint32_t* d_lpref = nullptr;
     uint32_t* d_tile_cls = nullptr;
     uint64_t* d_lcnt = nullptr;
     uint64_t* d_lpref_q = nullptr;
     uint32_t* d_nprobe = nullptr;
+    uint16_t* d_dense16 = nullptr;
+    uint32_t* d_dstart = nullptr;
+    uint32_t* d_ndense = nullptr;
+    uint32_t* d_dmode = nullptr;
+    uint32_t* d_sat = nullptr;
+    uint32_t sat_stride = 0;
+    uint32_t* d_err = nullptr;
+    uint64_t dense_keys = 0;        // sparse: keys whose lists have dense bitmaps, and their postings
+    uint64_t dense_postings = 0;
     // dense
     uint64_t batch = 0;
     uint64_t len = 0;               // bytes per query bitmap as given
@@ -208,6 +226,8 @@ abf_status download_vec(std::vector<T>& v, const T* src, uint64_t n) {
 
 uint64_t n_words_of(uint64_t n_bits) { return (n_bits + 31) / 32; }
 uint64_t round4(uint64_t x) { return (x + 3) & ~uint64_t(3); }
+// words of one query's saturation marks: a bit per 32-word tile
+uint32_t sat_words(const abf_index* ix) { return uint32_t((n_words_of(ix->n_ads) + 32u * 32u - 1u) / (32u * 32u)); }
 
 void default_tuning(abf_index* ix) {
     abf_tuning& t = ix->tuning;
@@ -365,7 +385,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     w->probe_stride = round4(n_words_of(ix->n_terms));
     w->chunks_per_q = abf::compact_chunks(std::max<uint64_t>(max_bits, ix->n_ads));
     const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
-    w->sat_stride = uint32_t((n_words_of(ix->n_ads) + 32u * 32u - 1u) / (32u * 32u));
+    w->sat_stride = sat_words(ix);
     abf_status st;
     if ((st = dev_alloc(&w->heavy, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->tile_cls, max_terms)) != ABF_OK ||
@@ -427,6 +447,61 @@ abf_status run_compact(abf_index* ix, const abf::CompactArgs& ca, cudaStream_t s
     return ABF_OK;
 }
 
+// The merge kernel's tile shape for n_q queries: a batch too small to fill the
+// GPU at the tuned shape (the tuner sees large batches) gets full 8-warp CTAs
+// first, then narrower tiles.
+abf_tuning tile_shape(const abf_index* ix, uint64_t n_q) {
+    abf_tuning t = ix->tuning;
+    if (t.fixed_tile_shape) return t;
+    const uint64_t n_words = n_words_of(ix->n_ads);
+    const uint64_t want = 4ull * uint64_t(ix->sm_count) * 256u;  // threads
+    auto threads = [&]() { return n_q * ((n_words + t.tile_words - 1) / t.tile_words) * t.warps_per_tile * 32u; };
+    while (t.warps_per_tile < 8 && threads() < want) t.warps_per_tile *= 2;
+    while (t.tile_words > 1024 && threads() < want) t.tile_words >>= 1;
+    return t;
+}
+
+// Tile width and stages of the dense group kernel for windows of wq queries
+// with about `lists` dense-list entries in all; off when the dense bitmaps
+// (plus the zero row) do not fit three TMA boxes of 256.
+struct GroupShape {
+    bool on = false;
+    uint32_t gw = 32, stages = 2;
+};
+// 64-word tiles (two words per lane: half the index work per word) in two
+// stages where those and the lists fit shared memory; else one 64-word stage
+// wherever it fits: the kernel keeps the window's lists in shared memory
+// beside it when they fit and reads them from global memory otherwise;
+// 32-word tiles cost twice the index work per word (c1, 512-query windows:
+// 5.60 against 7.46 ms per step). out8: the output rows are 8-byte aligned
+// (64-word tiles store two words at once; ORing into them needs no alignment).
+GroupShape group_shape(abf_index* ix, const abf::IndexView& v, uint32_t wq, uint64_t lists, bool out8) {
+    GroupShape g;
+    const uint32_t rows = v.n_dense + 1;
+    if (v.n_dense == 0 || rows > abf::kGroupMaxBoxes * abf::kGroupBoxRows) return g;
+    if (out8 && abf::dense_group_list_cap(rows, wq, 64, 2) >= lists) {
+        g.gw = 64;
+    } else if (out8 && abf::dense_group_list_cap(rows, wq, 64, 1) > 0) {
+        g.gw = 64;
+        g.stages = 1;
+    }
+    if (ix->tuning.group_tile_words == 32) {
+        g.gw = 32;
+        g.stages = abf::dense_group_list_cap(rows, wq, 32, 2) > 0 ? 2u : 1u;
+    }
+    g.on = true;
+    if (ix->dense_tmap_base != ix->dev.dense || ix->dense_tmap_rows != v.n_dense || ix->dense_tmap_gw != g.gw) {
+        if (abf::encode_dense_tmap(v, g.gw, ix->dense_tmap) == cudaSuccess) {
+            ix->dense_tmap_base = ix->dev.dense;
+            ix->dense_tmap_rows = v.n_dense;
+            ix->dense_tmap_gw = g.gw;
+        } else {
+            g.on = false;
+        }
+    }
+    return g;
+}
+
 abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const RunOpts& ro, cudaStream_t s) {
     if (b->n_queries == 0) return ABF_OK;
     if (b->n_queries > ws->max_q) return fail(ABF_ERR_CAPACITY, "batch has more queries than the workspace");
@@ -481,17 +556,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     ta.q_off = b->d_offsets;
     ta.heavy_min = ws->heavy;
     ta.n_q = b->n_queries;
-    // a batch too small to fill the GPU at the tuned tile shape (the tuner
-    // sees large batches) gets full 8-warp CTAs first, then narrower tiles
-    abf_tuning tt = t;
-    if (!t.fixed_tile_shape) {
-        const uint64_t want = 4ull * uint64_t(ix->sm_count) * 256u;  // threads
-        auto threads = [&]() {
-            return uint64_t(b->n_queries) * ((n_words + tt.tile_words - 1) / tt.tile_words) * tt.warps_per_tile * 32u;
-        };
-        while (tt.warps_per_tile < 8 && threads() < want) tt.warps_per_tile *= 2;
-        while (tt.tile_words > 1024 && threads() < want) tt.tile_words >>= 1;
-    }
+    const abf_tuning tt = tile_shape(ix, b->n_queries);
     ta.n_tiles = uint32_t((n_words + tt.tile_words - 1) / tt.tile_words);
     ta.out = b->d_bitmaps;
     ta.out_stride = b->bitmap_stride_words;
@@ -505,41 +570,16 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     ta.tile_list = ws->tile_list;
     ta.n_tile_list = ws->n_tile_list;
     // dense group kernel: the dense lists of every non-probe query in one pass per
-    // tile, when the batch is large enough and the dense bitmaps (plus the
-    // zero row) fit three TMA boxes of 256. Tiles of 64 words (two per lane:
-    // half the index work per word) where two such stages and the batch's
-    // lists (room for 64 per query) fit shared memory and the output rows
-    // are 8-byte aligned, else 32 words.
+    // tile, when the batch is large enough (room for 64 list entries per query)
     const uint32_t n_dense = v.n_dense;
-    bool group = t.group_min_queries && b->n_queries >= t.group_min_queries && n_dense > 0 &&
-                 n_dense + 1 <= abf::kGroupMaxBoxes * abf::kGroupBoxRows;
-    const uint32_t wq = std::min<uint32_t>(b->n_queries, abf::kGroupMaxQueries);
-    const bool out8 = reinterpret_cast<uintptr_t>(b->d_bitmaps) % 8 == 0 && b->bitmap_stride_words % 2 == 0;
-    uint32_t gw = 32, stages = 2;
-    if (out8 && abf::dense_group_list_cap(n_dense + 1, wq, 64, 2) >= 64u * wq) {
-        gw = 64;
-    } else if (out8 && abf::dense_group_list_cap(n_dense + 1, wq, 64, 1) > 0) {
-        // one 64-word stage wherever it fits: the kernel keeps the window's
-        // lists in shared memory beside it when they fit and reads them from
-        // global memory otherwise; 32-word tiles cost twice the index work
-        // per word (c1, 512-query windows: 5.60 against 7.46 ms per step)
-        gw = 64;
-        stages = 1;
+    GroupShape gs;
+    if (t.group_min_queries && b->n_queries >= t.group_min_queries) {
+        const uint32_t wq = std::min<uint32_t>(b->n_queries, abf::kGroupMaxQueries);
+        const bool out8 = reinterpret_cast<uintptr_t>(b->d_bitmaps) % 8 == 0 && b->bitmap_stride_words % 2 == 0;
+        gs = group_shape(ix, v, wq, 64ull * wq, out8);
     }
-    if (t.group_tile_words == 32) {
-        gw = 32;
-        stages = abf::dense_group_list_cap(n_dense + 1, wq, 32, 2) > 0 ? 2u : 1u;
-    }
-    if (group && (ix->dense_tmap_base != ix->dev.dense || ix->dense_tmap_rows != n_dense ||
-                  ix->dense_tmap_gw != gw)) {
-        if (abf::encode_dense_tmap(v, gw, ix->dense_tmap) == cudaSuccess) {
-            ix->dense_tmap_base = ix->dev.dense;
-            ix->dense_tmap_rows = n_dense;
-            ix->dense_tmap_gw = gw;
-        } else {
-            group = false;
-        }
-    }
+    const bool group = gs.on;
+    const uint32_t gw = gs.gw, stages = gs.stages;
     ta.skip_dense_only = group ? 1 : 0;
     // the group kernel marks each (query, tile) it leaves all ones; the
     // scatter then skips ORs into those tiles
@@ -580,6 +620,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         sa.sat = ws->sat;
         sa.sat_stride = ws->sat_stride;
         sa.sat_shift = gw == 64u ? 6u : 5u;
+        sa.sat_last = b->n_queries - 1;
     }
     TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
     if (maybe_probe) {
@@ -618,30 +659,172 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     return ABF_OK;
 }
 
-abf_status worker_plan_scratch(abf_worker* w, uint64_t n_q) {
-    ABF_TRY(dev_alloc(&w->d_heavy, n_q));
-    ABF_TRY(dev_alloc(&w->d_lpref, std::max<uint64_t>(w->n_keys, 1)));
-    ABF_TRY(dev_alloc(&w->d_tile_cls, std::max<uint64_t>(w->n_keys, 1)));
-    ABF_TRY(dev_alloc(&w->d_lcnt, n_q));
-    ABF_TRY(dev_alloc(&w->d_lpref_q, n_q + 1));
-    ABF_TRY(dev_alloc(&w->d_nprobe, 1));
+// ---- workers ----
+constexpr uint32_t kKeyRunCap = 256;    // runs of a keyed batch merged by the group kernel; later ones are scattered
+constexpr uint32_t kOneQueryKeys = 2048; // keys that one planning CTA takes in a few steps of 256
+constexpr uint32_t kTermWindow = 256;   // query bitmaps extracted and merged at a time
+
+// One allocation for all of a worker's arrays: take() once to size it, once
+// more over the allocation to place them.
+struct Arena {
+    char* base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, uint64_t n) {
+        used = (used + 255) & ~size_t(255);
+        if (base) p = reinterpret_cast<T*>(base + used);
+        used += std::max<uint64_t>(n, 1) * sizeof(T);
+    }
+};
+
+// arrays of a worker that plans at most n_q queries over w->term_cap terms
+void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
+    a.take(w->d_off1, 2);  // followed at once by the keys: one upload
+    w->d_keys = reinterpret_cast<uint32_t*>(w->d_off1 + 2);
+    a.used += uint64_t(w->term_cap) * sizeof(uint32_t);
+    a.take(w->d_off, n_q + 1);
+    a.take(w->d_heavy, n_q);
+    a.take(w->d_lpref, w->term_cap);
+    a.take(w->d_tile_cls, w->term_cap);
+    a.take(w->d_lcnt, n_q);
+    a.take(w->d_lpref_q, n_q + 1);
+    a.take(w->d_nprobe, 1);
+    a.take(w->d_n_q, 1);
+    a.take(w->d_err, 1);
+    a.take(w->d_dense16, w->term_cap + 8ull * w->q_cap + 16);
+    a.take(w->d_dstart, w->q_cap);
+    a.take(w->d_ndense, w->q_cap);
+    a.take(w->d_dmode, w->q_cap);
+    a.take(w->d_sat, (uint64_t(w->q_cap) + 1) * w->sat_stride);
+    if (w->kind == 0) a.take(w->d_slot, n_q);
+    else a.take(w->d_cnt, n_q);
+    if (w->kind == 1) a.take(w->d_qbm, std::max<uint64_t>(w->batch, 1) * w->qbm_stride);
+}
+
+abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
+    w->sat_stride = sat_words(w->ix);
+    Arena a;
+    worker_take(w, a, n_q);
+    char* p = nullptr;
+    ABF_TRY(dev_alloc(&p, a.used));
+    w->arena = p;
+    a = Arena{p, 0};
+    worker_take(w, a, n_q);
     return ABF_OK;
 }
 
 void worker_release(abf_worker* w) {
-    dev_free(w->d_keys);
-    dev_free(w->d_off1);
-    dev_free(w->d_offk);
-    dev_free(w->d_heavy);
-    dev_free(w->d_lpref);
-    dev_free(w->d_tile_cls);
-    dev_free(w->d_lcnt);
-    dev_free(w->d_lpref_q);
-    dev_free(w->d_nprobe);
-    dev_free(w->d_qbm);
+    if (w->arena) cudaFree(w->arena);
+    w->arena = nullptr;
 }
 
-// plan + scatter (and, for one query, merge tiles) of a sparse worker
+// Plan, merge and scatter of a worker's lists, ORed into d_res: n_q queries
+// (or, with d_n_q, at most n_q of them) over w->d_keys.
+struct WorkerRun {
+    const uint64_t* q_off;
+    uint32_t n_q;
+    const uint32_t* d_n_q = nullptr;
+    const uint32_t* out_slot = nullptr;
+    const uint32_t* key_slot = nullptr;
+    uint32_t* out;
+    uint64_t out_stride;
+    bool tiles;        // merge long lists with the tile kernel (one owner per bitmap)
+    GroupShape group;  // else, if on, with the dense group kernel; else scatter every list
+};
+
+abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const WorkerRun& r, cudaStream_t s) {
+    abf_index* ix = w->ix;
+    const abf_tuning& t = ix->tuning;
+    const uint64_t n_words = n_words_of(ix->n_ads);
+    const bool group = !r.tiles && r.group.on;
+    const uint32_t nd_q = std::min<uint32_t>(r.n_q, w->q_cap);  // queries with dense lists and marks
+    abf::PlanArgs pa{};
+    pa.terms = w->d_keys;
+    pa.q_off = r.q_off;
+    pa.n_q = r.n_q;
+    pa.d_n_q = r.d_n_q;
+    pa.path_uniform = r.tiles ? ABF_PATH_HYBRID : ABF_PATH_UNION;
+    pa.hybrid_min = t.heavy_min_len;
+    pa.heavy_min = w->d_heavy;
+    pa.term_lpref = w->d_lpref;
+    pa.q_light_cnt = w->d_lcnt;
+    pa.n_probe = w->d_nprobe;  // not reached: no query takes the probe path
+    pa.probe_cap = 0;
+    pa.max_terms = w->term_cap;
+    pa.dense_in_tile = r.tiles || group ? 1 : 0;
+    if (r.tiles) pa.tile_cls = w->d_tile_cls;
+    if (group) {
+        pa.no_dense_from = nd_q;
+        pa.q_dense16 = w->d_dense16;
+        pa.q_dstart = w->d_dstart;
+        pa.q_ndense = w->d_ndense;
+        pa.q_dmode = w->d_dmode;
+        CUDA_TRY(cudaMemsetAsync(w->d_sat, 0, (uint64_t(nd_q) + 1) * w->sat_stride * 4u, s));
+    }
+    TIMED(K_PLAN, abf::launch_plan(v, pa, s));
+    abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, r.n_q, r.d_n_q};
+    TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
+    if (group) {
+        abf::DenseGroupArgs ga{};
+        ga.q_dense16 = w->d_dense16;
+        ga.q_dstart = w->d_dstart;
+        ga.q_ndense = w->d_ndense;
+        ga.q_dmode = w->d_dmode;
+        ga.n_q = nd_q;
+        ga.d_n_q = r.d_n_q;
+        ga.n_rows = v.n_dense + 1;
+        ga.stages = r.group.stages;
+        ga.list_cap = abf::dense_group_list_cap(ga.n_rows, ga.n_q, r.group.gw, r.group.stages);
+        ga.n_tiles = uint32_t((n_words + r.group.gw - 1) / r.group.gw);
+        ga.out = r.out;
+        ga.out_stride = r.out_stride;
+        ga.out_slot = r.out_slot;
+        ga.n_words = n_words;
+        ga.err = w->d_err;
+        ga.spin_limit = abf::kDefaultSpinLimit;
+        ga.sat = w->d_sat;
+        ga.sat_stride = w->sat_stride;
+        ga.accumulate = 1;
+        TIMED(K_GROUP, abf::launch_dense_group(ix->dense_tmap, r.group.gw, ga, ix->sm_count, s));
+    }
+    if (r.tiles) {
+        const abf_tuning tt = tile_shape(ix, r.n_q);
+        abf::TileArgs ta{};
+        ta.tile_cls = w->d_tile_cls;
+        ta.q_off = r.q_off;
+        ta.heavy_min = w->d_heavy;
+        ta.n_q = r.n_q;
+        ta.n_tiles = uint32_t((n_words + tt.tile_words - 1) / tt.tile_words);
+        ta.out = r.out;
+        ta.out_stride = r.out_stride;
+        ta.n_words = n_words;
+        ta.accumulate = 1;
+        ta.vec_ok = (reinterpret_cast<uintptr_t>(r.out) % 16 == 0) && (r.out_stride % 4 == 0);
+        TIMED(K_TILE, abf::launch_tile_union(v, ta, tt, ix->sm_count, s));
+    }
+    abf::ScatterArgs sa{};
+    sa.terms = w->d_keys;
+    sa.q_off = r.q_off;
+    sa.term_lpref = w->d_lpref;
+    sa.q_light_pref = w->d_lpref_q;
+    sa.n_q = r.n_q;
+    sa.d_n_q = r.d_n_q;
+    sa.out_slot = r.out_slot;
+    sa.key_slot = r.key_slot;
+    sa.out = r.out;
+    sa.out_stride = r.out_stride;
+    sa.blocks_per_warp = std::max<uint32_t>(1u, t.scatter_blocks_per_warp);
+    if (group) {
+        sa.sat = w->d_sat;
+        sa.sat_stride = w->sat_stride;
+        sa.sat_shift = r.group.gw == 64u ? 6u : 5u;
+        sa.sat_last = nd_q;  // a row of zeros for the runs past it
+    }
+    TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
+    return ABF_OK;
+}
+
+// A sparse worker as one query, or keyed: key i into bitmap d_qidx[i].
 abf_status run_sparse(const abf_worker* w, uint32_t* d_res, bool keyed, const uint32_t* d_qidx,
                       uint64_t res_stride_words, cudaStream_t s) {
     abf_index* ix = w->ix;
@@ -650,65 +833,50 @@ abf_status run_sparse(const abf_worker* w, uint32_t* d_res, bool keyed, const ui
     if (w->n_keys == 0) return ABF_OK;
     CUDA_TRY(cudaSetDevice(ix->device));
     const abf::IndexView v = abf::view_of(ix);
-    const abf_tuning& t = ix->tuning;
-    const uint32_t n_q = keyed ? uint32_t(w->n_keys) : 1u;
-    const uint64_t* q_off = keyed ? w->d_offk : w->d_off1;
-    abf::PlanArgs pa{};
-    pa.terms = w->d_keys;
-    pa.q_off = q_off;
-    pa.n_q = n_q;
-    // keyed batches may map several keys to one bitmap: only atomic
-    // scatters are safe there; a single query merges its long lists per tile
-    pa.path_uniform = keyed ? ABF_PATH_UNION : ABF_PATH_HYBRID;
-    pa.hybrid_min = t.heavy_min_len;
-    pa.heavy_min = w->d_heavy;
-    pa.term_lpref = w->d_lpref;
-    pa.q_light_cnt = w->d_lcnt;
-    pa.n_probe = w->d_nprobe;
-    pa.probe_cap = 0;
-    pa.max_terms = w->n_keys;
-    pa.err = nullptr;
-    pa.dense_in_tile = keyed ? 0 : 1;
-    pa.tile_cls = w->d_tile_cls;
-    CUDA_TRY(cudaMemsetAsync(w->d_nprobe, 0, sizeof(uint32_t), s));
-    TIMED(K_PLAN, abf::launch_plan(v, pa, s));
-    abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, n_q};
-    TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
-    const uint64_t n_words = n_words_of(ix->n_ads);
+    WorkerRun r{};
+    r.out = d_res;
+    r.out_stride = res_stride_words;
     if (!keyed) {
-        abf::TileArgs ta{};
-        ta.tile_cls = w->d_tile_cls;
-        ta.q_off = q_off;
-        ta.heavy_min = w->d_heavy;
-        ta.n_q = 1;
-        ta.n_tiles = uint32_t((n_words + t.tile_words - 1) / t.tile_words);
-        ta.out = d_res;
-        ta.out_stride = n_words;
-        ta.n_words = n_words;
-        ta.accumulate = 1;
-        ta.vec_ok = (reinterpret_cast<uintptr_t>(d_res) % 16 == 0) && (n_words % 4 == 0);
-        TIMED(K_TILE, abf::launch_tile_union(v, ta, t, ix->sm_count, s));
+        r.q_off = w->d_off1;
+        r.n_q = 1;
+        r.tiles = true;
+        return run_worker_lists(w, v, r, s);
     }
-    abf::ScatterArgs sa{};
-    sa.terms = w->d_keys;
-    sa.q_off = q_off;
-    sa.term_lpref = w->d_lpref;
-    sa.q_light_pref = w->d_lpref_q;
-    sa.n_q = n_q;
-    sa.out_slot = keyed ? d_qidx : nullptr;
-    sa.out = d_res;
-    sa.out_stride = res_stride_words;
-    sa.blocks_per_warp = std::max<uint32_t>(1u, t.scatter_blocks_per_warp);
-    TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
-    return ABF_OK;
+    // The group kernel reads every dense bitmap once (n_dense * n_ads / 8
+    // bytes, ~6 TB/s) and then ORs 64-word rows; scattering the same lists
+    // costs one atomic per posting (~700 G/s measured on 32 queries of the
+    // quarter-scale workload). With ~15 us for the extra launches it pays from
+    // n_dense * n_ads / 64 + 2^23 postings on.
+    if (ix->tuning.group_min_queries && w->dense_postings >= uint64_t(v.n_dense) * v.n_ads / 64u + (1u << 23))
+        r.group = group_shape(ix, v, w->q_cap, w->dense_keys + 8ull * w->q_cap, true);
+    if (!r.group.on && w->n_keys <= kOneQueryKeys) {
+        // scattered whole: one query, a bitmap index per key
+        r.q_off = w->d_off1;
+        r.n_q = 1;
+        r.key_slot = d_qidx;
+        return run_worker_lists(w, v, r, s);
+    }
+    // several runs of keys may name one bitmap: every kernel ORs with atomics
+    abf::KeyRunsArgs ka{d_qidx, uint32_t(w->n_keys), w->d_off, w->d_slot, w->d_n_q};
+    TIMED(K_QUEUE, abf::launch_key_runs(ka, s));
+    r.q_off = w->d_off;
+    r.n_q = uint32_t(w->n_keys);
+    r.d_n_q = w->d_n_q;
+    r.out_slot = w->d_slot;
+    return run_worker_lists(w, v, r, s);
 }
 
+// The bitmap-probe operators: the query bitmaps' terms are listed, a window of
+// queries at a time, and merged as lists; a window whose terms exceed the
+// worker's room is answered by the scan of the whole index instead.
 abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_words, cudaStream_t s) {
     abf_index* ix = w->ix;
     ABF_TRY(need_device(ix));
     if (!d_res) return fail(ABF_ERR_INVALID, "null d_res");
     if (w->batch == 0) return ABF_OK;
     CUDA_TRY(cudaSetDevice(ix->device));
+    const abf::IndexView v = abf::view_of(ix);
+    const abf_tuning& t = ix->tuning;
     abf::ProbeArgs pr{};
     if (w->kind == 2) {
         pr.qbm = reinterpret_cast<const uint32_t*>(w->d_ext);
@@ -721,17 +889,38 @@ abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_w
         pr.qbm_words = uint32_t(w->qbm_stride);
         pr.staged_ok = 1;
     }
-    pr.d_n_probe = nullptr;
-    pr.n_probe_host = uint32_t(w->batch);
-    pr.out_slot = nullptr;
-    pr.out = d_res;
     pr.out_stride = res_stride_words;
-    pr.chunk_blocks = ix->tuning.probe_chunk_blocks;
-    abf_workspace* ws = nullptr;
-    ABF_TRY(own_ws(ix, 1, 1, ix->n_ads, &ws));
-    pr.err = ws->err;
-    pr.spin_limit = ws->spin_limit;
-    TIMED(K_PROBE, abf::launch_probe(abf::view_of(ix), pr, ix->tuning, ix->sm_count, s));
+    pr.chunk_blocks = t.probe_chunk_blocks;
+    pr.err = w->d_err;
+    pr.spin_limit = abf::kDefaultSpinLimit;
+    pr.only_if = w->d_n_q;
+    const uint32_t* qbm = pr.qbm;
+    for (uint64_t q0 = 0; q0 < w->batch; q0 += kTermWindow) {
+        WorkerRun r{};
+        r.q_off = w->d_off;
+        r.n_q = uint32_t(std::min<uint64_t>(kTermWindow, w->batch - q0));
+        r.out = d_res + q0 * res_stride_words;
+        r.out_stride = res_stride_words;
+        pr.qbm = qbm + q0 * pr.qbm_stride;
+        pr.n_probe_host = r.n_q;
+        pr.out = r.out;
+        abf::TermListArgs la{};
+        la.qbm = pr.qbm;
+        la.qbm_stride = pr.qbm_stride;
+        la.qbm_words = pr.qbm_words;
+        la.n_q = r.n_q;
+        la.n_terms = ix->n_terms;
+        la.cap = w->term_cap;
+        la.cnt = w->d_cnt;
+        la.terms = w->d_keys;
+        la.off = w->d_off;
+        la.overflow = w->d_n_q;
+        TIMED(K_PROBE, abf::launch_term_lists(la, s));
+        if (t.group_min_queries && r.n_q >= t.group_min_queries) r.group = group_shape(ix, v, r.n_q, 64ull * r.n_q, true);
+        r.tiles = !r.group.on;
+        ABF_TRY(run_worker_lists(w, v, r, s));
+        TIMED(K_PROBE, abf::launch_probe(v, pr, t, ix->sm_count, s));
+    }
     return ABF_OK;
 }
 
@@ -1004,21 +1193,22 @@ abf_status abf_prepare_sparse(abf_index* ix, const uint32_t* keys, uint64_t n_ke
     w->ix = ix;
     w->kind = 0;
     w->n_keys = n_keys;
-    std::vector<uint64_t> offk(n_keys + 1);
-    for (uint64_t i = 0; i <= n_keys; ++i) offk[i] = i;
-    uint64_t off1[2] = {0, n_keys};
-    abf_status st = ABF_OK;
-    if ((st = dev_alloc(&w->d_keys, n_keys)) != ABF_OK || (st = dev_alloc(&w->d_off1, 2)) != ABF_OK ||
-        (st = dev_alloc(&w->d_offk, n_keys + 1)) != ABF_OK ||
-        (st = worker_plan_scratch(w, std::max<uint64_t>(n_keys, 1))) != ABF_OK) {
-        worker_release(w);
+    w->term_cap = uint32_t(std::max<uint64_t>(n_keys, 1));
+    w->q_cap = std::min<uint32_t>(w->term_cap, kKeyRunCap);
+    for (uint64_t i = 0; i < n_keys; ++i) {
+        if (keys[i] >= ix->n_terms || ix->derived.term_dense[keys[i]] == abf::kNone) continue;
+        ++w->dense_keys;
+        w->dense_postings += ix->h_term_len[keys[i]];
+    }
+    std::vector<uint32_t> up(4 + n_keys);  // {0, n_keys} as 64-bit offsets, then the keys
+    up[2] = uint32_t(n_keys);
+    if (n_keys) std::memcpy(up.data() + 4, keys, n_keys * 4);
+    abf_status st = worker_alloc(w, w->term_cap);
+    if (st != ABF_OK) {
         delete w;
         return st;
     }
-    cudaError_t e = cudaSuccess;
-    if (n_keys) e = cudaMemcpy(w->d_keys, keys, n_keys * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(w->d_off1, off1, sizeof(off1), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(w->d_offk, offk.data(), offk.size() * 8, cudaMemcpyHostToDevice);
+    const cudaError_t e = cudaMemcpy(w->d_off1, up.data(), up.size() * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         worker_release(w);
         delete w;
@@ -1040,20 +1230,22 @@ static abf_status prepare_dense_impl(abf_index* ix, uint64_t batch, uint64_t len
     w->ix = ix;
     w->batch = batch;
     w->len = len;
-    if (device) {
-        w->kind = 2;
-        w->d_ext = bm;
-        *out = w;
-        return ABF_OK;
-    }
-    w->kind = 1;
-    // own copy, padded so every query covers all n_terms bits and starts
-    // 16-byte aligned (bulk copies into shared memory need both)
-    w->qbm_stride = round4(std::max<uint64_t>(n_words_of(ix->n_terms), 1));
-    abf_status st = dev_alloc(&w->d_qbm, std::max<uint64_t>(batch, 1) * w->qbm_stride);
+    w->kind = device ? 2 : 1;
+    if (device) w->d_ext = bm;
+    // own copy (host bitmaps), padded so every query covers all n_terms bits
+    // and starts 16-byte aligned (bulk copies into shared memory need both)
+    else w->qbm_stride = round4(std::max<uint64_t>(n_words_of(ix->n_terms), 1));
+    // room for 2,048 terms per query of a window on average, 24,576 at least
+    w->q_cap = uint32_t(std::min<uint64_t>(std::max<uint64_t>(batch, 1), kTermWindow));
+    w->term_cap = uint32_t(std::min<uint64_t>(uint64_t(w->q_cap) * ix->n_terms, std::max<uint64_t>(2048ull * w->q_cap, 24576)));
+    abf_status st = worker_alloc(w, w->q_cap);
     if (st != ABF_OK) {
         delete w;
         return st;
+    }
+    if (device) {
+        *out = w;
+        return ABF_OK;
     }
     const uint64_t copy = std::min<uint64_t>(len, w->qbm_stride * 4);
     cudaError_t e = cudaMemset(w->d_qbm, 0, std::max<uint64_t>(batch, 1) * w->qbm_stride * 4);

@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
     __shared__ plan_dev::PlannerSmem s_pl;
     static_assert(plan_dev::kFeatThreads == 256, "the planner code runs with the plan kernel's 256 threads");
     const uint32_t tid = threadIdx.x;
-    for (uint32_t q = blockIdx.x; q < a.n_q; q += gridDim.x) {
+    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
+    for (uint32_t q = blockIdx.x; q < n_q; q += gridDim.x) {
         uint64_t qb = a.q_off[q], qe = a.q_off[q + 1];
         if (qe < qb || qe > a.max_terms) {
             // offsets outside the scratch arrays: the query gets no work
@@ -351,7 +352,8 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
         const uint32_t hm = path == ABF_PATH_TILE ? 0u
                             : path == ABF_PATH_HYBRID ? a.hybrid_min
                             : probe ? kNoHeavy : kDenseOnly;
-        const bool want_d = a.q_dense16 != nullptr;
+        const bool merge_d = a.dense_in_tile && !(a.no_dense_from && q >= a.no_dense_from);
+        const bool want_d = a.q_dense16 != nullptr && merge_d;
         const uint32_t mw = (ix.n_dense + 31u) / 32u;
         if (want_d) {
             for (uint32_t i = tid; i < mw; i += 256) s_mask[i] = 0u;
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             if (i < qe && !probe) {
                 const uint32_t t = a.terms[i];
                 if (t < ix.n_terms) {
-                    const uint32_t d = a.dense_in_tile ? __ldg(ix.term_dense + t) : kNone;
+                    const uint32_t d = merge_d ? __ldg(ix.term_dense + t) : kNone;
                     const uint32_t len = __ldg(ix.term_len + t);
                     if (d != kNone) cls = kDenseFlag | d;
                     else if (len >= hm) cls = t;
@@ -429,11 +431,12 @@ __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
     __shared__ unsigned long long s_warp[32];
     __shared__ unsigned long long s_carry;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
+    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
     if (tid == 0) s_carry = 0;
     __syncthreads();
-    for (uint32_t c0 = 0; c0 < a.n_q; c0 += 1024) {
+    for (uint32_t c0 = 0; c0 < n_q; c0 += 1024) {
         const uint32_t i = c0 + tid;
-        const uint64_t v = i < a.n_q ? a.q_light_cnt[i] : 0ull;
+        const uint64_t v = i < n_q ? a.q_light_cnt[i] : 0ull;
         uint64_t x = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -453,12 +456,134 @@ __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
         }
         __syncthreads();
         const uint64_t base = s_carry + (warp ? s_warp[warp - 1] : 0ull);
-        if (i < a.n_q) a.q_light_pref[i] = base + x - v;
+        if (i < n_q) a.q_light_pref[i] = base + x - v;
         __syncthreads();
         if (tid == 0) s_carry += s_warp[31];
         __syncthreads();
     }
-    if (tid == 0) a.q_light_pref[a.n_q] = s_carry;
+    if (tid == 0) a.q_light_pref[n_q] = s_carry;
+}
+
+// Runs of consecutive keys with the same bitmap index, in one CTA: a flattened
+// batch of queries has a run per query. (A bitmap index may come back in a
+// later run: the kernels that follow OR with atomics.) Merged run by run, the
+// keys of 32 queries on 2^18 terms x 2^22 ads take 131 us; scattered key by
+// key, one atomic per posting of every list, they took 1,234.
+__global__ void __launch_bounds__(1024) key_runs_kernel(KeyRunsArgs a) {
+    __shared__ uint32_t s_warp[32];
+    const uint32_t tid = threadIdx.x;
+    uint32_t carry = 0;
+    for (uint64_t c0 = 0; c0 < a.n_keys; c0 += 4096) {
+        uint32_t v[4], heads = 0;
+        const uint64_t i0 = c0 + tid * 4u;
+        uint32_t prev = i0 && i0 <= a.n_keys ? a.qidx[i0 - 1] : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = i0 + k < a.n_keys ? a.qidx[i0 + k] : 0u;
+            if (i0 + k < a.n_keys && (i0 + k == 0 || v[k] != prev)) heads |= 1u << k;
+            prev = v[k];
+        }
+        uint32_t total;
+        uint32_t r = carry + block_excl_scan<1024>(uint32_t(__popc(heads)), s_warp, &total);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (heads >> k & 1u) {
+                a.off[r] = i0 + k;
+                a.slot[r] = v[k];
+                ++r;
+            }
+        }
+        carry += total;
+    }
+    if (tid == 0) {
+        a.off[carry] = a.n_keys;
+        *a.n_runs = carry;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// term bitmaps -> term lists (bitmap-probe operators)
+// ---------------------------------------------------------------------------
+// A query bitmap costs n_terms / 8 bytes to read and names a few hundred or
+// thousand lists; scanning the index's blocks for it reads 4 bytes of every
+// block and finds the hit blocks bunched in a few warps' shares. So the
+// bitmaps are turned into term lists (a CTA per query) and the list-union
+// kernels, which split the named blocks evenly, do the rest: 32 queries on
+// 2^18 terms x 2^22 ads 2,686 -> 142 us, on 2^20 x 2^24 6,290 -> 428 us; one
+// query on 2^16 x 2^20 138 -> 47 us.
+constexpr uint32_t kTermThreads = 512;
+__device__ __forceinline__ uint32_t term_word(const uint32_t* bm, uint32_t w, uint32_t n_terms) {
+    const uint32_t v = __ldg(bm + w), left = n_terms - w * 32u;
+    return left < 32u ? v & ((1u << left) - 1u) : v;
+}
+__device__ __forceinline__ uint32_t term_words(const TermListArgs& a) {
+    const uint32_t nw = (a.n_terms + 31u) / 32u;
+    return nw < a.qbm_words ? nw : a.qbm_words;
+}
+
+__global__ void __launch_bounds__(kTermThreads) term_count_kernel(TermListArgs a) {
+    __shared__ unsigned long long s_red[kTermThreads / 32];
+    const uint32_t nw = term_words(a);
+    for (uint32_t q = blockIdx.x; q < a.n_q; q += gridDim.x) {
+        const uint32_t* bm = a.qbm + uint64_t(q) * a.qbm_stride;
+        uint32_t c = 0;
+#pragma unroll 8
+        for (uint32_t w = threadIdx.x; w < nw; w += kTermThreads) c += __popc(term_word(bm, w, a.n_terms));
+        const uint64_t t = block_sum_u64<int(kTermThreads)>(c, s_red);
+        if (threadIdx.x == 0) a.cnt[q] = uint32_t(t);
+    }
+}
+
+__global__ void __launch_bounds__(kTermThreads) term_list_kernel(TermListArgs a) {
+    __shared__ unsigned long long s_red[kTermThreads / 32];
+    __shared__ uint32_t s_wcnt[kTermThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
+    constexpr uint32_t kNW = kTermThreads / 32u;
+    const uint32_t nw = term_words(a);
+    const uint32_t per = (nw + kNW * 32u - 1u) / (kNW * 32u) * 32u;  // words of a warp's share, whole warps' worth
+    for (uint32_t q = blockIdx.x; q < a.n_q; q += gridDim.x) {
+        uint64_t before = 0, all = 0;
+        for (uint32_t i = tid; i < a.n_q; i += kTermThreads) {
+            const uint32_t c = a.cnt[i];
+            all += c;
+            if (i < q) before += c;
+        }
+        all = block_sum_u64<int(kTermThreads)>(all, s_red);
+        before = block_sum_u64<int(kTermThreads)>(before, s_red);
+        const bool fits = all <= a.cap;
+        if (tid == 0) {
+            a.off[q] = fits ? before : 0u;
+            if (q == a.n_q - 1u) a.off[a.n_q] = fits ? all : 0u;
+            if (q == 0) *a.overflow = fits ? 0u : 1u;
+        }
+        if (!fits) continue;
+        const uint32_t* bm = a.qbm + uint64_t(q) * a.qbm_stride;
+        const uint32_t w0 = warp * per < nw ? warp * per : nw;
+        const uint32_t w1 = w0 + per < nw ? w0 + per : nw;
+        uint32_t c = 0;
+#pragma unroll 4
+        for (uint32_t w = w0 + lane; w < w1; w += 32u) c += __popc(term_word(bm, w, a.n_terms));
+        c = __reduce_add_sync(kFull, c);
+        if (lane == 0) s_wcnt[warp] = c;
+        __syncthreads();
+        uint32_t* dst = a.terms + before + __reduce_add_sync(kFull, lane < warp ? s_wcnt[lane] : 0u);
+        for (uint32_t wb = w0; wb < w1; wb += 32u) {
+            const uint32_t w = wb + lane;
+            uint32_t v = w < w1 ? term_word(bm, w, a.n_terms) : 0u;
+            if (!__any_sync(kFull, v != 0u)) continue;
+            const uint32_t n = __popc(v);
+            uint32_t x = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, x, o);
+                if (lane >= uint32_t(o)) x += y;
+            }
+            uint32_t* d = dst + (x - n);
+            for (; v; v &= v - 1u) *d++ = w * 32u + uint32_t(__ffs(v)) - 1u;
+            dst += __shfl_sync(kFull, x, 31);
+        }
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -597,7 +722,7 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
         // without dense bitmaps already has its dense lists in the output:
         // the tile starts from it and adds only the others
         const bool on_group = a.skip_dense_only && dmode == 2u && !a.accumulate;
-        for (uint32_t i = tid; i < uint32_t(W); i += NT) tile[i] = ((a.accumulate || on_group) && i < nw) ? dst[i] : 0u;
+        for (uint32_t i = tid; i < uint32_t(W); i += NT) tile[i] = (on_group && i < nw) ? dst[i] : 0u;
         if (tid == 0) s_ndense = 0;
         __syncthreads();
         for (uint64_t c0 = qb; c0 < qe; c0 += NT) {
@@ -692,7 +817,11 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
             if (tid == 0) s_ndense = 0;
             __syncthreads();
         }
-        if (a.vec_ok) {
+        if (a.accumulate) {
+            // the caller's bitmap may be ORed into by other calls at the same time
+            for (uint32_t i = tid; i < nw; i += NT)
+                if (tile[i]) atomicOr(dst + i, tile[i]);
+        } else if (a.vec_ok) {
             uint4* d4 = reinterpret_cast<uint4*>(dst);
             for (uint32_t j = tid; j * 4u + 3u < nw; j += NT) d4[j] = tile4[j];
             for (uint32_t i = (nw & ~3u) + tid; i < nw; i += NT) dst[i] = tile[i];
@@ -734,6 +863,15 @@ template <> __device__ __forceinline__ uint32_t zero_word<uint32_t>() { return 0
 template <> __device__ __forceinline__ uint2 zero_word<uint2>() { return make_uint2(0u, 0u); }
 __device__ __forceinline__ bool all_ones(uint32_t a) { return a == ~0u; }
 __device__ __forceinline__ bool all_ones(uint2 a) { return (a.x & a.y) == ~0u; }
+// OR of a lane's words (word w and on) into the output, by atomics: other
+// queries may share the bitmap
+__device__ __forceinline__ void or_words(uint32_t* o, uint32_t a, uint64_t w, uint64_t n_words) {
+    if (a && w < n_words) atomicOr(o, a);
+}
+__device__ __forceinline__ void or_words(uint32_t* o, uint2 a, uint64_t w, uint64_t n_words) {
+    if (a.x && w < n_words) atomicOr(o, a.x);
+    if (a.y && w + 1u < n_words) atomicOr(o + 1, a.y);
+}
 // true when the warp's whole tile slice is set: no further row can change it
 template <typename T>
 __device__ __forceinline__ bool tile_full(T acc) { return __all_sync(kFull, all_ones(acc)); }
@@ -793,7 +931,9 @@ __device__ __forceinline__ T or_list_rows(const uint8_t* B, const uint4* dl, uin
 // the 16-bit row lists are read from global memory). GW = 64 halves the
 // index work per word (each lane ORs two words per row) where two stages of
 // 64-word rows fit.
-template <uint32_t GW>
+// ACC: OR into the output with atomics (bitmaps may be shared, rows need no
+// alignment) instead of overwriting it.
+template <uint32_t GW, bool ACC>
 __global__ void __launch_bounds__(kGroupThreads, 1)
     dense_group_kernel(const __grid_constant__ CUtensorMap tmap_full, const __grid_constant__ CUtensorMap tmap_last,
                        DenseGroupArgs a) {
@@ -816,6 +956,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     constexpr uint32_t kNW = kGroupThreads / 32u;
     uint32_t t = blockIdx.x;
     if (t >= a.n_tiles) return;
+    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
     const uint32_t full_boxes = (a.n_rows - 1u) / kGroupBoxRows;  // boxes of 256 rows before the last
     auto issue = [&](uint32_t tile, uint32_t st) {  // thread 0 only
         fence_proxy_async();  // earlier reads of this stage (ordered by the barrier) before the copy
@@ -839,7 +980,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const uint32_t q = tid * 2u + r;
-        const bool dq = q < a.n_q && a.q_dmode[q];
+        // when ORing into the output, queries without dense bitmaps have nothing to add
+        const bool dq = q < n_q && a.q_dmode[q] && !(ACC && a.q_ndense[q] == 0u);
         len[r] = dq ? ((a.q_ndense[q] + 7u) & ~7u) : 0u;
         cnt[r] = dq ? 1u : 0u;
     }
@@ -909,9 +1051,13 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             const T acc = in_smem ? or_list_words<T>(B, s_lists + (m >> 16), nd)
                                   : or_list_rows<GW, T>(B, reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]),
                                                         nd);
-            uint32_t* o = a.out + uint64_t(q) * a.out_stride + w;
             if (a.sat && tile_full(acc) && lane == 0)
                 atomicOr(a.sat + uint64_t(q) * a.sat_stride + (t >> 5), 1u << (t & 31u));
+            if constexpr (ACC) {
+                or_words(a.out + uint64_t(a.out_slot ? a.out_slot[q] : q) * a.out_stride + w, acc, w, a.n_words);
+                continue;
+            }
+            uint32_t* o = a.out + uint64_t(q) * a.out_stride + w;
             if constexpr (GW == 64u) {
                 if (w + 1u < a.n_words) *reinterpret_cast<uint2*>(o) = acc;  // 8-byte aligned (checked at launch)
                 else if (w < a.n_words) o[0] = acc.x;
@@ -932,17 +1078,19 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
 // ---------------------------------------------------------------------------
 // list-union, scatter variant (load-balanced over the short lists' blocks)
 // ---------------------------------------------------------------------------
-template <int NW>
+// KEYED: one query whose term slots each have an output bitmap of their own.
+template <int NW, bool KEYED>
 __global__ void __launch_bounds__(NW * 32) scatter_kernel(IndexView ix, ScatterArgs a) {
     __shared__ __align__(16) uint4 stage[NW][32];
     const uint32_t warp = warp_id();
-    const uint64_t total = a.q_light_pref[a.n_q];
+    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
+    const uint64_t total = a.q_light_pref[n_q];
     const uint64_t bpw = a.blocks_per_warp;
     const uint64_t nwt = uint64_t(gridDim.x) * NW;
     for (uint64_t f0 = (uint64_t(blockIdx.x) * NW + warp) * bpw; f0 < total; f0 += nwt * bpw) {
         const uint64_t f1 = f0 + bpw < total ? f0 + bpw : total;
         // query: last q with q_light_pref[q] <= f0
-        uint32_t q0 = 0, q1 = a.n_q;
+        uint32_t q0 = 0, q1 = n_q;
         while (q1 - q0 > 1) {
             const uint32_t m = (q0 + q1) >> 1;
             if (a.q_light_pref[m] <= f0) q0 = m; else q1 = m;
@@ -959,8 +1107,8 @@ __global__ void __launch_bounds__(NW * 32) scatter_kernel(IndexView ix, ScatterA
         }
         uint64_t i = i0;
         uint32_t j = r - a.term_lpref[i];
-        uint32_t* out = a.out + uint64_t(a.out_slot ? a.out_slot[q] : q) * a.out_stride;
-        const uint32_t* sat = a.sat ? a.sat + uint64_t(q) * a.sat_stride : nullptr;
+        uint32_t* out = a.out + uint64_t(KEYED ? a.key_slot[i] : a.out_slot ? a.out_slot[q] : q) * a.out_stride;
+        const uint32_t* sat = a.sat ? a.sat + uint64_t(min(q, a.sat_last)) * a.sat_stride : nullptr;
         // (i, j) is a scattered block of query q; the walk moves to the next
         // one, crossing into later terms and queries as they run out
         auto advance = [&]() {
@@ -970,7 +1118,9 @@ __global__ void __launch_bounds__(NW * 32) scatter_kernel(IndexView ix, ScatterA
                 if (j < nb) return;
                 ++i;
                 j = 0;
-                if (i >= qe) {
+                if constexpr (KEYED) {
+                    out = a.out + uint64_t(a.key_slot[i]) * a.out_stride;
+                } else if (i >= qe) {
                     do {
                         ++q;
                     } while (a.q_light_pref[q + 1] == a.q_light_pref[q]);
@@ -979,7 +1129,7 @@ __global__ void __launch_bounds__(NW * 32) scatter_kernel(IndexView ix, ScatterA
                     qtot = uint32_t(a.q_light_pref[q + 1] - a.q_light_pref[q]);
                     i = qb;
                     out = a.out + uint64_t(a.out_slot ? a.out_slot[q] : q) * a.out_stride;
-                    if (a.sat) sat = a.sat + uint64_t(q) * a.sat_stride;
+                    if (a.sat) sat = a.sat + uint64_t(min(q, a.sat_last)) * a.sat_stride;
                 }
             }
         };
@@ -1031,6 +1181,7 @@ __global__ void __launch_bounds__(NW * 32) probe_kernel(IndexView ix, ProbeArgs 
     // the device counter also counts queries demoted past the slot capacity
     uint32_t n_probe = a.n_probe_host;
     if (a.d_n_probe && *a.d_n_probe < n_probe) n_probe = *a.d_n_probe;
+    if (a.only_if && *a.only_if == 0u) return;
     if (n_probe == 0 || ix.n_blocks == 0) return;
     if (tid == 0) {
         mbar_init(&bar, 1);
@@ -1499,8 +1650,9 @@ uint32_t compact_chunks(uint64_t n_bits) {
 
 cudaError_t launch_plan(const IndexView& v, const PlanArgs& a, cudaStream_t s) {
     if (a.n_q == 0) return cudaSuccess;
-    const uint32_t g = a.n_q < 65535u * 16u ? a.n_q : 65535u * 16u;
-    plan_kernel<<<g, 256, 0, s>>>(v, a);
+    // with a device count the bound may be far above it: a few waves of CTAs
+    const uint32_t most = a.d_n_q ? 148u * 16u : 65535u * 16u;
+    plan_kernel<<<a.n_q < most ? a.n_q : most, 256, 0, s>>>(v, a);
     count_launch();
     return cudaGetLastError();
 }
@@ -1508,6 +1660,22 @@ cudaError_t launch_plan(const IndexView& v, const PlanArgs& a, cudaStream_t s) {
 cudaError_t launch_queue_scan(const QueueArgs& a, cudaStream_t s) {
     queue_scan_kernel<<<1, 1024, 0, s>>>(a);
     count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_key_runs(const KeyRunsArgs& a, cudaStream_t s) {
+    key_runs_kernel<<<1, 1024, 0, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_term_lists(const TermListArgs& a, cudaStream_t s) {
+    if (a.n_q == 0) return cudaSuccess;
+    term_count_kernel<<<a.n_q, kTermThreads, 0, s>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    term_list_kernel<<<a.n_q, kTermThreads, 0, s>>>(a);
+    count_launch(2);
     return cudaGetLastError();
 }
 
@@ -1612,20 +1780,20 @@ uint32_t dense_group_list_cap(uint32_t n_rows, uint32_t n_q, uint32_t gw, uint32
 }
 
 namespace {
-template <uint32_t GW>
+template <uint32_t GW, bool ACC>
 cudaError_t launch_group_w(const CUtensorMap (&m)[2], const DenseGroupArgs& a, int sm_count, cudaStream_t s) {
     static std::atomic<uint64_t> done{0};  // devices whose attribute is set
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (!(done.load() >> dev & 1ull)) {
-        e = cudaFuncSetAttribute(dense_group_kernel<GW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(dense_group_kernel<GW, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(kGroupSmemBytes));
         if (e != cudaSuccess) return e;
         done.fetch_or(1ull << dev);
     }
     const uint32_t grid = a.n_tiles < uint32_t(sm_count) ? a.n_tiles : uint32_t(sm_count);
-    dense_group_kernel<GW><<<grid, kGroupThreads, kGroupSmemBytes, s>>>(m[0], m[1], a);
+    dense_group_kernel<GW, ACC><<<grid, kGroupThreads, kGroupSmemBytes, s>>>(m[0], m[1], a);
     return cudaGetLastError();
 }
 }  // namespace
@@ -1642,8 +1810,8 @@ cudaError_t launch_dense_group(const void* tmaps, uint32_t gw, const DenseGroupA
     CUtensorMap m[2];
     std::memcpy(m, tmaps, sizeof(m));
     cudaError_t e;
-    if (gw == 64u) e = launch_group_w<64>(m, a, sm_count, s);
-    else if (gw == 32u) e = launch_group_w<32>(m, a, sm_count, s);
+    if (gw == 64u) e = a.accumulate ? launch_group_w<64, true>(m, a, sm_count, s) : launch_group_w<64, false>(m, a, sm_count, s);
+    else if (gw == 32u) e = a.accumulate ? launch_group_w<32, true>(m, a, sm_count, s) : launch_group_w<32, false>(m, a, sm_count, s);
     else return cudaErrorInvalidValue;
     count_launch();
     return e;
@@ -1653,7 +1821,8 @@ cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_t
                            cudaStream_t s) {
     if (a.n_q == 0) return cudaSuccess;
     const int grid = grid_for(~0ull, sm_count, t.ctas_per_sm ? t.ctas_per_sm * 2u : 8u);
-    scatter_kernel<8><<<grid, 256, 0, s>>>(v, a);
+    if (a.key_slot) scatter_kernel<8, true><<<grid, 256, 0, s>>>(v, a);
+    else scatter_kernel<8, false><<<grid, 256, 0, s>>>(v, a);
     count_launch();
     return cudaGetLastError();
 }

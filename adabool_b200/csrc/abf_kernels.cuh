@@ -18,6 +18,10 @@
 //                      the probe queries' term-bitmap slices in shared memory
 //                      with bulk async copies (TMA engine), tests each block's
 //                      term and scatters hit blocks into their queries
+//   term_count / term_list_kernel  query term bitmaps -> term lists, for the
+//                      bitmap-probe operators (the list-union kernels then
+//                      merge them; the scan answers what does not fit)
+//   key_runs_kernel    runs of consecutive keys with one output bitmap
 //   compact_kernel     compaction: bitmap -> ascending uint32 ids in one pass
 //                      (chunk popcounts, decoupled look-back prefix, id
 //                      writes)
@@ -89,6 +93,9 @@ struct PlanArgs {
     uint32_t* q_ndense;       // out: per query, distinct dense bitmaps
     uint32_t* q_dmode;        // out: per query, 1 if every list it merges has a dense bitmap,
                               // 2 if it also merges lists without one, 0 for probe / empty
+    const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
+    uint32_t no_dense_from;   // queries from this one on scatter their dense-bitmap lists too
+                              // (0: none do; only with dense_in_tile)
 };
 
 constexpr uint32_t kDenseFlag = 0x80000000u;
@@ -97,6 +104,31 @@ struct QueueArgs {
     const uint64_t* q_light_cnt;
     uint64_t* q_light_pref;   // n_q + 1
     uint32_t n_q;
+    const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
+};
+
+// Consecutive keys with the same bitmap index form one run, which the kernels
+// above then treat as a query.
+struct KeyRunsArgs {
+    const uint32_t* qidx;
+    uint32_t n_keys;
+    uint64_t* off;            // out: first key of each run, then n_keys (n_keys + 1 entries)
+    uint32_t* slot;           // out: the run's bitmap index
+    uint32_t* n_runs;         // out
+};
+
+// Term bitmaps -> term lists (ascending), one list per bitmap, packed.
+struct TermListArgs {
+    const uint32_t* qbm;      // qbm_stride words apart
+    uint64_t qbm_stride;
+    uint32_t qbm_words;       // readable words per bitmap
+    uint32_t n_q;
+    uint32_t n_terms;         // bits at and past it are ignored
+    uint32_t cap;             // room in terms; if the lists do not fit, all come out empty and *overflow is 1
+    uint32_t* cnt;            // scratch: n_q
+    uint32_t* terms;          // out
+    uint64_t* off;            // out: n_q + 1
+    uint32_t* overflow;       // out: 0 or 1
 };
 
 struct TileArgs {
@@ -109,7 +141,7 @@ struct TileArgs {
     uint32_t* out;
     uint64_t out_stride;      // words between query bitmaps
     uint64_t n_words;         // words of one bitmap
-    int accumulate;           // 1: OR into the existing bitmap, 0: overwrite
+    int accumulate;           // 1: OR into the existing bitmap with atomics, 0: overwrite
     int vec_ok;               // out 16-byte aligned and out_stride % 4 == 0
     // optional (plan kernel): queries whose merged lists all have dense
     // bitmaps (q_dmode 1) take a barrier-free path that streams the OR of
@@ -151,6 +183,9 @@ struct DenseGroupArgs {
     uint32_t spin_limit;       // polls of an mbarrier wait before it gives up
     uint32_t* sat;             // optional, zeroed before launch: bit t of query q's sat_stride words
     uint32_t sat_stride;       //   is set when tile t of its bitmap came out all ones
+    const uint32_t* d_n_q;     // optional device count of queries (at most n_q)
+    int accumulate;            // 1: OR into the output with atomics (bitmaps may be shared), 0: overwrite
+    const uint32_t* out_slot;  // query -> output bitmap index (null: identity)
 };
 
 struct ScatterArgs {
@@ -160,12 +195,15 @@ struct ScatterArgs {
     const uint64_t* q_light_pref; // n_q + 1
     uint32_t n_q;
     const uint32_t* out_slot;  // query -> output bitmap index (null: identity)
+    const uint32_t* key_slot;  // instead, with n_q 1: term slot -> output bitmap index
     uint32_t* out;
     uint64_t out_stride;
     uint32_t blocks_per_warp;
     const uint32_t* sat;       // optional: the dense group kernel's saturated-tile bits
     uint32_t sat_stride;       //   (words per query); an OR into a word of such a tile
     uint32_t sat_shift;        //   is skipped; tile = word >> sat_shift
+    uint32_t sat_last;         // queries past this one share its row of marks (all zero then: no marks)
+    const uint32_t* d_n_q;     // optional device count of queries (at most n_q)
 };
 
 struct ProbeArgs {
@@ -181,6 +219,7 @@ struct ProbeArgs {
     uint32_t chunk_blocks;     // multiple of 128
     uint32_t* err;
     uint32_t spin_limit;       // polls of an mbarrier wait before it gives up
+    const uint32_t* only_if;   // optional: the kernel does nothing while this device word is 0
 };
 
 // Compaction of n_q bitmaps into one packed id array. Work item i is chunk
@@ -218,6 +257,8 @@ uint32_t dense_group_list_cap(uint32_t n_rows, uint32_t n_q, uint32_t gw, uint32
 cudaError_t launch_dense_group(const void* tmaps, uint32_t gw, const DenseGroupArgs& a, int sm_count,
                                cudaStream_t s);
 cudaError_t launch_queue_scan(const QueueArgs& a, cudaStream_t s);
+cudaError_t launch_key_runs(const KeyRunsArgs& a, cudaStream_t s);
+cudaError_t launch_term_lists(const TermListArgs& a, cudaStream_t s);
 cudaError_t launch_tile_union(const IndexView& v, const TileArgs& a, const abf_tuning& t, int sm_count,
                               cudaStream_t s);
 cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_tuning& t, int sm_count,

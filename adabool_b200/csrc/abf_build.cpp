@@ -294,6 +294,26 @@ void derive_tables(const HostIndex& h, uint32_t dense_div, int n_threads, Derive
         dense_terms.push_back(t);
     }
     out->n_dense = uint32_t(dense_terms.size());
+    // plain ids: the longest of the other lists, within the same budget
+    out->term_plain.assign(h.n_terms, kNone);
+    out->plain_term.clear();
+    out->plain_off.assign(1, 0u);
+    out->plain_dir_n = uint32_t(((uint64_t(h.n_ads) + (1ull << kBinShift) - 1) >> kBinShift) + 1);
+    cand.clear();
+    const uint32_t plain_min = plain_min_len(h.n_ads);
+    for (uint32_t t = 0; t < h.n_terms; ++t)
+        if (out->term_dense[t] == kNone && h.term_len[t] >= plain_min) cand.push_back(t);
+    std::sort(cand.begin(), cand.end(), [&](uint32_t a, uint32_t b) { return h.term_len[a] > h.term_len[b]; });
+    uint64_t units = 0, used = 0;
+    for (uint32_t t : cand) {
+        const uint64_t u = (uint64_t(h.term_len[t]) + 3) / 4;
+        used += u * 16 + out->plain_dir_n * 4ull;
+        if (used > budget || units + u >= (1ull << 30)) break;  // positions are 32-bit
+        units += u;
+        out->term_plain[t] = uint32_t(out->plain_term.size());
+        out->plain_term.push_back(t);
+        out->plain_off.push_back(uint32_t(units));
+    }
     std::vector<uint32_t> dir_terms;
     for (uint32_t t = 0; t < h.n_terms; ++t) {
         if (out->term_dense[t] != kNone) continue;

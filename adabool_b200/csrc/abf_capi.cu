@@ -56,9 +56,10 @@ using abf::fail;
 namespace {
 
 // ---- kernel timing (abf_profile_enable / abf_profile_read) ----
-enum Kid { K_PLAN, K_QUEUE, K_TILE, K_SCATTER, K_PROBE, K_COMPACT, K_PLANNER, K_GROUP, K_NKERNELS };
+enum Kid { K_PLAN, K_QUEUE, K_TILE, K_SCATTER, K_PROBE, K_COMPACT, K_PLANNER, K_GROUP, K_BIN, K_NKERNELS };
 const char* const kKernelNames[K_NKERNELS] = {"plan",  "queue_scan", "tile_union", "scatter_union",
-                                              "probe", "compact",    "planner",    "dense_group"};
+                                              "probe", "compact",    "planner",    "dense_group",
+                                              "bin_union"};
 
 struct Profiler {
     struct Rec {
@@ -124,7 +125,7 @@ struct abf_workspace {
     uint64_t probe_stride = 0;
     uint32_t chunks_per_q = 0;
     uint32_t* heavy = nullptr;
-    uint32_t* lpref = nullptr;
+    uint2* slot = nullptr;          // per term (see PlanArgs)
     uint32_t* tile_cls = nullptr;
     uint64_t* lcnt = nullptr;
     uint64_t* lpref_q = nullptr;
@@ -141,6 +142,11 @@ struct abf_workspace {
     uint32_t* q_ndense = nullptr;   // per query
     uint32_t* q_dmode = nullptr;    // per query
     uint32_t* err = nullptr;
+    uint32_t* bin_list = nullptr;   // the bin kernel's lists and work split (see PlanArgs, BinArgs)
+    uint32_t* q_nbin = nullptr;
+    uint32_t* q_bblk = nullptr;
+    uint32_t* parts_pref = nullptr;
+    uint32_t* bin_ticket = nullptr;
     uint32_t* tile_list = nullptr;  // queries the merge kernel visits beside the dense group kernel
     uint32_t* n_tile_list = nullptr;
     uint32_t* sat = nullptr;        // per query: the dense group kernel's all-ones tiles, one bit each
@@ -168,7 +174,7 @@ struct abf_worker {
     // marks cover the first q_cap queries or runs
     uint32_t q_cap = 0;
     uint32_t* d_heavy = nullptr;
-    uint32_t* d_lpref = nullptr;
+    uint2* d_tslot = nullptr;
     uint32_t* d_tile_cls = nullptr;
     uint64_t* d_lcnt = nullptr;
     uint64_t* d_lpref_q = nullptr;
@@ -179,6 +185,11 @@ struct abf_worker {
     uint32_t* d_dmode = nullptr;
     uint32_t* d_sat = nullptr;
     uint32_t sat_stride = 0;
+    uint32_t* d_bin_list = nullptr; // the bin kernel's lists and work split
+    uint32_t* d_nbin = nullptr;
+    uint32_t* d_bblk = nullptr;
+    uint32_t* d_parts = nullptr;
+    uint32_t* d_ticket = nullptr;
     uint32_t* d_err = nullptr;
     uint64_t dense_keys = 0;        // sparse: keys whose lists have dense bitmaps, and their postings
     uint64_t dense_postings = 0;
@@ -254,6 +265,15 @@ void default_tuning(abf_index* ix) {
     t.group_tile_words = 0;
 }
 
+void free_plain(abf_index* ix) {
+    auto& d = ix->dev;
+    dev_free(d.term_plain);
+    dev_free(d.plain_term);
+    dev_free(d.plain_off);
+    dev_free(d.plain);
+    dev_free(d.plain_dir);
+}
+
 void free_device(abf_index* ix) {
     auto& d = ix->dev;
     dev_free(d.term_blk);
@@ -267,6 +287,7 @@ void free_device(abf_index* ix) {
     dev_free(d.dense);
     dev_free(d.term_dir);
     dev_free(d.dir);
+    free_plain(ix);
     dev_free(d.term_cbytes);
     dev_free(d.planner);
     d.bytes = 0;
@@ -277,6 +298,40 @@ std::vector<uint32_t> cbytes32(const abf_index* ix) {
     std::vector<uint32_t> v(ix->h_term_bytes.size());
     for (size_t i = 0; i < v.size(); ++i) v[i] = uint32_t(std::min<uint64_t>(ix->h_term_bytes[i], 0xffffffffull));
     return v;
+}
+
+// The plain ids of h's choice of lists, unpacked on the device from the
+// uploaded blocks (synchronises). Where they do not fit the device's memory
+// the index does without them.
+abf_status make_plain(abf_index* ix, const abf::DerivedHost& h) {
+    auto& d = ix->dev;
+    const uint32_t n = h.n_plain();
+    if (n == 0) return ABF_OK;
+    const uint64_t before = d.bytes;
+    if (upload_vec(&d.term_plain, h.term_plain, &d.bytes) != ABF_OK ||
+        upload_vec(&d.plain_term, h.plain_term, &d.bytes) != ABF_OK ||
+        upload_vec(&d.plain_off, h.plain_off, &d.bytes) != ABF_OK ||
+        dev_alloc(&d.plain, uint64_t(h.plain_off[n]) * 4u, &d.bytes) != ABF_OK ||
+        dev_alloc(&d.plain_dir, uint64_t(n) * h.plain_dir_n, &d.bytes) != ABF_OK) {
+        cudaGetLastError();
+        abf::clear_error();
+        free_plain(ix);
+        d.bytes = before;
+        return ABF_OK;
+    }
+    abf::IndexView v = abf::view_of(ix);
+    v.plain_dir_n = h.plain_dir_n;
+    v.n_plain = n;
+    CUDA_TRY(abf::launch_plain_ids(v, d.plain_term, d.plain_off, d.plain, d.plain_dir, ix->sm_count, nullptr));
+    CUDA_TRY(cudaStreamSynchronize(nullptr));
+    return ABF_OK;
+}
+
+uint64_t plain_bytes(const abf_index* ix) {
+    const auto& h = ix->derived;
+    if (!ix->dev.plain) return 0;
+    return 4ull * (h.term_plain.size() + h.plain_term.size() + h.plain_off.size()) +
+           16ull * h.plain_off.back() + 4ull * uint64_t(h.n_plain()) * h.plain_dir_n;
 }
 
 abf_status upload(abf_index* ix, int device) {
@@ -300,7 +355,8 @@ abf_status upload(abf_index* ix, int device) {
         (st = upload_vec(&d.dense, ix->derived.dense, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.term_dir, ix->derived.term_dir, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.dir, ix->derived.dir, &d.bytes)) != ABF_OK ||
-        (st = upload_vec(&d.term_cbytes, cbytes32(ix), &d.bytes)) != ABF_OK) {
+        (st = upload_vec(&d.term_cbytes, cbytes32(ix), &d.bytes)) != ABF_OK ||
+        (st = make_plain(ix, ix->derived)) != ABF_OK) {
         free_device(ix);
         return st;
     }
@@ -353,7 +409,7 @@ abf_status need_device(const abf_index* ix) {
 
 void ws_release(abf_workspace* w) {
     dev_free(w->heavy);
-    dev_free(w->lpref);
+    dev_free(w->slot);
     dev_free(w->tile_cls);
     dev_free(w->lcnt);
     dev_free(w->lpref_q);
@@ -370,6 +426,11 @@ void ws_release(abf_workspace* w) {
     dev_free(w->q_ndense);
     dev_free(w->q_dmode);
     dev_free(w->err);
+    dev_free(w->bin_list);
+    dev_free(w->q_nbin);
+    dev_free(w->q_bblk);
+    dev_free(w->parts_pref);
+    dev_free(w->bin_ticket);
     dev_free(w->tile_list);
     dev_free(w->n_tile_list);
     dev_free(w->sat);
@@ -387,7 +448,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
     w->sat_stride = sat_words(ix);
     abf_status st;
-    if ((st = dev_alloc(&w->heavy, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref, max_terms)) != ABF_OK ||
+    if ((st = dev_alloc(&w->heavy, max_q)) != ABF_OK || (st = dev_alloc(&w->slot, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->tile_cls, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->lcnt, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref_q, uint64_t(max_q) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->probe_list, w->probe_cap)) != ABF_OK || (st = dev_alloc(&w->n_probe, 1)) != ABF_OK ||
@@ -399,7 +460,10 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
         (st = dev_alloc(&w->q_dense16, max_terms + 8ull * max_q + 16)) != ABF_OK ||
         (st = dev_alloc(&w->q_dstart, max_q)) != ABF_OK || (st = dev_alloc(&w->q_ndense, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->q_dmode, max_q)) != ABF_OK || (st = dev_alloc(&w->tile_list, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->n_tile_list, 1)) != ABF_OK ||
+        (st = dev_alloc(&w->n_tile_list, 1)) != ABF_OK || (st = dev_alloc(&w->bin_list, max_terms)) != ABF_OK ||
+        (st = dev_alloc(&w->q_nbin, max_q)) != ABF_OK || (st = dev_alloc(&w->q_bblk, max_q)) != ABF_OK ||
+        (st = dev_alloc(&w->parts_pref, uint64_t(max_q) + 1)) != ABF_OK ||
+        (st = dev_alloc(&w->bin_ticket, 1)) != ABF_OK ||
         (st = dev_alloc(&w->sat, uint64_t(max_q) * w->sat_stride)) != ABF_OK ||
         (st = dev_alloc(&w->q_terms, max_terms)) != ABF_OK || (st = dev_alloc(&w->q_off, 2)) != ABF_OK) {
         ws_release(w);
@@ -447,6 +511,11 @@ abf_status run_compact(abf_index* ix, const abf::CompactArgs& ca, cudaStream_t s
     return ABF_OK;
 }
 
+// consecutive blocks a scatter warp takes at a time
+uint32_t scatter_chunk(const abf_tuning& t) {
+    return std::min<uint32_t>(32u, 4u * std::max<uint32_t>(1u, std::min<uint32_t>(8u, t.scatter_blocks_per_warp)));
+}
+
 // The merge kernel's tile shape for n_q queries: a batch too small to fill the
 // GPU at the tuned shape (the tuner sees large batches) gets full 8-warp CTAs
 // first, then narrower tiles.
@@ -460,6 +529,13 @@ abf_tuning tile_shape(const abf_index* ix, uint64_t n_q) {
     while (t.tile_words > 1024 && threads() < want) t.tile_words >>= 1;
     return t;
 }
+
+// The bin kernel merges plain lists beside the dense group kernel. An item
+// moves a tile's 64 KB in and out at most, the scatter kernel a 32-byte sector
+// in and out per posting once the batch's bitmaps exceed L2: a query's lists
+// are binned from 16 blocks of 128 postings per tile on.
+uint32_t bin_tiles(uint64_t n_words) { return uint32_t((n_words + abf::kBinWords - 1) / abf::kBinWords); }
+uint32_t bin_min_blocks(uint64_t n_words) { return 16u * bin_tiles(n_words); }
 
 // Tile width and stages of the dense group kernel for windows of wq queries
 // with about `lists` dense-list entries in all; off when the dense bitmaps
@@ -512,6 +588,17 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     CUDA_TRY(cudaSetDevice(ix->device));
     const abf::IndexView v = abf::view_of(ix);
     const abf_tuning& t = ix->tuning;
+    // dense group kernel: the dense lists of every non-probe query in one pass per
+    // tile, when the batch is large enough (room for 64 list entries per query)
+    const uint32_t n_dense = v.n_dense, n_tiles_bin = bin_tiles(n_words);
+    GroupShape gs;
+    if (t.group_min_queries && b->n_queries >= t.group_min_queries) {
+        const uint32_t wq = std::min<uint32_t>(b->n_queries, abf::kGroupMaxQueries);
+        const bool out8 = reinterpret_cast<uintptr_t>(b->d_bitmaps) % 8 == 0 && b->bitmap_stride_words % 2 == 0;
+        gs = group_shape(ix, v, wq, 64ull * wq, out8);
+    }
+    const bool group = gs.on;
+    const uint32_t gw = gs.gw, stages = gs.stages;
     CUDA_TRY(cudaMemsetAsync(ws->n_probe, 0, sizeof(uint32_t), s));
     CUDA_TRY(cudaMemsetAsync(ws->n_tile_list, 0, sizeof(uint32_t), s));
     abf::PlanArgs pa{};
@@ -524,7 +611,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.probe_min_frac = t.probe_min_fraction;
     pa.fixed_hybrid_min = t.fixed_hybrid_min_len;
     pa.heavy_min = ws->heavy;
-    pa.term_lpref = ws->lpref;
+    pa.term_slot = ws->slot;
     pa.q_light_cnt = ws->lcnt;
     pa.probe_list = ws->probe_list;
     pa.n_probe = ws->n_probe;
@@ -546,8 +633,21 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.n_postings = ix->n_postings;
     pa.probe_bm = ws->probe_bm;
     pa.probe_stride = ws->probe_stride;
-    TIMED(K_PLAN, abf::launch_plan(v, pa, s));
     abf::QueueArgs qa{ws->lcnt, ws->lpref_q, b->n_queries};
+    const bool bins = group && v.n_plain > 0;
+    if (bins) {
+        pa.bin_list = ws->bin_list;
+        pa.bin_min_blocks = bin_min_blocks(n_words);
+        pa.q_nbin = ws->q_nbin;
+        pa.q_bblk = ws->q_bblk;
+        qa.q_nbin = ws->q_nbin;
+        qa.q_bblk = ws->q_bblk;
+        qa.parts_pref = ws->parts_pref;
+        qa.ticket = ws->bin_ticket;
+        qa.n_tiles = n_tiles_bin;
+        qa.slots = uint32_t(ix->sm_count) * abf::kBinCtasPerSm;
+    }
+    TIMED(K_PLAN, abf::launch_plan(v, pa, s));
     TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
     // the probe queries' term bitmaps are written by their plan CTAs
     const bool maybe_probe = ws->probe_cap > 0 && (b->d_paths || b->path == ABF_PATH_PROBE || b->path == ABF_PATH_AUTO);
@@ -569,17 +669,6 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     ta.q_dmode = ws->q_dmode;
     ta.tile_list = ws->tile_list;
     ta.n_tile_list = ws->n_tile_list;
-    // dense group kernel: the dense lists of every non-probe query in one pass per
-    // tile, when the batch is large enough (room for 64 list entries per query)
-    const uint32_t n_dense = v.n_dense;
-    GroupShape gs;
-    if (t.group_min_queries && b->n_queries >= t.group_min_queries) {
-        const uint32_t wq = std::min<uint32_t>(b->n_queries, abf::kGroupMaxQueries);
-        const bool out8 = reinterpret_cast<uintptr_t>(b->d_bitmaps) % 8 == 0 && b->bitmap_stride_words % 2 == 0;
-        gs = group_shape(ix, v, wq, 64ull * wq, out8);
-    }
-    const bool group = gs.on;
-    const uint32_t gw = gs.gw, stages = gs.stages;
     ta.skip_dense_only = group ? 1 : 0;
     // the group kernel marks each (query, tile) it leaves all ones; the
     // scatter then skips ORs into those tiles
@@ -610,17 +699,34 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     abf::ScatterArgs sa{};
     sa.terms = b->d_terms;
     sa.q_off = b->d_offsets;
-    sa.term_lpref = ws->lpref;
+    sa.term_slot = ws->slot;
     sa.q_light_pref = ws->lpref_q;
     sa.n_q = b->n_queries;
     sa.out = b->d_bitmaps;
     sa.out_stride = b->bitmap_stride_words;
-    sa.blocks_per_warp = std::max<uint32_t>(1u, t.scatter_blocks_per_warp);
+    sa.chunk_blocks = scatter_chunk(t);
     if (group) {
         sa.sat = ws->sat;
         sa.sat_stride = ws->sat_stride;
         sa.sat_shift = gw == 64u ? 6u : 5u;
         sa.sat_last = b->n_queries - 1;
+        abf::BinArgs ba{};
+        ba.bin_list = ws->bin_list;
+        ba.q_off = b->d_offsets;
+        ba.q_nbin = ws->q_nbin;
+        ba.parts_pref = ws->parts_pref;
+        ba.ticket = ws->bin_ticket;
+        ba.n_q = b->n_queries;
+        ba.n_tiles = n_tiles_bin;
+        ba.out = b->d_bitmaps;
+        ba.out_stride = b->bitmap_stride_words;
+        ba.n_words = n_words;
+        ba.vec_ok = ta.vec_ok;
+        ba.sat = sa.sat;
+        ba.sat_stride = sa.sat_stride;
+        ba.sat_shift = sa.sat_shift;
+        ba.sat_last = sa.sat_last;
+        if (bins) TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
     }
     TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
     if (maybe_probe) {
@@ -684,7 +790,7 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     a.used += uint64_t(w->term_cap) * sizeof(uint32_t);
     a.take(w->d_off, n_q + 1);
     a.take(w->d_heavy, n_q);
-    a.take(w->d_lpref, w->term_cap);
+    a.take(w->d_tslot, w->term_cap);
     a.take(w->d_tile_cls, w->term_cap);
     a.take(w->d_lcnt, n_q);
     a.take(w->d_lpref_q, n_q + 1);
@@ -696,6 +802,11 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     a.take(w->d_ndense, w->q_cap);
     a.take(w->d_dmode, w->q_cap);
     a.take(w->d_sat, (uint64_t(w->q_cap) + 1) * w->sat_stride);
+    a.take(w->d_bin_list, w->term_cap);
+    a.take(w->d_nbin, n_q);
+    a.take(w->d_bblk, n_q);
+    a.take(w->d_parts, n_q + 1);
+    a.take(w->d_ticket, 1);
     if (w->kind == 0) a.take(w->d_slot, n_q);
     else a.take(w->d_cnt, n_q);
     if (w->kind == 1) a.take(w->d_qbm, std::max<uint64_t>(w->batch, 1) * w->qbm_stride);
@@ -746,7 +857,7 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     pa.path_uniform = r.tiles ? ABF_PATH_HYBRID : ABF_PATH_UNION;
     pa.hybrid_min = t.heavy_min_len;
     pa.heavy_min = w->d_heavy;
-    pa.term_lpref = w->d_lpref;
+    pa.term_slot = w->d_tslot;
     pa.q_light_cnt = w->d_lcnt;
     pa.n_probe = w->d_nprobe;  // not reached: no query takes the probe path
     pa.probe_cap = 0;
@@ -761,8 +872,21 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         pa.q_dmode = w->d_dmode;
         CUDA_TRY(cudaMemsetAsync(w->d_sat, 0, (uint64_t(nd_q) + 1) * w->sat_stride * 4u, s));
     }
-    TIMED(K_PLAN, abf::launch_plan(v, pa, s));
     abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, r.n_q, r.d_n_q};
+    const bool bins = group && v.n_plain > 0;
+    if (bins) {
+        pa.bin_list = w->d_bin_list;
+        pa.bin_min_blocks = bin_min_blocks(n_words);
+        pa.q_nbin = w->d_nbin;
+        pa.q_bblk = w->d_bblk;
+        qa.q_nbin = w->d_nbin;
+        qa.q_bblk = w->d_bblk;
+        qa.parts_pref = w->d_parts;
+        qa.ticket = w->d_ticket;
+        qa.n_tiles = bin_tiles(n_words);
+        qa.slots = uint32_t(ix->sm_count) * abf::kBinCtasPerSm;
+    }
+    TIMED(K_PLAN, abf::launch_plan(v, pa, s));
     TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
     if (group) {
         abf::DenseGroupArgs ga{};
@@ -805,7 +929,7 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     abf::ScatterArgs sa{};
     sa.terms = w->d_keys;
     sa.q_off = r.q_off;
-    sa.term_lpref = w->d_lpref;
+    sa.term_slot = w->d_tslot;
     sa.q_light_pref = w->d_lpref_q;
     sa.n_q = r.n_q;
     sa.d_n_q = r.d_n_q;
@@ -813,12 +937,31 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     sa.key_slot = r.key_slot;
     sa.out = r.out;
     sa.out_stride = r.out_stride;
-    sa.blocks_per_warp = std::max<uint32_t>(1u, t.scatter_blocks_per_warp);
+    sa.chunk_blocks = scatter_chunk(t);
     if (group) {
         sa.sat = w->d_sat;
         sa.sat_stride = w->sat_stride;
         sa.sat_shift = r.group.gw == 64u ? 6u : 5u;
         sa.sat_last = nd_q;  // a row of zeros for the runs past it
+        abf::BinArgs ba{};
+        ba.bin_list = w->d_bin_list;
+        ba.q_off = r.q_off;
+        ba.q_nbin = w->d_nbin;
+        ba.parts_pref = w->d_parts;
+        ba.ticket = w->d_ticket;
+        ba.n_q = r.n_q;
+        ba.d_n_q = r.d_n_q;
+        ba.n_tiles = bin_tiles(n_words);
+        ba.out = r.out;
+        ba.out_stride = r.out_stride;
+        ba.out_slot = r.out_slot;
+        ba.n_words = n_words;
+        ba.accumulate = 1;
+        ba.sat = sa.sat;
+        ba.sat_stride = sa.sat_stride;
+        ba.sat_shift = sa.sat_shift;
+        ba.sat_last = nd_q;
+        if (bins) TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
     }
     TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
     return ABF_OK;
@@ -1102,17 +1245,18 @@ abf_status abf_index_set_dense_div(abf_index* ix, uint32_t dense_div) {
         auto& dv = ix->dev;
         const uint64_t old = 4ull * (ix->derived.term_dense.size() + ix->derived.term_dir.size()) +
                              4ull * uint64_t(ix->derived.n_dense) * ix->derived.dense_stride +
-                             4ull * uint64_t(ix->derived.n_dir) * ix->derived.dir_n;
+                             4ull * uint64_t(ix->derived.n_dir) * ix->derived.dir_n + plain_bytes(ix);
         dev_free(dv.term_dense);
         dev_free(dv.dense);
         dev_free(dv.term_dir);
         dev_free(dv.dir);
+        free_plain(ix);
         dv.bytes = dv.bytes > old ? dv.bytes - old : 0;
         abf_status st;
         if ((st = upload_vec(&dv.term_dense, d.term_dense, &dv.bytes)) != ABF_OK ||
             (st = upload_vec(&dv.dense, d.dense, &dv.bytes)) != ABF_OK ||
             (st = upload_vec(&dv.term_dir, d.term_dir, &dv.bytes)) != ABF_OK ||
-            (st = upload_vec(&dv.dir, d.dir, &dv.bytes)) != ABF_OK) {
+            (st = upload_vec(&dv.dir, d.dir, &dv.bytes)) != ABF_OK || (st = make_plain(ix, d)) != ABF_OK) {
             free_device(ix);
             return st;
         }

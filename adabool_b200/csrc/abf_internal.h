@@ -74,10 +74,16 @@ struct HostIndex {
 //     merge kernel ORs its tile slice instead of decoding the blocks;
 //   - block directory: for long lists without a dense bitmap, dir[j] is
 //     the first block whose last id is >= j * 2^kDirShift, so a tile finds
-//     its blocks with three loads instead of two binary searches.
+//     its blocks with three loads instead of two binary searches;
+//   - plain ids: lists without a dense bitmap of at least plain_min_len()
+//     postings (longest first, within a memory budget) also keep their ids as
+//     plain uint32 arrays, unpacked on the device after the upload, with each
+//     list's position at every multiple of 2^kBinShift ads. Large batches
+//     merge them per tile without decoding (bin_kernel).
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint32_t kDirShift = 13;      // directory granularity: 8192 ids = 256 words
 constexpr uint32_t kDefaultDenseDiv = 128;
+constexpr uint32_t kBinShift = 19;      // ads per tile of the bin kernel: 2^19 (16,384 words)
 constexpr uint32_t kDirDiv = 512;       // lists with len * kDirDiv >= n_ads get a directory
 
 struct DerivedHost {
@@ -89,7 +95,19 @@ struct DerivedHost {
     std::vector<uint32_t> dir;          // n_dir * dir_n absolute block indices
     uint32_t dir_n = 0;                 // entries per list: ceil(n_ads / 2^kDirShift) + 1
     uint32_t n_dir = 0;
+    std::vector<uint32_t> term_plain;   // n_terms: plain list index or kNone
+    std::vector<uint32_t> plain_term;   // n_plain: its term
+    std::vector<uint32_t> plain_off;    // n_plain + 1: first id in the plain ids, in units of 4
+    uint32_t plain_dir_n = 0;           // positions per list: ceil(n_ads / 2^kBinShift) + 1
+    uint32_t n_plain() const { return uint32_t(plain_term.size()); }
 };
+
+// Shortest list that gets plain ids: below it a list's few postings per tile
+// cost less as atomics than the look-up of the tile's range.
+inline uint32_t plain_min_len(uint32_t n_ads) {
+    const uint32_t m = n_ads / 32768u;
+    return m > 256u ? m : 256u;
+}
 
 // Device copies of the same arrays.
 struct DeviceIndex {
@@ -104,6 +122,11 @@ struct DeviceIndex {
     uint32_t* dense = nullptr;
     uint32_t* term_dir = nullptr;
     uint32_t* dir = nullptr;
+    uint32_t* term_plain = nullptr;
+    uint32_t* plain_term = nullptr;
+    uint32_t* plain_off = nullptr;
+    uint32_t* plain = nullptr;        // ids
+    uint32_t* plain_dir = nullptr;    // n_plain x plain_dir_n positions in `plain`
     uint32_t* term_cbytes = nullptr;  // compressed bytes per term (planner feature)
     float* planner = nullptr;         // planner parameters (ABF_PLANNER_PARAMS) or null
     uint64_t bytes = 0;
@@ -123,6 +146,11 @@ struct IndexView {
     const uint32_t* term_dir;
     const uint32_t* dir;
     const uint32_t* term_cbytes;
+    const uint32_t* term_plain;
+    const uint32_t* plain;
+    const uint32_t* plain_dir;
+    uint32_t plain_dir_n;
+    uint32_t n_plain;
     uint64_t dense_stride;
     uint32_t n_dense;
     uint32_t dir_n;

@@ -138,24 +138,6 @@ __device__ __forceinline__ bool in_full_tile(const uint32_t* sat, uint32_t sat_s
     return (__ldg(sat + (t >> 5)) >> (t & 31u)) & 1u;
 }
 
-// true when every tile that ids [lo, hi) can touch is marked all ones
-// (tile = word >> sat_shift): the whole block can be skipped, decode
-// included. Ranges over more than 32 words of marks are not checked.
-__device__ __forceinline__ bool range_saturated(const uint32_t* sat, uint32_t sat_shift, uint32_t lo, uint32_t hi) {
-    const uint32_t t0 = (lo >> 5) >> sat_shift, t1 = ((hi - 1u) >> 5) >> sat_shift;
-    const uint32_t w0 = t0 >> 5, nw = (t1 >> 5) - w0 + 1u;
-    if (nw > 32u) return false;  // warp-uniform
-    const uint32_t lane = lane_id();
-    bool ok = true;
-    if (lane < nw) {
-        uint32_t m = ~0u;
-        if (lane == 0) m &= ~0u << (t0 & 31u);
-        if (lane + 1u == nw) m &= ~0u >> (31u - (t1 & 31u));
-        ok = (__ldg(sat + w0 + lane) & m) == m;
-    }
-    return __all_sync(kFull, ok);
-}
-
 // OR of this lane's four ids into the bitmap, one atomic per distinct word;
 // with sat (the dense group kernel's saturated-tile bits of this bitmap),
 // words inside an all-ones tile are skipped: the OR cannot change them
@@ -274,13 +256,24 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return true;
 }
 
+// async 4- and 16-byte copies global -> shared (LDGSTS: no register round trip)
+__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // planning
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) {
     __shared__ uint32_t s_warp[32];
     __shared__ unsigned long long s_red[8];
-    __shared__ uint32_t s_path, s_max, s_slot;
+    __shared__ uint32_t s_path, s_max, s_slot, s_nbin;
     __shared__ uint32_t s_mask[2048];  // the query's dense bitmaps (n_dense <= 65535)
     __shared__ plan_dev::PlannerSmem s_pl;
     static_assert(plan_dev::kFeatThreads == 256, "the planner code runs with the plan kernel's 256 threads");
@@ -359,24 +352,42 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             for (uint32_t i = tid; i < mw; i += 256) s_mask[i] = 0u;
             __syncthreads();
         }
+        bool bin = false;
+        if (a.bin_list) {
+            uint64_t nb = 0;
+            for (uint64_t i = qb + tid; i < qe && !probe; i += 256) {
+                const uint32_t t = a.terms[i];
+                if (t < ix.n_terms && __ldg(ix.term_plain + t) != kNone)
+                    nb += (__ldg(ix.term_len + t) + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS;
+            }
+            if (tid == 0) s_nbin = 0;
+            nb = block_sum_u64<256>(nb, s_red);  // its barriers also order the s_nbin reset
+            bin = nb >= a.bin_min_blocks && nb < 0xffffffffull;
+            if (tid == 0) a.q_bblk[q] = bin ? uint32_t(nb) : 0u;
+        }
         uint32_t carry = 0, nmerge = 0;
         for (uint64_t c0 = qb; c0 < qe; c0 += 256) {
             const uint64_t i = c0 + tid;
-            uint32_t cnt = 0, cls = kNone;
+            uint32_t cnt = 0, cls = kNone, blk = 0, pl;
             if (i < qe && !probe) {
                 const uint32_t t = a.terms[i];
                 if (t < ix.n_terms) {
                     const uint32_t d = merge_d ? __ldg(ix.term_dense + t) : kNone;
                     const uint32_t len = __ldg(ix.term_len + t);
                     if (d != kNone) cls = kDenseFlag | d;
-                    else if (len >= hm) cls = t;
-                    else cnt = __ldg(ix.term_blk + t + 1) - __ldg(ix.term_blk + t);
+                    else if (bin && (pl = __ldg(ix.term_plain + t)) != kNone) {
+                        a.bin_list[qb + atomicAdd(&s_nbin, 1u)] = pl;
+                    } else if (len >= hm) cls = t;
+                    else {
+                        blk = __ldg(ix.term_blk + t);
+                        cnt = __ldg(ix.term_blk + t + 1) - blk;
+                    }
                 }
             }
             if (i < qe && a.tile_cls) a.tile_cls[i] = cls;
             uint32_t tot;
             const uint32_t ex = block_excl_scan<256>(cnt, s_warp, &tot);
-            if (i < qe) a.term_lpref[i] = carry + ex;
+            if (i < qe) a.term_slot[i] = make_uint2(carry + ex, blk);
             carry += tot;
             if (want_d && cls != kNone) {
                 if (cls & kDenseFlag) {
@@ -419,6 +430,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             }
         }
         if (tid == 0) {
+            if (a.bin_list) a.q_nbin[q] = bin ? s_nbin : 0u;  // the scans' barriers order the last add
             a.heavy_min[q] = probe ? kNoHeavy : hm;
             a.q_light_cnt[q] = carry;
             if (a.path_out) a.path_out[q] = uint8_t(path);
@@ -462,6 +474,30 @@ __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
         __syncthreads();
     }
     if (tid == 0) a.q_light_pref[n_q] = s_carry;
+    if (!a.q_bblk) return;
+    // The bin kernel's items: every tile x every part of every query. A query
+    // is cut into parts by its lists so that no item has much more than half
+    // an even share of the work (or 128 blocks).
+    uint64_t sum = 0;
+    for (uint32_t i = tid; i < n_q; i += 1024) sum += a.q_bblk[i];
+    sum = block_sum_u64<1024>(sum, s_warp);
+    const uint64_t lim64 = max(128ull, static_cast<unsigned long long>(sum) / (2ull * a.slots)) * a.n_tiles;
+    const uint32_t lim = lim64 < 0xffffffffull ? uint32_t(lim64) : kFull;
+    uint32_t carry = 0;
+    __shared__ uint32_t s_w32[32];
+    for (uint32_t c0 = 0; c0 < n_q; c0 += 1024) {
+        const uint32_t i = c0 + tid;
+        uint32_t parts = 0;
+        if (i < n_q && a.q_bblk[i]) parts = min((a.q_bblk[i] - 1u) / lim + 1u, a.q_nbin[i]);
+        uint32_t tot;
+        const uint32_t ex = block_excl_scan<1024>(parts, s_w32, &tot);
+        if (i < n_q) a.parts_pref[i] = carry + ex;
+        carry += tot;
+    }
+    if (tid == 0) {
+        a.parts_pref[n_q] = carry;
+        *a.ticket = 0;
+    }
 }
 
 // Runs of consecutive keys with the same bitmap index, in one CTA: a flattened
@@ -668,7 +704,10 @@ __device__ __forceinline__ void dense_only_tile(const IndexView& ix, const uint1
     }
 }
 
-template <int W, int NW>
+// ACC: OR into the caller's bitmaps with atomics (other calls may do so at the
+// same time) instead of overwriting them. (A template: as a run-time flag it
+// cost the overwriting kernel 8 registers and a fifth of its occupancy.)
+template <int W, int NW, bool ACC>
 __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileArgs a) {
     constexpr int NT = NW * 32;
     constexpr uint32_t SPAN = uint32_t(W) * 32u;
@@ -704,12 +743,12 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
         const uint64_t left = a.n_words - uint64_t(t) * W;
         const uint32_t nw = left < uint64_t(W) ? uint32_t(left) : uint32_t(W);
         if (hm == kNoHeavy || qb == qe) {  // nothing to merge: leave or zero the tile
-            if (!a.accumulate)
+            if (!ACC)
                 for (uint32_t i = tid; i < nw; i += NT) dst[i] = 0u;
             continue;
         }
         const uint32_t dmode = a.q_dense16 ? a.q_dmode[q] : 0u;
-        if (a.q_dense16 && !a.accumulate && dmode == 1u) {
+        if (!ACC && a.q_dense16 && dmode == 1u) {
             // every merged list has a dense bitmap: the dense group kernel
             // writes this tile, or each thread ORs its 16-byte slots over the
             // query's dense slices, KT loads in flight, and stores the
@@ -721,7 +760,7 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
         // with the dense group kernel on, a query that also merges lists
         // without dense bitmaps already has its dense lists in the output:
         // the tile starts from it and adds only the others
-        const bool on_group = a.skip_dense_only && dmode == 2u && !a.accumulate;
+        const bool on_group = a.skip_dense_only && dmode == 2u && !ACC;
         for (uint32_t i = tid; i < uint32_t(W); i += NT) tile[i] = (on_group && i < nw) ? dst[i] : 0u;
         if (tid == 0) s_ndense = 0;
         __syncthreads();
@@ -817,8 +856,7 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
             if (tid == 0) s_ndense = 0;
             __syncthreads();
         }
-        if (a.accumulate) {
-            // the caller's bitmap may be ORed into by other calls at the same time
+        if constexpr (ACC) {
             for (uint32_t i = tid; i < nw; i += NT)
                 if (tile[i]) atomicOr(dst + i, tile[i]);
         } else if (a.vec_ok) {
@@ -1078,94 +1116,464 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
 // ---------------------------------------------------------------------------
 // list-union, scatter variant (load-balanced over the short lists' blocks)
 // ---------------------------------------------------------------------------
+// Lean decode of one block by one warp, from payload words read straight into
+// registers: lane l takes gap slots 4l .. 4l+3, that is ids 4l+1 .. 4l+4, and
+// the last lane's fourth position (a block has at most 127 gaps) stands for
+// the block's first id. Only for bits <= 16: the lane's four gaps then lie in
+// the 64 bits from bit 4 * bits * l, three words at most.
+struct GapWords {
+    uint32_t x0, x1, x2;
+};
+__device__ __forceinline__ GapWords load_gaps(const IndexView& ix, uint32_t unit, uint32_t meta) {
+    const uint32_t bits = meta & 63u, gaps = (meta >> 8) & 127u;
+    GapWords g{0u, 0u, 0u};
+    // a lane whose first slot exists reads at most two words past the block's
+    // last one: inside the payload's padding unit
+    if (4u * lane_id() < gaps) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(ix.payload + unit) + ((4u * bits * lane_id()) >> 5);
+        g.x0 = __ldg(w);
+        g.x1 = __ldg(w + 1);
+        g.x2 = __ldg(w + 2);
+    }
+    return g;
+}
+__device__ __forceinline__ void gaps_to_ids(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, uint32_t first,
+                                            uint32_t (&id)[4]) {
+    const uint32_t lane = lane_id();
+    const uint32_t p0 = v0 + 1u, p1 = p0 + v1 + 1u, p2 = p1 + v2 + 1u, run = p2 + v3 + 1u;
+    uint32_t x = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= uint32_t(o)) x += y;
+    }
+    const uint32_t base = first + (x - run);
+    id[0] = base + p0;
+    id[1] = base + p1;
+    id[2] = base + p2;
+    id[3] = lane == 31u ? first : base + run;
+}
+// ids of this lane's four positions; position k is valid when 4 * lane + k <
+// gaps, and lane 31's fourth always is
+__device__ __forceinline__ void decode_gaps(const GapWords& g, uint32_t first, uint32_t meta, uint32_t (&id)[4]) {
+    const uint32_t lane = lane_id(), bits = meta & 63u, mask = (1u << bits) - 1u;
+    const uint32_t off = (4u * bits * lane) & 31u;
+    uint32_t lo = __funnelshift_r(g.x0, g.x1, off), hi = __funnelshift_r(g.x1, g.x2, off);
+    const uint32_t v0 = lo & mask, v1 = __funnelshift_r(lo, hi, bits) & mask;
+    lo = __funnelshift_rc(lo, hi, 2u * bits);
+    hi = __funnelshift_rc(hi, 0u, 2u * bits);
+    const uint32_t v2 = lo & mask, v3 = __funnelshift_r(lo, hi, bits) & mask;
+    gaps_to_ids(v0, v1, v2, v3, first, id);
+}
+// The same for any width, with each gap's two words read on their own: lists
+// whose gaps do not fit 16 bits are short or very uneven.
+__device__ __noinline__ void decode_wide(const IndexView& ix, uint32_t unit, uint32_t first, uint32_t meta,
+                                         uint32_t (&id)[4]) {
+    const uint32_t bits = meta & 63u, gaps = (meta >> 8) & 127u;
+    const uint32_t mask = bits >= 32u ? kFull : (1u << bits) - 1u;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(ix.payload + unit);
+    uint32_t v[4];
+#pragma unroll
+    for (uint32_t e = 0; e < 4u; ++e) {
+        const uint32_t s = 4u * lane_id() + e, pos = s * bits;
+        v[e] = s < gaps ? __funnelshift_r(__ldg(w + (pos >> 5)), __ldg(w + (pos >> 5) + 1), pos & 31u) & mask : 0u;
+    }
+    gaps_to_ids(v[0], v[1], v[2], v[3], first, id);
+}
+
+// last i in [0, n) with at(i) <= key, by the whole warp (32 probes a step);
+// at(0) <= key, at ascending
+template <typename At, typename Key>
+__device__ __forceinline__ uint32_t warp_last_le(At at, uint32_t n, Key key) {
+    uint32_t lo = 0;
+    while (n > 1u) {
+        const uint32_t step = (n + 31u) / 32u, i = lane_id() * step;
+        const bool le = i < n && at(lo + i) <= key;
+        const uint32_t k = uint32_t(__popc(__ballot_sync(kFull, le))) - 1u;
+        lo += k * step;
+        n = n - k * step < step ? n - k * step : step;
+    }
+    return lo;
+}
+
+// Load-balanced warps over the short lists' blocks. A warp takes a chunk of up
+// to 32 consecutive blocks of the flat block order (queries, then their term
+// slots, then the slots' blocks) and works in two parts:
+//  * a lane per block: find the block's query and term slot, read its bounds
+//    and descriptor, and test its id range against the saturation marks of its
+//    bitmap. Blocks in all-ones tiles only are dropped here, before any of
+//    their payload is read;
+//  * a warp per remaining block: decode (the next block's payload loads in
+//    flight) and OR, one atomic per word a lane's ids touch; a block of which
+//    some tiles are all ones skips the ORs into those.
+// Bound: the atomics' way to L2 (see bin_kernel). Walking the blocks one by
+// one (slot arithmetic, bound and descriptor loads by the whole warp, gaps
+// staged in shared memory) took about 300 instructions per block of 128 ids
+// and a chain of ~20 loads per chunk: one query's few hundred blocks 16.5 us
+// where they now take 4 (c0), 32 queries' 94 thousand 49 instead of 55.
 // KEYED: one query whose term slots each have an output bitmap of their own.
 template <int NW, bool KEYED>
-__global__ void __launch_bounds__(NW * 32) scatter_kernel(IndexView ix, ScatterArgs a) {
-    __shared__ __align__(16) uint4 stage[NW][32];
-    const uint32_t warp = warp_id();
+__global__ void __launch_bounds__(NW * 32, 6) scatter_kernel(IndexView ix, ScatterArgs a) {
+    __shared__ __align__(16) uint4 s_blk[NW][32];  // {payload unit, first id, meta | kMixed, output bitmap}
+    __shared__ uint32_t s_row[NW][32];             // row of saturation marks
+    constexpr uint32_t kMixed = 0x80000000u;       // some of the block's tiles are all ones
+    const uint32_t warp = warp_id(), lane = lane_id();
     const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
+    if (n_q == 0) return;
     const uint64_t total = a.q_light_pref[n_q];
-    const uint64_t bpw = a.blocks_per_warp;
     const uint64_t nwt = uint64_t(gridDim.x) * NW;
-    for (uint64_t f0 = (uint64_t(blockIdx.x) * NW + warp) * bpw; f0 < total; f0 += nwt * bpw) {
-        const uint64_t f1 = f0 + bpw < total ? f0 + bpw : total;
-        // query: last q with q_light_pref[q] <= f0
-        uint32_t q0 = 0, q1 = n_q;
-        while (q1 - q0 > 1) {
-            const uint32_t m = (q0 + q1) >> 1;
-            if (a.q_light_pref[m] <= f0) q0 = m; else q1 = m;
+    // few blocks: fewer per warp, so that every warp has some
+    const uint64_t per = (total + nwt - 1) / nwt;
+    const uint32_t chunk = per < a.chunk_blocks ? uint32_t(per) : a.chunk_blocks;
+    const uint32_t tshift = a.sat_shift + 5u;  // id -> tile
+    for (uint64_t f0 = (uint64_t(blockIdx.x) * NW + warp) * chunk; f0 < total; f0 += nwt * chunk) {
+        // ---- a lane per block ----
+        const bool mine = lane < chunk && f0 + lane < total;
+        const uint64_t f = mine ? f0 + lane : f0;
+        uint32_t q = warp_last_le([&](uint32_t i) { return a.q_light_pref[i]; }, n_q, f0);
+        uint64_t pq = a.q_light_pref[q];
+        for (uint64_t nx; (nx = a.q_light_pref[q + 1]) <= f; pq = nx) ++q;
+        const uint32_t r = uint32_t(f - pq);
+        uint64_t slot = 0;
+        uint2 sl = make_uint2(0u, 0u);  // the slot's first block: flat in its query, and in the index
+        for (uint32_t todo = kFull; todo;) {
+            const int lead = __ffs(todo) - 1;
+            const uint32_t ql = __shfl_sync(kFull, q, lead);
+            const uint32_t rl = __shfl_sync(kFull, r, lead);
+            const uint64_t qb = a.q_off[ql];
+            const uint32_t n = uint32_t(a.q_off[ql + 1] - qb);
+            uint32_t base = warp_last_le([&](uint32_t i) { return a.term_slot[qb + i].x; }, n, rl);
+            // 32 slots at a time: rank of each of this query's lanes among their prefixes
+            for (uint32_t left = __ballot_sync(kFull, (todo >> lane & 1u) && q == ql);; base += 31u) {
+                const uint2 p = base + lane < n ? a.term_slot[qb + base + lane] : make_uint2(kFull, 0u);
+                uint32_t at = 0;
+#pragma unroll
+                for (uint32_t h = 16; h; h >>= 1) {
+                    const uint32_t y = __shfl_sync(kFull, p.x, at + h);
+                    if (y <= r) at += h;
+                }
+                const uint32_t px = __shfl_sync(kFull, p.x, at), py = __shfl_sync(kFull, p.y, at);
+                const bool in = left >> lane & 1u;
+                const bool done = in && at < 31u;
+                if (done) {
+                    slot = qb + base + at;
+                    sl = make_uint2(px, py);
+                }
+                const uint32_t d = __ballot_sync(kFull, done);
+                left &= ~d;
+                todo &= ~d;
+                if (!left) break;
+            }
         }
-        uint32_t q = q0;
-        uint64_t qb = a.q_off[q], qe = a.q_off[q + 1];
-        uint32_t qtot = uint32_t(a.q_light_pref[q + 1] - a.q_light_pref[q]);
-        const uint32_t r = uint32_t(f0 - a.q_light_pref[q]);
-        // term slot: last i with term_lpref[i] <= r
-        uint64_t i0 = qb, i1 = qe;
-        while (i1 - i0 > 1) {
-            const uint64_t m = (i0 + i1) >> 1;
-            if (a.term_lpref[m] <= r) i0 = m; else i1 = m;
+        const uint32_t b = sl.y + (r - sl.x);
+        const uint32_t first = __ldg(ix.blk_first + b);
+        const uint2 desc = __ldg(ix.blk_desc + b);
+        const uint32_t out_i = KEYED ? a.key_slot[slot] : a.out_slot ? a.out_slot[q] : q;
+        uint32_t meta = desc.y;
+        bool live = mine;
+        if (a.sat) {
+            const uint32_t row = min(q, a.sat_last);
+            const uint32_t* sat = a.sat + uint64_t(row) * a.sat_stride;
+            const uint32_t t0 = first >> tshift, t1 = __ldg(ix.blk_last + b) >> tshift;
+            const uint32_t w0 = t0 >> 5, w1 = t1 >> 5;
+            bool all = true, some = false;
+            if (w1 - w0 < 32u) {
+                for (uint32_t w = w0; w <= w1; ++w) {
+                    uint32_t m = kFull;
+                    if (w == w0) m &= kFull << (t0 & 31u);
+                    if (w == w1) m &= kFull >> (31u - (t1 & 31u));
+                    const uint32_t v = __ldg(sat + w) & m;
+                    all &= v == m;
+                    some |= v != 0u;
+                }
+            } else {  // a wide range is not checked as a whole
+                all = false;
+                some = true;
+            }
+            live = mine && !all;
+            if (some) meta |= kMixed;
+            s_row[warp][lane] = row;
         }
-        uint64_t i = i0;
-        uint32_t j = r - a.term_lpref[i];
-        uint32_t* out = a.out + uint64_t(KEYED ? a.key_slot[i] : a.out_slot ? a.out_slot[q] : q) * a.out_stride;
-        const uint32_t* sat = a.sat ? a.sat + uint64_t(min(q, a.sat_last)) * a.sat_stride : nullptr;
-        // (i, j) is a scattered block of query q; the walk moves to the next
-        // one, crossing into later terms and queries as they run out
-        auto advance = [&]() {
-            ++j;
-            for (;;) {
-                const uint32_t nb = (i + 1 < qe ? a.term_lpref[i + 1] : qtot) - a.term_lpref[i];
-                if (j < nb) return;
-                ++i;
-                j = 0;
-                if constexpr (KEYED) {
-                    out = a.out + uint64_t(a.key_slot[i]) * a.out_stride;
-                } else if (i >= qe) {
-                    do {
-                        ++q;
-                    } while (a.q_light_pref[q + 1] == a.q_light_pref[q]);
-                    qb = a.q_off[q];
-                    qe = a.q_off[q + 1];
-                    qtot = uint32_t(a.q_light_pref[q + 1] - a.q_light_pref[q]);
-                    i = qb;
-                    out = a.out + uint64_t(a.out_slot ? a.out_slot[q] : q) * a.out_stride;
-                    if (a.sat) sat = a.sat + uint64_t(min(q, a.sat_last)) * a.sat_stride;
+        __syncwarp();
+        s_blk[warp][lane] = make_uint4(desc.x, first, meta, out_i);
+        __syncwarp();
+        // ---- a warp per block ----
+        uint32_t todo = __ballot_sync(kFull, live);
+        if (!todo) continue;
+        uint32_t k = uint32_t(__ffs(todo)) - 1u;
+        uint4 nb = s_blk[warp][k];
+        GapWords ng = load_gaps(ix, nb.x, nb.z);
+        while (todo) {
+            const uint4 cb = nb;
+            const GapWords cg = ng;
+            const uint32_t ck = k;
+            todo &= todo - 1u;
+            if (todo) {
+                k = uint32_t(__ffs(todo)) - 1u;
+                nb = s_blk[warp][k];
+                ng = load_gaps(ix, nb.x, nb.z);
+            }
+            uint32_t* out = a.out + uint64_t(cb.w) * a.out_stride;
+            const uint32_t* sat = cb.z & kMixed ? a.sat + uint64_t(s_row[warp][ck]) * a.sat_stride : nullptr;
+            uint32_t id[4];
+            if ((cb.z & 63u) > 16u) decode_wide(ix, cb.x, cb.y, cb.z, id);
+            else decode_gaps(cg, cb.y, cb.z, id);
+            const uint32_t gaps = (cb.z >> 8) & 127u;
+            uint32_t m[4];
+#pragma unroll
+            for (uint32_t e = 0; e < 4u; ++e) m[e] = 1u << (id[e] & 31u);
+            if (gaps != 127u) {  // warp-uniform: a list's last block
+#pragma unroll
+                for (uint32_t e = 0; e < 4u; ++e)
+                    if (4u * lane + e >= gaps && !(e == 3u && lane == 31u)) m[e] = 0u;
+            }
+            if (sat) {
+#pragma unroll
+                for (uint32_t e = 0; e < 4u; ++e) {
+                    const uint32_t t = id[e] >> tshift;
+                    if (m[e] && (__ldg(sat + (t >> 5)) >> (t & 31u) & 1u)) m[e] = 0u;
                 }
             }
-        };
-        // exclusive bound on the ids of block b, the j-th of slot i: the next
-        // block's first id, or n_ads after the term's last block (only
-        // needed with saturation marks)
-        auto block_hi = [&](uint32_t b) -> uint32_t {
-            if (!a.sat) return ix.n_ads;
-            const uint32_t nb = (i + 1 < qe ? a.term_lpref[i + 1] : qtot) - a.term_lpref[i];
-            return j + 1u < nb ? __ldg(ix.blk_first + b + 1u) : ix.n_ads;
-        };
-        uint32_t b = __ldg(ix.term_blk + a.terms[i]) + j;
-        Fetched nxt = fetch_block(ix, b);
-        uint32_t nxt_hi = block_hi(b);
-        uint32_t* nxt_out = out;
-        const uint32_t* nxt_sat = sat;
-        for (uint64_t f = f0; f < f1; ++f) {
-            const Fetched cur = nxt;
-            const uint32_t cur_hi = nxt_hi;
-            uint32_t* cur_out = nxt_out;
-            const uint32_t* cur_sat = nxt_sat;
-            if (f + 1 < f1) {  // next block's loads in flight during this decode
-                advance();
-                b = __ldg(ix.term_blk + a.terms[i]) + j;
-                nxt = fetch_block(ix, b);
-                nxt_hi = block_hi(b);
-                nxt_out = out;
-                nxt_sat = sat;
+            // ids of one word become one atomic
+#pragma unroll
+            for (uint32_t e = 0; e < 3u; ++e) {
+                if ((id[e] ^ id[e + 1]) < 32u) {
+                    m[e + 1] |= m[e];
+                    m[e] = 0u;
+                }
             }
-            // a block whose whole id range lies in tiles the dense lists
-            // already filled changes nothing: skip its decode and ORs
-            if (cur_sat && range_saturated(cur_sat, a.sat_shift, cur.first, cur_hi)) continue;
-            uint32_t id[4], cnt;
-            decode_fetched(cur, stage[warp], id, cnt);
-            or_global(cur_out, ix.n_ads, id, cnt, cur_sat, a.sat_shift);
+#pragma unroll
+            for (uint32_t e = 0; e < 4u; ++e)
+                if (m[e]) atomicOr(out + (id[e] >> 5), m[e]);
         }
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// list-union, binned variant
+// ---------------------------------------------------------------------------
+// The plain ids of the lists in plain_term, a warp per block.
+__global__ void __launch_bounds__(256) plain_ids_kernel(IndexView ix, const uint32_t* plain_off, uint32_t* plain) {
+    const uint64_t nw = uint64_t(gridDim.x) * 8u;
+    for (uint64_t b = uint64_t(blockIdx.x) * 8u + warp_id(); b < ix.n_blocks; b += nw) {
+        const uint32_t t = __ldg(ix.blk_term + b), p = __ldg(ix.term_plain + t);
+        if (p == kNone) continue;
+        const uint2 d = __ldg(ix.blk_desc + b);
+        const uint32_t first = __ldg(ix.blk_first + b), gaps = d.y >> 8;
+        uint32_t id[4];
+        if ((d.y & 63u) > 16u) decode_wide(ix, d.x, first, d.y, id);
+        else decode_gaps(load_gaps(ix, d.x, d.y), first, d.y, id);
+        uint32_t* dst = plain + uint64_t(__ldg(plain_off + p)) * 4u + (b - __ldg(ix.term_blk + t)) * ABF_BLOCK_POSTINGS;
+#pragma unroll
+        for (uint32_t e = 0; e < 4u; ++e) {
+            const uint32_t s = 4u * lane_id() + e;  // gap slot: the id after it
+            if (s < gaps) dst[s + 1u] = id[e];
+            else if (s == ABF_BLOCK_POSTINGS - 1u) dst[0] = first;
+        }
+    }
+}
+
+// position in the plain ids of each list's first id at or past every tile start
+__global__ void __launch_bounds__(256) plain_dir_kernel(IndexView ix, const uint32_t* plain_term,
+                                                        const uint32_t* plain_off, uint32_t* dir) {
+    const uint64_t n = uint64_t(ix.n_plain) * ix.plain_dir_n;
+    for (uint64_t i = uint64_t(blockIdx.x) * 256u + threadIdx.x; i < n; i += uint64_t(gridDim.x) * 256u) {
+        const uint32_t p = uint32_t(i / ix.plain_dir_n), j = uint32_t(i - uint64_t(p) * ix.plain_dir_n);
+        const uint32_t len = __ldg(ix.term_len + plain_term[p]), a0 = plain_off[p] * 4u;
+        const uint64_t key = uint64_t(j) << kBinShift;
+        dir[i] = a0 + (key >= ix.n_ads ? len : lower_bound_g(ix.plain + a0, 0u, len, uint32_t(key)));
+    }
+}
+
+// A lane's global atomic is a 32-byte sector of its own on the way to L2: an
+// SM sends about one per clock, so the scatter kernel stops at ~300 G
+// postings/s however few instructions it takes, and where the batch's bitmaps
+// exceed L2 each such sector is read from and written to HBM. Shared-memory
+// atomics go at about ten lanes a clock. So in large batches the lists of mid
+// length (plain ids, no dense bitmap) are merged per tile: a CTA takes one
+// (tile, query, part) item at a time from a ticket counter, loads its 16,384
+// words of the bitmap (the group kernel's output), looks up each list's ids in
+// the tile (a thread per list), cuts them into chunks of at most 256 (a thread
+// per chunk), ORs the chunks (a warp per chunk, eight ids a lane) and writes
+// the tile back. Tiles-of-64 that are all ones already are neither read nor
+// written. Items run tile by tile, so that the ids that queries share are read
+// from L2. A query with more than its share of ids is cut into parts by its
+// lists; their tiles start at zero and are ORed into the output by coalesced
+// atomics.
+// 512 queries of config c1: 550 us (333 of them the tiles' round trip through
+// HBM), and the scatter kernel's share falls from 1,269 to 110; 2,048 queries
+// of config c2: 2.65 and 0.47 ms where the scatter took 9.72. The same from
+// the packed blocks (bounds, decode and range tests per block and tile, ~160
+// instructions for 128 ids) took 868 us on c1; testing every id's mark before
+// its shared atomic 649; without the shared atomics it takes as long as with.
+template <bool ACC>
+__global__ void __launch_bounds__(kBinThreads, kBinCtasPerSm) bin_kernel(IndexView ix, BinArgs a) {
+    constexpr uint32_t W = kBinWords, NT = kBinThreads, NW = NT / 32u;
+    constexpr uint32_t kSub = W / 64u;  // tiles-of-64 of an item, one mark each
+    constexpr uint32_t kChunk = 256u;   // ids a warp ORs at a time
+    extern __shared__ __align__(16) uint32_t tile[];
+    __shared__ uint32_t s_lo[NT], s_n[NT], s_pref[NT + 1], s_warp[32], s_sat[kSub / 32u];
+    __shared__ uint2 s_chunk[NT];                 // {position of the first id, ids}
+    __shared__ uint64_t s_qb[2];                  // of the current and the next item: first slot of the query,
+    __shared__ uint32_t s_it[2][6];                // {item left?, tile, query, part, parts, lists of the query}
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
+    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
+    if (n_q == 0) return;
+    const uint32_t n_parts = a.parts_pref[n_q];
+    if (n_parts == 0) return;
+    const uint64_t items = uint64_t(n_parts) * a.n_tiles;
+    uint4* tile4 = reinterpret_cast<uint4*>(tile);
+    uint8_t* tile_b = reinterpret_cast<uint8_t*>(tile);
+    // warp 0 claims an item and looks it up, one item ahead of the CTA's work
+    auto claim = [&](uint32_t slot) {
+        uint32_t item = 0;
+        if (lane == 0) item = atomicAdd(a.ticket, 1u);
+        item = __shfl_sync(kFull, item, 0);
+        if (item < items) {
+            const uint32_t t = item / n_parts, g = item - t * n_parts;
+            const uint32_t q = warp_last_le([&](uint32_t i) { return a.parts_pref[i]; }, n_q, g);
+            const uint32_t p0 = a.parts_pref[q], p1 = a.parts_pref[q + 1];
+            if (lane == 0) {
+                s_qb[slot] = a.q_off[q];
+                s_it[slot][1] = t;
+                s_it[slot][2] = q;
+                s_it[slot][3] = g - p0;
+                s_it[slot][4] = p1 - p0;
+                s_it[slot][5] = a.q_nbin[q];
+            }
+        }
+        if (lane == 0) s_it[slot][0] = item < items ? 1u : 0u;
+    };
+    if (warp == 0) claim(0);
+    __syncthreads();
+    for (uint32_t cur = 0;; cur ^= 1u) {
+        if (!s_it[cur][0]) return;
+        const uint32_t t = s_it[cur][1], q = s_it[cur][2], part = s_it[cur][3], parts = s_it[cur][4];
+        const uint64_t qb = s_qb[cur];
+        const uint32_t nm = (s_it[cur][5] + parts - 1u - part) / parts;  // this part's lists: part, part + parts, ..
+        const bool own = !ACC && parts == 1u;  // nobody else ORs into this tile
+        uint32_t* dst = a.out + uint64_t(a.out_slot ? a.out_slot[q] : q) * a.out_stride + uint64_t(t) * W;
+        const uint64_t left = a.n_words - uint64_t(t) * W;
+        const uint32_t nw = left < uint64_t(W) ? uint32_t(left) : W;
+        // marks of the tile; a tile that is all ones needs nothing
+        bool full = true;
+        if (tid < kSub / 32u) {
+            const uint32_t* sat = a.sat + uint64_t(min(q, a.sat_last)) * a.sat_stride;
+            uint32_t v = 0;
+            if (a.sat_shift == 6u) {
+                const uint32_t w = t * (kSub / 32u) + tid;
+                if (w < a.sat_stride) v = sat[w];
+            } else {  // marks of 32-word tiles: both halves
+                for (uint32_t h = 0; h < 2u; ++h) {
+                    const uint32_t w = (t * (kSub / 32u) + tid) * 2u + h;
+                    const uint32_t x = w < a.sat_stride ? sat[w] : 0u;
+                    for (uint32_t b = 0; b < 16u; ++b) v |= ((x >> (2u * b) & 3u) == 3u ? 1u : 0u) << (h * 16u + b);
+                }
+            }
+            s_sat[tid] = v;
+            const uint32_t n = (nw + 63u) / 64u;  // marks in use
+            const uint32_t used = tid * 32u >= n ? 0u : n - tid * 32u >= 32u ? kFull : (1u << (n - tid * 32u)) - 1u;
+            full = (v & used) == used;
+        }
+        const bool skip = __syncthreads_and(full);
+        if (warp == 0) claim(cur ^ 1u);
+        if (skip) {
+            __syncthreads();
+            continue;
+        }
+        // the tile's words come in while the lists are looked up. Thread tid's
+        // 16-byte slots are tid + NT * k, in tiles-of-64 tid / 16 + 32 * k: bit
+        // tid / 16 of mark word k
+        const uint32_t mbit = 1u << (tid >> 4);
+        static_assert(NT == 512 && kSub == 256, "mark word k covers the slots tid + NT * k");
+        if (own && a.vec_ok && nw == W) {
+#pragma unroll
+            for (uint32_t k = 0; k < kSub / 32u; ++k)
+                if (!(s_sat[k] & mbit)) cp_async16(tile4 + tid + NT * k, dst + (tid + NT * k) * 4u);
+        } else if (own) {
+            for (uint32_t i = tid; i < W; i += NT) tile[i] = i < nw ? dst[i] : 0u;
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < kSub / 32u; ++k) tile4[tid + NT * k] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (uint32_t c0 = 0; c0 < nm; c0 += NT) {
+            uint32_t lo = 0, n = 0;
+            if (c0 + tid < nm) {
+                const uint32_t* d = ix.plain_dir +
+                                    uint64_t(a.bin_list[qb + part + uint64_t(c0 + tid) * parts]) * ix.plain_dir_n + t;
+                lo = __ldg(d);
+                n = __ldg(d + 1) - lo;
+            }
+            uint32_t total;
+            const uint32_t ex = block_excl_scan<int(NT)>((n + kChunk - 1u) / kChunk, s_warp, &total);
+            s_lo[tid] = lo;
+            s_n[tid] = n;
+            s_pref[tid] = ex;
+            if (tid == NT - 1u) s_pref[NT] = ex + (n + kChunk - 1u) / kChunk;
+            cp_async_wait_all();
+            __syncthreads();  // also: the tile is loaded
+            for (uint32_t f0 = 0; f0 < total; f0 += NT) {
+                const uint32_t m = min(NT, total - f0);
+                if (tid < m) {
+                    const uint32_t s = find_slot<int(NT)>(s_pref, f0 + tid), k = (f0 + tid - s_pref[s]) * kChunk;
+                    s_chunk[tid] = make_uint2(s_lo[s] + k, min(kChunk, s_n[s] - k));
+                }
+                __syncthreads();
+                // the next chunk's ids are in flight while one is ORed
+                constexpr uint32_t E = kChunk / 32u;
+                uint32_t nx[E], nn = 0;
+                auto fetch = [&](uint32_t i) {
+                    const uint2 c = s_chunk[i];
+                    const uint32_t* src = ix.plain + c.x + lane;
+                    nn = c.y;
+#pragma unroll
+                    for (uint32_t e = 0; e < E; ++e)
+                        if (lane + 32u * e < c.y) nx[e] = __ldg(src + 32u * e);
+                };
+                if (warp < m) fetch(warp);
+                for (uint32_t i = warp; i < m; i += NW) {
+                    uint32_t x[E];
+                    const uint32_t cn = nn;
+#pragma unroll
+                    for (uint32_t e = 0; e < E; ++e) x[e] = nx[e];
+                    if (i + NW < m) fetch(i + NW);
+                    // a tile starts at a multiple of 2^19 ads: the byte of an
+                    // id's word in it is (id >> 3) mod 64 K, less two bits
+                    auto put = [&](uint32_t e) {
+                        atomicOr(reinterpret_cast<uint32_t*>(tile_b + (x[e] >> 3 & (W * 4u - 4u))), 1u << (x[e] & 31u));
+                    };
+                    if (cn == kChunk) {
+#pragma unroll
+                        for (uint32_t e = 0; e < E; ++e) put(e);
+                    } else {
+#pragma unroll
+                        for (uint32_t e = 0; e < E; ++e)
+                            if (lane + 32u * e < cn) put(e);
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (own) {
+            if (a.vec_ok && nw == W) {
+#pragma unroll
+                for (uint32_t k = 0; k < kSub / 32u; ++k)
+                    if (!(s_sat[k] & mbit)) reinterpret_cast<uint4*>(dst)[tid + NT * k] = tile4[tid + NT * k];
+            } else {
+                for (uint32_t i = tid; i < nw; i += NT) dst[i] = tile[i];
+            }
+        } else if (nw == W) {
+#pragma unroll 8
+            for (uint32_t i = tid; i < W; i += NT) {
+                const uint32_t v = tile[i];
+                if (v) atomicOr(dst + i, v);
+            }
+        } else {
+            for (uint32_t i = tid; i < nw; i += NT)
+                if (tile[i]) atomicOr(dst + i, tile[i]);
+        }
+        __syncthreads();  // the tile and the marks are read, the next item is there
     }
 }
 
@@ -1409,14 +1817,6 @@ __device__ __forceinline__ void expand_lane_word(uint32_t v, uint32_t ex, uint32
     }
 }
 
-// async 4-byte copy global -> shared (LDGSTS: no register round trip)
-__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(sdst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 // One warp claims the next work item and makes it ready for the CTA: the
 // chunk's words into buf (lane l: word 32 m + l), each warp slice's id count
 // into s_wtot, the decoupled look-back's exclusive prefix into *s_prefix.
@@ -1634,6 +2034,11 @@ IndexView view_of(const abf_index* ix) {
     v.term_dir = ix->dev.term_dir;
     v.dir = ix->dev.dir;
     v.term_cbytes = ix->dev.term_cbytes;
+    v.term_plain = ix->dev.term_plain;
+    v.plain = ix->dev.plain;
+    v.plain_dir = ix->dev.plain_dir;
+    v.plain_dir_n = ix->derived.plain_dir_n;
+    v.n_plain = ix->dev.plain ? ix->derived.n_plain() : 0u;
     v.dense_stride = ix->derived.dense_stride;
     v.dir_n = ix->derived.dir_n;
     v.n_dense = ix->derived.n_dense;
@@ -1679,7 +2084,7 @@ cudaError_t launch_term_lists(const TermListArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int W, int NW>
+template <int W, int NW, bool ACC>
 static cudaError_t tile_launch(const IndexView& v, const TileArgs& a, int grid, cudaStream_t s) {
     constexpr int smem = W * 4;
     if (smem > 48 * 1024) {
@@ -1692,22 +2097,22 @@ static cudaError_t tile_launch(const IndexView& v, const TileArgs& a, int grid, 
         if (e != cudaSuccess) return e;
         const uint64_t bit = 1ull << (dev & 63);
         if (!(done.load() & bit)) {
-            e = cudaFuncSetAttribute(tile_union_kernel<W, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = cudaFuncSetAttribute(tile_union_kernel<W, NW, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
             done.fetch_or(bit);
         }
     }
-    tile_union_kernel<W, NW><<<grid, NW * 32, smem, s>>>(v, a);
+    tile_union_kernel<W, NW, ACC><<<grid, NW * 32, smem, s>>>(v, a);
     return cudaGetLastError();
 }
 
 template <int W>
 static cudaError_t tile_dispatch_w(const IndexView& v, const TileArgs& a, uint32_t nw, int grid, cudaStream_t s) {
     switch (nw) {
-        case 1: return tile_launch<W, 1>(v, a, grid, s);
-        case 2: return tile_launch<W, 2>(v, a, grid, s);
-        case 4: return tile_launch<W, 4>(v, a, grid, s);
-        default: return tile_launch<W, 8>(v, a, grid, s);
+        case 1: return a.accumulate ? tile_launch<W, 1, true>(v, a, grid, s) : tile_launch<W, 1, false>(v, a, grid, s);
+        case 2: return a.accumulate ? tile_launch<W, 2, true>(v, a, grid, s) : tile_launch<W, 2, false>(v, a, grid, s);
+        case 4: return a.accumulate ? tile_launch<W, 4, true>(v, a, grid, s) : tile_launch<W, 4, false>(v, a, grid, s);
+        default: return a.accumulate ? tile_launch<W, 8, true>(v, a, grid, s) : tile_launch<W, 8, false>(v, a, grid, s);
     }
 }
 
@@ -1820,11 +2225,47 @@ cudaError_t launch_dense_group(const void* tmaps, uint32_t gw, const DenseGroupA
 cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_tuning& t, int sm_count,
                            cudaStream_t s) {
     if (a.n_q == 0) return cudaSuccess;
-    const int grid = grid_for(~0ull, sm_count, t.ctas_per_sm ? t.ctas_per_sm * 2u : 8u);
+    // one wave of resident CTAs (6 of 8 warps per SM) at most
+    const int grid = grid_for(~0ull, sm_count, std::min<uint32_t>(t.ctas_per_sm ? t.ctas_per_sm * 2u : 6u, 6u));
     if (a.key_slot) scatter_kernel<8, true><<<grid, 256, 0, s>>>(v, a);
     else scatter_kernel<8, false><<<grid, 256, 0, s>>>(v, a);
     count_launch();
     return cudaGetLastError();
+}
+
+namespace {
+template <bool ACC>
+cudaError_t launch_bin_acc(const IndexView& v, const BinArgs& a, int sm_count, cudaStream_t s) {
+    static std::atomic<uint64_t> done{0};  // devices whose attribute is set
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (!(done.load() >> (dev & 63) & 1ull)) {
+        e = cudaFuncSetAttribute(bin_kernel<ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBinWords * 4u));
+        if (e != cudaSuccess) return e;
+        done.fetch_or(1ull << (dev & 63));
+    }
+    bin_kernel<ACC><<<uint32_t(sm_count) * kBinCtasPerSm, kBinThreads, kBinWords * 4u, s>>>(v, a);
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_plain_ids(const IndexView& v, const uint32_t* plain_term, const uint32_t* plain_off, uint32_t* plain,
+                             uint32_t* plain_dir, int sm_count, cudaStream_t s) {
+    if (v.n_plain == 0) return cudaSuccess;
+    plain_ids_kernel<<<sm_count * 8, 256, 0, s>>>(v, plain_off, plain);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    plain_dir_kernel<<<sm_count * 8, 256, 0, s>>>(v, plain_term, plain_off, plain_dir);
+    count_launch(2);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bin(const IndexView& v, const BinArgs& a, int sm_count, cudaStream_t s) {
+    if (a.n_q == 0 || a.n_tiles == 0) return cudaSuccess;
+    const cudaError_t e = a.accumulate ? launch_bin_acc<true>(v, a, sm_count, s) : launch_bin_acc<false>(v, a, sm_count, s);
+    count_launch();
+    return e;
 }
 
 cudaError_t launch_probe(const IndexView& v, const ProbeArgs& a, const abf_tuning& t, int sm_count, cudaStream_t s) {

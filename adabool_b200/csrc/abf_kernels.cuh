@@ -14,6 +14,10 @@
 //   scatter_kernel     list-union, scatter variant: load-balanced warps decode
 //                      the short lists' blocks and OR into the global bitmap
 //                      with lane-combined atomicOr
+//   bin_kernel         list-union, binned variant: the mid-length lists of large
+//                      batches, from plain ids, per 16,384-word tile in shared
+//                      memory
+//   plain_ids / plain_dir_kernel  the plain ids, when an index is uploaded
 //   probe_kernel       bitmap-probe: scans every block of the index, stages
 //                      the probe queries' term-bitmap slices in shared memory
 //                      with bulk async copies (TMA engine), tests each block's
@@ -66,7 +70,8 @@ struct PlanArgs {
     uint32_t fixed_hybrid_min;  // fixed rule otherwise: HYBRID when a list has >= this many
                                 // postings (0: never), else UNION
     uint32_t* heavy_min;      // out: per query
-    uint32_t* term_lpref;     // out: per term slot, exclusive prefix of scattered blocks
+    uint2* term_slot;         // out: per term slot, exclusive prefix (in its query) of scattered blocks
+                              // and the list's first block
     uint64_t* q_light_cnt;    // out: per query scattered blocks
     uint32_t* probe_list;     // out: probe slot -> query
     uint32_t* n_probe;        // in/out: zeroed before launch
@@ -94,6 +99,12 @@ struct PlanArgs {
     uint32_t* q_dmode;        // out: per query, 1 if every list it merges has a dense bitmap,
                               // 2 if it also merges lists without one, 0 for probe / empty
     const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
+    // optional binning (bin_list set): lists with plain ids go to the bin
+    // kernel, in queries where they hold at least bin_min_blocks blocks in all
+    uint32_t* bin_list;       // out: from slot q_off[q] on, their plain list indices
+    uint32_t* q_nbin;         // out: per query, such lists
+    uint32_t* q_bblk;         // out: per query, their blocks
+    uint32_t bin_min_blocks;
     uint32_t no_dense_from;   // queries from this one on scatter their dense-bitmap lists too
                               // (0: none do; only with dense_in_tile)
 };
@@ -105,6 +116,13 @@ struct QueueArgs {
     uint64_t* q_light_pref;   // n_q + 1
     uint32_t n_q;
     const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
+    // optional (q_bblk): the bin kernel's work split, see BinArgs
+    const uint32_t* q_bblk;
+    const uint32_t* q_nbin;
+    uint32_t* parts_pref;     // out: n_q + 1
+    uint32_t* ticket;         // out: zeroed
+    uint32_t n_tiles;
+    uint32_t slots;           // CTAs of the bin kernel that run at a time
 };
 
 // Consecutive keys with the same bitmap index form one run, which the kernels
@@ -188,17 +206,42 @@ struct DenseGroupArgs {
     const uint32_t* out_slot;  // query -> output bitmap index (null: identity)
 };
 
+// bin kernel: tiles of kBinWords words
+constexpr uint32_t kBinWords = (1u << kBinShift) / 32u;
+constexpr uint32_t kBinThreads = 512;
+constexpr uint32_t kBinCtasPerSm = 3;
+struct BinArgs {
+    const uint32_t* bin_list;  // per query: plain list indices, from slot q_off[q] on
+    const uint64_t* q_off;
+    const uint32_t* q_nbin;
+    const uint32_t* parts_pref;  // exclusive prefix (n_q + 1) of the parts that each query's lists are cut into
+    uint32_t* ticket;          // item counter, zero
+    uint32_t n_q;
+    const uint32_t* d_n_q;     // optional device count of queries (at most n_q)
+    uint32_t n_tiles;
+    uint32_t* out;
+    uint64_t out_stride;
+    const uint32_t* out_slot;  // query -> output bitmap index (null: identity)
+    uint64_t n_words;
+    int accumulate;            // 1: bitmaps may be shared, OR with atomics always
+    int vec_ok;                // out 16-byte aligned and out_stride % 4 == 0
+    const uint32_t* sat;       // the dense group kernel's marks (see ScatterArgs)
+    uint32_t sat_stride;
+    uint32_t sat_shift;
+    uint32_t sat_last;
+};
+
 struct ScatterArgs {
     const uint32_t* terms;
     const uint64_t* q_off;
-    const uint32_t* term_lpref;
+    const uint2* term_slot;
     const uint64_t* q_light_pref; // n_q + 1
     uint32_t n_q;
     const uint32_t* out_slot;  // query -> output bitmap index (null: identity)
     const uint32_t* key_slot;  // instead, with n_q 1: term slot -> output bitmap index
     uint32_t* out;
     uint64_t out_stride;
-    uint32_t blocks_per_warp;
+    uint32_t chunk_blocks;     // consecutive blocks a warp takes at a time (at most 32)
     const uint32_t* sat;       // optional: the dense group kernel's saturated-tile bits
     uint32_t sat_stride;       //   (words per query); an OR into a word of such a tile
     uint32_t sat_shift;        //   is skipped; tile = word >> sat_shift
@@ -263,6 +306,10 @@ cudaError_t launch_tile_union(const IndexView& v, const TileArgs& a, const abf_t
                               cudaStream_t s);
 cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_tuning& t, int sm_count,
                            cudaStream_t s);
+// ids and positions of the plain lists (IndexView::plain, plain_dir) from the blocks
+cudaError_t launch_plain_ids(const IndexView& v, const uint32_t* plain_term, const uint32_t* plain_off, uint32_t* plain,
+                             uint32_t* plain_dir, int sm_count, cudaStream_t s);
+cudaError_t launch_bin(const IndexView& v, const BinArgs& a, int sm_count, cudaStream_t s);
 cudaError_t launch_probe(const IndexView& v, const ProbeArgs& a, const abf_tuning& t, int sm_count,
                          cudaStream_t s);
 // planner (abf_planner.cu)

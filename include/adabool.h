@@ -144,7 +144,9 @@ typedef struct abf_tuning {
     uint32_t heavy_min_len;   /* HYBRID: lists with >= this many postings are merged
                                  per tile, shorter lists are scattered */
     uint32_t probe_chunk_blocks; /* blocks per CTA in the bitmap-probe scan */
-    uint32_t scatter_blocks_per_warp; /* consecutive blocks a union warp takes */
+    uint32_t scatter_blocks_per_warp; /* consecutive blocks a union warp takes at a time, in fours
+                                 (8 and more: 32); fewer where there are not enough for
+                                 every warp */
     uint32_t ctas_per_sm;     /* grid = SMs x this, for the persistent kernels */
     uint32_t probe_cap;       /* queries of one batch that may take the probe path (<= 65536) */
     float probe_min_fraction; /* fixed rule (ABF_PATH_AUTO without a planner): probe

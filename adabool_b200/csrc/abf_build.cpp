@@ -294,6 +294,9 @@ void derive_tables(const HostIndex& h, uint32_t dense_div, int n_threads, Derive
         dense_terms.push_back(t);
     }
     out->n_dense = uint32_t(dense_terms.size());
+    out->max_other_len = 0;
+    for (uint32_t t = 0; t < h.n_terms; ++t)
+        if (out->term_dense[t] == kNone) out->max_other_len = std::max(out->max_other_len, h.term_len[t]);
     // plain ids: the longest of the other lists, within the same budget
     out->term_plain.assign(h.n_terms, kNone);
     out->plain_term.clear();

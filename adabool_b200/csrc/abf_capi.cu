@@ -56,10 +56,10 @@ using abf::fail;
 namespace {
 
 // ---- kernel timing (abf_profile_enable / abf_profile_read) ----
-enum Kid { K_PLAN, K_QUEUE, K_TILE, K_SCATTER, K_PROBE, K_COMPACT, K_PLANNER, K_GROUP, K_BIN, K_NKERNELS };
+enum Kid { K_PLAN, K_QUEUE, K_TILE, K_SCATTER, K_PROBE, K_COMPACT, K_PLANNER, K_GROUP, K_BIN, K_STREAM, K_NKERNELS };
 const char* const kKernelNames[K_NKERNELS] = {"plan",  "queue_scan", "tile_union", "scatter_union",
                                               "probe", "compact",    "planner",    "dense_group",
-                                              "bin_union"};
+                                              "bin_union", "dense_stream"};
 
 struct Profiler {
     struct Rec {
@@ -124,7 +124,6 @@ struct abf_workspace {
     uint32_t probe_cap = 0;
     uint64_t probe_stride = 0;
     uint32_t chunks_per_q = 0;
-    uint32_t* heavy = nullptr;
     uint2* slot = nullptr;          // per term (see PlanArgs)
     uint32_t* tile_cls = nullptr;
     uint64_t* lcnt = nullptr;
@@ -140,7 +139,6 @@ struct abf_workspace {
     uint16_t* q_dense16 = nullptr;  // the queries' dense bitmap lists (see PlanArgs)
     uint32_t* q_dstart = nullptr;   // per query
     uint32_t* q_ndense = nullptr;   // per query
-    uint32_t* q_dmode = nullptr;    // per query
     uint32_t* err = nullptr;
     uint32_t* bin_list = nullptr;   // the bin kernel's lists and work split (see PlanArgs, BinArgs)
     uint32_t* q_nbin = nullptr;
@@ -173,16 +171,16 @@ struct abf_worker {
     // planning scratch (see PlanArgs); the dense-bitmap lists and saturation
     // marks cover the first q_cap queries or runs
     uint32_t q_cap = 0;
-    uint32_t* d_heavy = nullptr;
     uint2* d_tslot = nullptr;
     uint32_t* d_tile_cls = nullptr;
     uint64_t* d_lcnt = nullptr;
     uint64_t* d_lpref_q = nullptr;
     uint32_t* d_nprobe = nullptr;
+    uint32_t* d_tile_list = nullptr;
+    uint32_t* d_n_tile_list = nullptr;
     uint16_t* d_dense16 = nullptr;
     uint32_t* d_dstart = nullptr;
     uint32_t* d_ndense = nullptr;
-    uint32_t* d_dmode = nullptr;
     uint32_t* d_sat = nullptr;
     uint32_t sat_stride = 0;
     uint32_t* d_bin_list = nullptr; // the bin kernel's lists and work split
@@ -408,7 +406,6 @@ abf_status need_device(const abf_index* ix) {
 }
 
 void ws_release(abf_workspace* w) {
-    dev_free(w->heavy);
     dev_free(w->slot);
     dev_free(w->tile_cls);
     dev_free(w->lcnt);
@@ -424,7 +421,6 @@ void ws_release(abf_workspace* w) {
     dev_free(w->q_dense16);
     dev_free(w->q_dstart);
     dev_free(w->q_ndense);
-    dev_free(w->q_dmode);
     dev_free(w->err);
     dev_free(w->bin_list);
     dev_free(w->q_nbin);
@@ -448,7 +444,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
     w->sat_stride = sat_words(ix);
     abf_status st;
-    if ((st = dev_alloc(&w->heavy, max_q)) != ABF_OK || (st = dev_alloc(&w->slot, max_terms)) != ABF_OK ||
+    if ((st = dev_alloc(&w->slot, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->tile_cls, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->lcnt, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref_q, uint64_t(max_q) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->probe_list, w->probe_cap)) != ABF_OK || (st = dev_alloc(&w->n_probe, 1)) != ABF_OK ||
@@ -459,7 +455,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
         (st = dev_alloc(&w->auto_paths, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->q_dense16, max_terms + 8ull * max_q + 16)) != ABF_OK ||
         (st = dev_alloc(&w->q_dstart, max_q)) != ABF_OK || (st = dev_alloc(&w->q_ndense, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->q_dmode, max_q)) != ABF_OK || (st = dev_alloc(&w->tile_list, max_q)) != ABF_OK ||
+        (st = dev_alloc(&w->tile_list, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->n_tile_list, 1)) != ABF_OK || (st = dev_alloc(&w->bin_list, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->q_nbin, max_q)) != ABF_OK || (st = dev_alloc(&w->q_bblk, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->parts_pref, uint64_t(max_q) + 1)) != ABF_OK ||
@@ -610,7 +606,6 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.hybrid_min = t.heavy_min_len;
     pa.probe_min_frac = t.probe_min_fraction;
     pa.fixed_hybrid_min = t.fixed_hybrid_min_len;
-    pa.heavy_min = ws->heavy;
     pa.term_slot = ws->slot;
     pa.q_light_cnt = ws->lcnt;
     pa.probe_list = ws->probe_list;
@@ -624,7 +619,6 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.q_dense16 = ws->q_dense16;
     pa.q_dstart = ws->q_dstart;
     pa.q_ndense = ws->q_ndense;
-    pa.q_dmode = ws->q_dmode;
     pa.tile_list = ws->tile_list;
     pa.n_tile_list = ws->n_tile_list;
     // learned planner: the plan kernel runs its feature + MLP code for the
@@ -649,12 +643,16 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     }
     TIMED(K_PLAN, abf::launch_plan(v, pa, s));
     TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
+    // the merge kernel has work only where a query can merge a list that has
+    // no dense bitmap: never on UNION and PROBE
+    const bool may_merge = b->d_paths || b->path == ABF_PATH_TILE ||
+                           ((b->path == ABF_PATH_AUTO || b->path == ABF_PATH_HYBRID) &&
+                            ix->derived.max_other_len >= t.heavy_min_len);
     // the probe queries' term bitmaps are written by their plan CTAs
     const bool maybe_probe = ws->probe_cap > 0 && (b->d_paths || b->path == ABF_PATH_PROBE || b->path == ABF_PATH_AUTO);
     abf::TileArgs ta{};
     ta.tile_cls = ws->tile_cls;
     ta.q_off = b->d_offsets;
-    ta.heavy_min = ws->heavy;
     ta.n_q = b->n_queries;
     const abf_tuning tt = tile_shape(ix, b->n_queries);
     ta.n_tiles = uint32_t((n_words + tt.tile_words - 1) / tt.tile_words);
@@ -663,16 +661,11 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     ta.n_words = n_words;
     ta.accumulate = 0;
     ta.vec_ok = (reinterpret_cast<uintptr_t>(b->d_bitmaps) % 16 == 0) && (b->bitmap_stride_words % 4 == 0);
-    ta.q_dense16 = ws->q_dense16;
-    ta.q_dstart = ws->q_dstart;
-    ta.q_ndense = ws->q_ndense;
-    ta.q_dmode = ws->q_dmode;
     ta.tile_list = ws->tile_list;
     ta.n_tile_list = ws->n_tile_list;
-    ta.skip_dense_only = group ? 1 : 0;
-    // the group kernel marks each (query, tile) it leaves all ones; the
+    // the dense kernels mark each (query, tile) they leave all ones; the
     // scatter then skips ORs into those tiles
-    if (group) CUDA_TRY(cudaMemsetAsync(ws->sat, 0, uint64_t(b->n_queries) * ws->sat_stride * 4u, s));
+    CUDA_TRY(cudaMemsetAsync(ws->sat, 0, uint64_t(b->n_queries) * ws->sat_stride * 4u, s));
     // one launch per window of at most kGroupMaxQueries queries (their
     // per-query state must fit the kernel's shared memory)
     for (uint32_t q0 = 0; group && q0 < b->n_queries; q0 += abf::kGroupMaxQueries) {
@@ -680,7 +673,6 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         ga.q_dense16 = ws->q_dense16;
         ga.q_dstart = ws->q_dstart + q0;
         ga.q_ndense = ws->q_ndense + q0;
-        ga.q_dmode = ws->q_dmode + q0;
         ga.n_q = std::min<uint32_t>(abf::kGroupMaxQueries, b->n_queries - q0);
         ga.n_rows = n_dense + 1;
         ga.stages = stages;
@@ -695,7 +687,21 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         ga.sat_stride = ws->sat_stride;
         TIMED(K_GROUP, abf::launch_dense_group(ix->dense_tmap, gw, ga, ix->sm_count, s));
     }
-    TIMED(K_TILE, abf::launch_tile_union(v, ta, tt, ix->sm_count, s));
+    if (!group) {
+        abf::DenseStreamArgs da{};
+        da.q_dense16 = ws->q_dense16;
+        da.q_dstart = ws->q_dstart;
+        da.q_ndense = ws->q_ndense;
+        da.n_q = b->n_queries;
+        da.out = b->d_bitmaps;
+        da.out_stride = b->bitmap_stride_words;
+        da.n_words = n_words;
+        da.vec_ok = ta.vec_ok;
+        da.sat = ws->sat;
+        da.sat_stride = ws->sat_stride;
+        TIMED(K_STREAM, abf::launch_dense_stream(v, da, ix->sm_count, s));
+    }
+    if (may_merge) TIMED(K_TILE, abf::launch_tile_union(v, ta, tt, ix->sm_count, s));
     abf::ScatterArgs sa{};
     sa.terms = b->d_terms;
     sa.q_off = b->d_offsets;
@@ -705,11 +711,11 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     sa.out = b->d_bitmaps;
     sa.out_stride = b->bitmap_stride_words;
     sa.chunk_blocks = scatter_chunk(t);
-    if (group) {
-        sa.sat = ws->sat;
-        sa.sat_stride = ws->sat_stride;
-        sa.sat_shift = gw == 64u ? 6u : 5u;
-        sa.sat_last = b->n_queries - 1;
+    sa.sat = ws->sat;
+    sa.sat_stride = ws->sat_stride;
+    sa.sat_shift = group && gw == 32u ? 5u : 6u;
+    sa.sat_last = b->n_queries - 1;
+    if (bins) {
         abf::BinArgs ba{};
         ba.bin_list = ws->bin_list;
         ba.q_off = b->d_offsets;
@@ -726,7 +732,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         ba.sat_stride = sa.sat_stride;
         ba.sat_shift = sa.sat_shift;
         ba.sat_last = sa.sat_last;
-        if (bins) TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
+        TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
     }
     TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
     if (maybe_probe) {
@@ -789,18 +795,18 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     w->d_keys = reinterpret_cast<uint32_t*>(w->d_off1 + 2);
     a.used += uint64_t(w->term_cap) * sizeof(uint32_t);
     a.take(w->d_off, n_q + 1);
-    a.take(w->d_heavy, n_q);
     a.take(w->d_tslot, w->term_cap);
     a.take(w->d_tile_cls, w->term_cap);
     a.take(w->d_lcnt, n_q);
     a.take(w->d_lpref_q, n_q + 1);
     a.take(w->d_nprobe, 1);
+    a.take(w->d_n_tile_list, 1);
+    a.take(w->d_tile_list, w->q_cap);
     a.take(w->d_n_q, 1);
     a.take(w->d_err, 1);
     a.take(w->d_dense16, w->term_cap + 8ull * w->q_cap + 16);
     a.take(w->d_dstart, w->q_cap);
     a.take(w->d_ndense, w->q_cap);
-    a.take(w->d_dmode, w->q_cap);
     a.take(w->d_sat, (uint64_t(w->q_cap) + 1) * w->sat_stride);
     a.take(w->d_bin_list, w->term_cap);
     a.take(w->d_nbin, n_q);
@@ -839,37 +845,41 @@ struct WorkerRun {
     const uint32_t* key_slot = nullptr;
     uint32_t* out;
     uint64_t out_stride;
-    bool tiles;        // merge long lists with the tile kernel (one owner per bitmap)
-    GroupShape group;  // else, if on, with the dense group kernel; else scatter every list
+    bool stream;       // dense bitmaps by the stream kernel, other long lists by the merge kernel
+    GroupShape group;  // else, if on, by the dense group kernel; else scatter every list
 };
 
 abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const WorkerRun& r, cudaStream_t s) {
     abf_index* ix = w->ix;
     const abf_tuning& t = ix->tuning;
     const uint64_t n_words = n_words_of(ix->n_ads);
-    const bool group = !r.tiles && r.group.on;
+    const bool group = !r.stream && r.group.on;
     const uint32_t nd_q = std::min<uint32_t>(r.n_q, w->q_cap);  // queries with dense lists and marks
     abf::PlanArgs pa{};
     pa.terms = w->d_keys;
     pa.q_off = r.q_off;
     pa.n_q = r.n_q;
     pa.d_n_q = r.d_n_q;
-    pa.path_uniform = r.tiles ? ABF_PATH_HYBRID : ABF_PATH_UNION;
+    const bool merge = r.stream && ix->derived.max_other_len >= t.heavy_min_len;
+    pa.path_uniform = merge ? ABF_PATH_HYBRID : ABF_PATH_UNION;
     pa.hybrid_min = t.heavy_min_len;
-    pa.heavy_min = w->d_heavy;
     pa.term_slot = w->d_tslot;
     pa.q_light_cnt = w->d_lcnt;
     pa.n_probe = w->d_nprobe;  // not reached: no query takes the probe path
     pa.probe_cap = 0;
     pa.max_terms = w->term_cap;
-    pa.dense_in_tile = r.tiles || group ? 1 : 0;
-    if (r.tiles) pa.tile_cls = w->d_tile_cls;
-    if (group) {
-        pa.no_dense_from = nd_q;
+    pa.dense_in_tile = r.stream || group ? 1 : 0;
+    if (merge) {
+        pa.tile_cls = w->d_tile_cls;
+        pa.tile_list = w->d_tile_list;
+        pa.n_tile_list = w->d_n_tile_list;
+        CUDA_TRY(cudaMemsetAsync(w->d_n_tile_list, 0, sizeof(uint32_t), s));
+    }
+    if (pa.dense_in_tile) {
         pa.q_dense16 = w->d_dense16;
         pa.q_dstart = w->d_dstart;
         pa.q_ndense = w->d_ndense;
-        pa.q_dmode = w->d_dmode;
+        if (group) pa.no_dense_from = nd_q;
         CUDA_TRY(cudaMemsetAsync(w->d_sat, 0, (uint64_t(nd_q) + 1) * w->sat_stride * 4u, s));
     }
     abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, r.n_q, r.d_n_q};
@@ -893,7 +903,6 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         ga.q_dense16 = w->d_dense16;
         ga.q_dstart = w->d_dstart;
         ga.q_ndense = w->d_ndense;
-        ga.q_dmode = w->d_dmode;
         ga.n_q = nd_q;
         ga.d_n_q = r.d_n_q;
         ga.n_rows = v.n_dense + 1;
@@ -911,19 +920,36 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         ga.accumulate = 1;
         TIMED(K_GROUP, abf::launch_dense_group(ix->dense_tmap, r.group.gw, ga, ix->sm_count, s));
     }
-    if (r.tiles) {
+    const bool vec_ok = (reinterpret_cast<uintptr_t>(r.out) % 16 == 0) && (r.out_stride % 4 == 0);
+    if (r.stream) {
+        abf::DenseStreamArgs da{};
+        da.q_dense16 = w->d_dense16;
+        da.q_dstart = w->d_dstart;
+        da.q_ndense = w->d_ndense;
+        da.n_q = r.n_q;
+        da.out = r.out;
+        da.out_stride = r.out_stride;
+        da.n_words = n_words;
+        da.accumulate = 1;
+        da.vec_ok = vec_ok;
+        da.sat = w->d_sat;
+        da.sat_stride = w->sat_stride;
+        TIMED(K_STREAM, abf::launch_dense_stream(v, da, ix->sm_count, s));
+    }
+    if (merge) {
         const abf_tuning tt = tile_shape(ix, r.n_q);
         abf::TileArgs ta{};
         ta.tile_cls = w->d_tile_cls;
+        ta.tile_list = w->d_tile_list;
+        ta.n_tile_list = w->d_n_tile_list;
         ta.q_off = r.q_off;
-        ta.heavy_min = w->d_heavy;
         ta.n_q = r.n_q;
         ta.n_tiles = uint32_t((n_words + tt.tile_words - 1) / tt.tile_words);
         ta.out = r.out;
         ta.out_stride = r.out_stride;
         ta.n_words = n_words;
         ta.accumulate = 1;
-        ta.vec_ok = (reinterpret_cast<uintptr_t>(r.out) % 16 == 0) && (r.out_stride % 4 == 0);
+        ta.vec_ok = vec_ok;
         TIMED(K_TILE, abf::launch_tile_union(v, ta, tt, ix->sm_count, s));
     }
     abf::ScatterArgs sa{};
@@ -938,11 +964,13 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     sa.out = r.out;
     sa.out_stride = r.out_stride;
     sa.chunk_blocks = scatter_chunk(t);
-    if (group) {
+    if (pa.dense_in_tile) {
         sa.sat = w->d_sat;
         sa.sat_stride = w->sat_stride;
-        sa.sat_shift = r.group.gw == 64u ? 6u : 5u;
+        sa.sat_shift = group && r.group.gw == 32u ? 5u : 6u;
         sa.sat_last = nd_q;  // a row of zeros for the runs past it
+    }
+    if (bins) {
         abf::BinArgs ba{};
         ba.bin_list = w->d_bin_list;
         ba.q_off = r.q_off;
@@ -961,7 +989,7 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         ba.sat_stride = sa.sat_stride;
         ba.sat_shift = sa.sat_shift;
         ba.sat_last = nd_q;
-        if (bins) TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
+        TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
     }
     TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
     return ABF_OK;
@@ -982,7 +1010,7 @@ abf_status run_sparse(const abf_worker* w, uint32_t* d_res, bool keyed, const ui
     if (!keyed) {
         r.q_off = w->d_off1;
         r.n_q = 1;
-        r.tiles = true;
+        r.stream = true;
         return run_worker_lists(w, v, r, s);
     }
     // The group kernel reads every dense bitmap once (n_dense * n_ads / 8
@@ -1060,7 +1088,7 @@ abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_w
         la.overflow = w->d_n_q;
         TIMED(K_PROBE, abf::launch_term_lists(la, s));
         if (t.group_min_queries && r.n_q >= t.group_min_queries) r.group = group_shape(ix, v, r.n_q, 64ull * r.n_q, true);
-        r.tiles = !r.group.on;
+        r.stream = !r.group.on;
         ABF_TRY(run_worker_lists(w, v, r, s));
         TIMED(K_PROBE, abf::launch_probe(v, pr, t, ix->sm_count, s));
     }

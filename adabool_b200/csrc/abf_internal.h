@@ -95,6 +95,7 @@ struct DerivedHost {
     std::vector<uint32_t> dir;          // n_dir * dir_n absolute block indices
     uint32_t dir_n = 0;                 // entries per list: ceil(n_ads / 2^kDirShift) + 1
     uint32_t n_dir = 0;
+    uint32_t max_other_len = 0;         // longest list without a dense bitmap
     std::vector<uint32_t> term_plain;   // n_terms: plain list index or kNone
     std::vector<uint32_t> plain_term;   // n_plain: its term
     std::vector<uint32_t> plain_off;    // n_plain + 1: first id in the plain ids, in units of 4

@@ -368,13 +368,13 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
         uint32_t carry = 0, nmerge = 0;
         for (uint64_t c0 = qb; c0 < qe; c0 += 256) {
             const uint64_t i = c0 + tid;
-            uint32_t cnt = 0, cls = kNone, blk = 0, pl;
+            uint32_t cnt = 0, cls = kNone, blk = 0, dense = kNone, pl;
             if (i < qe && !probe) {
                 const uint32_t t = a.terms[i];
                 if (t < ix.n_terms) {
                     const uint32_t d = merge_d ? __ldg(ix.term_dense + t) : kNone;
                     const uint32_t len = __ldg(ix.term_len + t);
-                    if (d != kNone) cls = kDenseFlag | d;
+                    if (d != kNone) dense = d;
                     else if (bin && (pl = __ldg(ix.term_plain + t)) != kNone) {
                         a.bin_list[qb + atomicAdd(&s_nbin, 1u)] = pl;
                     } else if (len >= hm) cls = t;
@@ -389,14 +389,8 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             const uint32_t ex = block_excl_scan<256>(cnt, s_warp, &tot);
             if (i < qe) a.term_slot[i] = make_uint2(carry + ex, blk);
             carry += tot;
-            if (want_d && cls != kNone) {
-                if (cls & kDenseFlag) {
-                    const uint32_t d = cls & ~kDenseFlag;
-                    atomicOr(&s_mask[d >> 5], 1u << (d & 31u));
-                } else {
-                    ++nmerge;
-                }
-            }
+            if (want_d && dense != kNone) atomicOr(&s_mask[dense >> 5], 1u << (dense & 31u));
+            if (cls != kNone) ++nmerge;
         }
         if (want_d) {
             // the query's distinct dense bitmaps in ascending order: each
@@ -422,16 +416,11 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             if (tid == 0) {
                 a.q_dstart[q] = start;
                 a.q_ndense[q] = nd;
-                // 1: every list it merges has a dense bitmap; 2: it also merges
-                // lists without one; 0: probe or empty (no dense merge at all)
-                const uint32_t dmode = (!probe && qe > qb) ? (any_merge ? 2u : 1u) : 0u;
-                a.q_dmode[q] = dmode;
-                if (a.tile_list && dmode != 1u) a.tile_list[atomicAdd(a.n_tile_list, 1u)] = q;
+                if (a.tile_list && any_merge) a.tile_list[atomicAdd(a.n_tile_list, 1u)] = q;
             }
         }
         if (tid == 0) {
             if (a.bin_list) a.q_nbin[q] = bin ? s_nbin : 0u;  // the scans' barriers order the last add
-            a.heavy_min[q] = probe ? kNoHeavy : hm;
             a.q_light_cnt[q] = carry;
             if (a.path_out) a.path_out[q] = uint8_t(path);
         }
@@ -656,57 +645,80 @@ __device__ __forceinline__ uint32_t find_slot(const uint32_t* s_pref, uint32_t f
     return a0;
 }
 
-// One tile of a query whose merged lists all have dense bitmaps: the OR of
-// the nd slices [t*W, t*W + nw) of the bitmaps listed in dl, written to dst.
-template <int W, int NT>
-__device__ __forceinline__ void dense_only_tile(const IndexView& ix, const uint16_t* dl, uint32_t nd, uint32_t t,
-                                                uint32_t* dst, uint32_t nw, bool vec_ok) {
-    constexpr uint32_t KT = 8;
-    const uint32_t tid = threadIdx.x;
-    const uint64_t tw = uint64_t(t) * W;
-    if (vec_ok) {
-        const uint4* base = reinterpret_cast<const uint4*>(ix.dense + tw);
-        const uint64_t st4 = ix.dense_stride / 4;
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
-        const uint32_t n4 = nw / 4u;
-        for (uint32_t j = tid; j < n4; j += NT) {
-            uint4 acc = make_uint4(0u, 0u, 0u, 0u);
-            uint32_t k = 0;
-            for (; k + KT <= nd; k += KT) {
-                uint4 x[KT];
+// list-union, streamed variant of the dense merge, for batches too small for
+// the dense group kernel: a thread ORs one 16-byte column of a query's dense
+// bitmaps, eight rows in flight, and writes it; no shared memory, no barrier.
+// Bound by HBM / L2 (every named row read; column-major item order, so the
+// queries that share a row read it from L2). Rows come longest list first: a
+// warp whose columns are all ones reads no more. Half-warps whose 64 words
+// came out all ones mark them for the scatter kernel.
+// The merge kernel did this with a quarter of its threads at 256-word tiles:
+// seven queries of the serving mix on c1 135 to 186 us, here 74 to 122; one
+// query 17 to 26, here 12 to 18.
+// ACC: OR into the output with atomics (other calls may do so at the same
+// time). V: uint4, or uint32_t where rows are not 16-byte aligned.
+__device__ __forceinline__ void or_in(uint4& a, uint4 b) { a.x |= b.x; a.y |= b.y; a.z |= b.z; a.w |= b.w; }
+__device__ __forceinline__ void or_in(uint32_t& a, uint32_t b) { a |= b; }
+__device__ __forceinline__ bool full_vec(uint4 a) { return (a.x & a.y & a.z & a.w) == ~0u; }
+__device__ __forceinline__ bool full_vec(uint32_t a) { return a == ~0u; }
+
+constexpr uint32_t kStreamThreads = 256;
+template <typename V, bool ACC>
+__global__ void __launch_bounds__(kStreamThreads) dense_stream_kernel(IndexView ix, DenseStreamArgs a) {
+    constexpr uint32_t KT = 8, VW = sizeof(V) / 4u;
+    const uint64_t n_v = (a.n_words + VW - 1u) / VW;  // columns (the last may be partial)
+    const uint32_t n_cb = uint32_t((n_v + kStreamThreads - 1u) / kStreamThreads);
+    const uint64_t items = uint64_t(n_cb) * a.n_q;
+    const uint64_t st = ix.dense_stride / VW;
+    for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint32_t cb = uint32_t(item / a.n_q), q = uint32_t(item - uint64_t(cb) * a.n_q);
+        const uint32_t nd = a.q_ndense[q];
+        if (ACC && nd == 0) continue;
+        const uint64_t j = uint64_t(cb) * kStreamThreads + threadIdx.x;
+        const bool in = j < n_v;
+        V acc = V();
+        const uint4* dl = reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]);  // eight rows each
+        const V* base = reinterpret_cast<const V*>(ix.dense) + (in ? j : 0u);
+        for (uint32_t k = 0; k < nd; k += KT) {
+            const uint4 r = __ldg(dl + k / KT);
+            const uint32_t row[KT] = {r.x & 0xffffu, r.x >> 16, r.y & 0xffffu, r.y >> 16,
+                                      r.z & 0xffffu, r.z >> 16, r.w & 0xffffu, r.w >> 16};
+            V x[KT];
 #pragma unroll
-                for (uint32_t e = 0; e < KT; ++e) x[e] = __ldg(base + uint64_t(__ldg(dl + k + e)) * st4 + j);
+            for (uint32_t e = 0; e < KT; ++e)  // past the list: its first row of the eight again
+                x[e] = __ldg(base + uint64_t(k + e < nd ? row[e] : row[0]) * st);
 #pragma unroll
-                for (uint32_t e = 0; e < KT; ++e) {
-                    acc.x |= x[e].x; acc.y |= x[e].y; acc.z |= x[e].z; acc.w |= x[e].w;
+            for (uint32_t e = 0; e < KT; ++e) or_in(acc, x[e]);
+            if (__all_sync(kFull, full_vec(acc) || !in)) break;
+        }
+        const uint32_t ones = __ballot_sync(kFull, in && full_vec(acc));
+        if (a.sat && VW == 4u && (lane_id() & 15u) == 0 && (ones >> lane_id() & 0xffffu) == 0xffffu) {
+            const uint32_t t = uint32_t(j / 16u);  // tile-of-64
+            atomicOr(a.sat + uint64_t(q) * a.sat_stride + (t >> 5), 1u << (t & 31u));
+        }
+        if (!in) continue;
+        uint32_t* dst = a.out + uint64_t(q) * a.out_stride + j * VW;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(&acc);
+        const uint64_t left = a.n_words - j * VW;
+        if (!ACC && left >= VW) {
+            *reinterpret_cast<V*>(dst) = acc;
+        } else {
+#pragma unroll
+            for (uint32_t e = 0; e < VW; ++e)
+                if (e < left) {
+                    if (!ACC) dst[e] = w[e];
+                    else if (w[e]) atomicOr(dst + e, w[e]);
                 }
-                // lists come longest first: a saturated slice reads no more rows
-                if ((acc.x & acc.y & acc.z & acc.w) == ~0u) break;
-            }
-            if ((acc.x & acc.y & acc.z & acc.w) == ~0u) k = nd;
-            for (; k < nd; ++k) {
-                const uint4 x = __ldg(base + uint64_t(__ldg(dl + k)) * st4 + j);
-                acc.x |= x.x; acc.y |= x.y; acc.z |= x.z; acc.w |= x.w;
-            }
-            d4[j] = acc;
-        }
-        for (uint32_t i = n4 * 4u + tid; i < nw; i += NT) {
-            uint32_t acc = 0;
-            for (uint32_t k = 0; k < nd; ++k) acc |= __ldg(ix.dense + uint64_t(__ldg(dl + k)) * ix.dense_stride + tw + i);
-            dst[i] = acc;
-        }
-    } else {
-        for (uint32_t i = tid; i < nw; i += NT) {
-            uint32_t acc = 0;
-            for (uint32_t k = 0; k < nd; ++k) acc |= __ldg(ix.dense + uint64_t(__ldg(dl + k)) * ix.dense_stride + tw + i);
-            dst[i] = acc;
         }
     }
 }
 
-// ACC: OR into the caller's bitmaps with atomics (other calls may do so at the
-// same time) instead of overwriting them. (A template: as a run-time flag it
-// cost the overwriting kernel 8 registers and a fifth of its occupancy.)
+// list-union, merge variant, for lists without dense bitmaps that HYBRID and
+// TILE queries merge per tile (the dense ones are in the output already): the
+// queries the plan kernel listed, tile by tile; blocks that overlap the tile
+// are decoded a warp each into the tile in shared memory.
+// ACC: start from an empty tile and OR it into the caller's bitmap with
+// atomics (other calls may do so at the same time).
 template <int W, int NW, bool ACC>
 __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileArgs a) {
     constexpr int NT = NW * 32;
@@ -715,117 +727,38 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
     __shared__ __align__(16) uint4 stage[NW][32];
     __shared__ uint32_t s_lo[NT];
     __shared__ uint32_t s_pref[NT + 1];
-    __shared__ uint32_t s_dense[NT];
     __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_ndense;
     const uint32_t tid = threadIdx.x, warp = warp_id();
-    // with the dense group kernel writing the dense-only queries, only the
-    // plan kernel's list of the other queries is visited (often none)
-    const bool listed = a.skip_dense_only && a.tile_list;
-    const uint32_t n_q = listed ? *a.n_tile_list : a.n_q;
+    const uint32_t n_q = *a.n_tile_list;
     const uint64_t items = uint64_t(n_q) * a.n_tiles;
     uint4* tile4 = reinterpret_cast<uint4*>(tile);
     for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
         // tile-major order: the CTAs resident together work on one region of
-        // the ad space for many queries, so the blocks and dense slices of
-        // lists those queries share are read from L2
+        // the ad space for many queries, so the blocks of lists those queries
+        // share are read from L2
         const uint32_t t = uint32_t(item / n_q);
-        const uint32_t qi = uint32_t(item - uint64_t(t) * n_q);
-        const uint32_t q = listed ? a.tile_list[qi] : qi;
+        const uint32_t q = a.tile_list[uint32_t(item - uint64_t(t) * n_q)];
         const uint32_t lo_id = t * SPAN;
         const uint32_t hi_id = (uint64_t(lo_id) + SPAN > ix.n_ads) ? ix.n_ads : lo_id + SPAN;
         const uint32_t dj0 = lo_id >> kDirShift;
         uint32_t dj1 = uint32_t((uint64_t(lo_id) + SPAN) >> kDirShift);
         if (dj1 > ix.dir_n - 1) dj1 = ix.dir_n - 1;
-        const uint32_t hm = a.heavy_min ? a.heavy_min[q] : a.heavy_all;
         const uint64_t qb = a.q_off[q], qe = a.q_off[q + 1];
         uint32_t* dst = a.out + uint64_t(q) * a.out_stride + uint64_t(t) * W;
         const uint64_t left = a.n_words - uint64_t(t) * W;
         const uint32_t nw = left < uint64_t(W) ? uint32_t(left) : uint32_t(W);
-        if (hm == kNoHeavy || qb == qe) {  // nothing to merge: leave or zero the tile
-            if (!ACC)
-                for (uint32_t i = tid; i < nw; i += NT) dst[i] = 0u;
-            continue;
-        }
-        const uint32_t dmode = a.q_dense16 ? a.q_dmode[q] : 0u;
-        if (!ACC && a.q_dense16 && dmode == 1u) {
-            // every merged list has a dense bitmap: the dense group kernel
-            // writes this tile, or each thread ORs its 16-byte slots over the
-            // query's dense slices, KT loads in flight, and stores the
-            // result; no shared tile, no barrier
-            if (!a.skip_dense_only)
-                dense_only_tile<W, NT>(ix, a.q_dense16 + a.q_dstart[q], a.q_ndense[q], t, dst, nw, a.vec_ok != 0);
-            continue;
-        }
-        // with the dense group kernel on, a query that also merges lists
-        // without dense bitmaps already has its dense lists in the output:
-        // the tile starts from it and adds only the others
-        const bool on_group = a.skip_dense_only && dmode == 2u && !ACC;
-        for (uint32_t i = tid; i < uint32_t(W); i += NT) tile[i] = (on_group && i < nw) ? dst[i] : 0u;
-        if (tid == 0) s_ndense = 0;
+        for (uint32_t i = tid; i < uint32_t(W); i += NT) tile[i] = (!ACC && i < nw) ? dst[i] : 0u;
         __syncthreads();
         for (uint64_t c0 = qb; c0 < qe; c0 += NT) {
             const uint64_t i = c0 + tid;
             uint32_t lo = 0, cnt = 0;
             const uint32_t cls = i < qe ? __ldg(a.tile_cls + i) : kNone;
-            if (cls != kNone) {
-                if (cls & kDenseFlag) {
-                    if (!on_group) s_dense[atomicAdd(&s_ndense, 1u)] = cls & ~kDenseFlag;
-                } else {
-                    tile_block_range(ix, cls, lo_id, hi_id, dj0, dj1, lo, cnt);
-                }
-            }
+            if (cls != kNone) tile_block_range(ix, cls, lo_id, hi_id, dj0, dj1, lo, cnt);
             uint32_t total;
             const uint32_t ex = block_excl_scan<NT>(cnt, s_warp, &total);
             s_lo[tid] = lo;
             s_pref[tid] = ex;
             if (tid == NT - 1) s_pref[NT] = ex + cnt;
-            __syncthreads();
-            // dense lists: OR their slice of this tile, 16 bytes per thread and
-            // slot, four lists' loads in flight at once; finished before any
-            // decode warp starts its shared atomics
-            const uint32_t nd = s_ndense;
-            if (nd) {
-                // each thread keeps VG of its 16-byte slots in registers and
-                // issues VG x KT independent loads per step (KT lists at once)
-                constexpr int V = (W / 4 + NT - 1) / NT;
-                constexpr int VG = V < 4 ? V : 4;
-                constexpr int KT = VG >= 4 ? 2 : (VG == 2 ? 4 : 8);
-                const uint4* base = reinterpret_cast<const uint4*>(ix.dense + uint64_t(t) * W);
-                const uint64_t st4 = ix.dense_stride / 4;
-                for (int vg = 0; vg < V; vg += VG) {
-                    uint4 acc[VG];
-#pragma unroll
-                    for (int v = 0; v < VG; ++v) {
-                        const uint32_t j = tid + uint32_t(vg + v) * NT;
-                        acc[v] = j * 4u < nw ? tile4[j] : make_uint4(0u, 0u, 0u, 0u);
-                    }
-                    for (uint32_t k = 0; k < nd; k += KT) {
-                        const uint4* src[KT];
-#pragma unroll
-                        for (int e = 0; e < KT; ++e)
-                            src[e] = base + uint64_t(s_dense[k + e < nd ? k + e : k]) * st4;
-#pragma unroll
-                        for (int v = 0; v < VG; ++v) {
-                            const uint32_t j = tid + uint32_t(vg + v) * NT;
-                            if (j * 4u < nw) {
-                                uint4 x[KT];
-#pragma unroll
-                                for (int e = 0; e < KT; ++e) x[e] = __ldg(src[e] + j);
-#pragma unroll
-                                for (int e = 0; e < KT; ++e) {
-                                    acc[v].x |= x[e].x; acc[v].y |= x[e].y; acc[v].z |= x[e].z; acc[v].w |= x[e].w;
-                                }
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int v = 0; v < VG; ++v) {
-                        const uint32_t j = tid + uint32_t(vg + v) * NT;
-                        if (j * 4u < nw) tile4[j] = acc[v];
-                    }
-                }
-            }
             __syncthreads();
             // decode the blocks: warp w takes a contiguous share of the flat
             // block range, finds its first (slot, block) once and walks on,
@@ -853,7 +786,6 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
                     or_tile(tile, lo_id, SPAN, id, cnt_b);
                 }
             }
-            if (tid == 0) s_ndense = 0;
             __syncthreads();
         }
         if constexpr (ACC) {
@@ -988,7 +920,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     const bool dbl = a.stages == 2u;  // two stages: the next tile's copy overlaps this tile's merge
     uint32_t* stage0 = reinterpret_cast<uint32_t*>(base);
     uint32_t* s_meta = reinterpret_cast<uint32_t*>(base + a.stages * stage_bytes);  // n_q: list offset / 8 << 16 | nd
-    uint16_t* s_qlist = reinterpret_cast<uint16_t*>(s_meta + a.n_q);               // queries with q_dmode != 0
+    uint16_t* s_qlist = reinterpret_cast<uint16_t*>(s_meta + a.n_q);               // queries with work
     uint4* s_lists = reinterpret_cast<uint4*>(base + a.stages * stage_bytes + ((6u * a.n_q + 15u) & ~15u));
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     constexpr uint32_t kNW = kGroupThreads / 32u;
@@ -1019,7 +951,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     for (int r = 0; r < 2; ++r) {
         const uint32_t q = tid * 2u + r;
         // when ORing into the output, queries without dense bitmaps have nothing to add
-        const bool dq = q < n_q && a.q_dmode[q] && !(ACC && a.q_ndense[q] == 0u);
+        const bool dq = q < n_q && !(ACC && a.q_ndense[q] == 0u);
         len[r] = dq ? ((a.q_ndense[q] + 7u) & ~7u) : 0u;
         cnt[r] = dq ? 1u : 0u;
     }
@@ -2114,6 +2046,25 @@ static cudaError_t tile_dispatch_w(const IndexView& v, const TileArgs& a, uint32
         case 4: return a.accumulate ? tile_launch<W, 4, true>(v, a, grid, s) : tile_launch<W, 4, false>(v, a, grid, s);
         default: return a.accumulate ? tile_launch<W, 8, true>(v, a, grid, s) : tile_launch<W, 8, false>(v, a, grid, s);
     }
+}
+
+namespace {
+template <typename V, bool ACC>
+void stream_launch(const IndexView& v, const DenseStreamArgs& a, int sm_count, cudaStream_t s) {
+    const uint64_t cols = (a.n_words + sizeof(V) / 4u - 1u) / (sizeof(V) / 4u);
+    const uint64_t items = (cols + kStreamThreads - 1u) / kStreamThreads * a.n_q;
+    dense_stream_kernel<V, ACC><<<grid_for(items, sm_count, 64), kStreamThreads, 0, s>>>(v, a);
+}
+}  // namespace
+
+cudaError_t launch_dense_stream(const IndexView& v, const DenseStreamArgs& a, int sm_count, cudaStream_t s) {
+    if (a.n_q == 0 || a.n_words == 0) return cudaSuccess;
+    if (a.vec_ok && a.accumulate) stream_launch<uint4, true>(v, a, sm_count, s);
+    else if (a.vec_ok) stream_launch<uint4, false>(v, a, sm_count, s);
+    else if (a.accumulate) stream_launch<uint32_t, true>(v, a, sm_count, s);
+    else stream_launch<uint32_t, false>(v, a, sm_count, s);
+    count_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_tile_union(const IndexView& v, const TileArgs& a, const abf_tuning& t, int sm_count,

@@ -7,10 +7,14 @@
 //                      lists' block counts, claim a bitmap-probe slot and
 //                      write the probe query's term bitmap
 //   queue_scan_kernel  exclusive scan of the per-query scattered block counts
+//   dense_stream_kernel  list-union, dense bitmaps of small batches: every
+//                      thread ORs one 16-byte column of a query's rows
+//   dense_group_kernel list-union, dense bitmaps of large batches: every row
+//                      staged once per tile, ORed per query in shared memory
 //   tile_union_kernel  list-union, merge variant: one CTA owns a tile of one
 //                      query's output bitmap in shared memory, decodes every
-//                      block of the long lists that overlaps the tile, ORs
-//                      with shared-memory atomics and writes the tile once
+//                      block of the long lists without dense bitmaps that
+//                      overlaps the tile and ORs with shared-memory atomics
 //   scatter_kernel     list-union, scatter variant: load-balanced warps decode
 //                      the short lists' blocks and OR into the global bitmap
 //                      with lane-combined atomicOr
@@ -69,7 +73,6 @@ struct PlanArgs {
     float probe_min_frac;     // fixed rule: probe when touched blocks / all blocks > this
     uint32_t fixed_hybrid_min;  // fixed rule otherwise: HYBRID when a list has >= this many
                                 // postings (0: never), else UNION
-    uint32_t* heavy_min;      // out: per query
     uint2* term_slot;         // out: per term slot, exclusive prefix (in its query) of scattered blocks
                               // and the list's first block
     uint64_t* q_light_cnt;    // out: per query scattered blocks
@@ -81,23 +84,20 @@ struct PlanArgs {
     uint8_t* path_out;        // out (optional): resolved path per query
     uint64_t max_terms;       // term slots of the scratch arrays; queries past it get no work
     uint32_t* err;            // device error flag (optional)
-    // optional: queries the merge kernel still has to visit when the dense
-    // group kernel writes the dense-only ones (q_dmode != 1), compacted in
-    // any order; n_tile_list is zeroed before launch
+    // optional: queries that (also) merge lists without dense bitmaps, in any
+    // order; n_tile_list is zeroed before launch
     uint32_t* tile_list;
     uint32_t* n_tile_list;
     int dense_in_tile;        // 1: dense-bitmap lists go to the merge kernel, 0: scattered too
     uint32_t* tile_cls;       // out: per term slot, what the merge kernel does with it
-                              // (kNone: nothing, kDenseFlag | d: dense bitmap d, else the term)
-    // optional per-query dense-bitmap lists (all four set, or q_dense16 null):
+                              // (kNone: nothing, else the term)
+    // optional per-query dense-bitmap lists (all three set, or q_dense16 null):
     // the query's distinct dense bitmap indices in ascending order, as 16-bit
     // values from q_dense16 + q_dstart[q] (16-byte aligned), padded to a
     // multiple of 8 with the index n_dense (an all-zero row for the TMA path)
     uint16_t* q_dense16;      // out: max_terms + 8 * n_q + 16 entries
     uint32_t* q_dstart;       // out: per query
     uint32_t* q_ndense;       // out: per query, distinct dense bitmaps
-    uint32_t* q_dmode;        // out: per query, 1 if every list it merges has a dense bitmap,
-                              // 2 if it also merges lists without one, 0 for probe / empty
     const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
     // optional binning (bin_list set): lists with plain ids go to the bin
     // kernel, in queries where they hold at least bin_min_blocks blocks in all
@@ -108,8 +108,6 @@ struct PlanArgs {
     uint32_t no_dense_from;   // queries from this one on scatter their dense-bitmap lists too
                               // (0: none do; only with dense_in_tile)
 };
-
-constexpr uint32_t kDenseFlag = 0x80000000u;
 
 struct QueueArgs {
     const uint64_t* q_light_cnt;
@@ -152,33 +150,33 @@ struct TermListArgs {
 struct TileArgs {
     const uint32_t* tile_cls;  // per term slot, from the plan kernel
     const uint64_t* q_off;
-    const uint32_t* heavy_min; // per query (null: heavy_all for every query)
-    uint32_t heavy_all;
-    uint32_t n_q;
+    uint32_t n_q;              // most queries that can be listed
     uint32_t n_tiles;
-    uint32_t* out;
+    uint32_t* out;             // holds the queries' dense bitmaps' OR already
     uint64_t out_stride;      // words between query bitmaps
     uint64_t n_words;         // words of one bitmap
-    int accumulate;           // 1: OR into the existing bitmap with atomics, 0: overwrite
+    int accumulate;           // 1: OR into the existing bitmap with atomics, 0: load, add, store
     int vec_ok;               // out 16-byte aligned and out_stride % 4 == 0
-    // optional (plan kernel): queries whose merged lists all have dense
-    // bitmaps (q_dmode 1) take a barrier-free path that streams the OR of
-    // their slices straight to the output, or are skipped when the dense
-    // group kernel covers them; with the group kernel on (skip_dense_only),
-    // q_dmode 2 queries start their tiles from its output and merge only
-    // their lists without dense bitmaps
-    const uint16_t* q_dense16;
-    const uint32_t* q_dstart;
-    const uint32_t* q_ndense;
-    const uint32_t* q_dmode;
-    int skip_dense_only;
-    // with skip_dense_only: the plan kernel's list of the queries that are
-    // not dense-only (the only ones this kernel visits) and its length
-    const uint32_t* tile_list;
+    const uint32_t* tile_list;  // the plan kernel's list of the queries to visit, and its length
     const uint32_t* n_tile_list;
 };
 
-// dense group kernel: one pass per 32- or 64-word tile over all dense-only queries
+// dense stream kernel: the dense bitmaps of every query, for small batches
+struct DenseStreamArgs {
+    const uint16_t* q_dense16;
+    const uint32_t* q_dstart;
+    const uint32_t* q_ndense;
+    uint32_t n_q;
+    uint32_t* out;
+    uint64_t out_stride;
+    uint64_t n_words;
+    int accumulate;            // 1: OR into the output with atomics, 0: overwrite
+    int vec_ok;                // out 16-byte aligned and out_stride % 4 == 0
+    uint32_t* sat;             // optional, zeroed: marks of all-ones tiles-of-64 (only with vec_ok)
+    uint32_t sat_stride;
+};
+
+// dense group kernel: one pass per 32- or 64-word tile over all queries
 constexpr uint32_t kGroupBoxRows = 256;   // dense bitmaps per TMA box
 constexpr uint32_t kGroupMaxBoxes = 3;    // up to 767 dense bitmaps plus the zero row
 constexpr uint32_t kGroupMaxQueries = 2048;
@@ -188,7 +186,6 @@ struct DenseGroupArgs {
     const uint16_t* q_dense16;
     const uint32_t* q_dstart;
     const uint32_t* q_ndense;
-    const uint32_t* q_dmode;
     uint32_t n_q;              // <= kGroupMaxQueries
     uint32_t n_rows;           // n_dense + 1 (the last row reads as zeros)
     uint32_t list_cap;         // list entries (16-bit row word offsets) that fit in shared memory
@@ -299,6 +296,7 @@ cudaError_t encode_dense_tmap(const IndexView& v, uint32_t gw, void* out);
 uint32_t dense_group_list_cap(uint32_t n_rows, uint32_t n_q, uint32_t gw, uint32_t stages);
 cudaError_t launch_dense_group(const void* tmaps, uint32_t gw, const DenseGroupArgs& a, int sm_count,
                                cudaStream_t s);
+cudaError_t launch_dense_stream(const IndexView& v, const DenseStreamArgs& a, int sm_count, cudaStream_t s);
 cudaError_t launch_queue_scan(const QueueArgs& a, cudaStream_t s);
 cudaError_t launch_key_runs(const KeyRunsArgs& a, cudaStream_t s);
 cudaError_t launch_term_lists(const TermListArgs& a, cudaStream_t s);

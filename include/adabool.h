@@ -153,7 +153,7 @@ typedef struct abf_tuning {
                                  when the query's lists hold more than this fraction
                                  of all blocks, else HYBRID or list-union (below) */
     uint32_t group_min_queries; /* batches of at least this many queries merge the
-                                 dense bitmaps of all their dense-only queries in one
+                                 dense bitmaps of all their queries in one
                                  pass per 64- or 32-word tile (each tile's slice of every
                                  dense bitmap staged once in shared memory by TMA, then
                                  ORed per query); needs at most 767 dense bitmaps;

@@ -129,9 +129,14 @@ struct abf_workspace {
     uint64_t* lcnt = nullptr;
     uint64_t* lpref_q = nullptr;
     uint32_t* probe_list = nullptr;
+    // counters of one batch, zeroed together: probe slots taken, merge list
+    // length, plan CTAs finished, compaction ticket (8 bytes); before the
+    // single-query staging, so that abf_query uploads the zeros with its terms
+    uint32_t* ctl = nullptr;
     uint32_t* n_probe = nullptr;
     uint32_t* probe_bm = nullptr;
     uint64_t* scan_status = nullptr;         // compaction look-back words, one per chunk (+1)
+    uint32_t* plan_done = nullptr;
     unsigned long long* ticket = nullptr;   // compaction item counter
     uint64_t* id_off = nullptr;
     uint8_t* path_out = nullptr;
@@ -178,6 +183,7 @@ struct abf_worker {
     uint32_t* d_nprobe = nullptr;
     uint32_t* d_tile_list = nullptr;
     uint32_t* d_n_tile_list = nullptr;
+    uint32_t* d_plan_done = nullptr;
     uint16_t* d_dense16 = nullptr;
     uint32_t* d_dstart = nullptr;
     uint32_t* d_ndense = nullptr;
@@ -285,6 +291,7 @@ void free_device(abf_index* ix) {
     dev_free(d.dense);
     dev_free(d.term_dir);
     dev_free(d.dir);
+    dev_free(d.term_info);
     free_plain(ix);
     dev_free(d.term_cbytes);
     dev_free(d.planner);
@@ -325,6 +332,16 @@ abf_status make_plain(abf_index* ix, const abf::DerivedHost& h) {
     return ABF_OK;
 }
 
+// The plan kernel's table, from the tables above (synchronises).
+abf_status make_term_info(abf_index* ix, const abf::DerivedHost& h) {
+    if (!ix->dev.term_info) ABF_TRY(dev_alloc(&ix->dev.term_info, ix->n_terms, &ix->dev.bytes));
+    abf::IndexView v = abf::view_of(ix);
+    v.n_plain = ix->dev.plain ? h.n_plain() : 0u;
+    CUDA_TRY(abf::launch_term_info(v, ix->dev.term_info, ix->sm_count, nullptr));
+    CUDA_TRY(cudaStreamSynchronize(nullptr));
+    return ABF_OK;
+}
+
 uint64_t plain_bytes(const abf_index* ix) {
     const auto& h = ix->derived;
     if (!ix->dev.plain) return 0;
@@ -354,7 +371,7 @@ abf_status upload(abf_index* ix, int device) {
         (st = upload_vec(&d.term_dir, ix->derived.term_dir, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.dir, ix->derived.dir, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.term_cbytes, cbytes32(ix), &d.bytes)) != ABF_OK ||
-        (st = make_plain(ix, ix->derived)) != ABF_OK) {
+        (st = make_plain(ix, ix->derived)) != ABF_OK || (st = make_term_info(ix, ix->derived)) != ABF_OK) {
         free_device(ix);
         return st;
     }
@@ -411,10 +428,8 @@ void ws_release(abf_workspace* w) {
     dev_free(w->lcnt);
     dev_free(w->lpref_q);
     dev_free(w->probe_list);
-    dev_free(w->n_probe);
     dev_free(w->probe_bm);
     dev_free(w->scan_status);
-    dev_free(w->ticket);
     dev_free(w->id_off);
     dev_free(w->path_out);
     dev_free(w->auto_paths);
@@ -428,11 +443,11 @@ void ws_release(abf_workspace* w) {
     dev_free(w->parts_pref);
     dev_free(w->bin_ticket);
     dev_free(w->tile_list);
-    dev_free(w->n_tile_list);
     dev_free(w->sat);
-    dev_free(w->q_terms);
-    dev_free(w->q_off);
+    dev_free(w->ctl);
 }
+
+constexpr uint32_t kCtlWords = 8;
 
 abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t max_bits, abf_workspace* w) {
     w->ix = ix;
@@ -447,24 +462,30 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     if ((st = dev_alloc(&w->slot, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->tile_cls, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->lcnt, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref_q, uint64_t(max_q) + 1)) != ABF_OK ||
-        (st = dev_alloc(&w->probe_list, w->probe_cap)) != ABF_OK || (st = dev_alloc(&w->n_probe, 1)) != ABF_OK ||
+        (st = dev_alloc(&w->probe_list, w->probe_cap)) != ABF_OK ||
         (st = dev_alloc(&w->probe_bm, uint64_t(w->probe_cap) * w->probe_stride)) != ABF_OK ||
-        (st = dev_alloc(&w->scan_status, chunks + 1)) != ABF_OK || (st = dev_alloc(&w->ticket, 1)) != ABF_OK ||
+        (st = dev_alloc(&w->scan_status, chunks + 1)) != ABF_OK ||
         (st = dev_alloc(&w->id_off, uint64_t(max_q) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->path_out, max_q)) != ABF_OK || (st = dev_alloc(&w->err, 1)) != ABF_OK ||
         (st = dev_alloc(&w->auto_paths, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->q_dense16, max_terms + 8ull * max_q + 16)) != ABF_OK ||
         (st = dev_alloc(&w->q_dstart, max_q)) != ABF_OK || (st = dev_alloc(&w->q_ndense, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->tile_list, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->n_tile_list, 1)) != ABF_OK || (st = dev_alloc(&w->bin_list, max_terms)) != ABF_OK ||
+        (st = dev_alloc(&w->bin_list, max_terms)) != ABF_OK ||
         (st = dev_alloc(&w->q_nbin, max_q)) != ABF_OK || (st = dev_alloc(&w->q_bblk, max_q)) != ABF_OK ||
         (st = dev_alloc(&w->parts_pref, uint64_t(max_q) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->bin_ticket, 1)) != ABF_OK ||
         (st = dev_alloc(&w->sat, uint64_t(max_q) * w->sat_stride)) != ABF_OK ||
-        (st = dev_alloc(&w->q_terms, max_terms)) != ABF_OK || (st = dev_alloc(&w->q_off, 2)) != ABF_OK) {
+        (st = dev_alloc(&w->ctl, kCtlWords + 4 + max_terms)) != ABF_OK) {
         ws_release(w);
         return st;
     }
+    w->n_probe = w->ctl;
+    w->n_tile_list = w->ctl + 1;
+    w->plan_done = w->ctl + 2;
+    w->ticket = reinterpret_cast<unsigned long long*>(w->ctl + 4);
+    w->q_off = reinterpret_cast<uint64_t*>(w->ctl + kCtlWords);
+    w->q_terms = w->ctl + kCtlWords + 4;
     CUDA_TRY(cudaMemset(w->err, 0, sizeof(uint32_t)));
     return ABF_OK;
 }
@@ -500,6 +521,7 @@ abf_status own_ws(abf_index* ix, uint32_t n_q, uint64_t n_terms, uint64_t n_bits
 
 struct RunOpts {
     uint64_t* id_counts = nullptr;
+    bool ctl_zeroed = false;  // the workspace's counters are zero already
 };
 
 abf_status run_compact(abf_index* ix, const abf::CompactArgs& ca, cudaStream_t s) {
@@ -595,8 +617,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     }
     const bool group = gs.on;
     const uint32_t gw = gs.gw, stages = gs.stages;
-    CUDA_TRY(cudaMemsetAsync(ws->n_probe, 0, sizeof(uint32_t), s));
-    CUDA_TRY(cudaMemsetAsync(ws->n_tile_list, 0, sizeof(uint32_t), s));
+    if (!ro.ctl_zeroed) CUDA_TRY(cudaMemsetAsync(ws->ctl, 0, kCtlWords * 4u, s));
     abf::PlanArgs pa{};
     pa.terms = b->d_terms;
     pa.q_off = b->d_offsets;
@@ -641,8 +662,22 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         qa.n_tiles = n_tiles_bin;
         qa.slots = uint32_t(ix->sm_count) * abf::kBinCtasPerSm;
     }
+    // the dense kernels mark each (query, tile) they leave all ones; the
+    // scatter then skips ORs into those tiles
+    pa.sat = ws->sat;
+    pa.sat_stride = ws->sat_stride;
+    const bool ids = b->d_ids || ro.id_counts;
+    if (ids) {
+        pa.status = ws->scan_status;
+        pa.n_chunks = abf::compact_chunks(ix->n_ads);
+        pa.id_counts = ro.id_counts;
+    }
+    if (b->n_queries <= abf::kScanInPlan) {
+        pa.done = ws->plan_done;
+        pa.queue = qa;
+    }
     TIMED(K_PLAN, abf::launch_plan(v, pa, s));
-    TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
+    if (!pa.done) TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
     // the merge kernel has work only where a query can merge a list that has
     // no dense bitmap: never on UNION and PROBE
     const bool may_merge = b->d_paths || b->path == ABF_PATH_TILE ||
@@ -663,9 +698,6 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     ta.vec_ok = (reinterpret_cast<uintptr_t>(b->d_bitmaps) % 16 == 0) && (b->bitmap_stride_words % 4 == 0);
     ta.tile_list = ws->tile_list;
     ta.n_tile_list = ws->n_tile_list;
-    // the dense kernels mark each (query, tile) they leave all ones; the
-    // scatter then skips ORs into those tiles
-    CUDA_TRY(cudaMemsetAsync(ws->sat, 0, uint64_t(b->n_queries) * ws->sat_stride * 4u, s));
     // one launch per window of at most kGroupMaxQueries queries (their
     // per-query state must fit the kernel's shared memory)
     for (uint32_t q0 = 0; group && q0 < b->n_queries; q0 += abf::kGroupMaxQueries) {
@@ -751,8 +783,9 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         pr.spin_limit = ws->spin_limit;
         TIMED(K_PROBE, abf::launch_probe(v, pr, t, ix->sm_count, s));
     }
-    if (b->d_ids || ro.id_counts) {
+    if (ids) {
         abf::CompactArgs ca{};
+        ca.zeroed = 1;
         ca.bm = b->d_bitmaps;
         ca.stride = b->bitmap_stride_words;
         ca.n_q = b->n_queries;
@@ -799,8 +832,9 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     a.take(w->d_tile_cls, w->term_cap);
     a.take(w->d_lcnt, n_q);
     a.take(w->d_lpref_q, n_q + 1);
-    a.take(w->d_nprobe, 1);
-    a.take(w->d_n_tile_list, 1);
+    a.take(w->d_nprobe, 4);
+    w->d_n_tile_list = w->d_nprobe + 1;
+    w->d_plan_done = w->d_nprobe + 2;
     a.take(w->d_tile_list, w->q_cap);
     a.take(w->d_n_q, 1);
     a.take(w->d_err, 1);
@@ -873,15 +907,22 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         pa.tile_cls = w->d_tile_cls;
         pa.tile_list = w->d_tile_list;
         pa.n_tile_list = w->d_n_tile_list;
-        CUDA_TRY(cudaMemsetAsync(w->d_n_tile_list, 0, sizeof(uint32_t), s));
     }
     if (pa.dense_in_tile) {
         pa.q_dense16 = w->d_dense16;
         pa.q_dstart = w->d_dstart;
         pa.q_ndense = w->d_ndense;
         if (group) pa.no_dense_from = nd_q;
-        CUDA_TRY(cudaMemsetAsync(w->d_sat, 0, (uint64_t(nd_q) + 1) * w->sat_stride * 4u, s));
+        // the plan kernel zeroes the marks of the queries there are; with more
+        // runs than rows, all rows (the last one stands for the runs past it)
+        if (r.d_n_q && r.n_q > w->q_cap) {
+            CUDA_TRY(cudaMemsetAsync(w->d_sat, 0, (uint64_t(nd_q) + 1) * w->sat_stride * 4u, s));
+        } else {
+            pa.sat = w->d_sat;
+            pa.sat_stride = w->sat_stride;
+        }
     }
+    CUDA_TRY(cudaMemsetAsync(w->d_nprobe, 0, 4 * sizeof(uint32_t), s));  // and the other counters
     abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, r.n_q, r.d_n_q};
     const bool bins = group && v.n_plain > 0;
     if (bins) {
@@ -896,8 +937,12 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         qa.n_tiles = bin_tiles(n_words);
         qa.slots = uint32_t(ix->sm_count) * abf::kBinCtasPerSm;
     }
+    if (r.n_q <= abf::kScanInPlan) {
+        pa.done = w->d_plan_done;
+        pa.queue = qa;
+    }
     TIMED(K_PLAN, abf::launch_plan(v, pa, s));
-    TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
+    if (!pa.done) TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
     if (group) {
         abf::DenseGroupArgs ga{};
         ga.q_dense16 = w->d_dense16;
@@ -1284,7 +1329,8 @@ abf_status abf_index_set_dense_div(abf_index* ix, uint32_t dense_div) {
         if ((st = upload_vec(&dv.term_dense, d.term_dense, &dv.bytes)) != ABF_OK ||
             (st = upload_vec(&dv.dense, d.dense, &dv.bytes)) != ABF_OK ||
             (st = upload_vec(&dv.term_dir, d.term_dir, &dv.bytes)) != ABF_OK ||
-            (st = upload_vec(&dv.dir, d.dir, &dv.bytes)) != ABF_OK || (st = make_plain(ix, d)) != ABF_OK) {
+            (st = upload_vec(&dv.dir, d.dir, &dv.bytes)) != ABF_OK || (st = make_plain(ix, d)) != ABF_OK ||
+            (st = make_term_info(ix, d)) != ABF_OK) {
             free_device(ix);
             return st;
         }
@@ -1762,7 +1808,7 @@ abf_status abf_query(abf_index* ix, const uint32_t* terms, uint32_t n_terms, abf
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     abf_workspace* ws = nullptr;
     ABF_TRY(own_ws(ix, 1, n_terms, ix->n_ads, &ws));
-    const size_t need = size_t(n_terms) * 4 + 16;
+    const size_t need = (kCtlWords + 4 + size_t(n_terms)) * 4;  // zeroed counters, offsets, terms
     if (!ix->stage_event) {
         cudaEvent_t ev;
         CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -1777,12 +1823,11 @@ abf_status abf_query(abf_index* ix, const uint32_t* terms, uint32_t n_terms, abf
         CUDA_TRY(cudaMallocHost(&ix->h_stage, std::max<size_t>(need, 4096)));
         ix->h_stage_bytes = std::max<size_t>(need, 4096);
     }
-    uint64_t* off = static_cast<uint64_t*>(ix->h_stage);
-    off[0] = 0;
-    off[1] = n_terms;
-    if (n_terms) std::memcpy(off + 2, terms, size_t(n_terms) * 4);
-    CUDA_TRY(cudaMemcpyAsync(ws->q_off, off, 16, cudaMemcpyHostToDevice, s));
-    if (n_terms) CUDA_TRY(cudaMemcpyAsync(ws->q_terms, off + 2, size_t(n_terms) * 4, cudaMemcpyHostToDevice, s));
+    uint32_t* up = static_cast<uint32_t*>(ix->h_stage);
+    std::memset(up, 0, (kCtlWords + 4) * 4);
+    up[kCtlWords + 2] = n_terms;  // {0, n_terms} as 64-bit offsets
+    if (n_terms) std::memcpy(up + kCtlWords + 4, terms, size_t(n_terms) * 4);
+    CUDA_TRY(cudaMemcpyAsync(ws->ctl, up, need, cudaMemcpyHostToDevice, s));
     CUDA_TRY(cudaEventRecord(ev, s));
     abf_batch b{};
     b.d_terms = ws->q_terms;
@@ -1796,6 +1841,7 @@ abf_status abf_query(abf_index* ix, const uint32_t* terms, uint32_t n_terms, abf
     b.d_id_offsets = ws->id_off;
     RunOpts ro;
     ro.id_counts = d_count;
+    ro.ctl_zeroed = true;
     return run_batch(ix, ws, &b, ro, s);
     API_END
 }

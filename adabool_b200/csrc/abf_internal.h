@@ -123,6 +123,7 @@ struct DeviceIndex {
     uint32_t* dense = nullptr;
     uint32_t* term_dir = nullptr;
     uint32_t* dir = nullptr;
+    abf_u4* term_info = nullptr;      // per term {first block, postings, dense bitmap, plain list}
     uint32_t* term_plain = nullptr;
     uint32_t* plain_term = nullptr;
     uint32_t* plain_off = nullptr;
@@ -147,6 +148,7 @@ struct IndexView {
     const uint32_t* term_dir;
     const uint32_t* dir;
     const uint32_t* term_cbytes;
+    const abf_u4* term_info;
     const uint32_t* term_plain;
     const uint32_t* plain;
     const uint32_t* plain_dir;

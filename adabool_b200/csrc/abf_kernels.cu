@@ -32,6 +32,15 @@ constexpr uint64_t kFlagAgg = 1ull << 62;   // the item's own id count is known
 constexpr uint64_t kFlagIncl = 2ull << 62;  // the ids of the item and all before it
 constexpr uint64_t kValMask = (1ull << 62) - 1;
 
+// Programmatic launch order: the kernels of a batch are launched so that each
+// may come up while the one before it finishes. Every kernel begins with this
+// wait, before it reads or writes any global memory, and on every CTA (a
+// kernel is complete only when the ones before it are).
+__device__ __forceinline__ void wait_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 __device__ __forceinline__ uint32_t warp_id() { return threadIdx.x >> 5; }
 
@@ -193,6 +202,30 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
     return wex + x - v;
 }
 
+// exclusive scan of 64-bit values over the CTA (s: NT / 32 entries)
+template <int NT>
+__device__ __forceinline__ uint64_t block_excl_scan64(uint64_t v, unsigned long long* s, uint64_t* total) {
+    const uint32_t lane = lane_id(), warp = warp_id();
+    uint64_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= uint32_t(o)) x += y;
+    }
+    if (lane == 31) s[warp] = x;
+    __syncthreads();
+    uint64_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < uint32_t(NT / 32); ++i) {
+        const uint64_t y = s[i];
+        if (i < warp) before += y;
+        all += y;
+    }
+    __syncthreads();
+    *total = all;
+    return before + x - v;
+}
+
 template <int NT>
 __device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, unsigned long long* s) {
     const uint32_t lane = lane_id(), warp = warp_id();
@@ -270,6 +303,58 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // ---------------------------------------------------------------------------
 // planning
 // ---------------------------------------------------------------------------
+// Exclusive scan of the queries' scattered block counts and, where the bin
+// kernel runs, its work split; by one CTA. The counts may come from other CTAs
+// of the same kernel: they are read past L1.
+template <int NT>
+__device__ __forceinline__ void queue_scan_body(const QueueArgs& a, uint32_t n_q, unsigned long long* s64,
+                                                uint32_t* s32) {
+    const uint32_t tid = threadIdx.x;
+    uint64_t carry = 0, sum = 0;
+    for (uint32_t c0 = 0; c0 < n_q; c0 += NT) {
+        const uint32_t i = c0 + tid;
+        const uint64_t v = i < n_q ? __ldcg(a.q_light_cnt + i) : 0ull;
+        if (a.q_bblk && i < n_q) sum += __ldcg(a.q_bblk + i);
+        uint64_t tot;
+        const uint64_t ex = block_excl_scan64<NT>(v, s64, &tot);
+        if (i < n_q) a.q_light_pref[i] = carry + ex;
+        carry += tot;
+    }
+    if (tid == 0) a.q_light_pref[n_q] = carry;
+    if (!a.q_bblk) return;
+    // The bin kernel's items: every tile x every part of every query. A query
+    // is cut into parts by its lists so that no item has much more than half
+    // an even share of the work (or 128 blocks).
+    sum = block_sum_u64<NT>(sum, s64);
+    const uint64_t lim64 = max(128ull, static_cast<unsigned long long>(sum) / (2ull * a.slots)) * a.n_tiles;
+    const uint32_t lim = lim64 < 0xffffffffull ? uint32_t(lim64) : kFull;
+    uint32_t pc = 0;
+    for (uint32_t c0 = 0; c0 < n_q; c0 += NT) {
+        const uint32_t i = c0 + tid;
+        uint32_t parts = 0;
+        if (i < n_q) {
+            const uint32_t nb = __ldcg(a.q_bblk + i);
+            if (nb) parts = min((nb - 1u) / lim + 1u, __ldcg(a.q_nbin + i));
+        }
+        uint32_t tot;
+        const uint32_t ex = block_excl_scan<NT>(parts, s32, &tot);
+        if (i < n_q) a.parts_pref[i] = pc + ex;
+        pc += tot;
+    }
+    if (tid == 0) {
+        a.parts_pref[n_q] = pc;
+        *a.ticket = 0;
+    }
+}
+
+// A CTA per query at a time, four terms per thread and step (one 16-byte load
+// of a term's table entry each): a step's latency, not its work, is what the
+// longest queries' CTAs wait for, and they end last (one term per step from
+// four tables: 62 us for 512 queries of c1, 245 for 2,048 of c2; here 26 and
+// 119 with the scan). The CTA that finishes
+// last runs the scan over the queries (batches of up to kScanInPlan), which
+// saves that launch.
+constexpr uint32_t kPlanTerms = 4;
 __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) {
     __shared__ uint32_t s_warp[32];
     __shared__ unsigned long long s_red[8];
@@ -278,6 +363,9 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
     __shared__ plan_dev::PlannerSmem s_pl;
     static_assert(plan_dev::kFeatThreads == 256, "the planner code runs with the plan kernel's 256 threads");
     const uint32_t tid = threadIdx.x;
+    constexpr uint32_t kStep = 256u * kPlanTerms;
+    if (a.planner) plan_dev::load_params(a.planner, s_pl);  // not written by any kernel of a batch
+    wait_previous();
     const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
     for (uint32_t q = blockIdx.x; q < n_q; q += gridDim.x) {
         uint64_t qb = a.q_off[q], qe = a.q_off[q + 1];
@@ -286,22 +374,45 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             if (tid == 0 && a.err) atomicOr(a.err, kErrTermRange);
             qe = qb = 0;
         }
+        // what the later kernels find zeroed: the query's saturation marks,
+        // its chunks' look-back words and its id count
+        if (a.sat)
+            for (uint32_t i = tid; i < a.sat_stride; i += 256) a.sat[uint64_t(q) * a.sat_stride + i] = 0u;
+        if (a.status)
+            for (uint32_t i = tid; i < a.n_chunks; i += 256) a.status[uint64_t(q) * a.n_chunks + i] = 0ull;
+        if (a.id_counts && tid == 0) a.id_counts[q] = 0ull;
+        // table entries of this thread's terms of the step at c0: {first
+        // block, postings, dense bitmap, plain list}; no postings: skip it
+        auto load_step = [&](uint64_t c0, uint4 (&e)[kPlanTerms]) {
+            uint32_t t[kPlanTerms];
+#pragma unroll
+            for (uint32_t k = 0; k < kPlanTerms; ++k) {
+                const uint64_t i = c0 + tid * kPlanTerms + k;
+                t[k] = i < qe ? a.terms[i] : kNone;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kPlanTerms; ++k)
+                e[k] = t[k] < ix.n_terms ? __ldg(ix.term_info + t[k]) : make_uint4(0u, 0u, kNone, kNone);
+        };
+        auto blocks_of = [](uint32_t len) { return (len + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS; };
         uint32_t path = a.paths ? a.paths[q] : a.path_uniform;
         if (path == ABF_PATH_AUTO && a.planner) {
             // learned planner: features + MLP of this query, inline
-            path = plan_dev::planner_path(ix, a.planner, a.terms, a.q_off, q,
-                                          plan_dev::FeatCtx{a.hybrid_min, a.n_postings, a.n_q}, s_pl);
+            path = plan_dev::planner_path(ix, a.terms, a.q_off, q, plan_dev::FeatCtx{a.hybrid_min, a.n_postings, a.n_q},
+                                          s_pl);
         } else if (path == ABF_PATH_AUTO) {
             // fixed rule: probe when the query's lists cover more than
             // probe_min_frac of all blocks; else HYBRID when one of its lists
             // has at least fixed_hybrid_min postings; else list-union
             uint64_t nb = 0;
             uint32_t mx = 0;
-            for (uint64_t i = qb + tid; i < qe; i += 256) {
-                const uint32_t t = a.terms[i];
-                if (t < ix.n_terms) {
-                    nb += __ldg(ix.term_blk + t + 1) - __ldg(ix.term_blk + t);
-                    mx = max(mx, __ldg(ix.term_len + t));
+            for (uint64_t c0 = qb; c0 < qe; c0 += kStep) {
+                uint4 e[kPlanTerms];
+                load_step(c0, e);
+#pragma unroll
+                for (uint32_t k = 0; k < kPlanTerms; ++k) {
+                    nb += blocks_of(e[k].y);
+                    mx = max(mx, e[k].y);
                 }
             }
             if (tid == 0) s_max = 0;
@@ -326,7 +437,13 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
                 }
             }
             s_path = path;
+            s_nbin = 0;
         }
+        const bool merge_d = a.dense_in_tile && !(a.no_dense_from && q >= a.no_dense_from);
+        const bool want_d = a.q_dense16 != nullptr && merge_d;
+        const uint32_t mw = (ix.n_dense + 31u) / 32u;
+        if (want_d)
+            for (uint32_t i = tid; i < mw; i += 256) s_mask[i] = 0u;
         __syncthreads();
         path = s_path;
         const bool probe = path == ABF_PATH_PROBE;
@@ -345,52 +462,55 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
         const uint32_t hm = path == ABF_PATH_TILE ? 0u
                             : path == ABF_PATH_HYBRID ? a.hybrid_min
                             : probe ? kNoHeavy : kDenseOnly;
-        const bool merge_d = a.dense_in_tile && !(a.no_dense_from && q >= a.no_dense_from);
-        const bool want_d = a.q_dense16 != nullptr && merge_d;
-        const uint32_t mw = (ix.n_dense + 31u) / 32u;
-        if (want_d) {
-            for (uint32_t i = tid; i < mw; i += 256) s_mask[i] = 0u;
-            __syncthreads();
-        }
         bool bin = false;
         if (a.bin_list) {
             uint64_t nb = 0;
-            for (uint64_t i = qb + tid; i < qe && !probe; i += 256) {
-                const uint32_t t = a.terms[i];
-                if (t < ix.n_terms && __ldg(ix.term_plain + t) != kNone)
-                    nb += (__ldg(ix.term_len + t) + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS;
+            for (uint64_t c0 = qb; c0 < qe && !probe; c0 += kStep) {
+                uint4 e[kPlanTerms];
+                load_step(c0, e);
+#pragma unroll
+                for (uint32_t k = 0; k < kPlanTerms; ++k)
+                    if (e[k].w != kNone) nb += blocks_of(e[k].y);
             }
-            if (tid == 0) s_nbin = 0;
-            nb = block_sum_u64<256>(nb, s_red);  // its barriers also order the s_nbin reset
+            nb = block_sum_u64<256>(nb, s_red);
             bin = nb >= a.bin_min_blocks && nb < 0xffffffffull;
             if (tid == 0) a.q_bblk[q] = bin ? uint32_t(nb) : 0u;
         }
         uint32_t carry = 0, nmerge = 0;
-        for (uint64_t c0 = qb; c0 < qe; c0 += 256) {
-            const uint64_t i = c0 + tid;
-            uint32_t cnt = 0, cls = kNone, blk = 0, dense = kNone, pl;
-            if (i < qe && !probe) {
-                const uint32_t t = a.terms[i];
-                if (t < ix.n_terms) {
-                    const uint32_t d = merge_d ? __ldg(ix.term_dense + t) : kNone;
-                    const uint32_t len = __ldg(ix.term_len + t);
-                    if (d != kNone) dense = d;
-                    else if (bin && (pl = __ldg(ix.term_plain + t)) != kNone) {
-                        a.bin_list[qb + atomicAdd(&s_nbin, 1u)] = pl;
-                    } else if (len >= hm) cls = t;
-                    else {
-                        blk = __ldg(ix.term_blk + t);
-                        cnt = __ldg(ix.term_blk + t + 1) - blk;
+        for (uint64_t c0 = qb; c0 < qe; c0 += kStep) {
+            uint4 e[kPlanTerms];
+            load_step(c0, e);
+            uint32_t cnt[kPlanTerms], sum = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kPlanTerms; ++k) {
+                const uint64_t i = c0 + tid * kPlanTerms + k;
+                const uint32_t d = merge_d ? e[k].z : kNone;
+                uint32_t cls = kNone;
+                cnt[k] = 0;
+                if (i < qe && !probe && e[k].y) {
+                    if (d != kNone) {
+                        if (want_d) atomicOr(&s_mask[d >> 5], 1u << (d & 31u));
+                    } else if (bin && e[k].w != kNone) {
+                        a.bin_list[qb + atomicAdd(&s_nbin, 1u)] = e[k].w;
+                    } else if (e[k].y >= hm) {
+                        cls = a.terms[i];
+                        ++nmerge;
+                    } else {
+                        cnt[k] = blocks_of(e[k].y);
                     }
                 }
+                if (i < qe && a.tile_cls) a.tile_cls[i] = cls;
+                sum += cnt[k];
             }
-            if (i < qe && a.tile_cls) a.tile_cls[i] = cls;
             uint32_t tot;
-            const uint32_t ex = block_excl_scan<256>(cnt, s_warp, &tot);
-            if (i < qe) a.term_slot[i] = make_uint2(carry + ex, blk);
+            uint32_t ex = carry + block_excl_scan<256>(sum, s_warp, &tot);
+#pragma unroll
+            for (uint32_t k = 0; k < kPlanTerms; ++k) {
+                const uint64_t i = c0 + tid * kPlanTerms + k;
+                if (i < qe) a.term_slot[i] = make_uint2(ex, e[k].x);
+                ex += cnt[k];
+            }
             carry += tot;
-            if (want_d && dense != kNone) atomicOr(&s_mask[dense >> 5], 1u << (dense & 31u));
-            if (cls != kNone) ++nmerge;
         }
         if (want_d) {
             // the query's distinct dense bitmaps in ascending order: each
@@ -426,67 +546,22 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
         }
         __syncthreads();
     }
+    if (!a.done) return;
+    __threadfence();  // this CTA's counts before its arrival
+    __syncthreads();
+    if (tid == 0) s_slot = atomicAdd(a.done, 1u);
+    __syncthreads();
+    if (s_slot == gridDim.x - 1u) {
+        __threadfence();
+        queue_scan_body<256>(a.queue, n_q, s_red, s_warp);
+    }
 }
 
 __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
-    __shared__ unsigned long long s_warp[32];
-    __shared__ unsigned long long s_carry;
-    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
-    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
-    if (tid == 0) s_carry = 0;
-    __syncthreads();
-    for (uint32_t c0 = 0; c0 < n_q; c0 += 1024) {
-        const uint32_t i = c0 + tid;
-        const uint64_t v = i < n_q ? a.q_light_cnt[i] : 0ull;
-        uint64_t x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(kFull, x, o);
-            if (lane >= uint32_t(o)) x += y;
-        }
-        if (lane == 31) s_warp[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            uint64_t w = s_warp[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint64_t y = __shfl_up_sync(kFull, w, o);
-                if (lane >= uint32_t(o)) w += y;
-            }
-            s_warp[lane] = w;
-        }
-        __syncthreads();
-        const uint64_t base = s_carry + (warp ? s_warp[warp - 1] : 0ull);
-        if (i < n_q) a.q_light_pref[i] = base + x - v;
-        __syncthreads();
-        if (tid == 0) s_carry += s_warp[31];
-        __syncthreads();
-    }
-    if (tid == 0) a.q_light_pref[n_q] = s_carry;
-    if (!a.q_bblk) return;
-    // The bin kernel's items: every tile x every part of every query. A query
-    // is cut into parts by its lists so that no item has much more than half
-    // an even share of the work (or 128 blocks).
-    uint64_t sum = 0;
-    for (uint32_t i = tid; i < n_q; i += 1024) sum += a.q_bblk[i];
-    sum = block_sum_u64<1024>(sum, s_warp);
-    const uint64_t lim64 = max(128ull, static_cast<unsigned long long>(sum) / (2ull * a.slots)) * a.n_tiles;
-    const uint32_t lim = lim64 < 0xffffffffull ? uint32_t(lim64) : kFull;
-    uint32_t carry = 0;
-    __shared__ uint32_t s_w32[32];
-    for (uint32_t c0 = 0; c0 < n_q; c0 += 1024) {
-        const uint32_t i = c0 + tid;
-        uint32_t parts = 0;
-        if (i < n_q && a.q_bblk[i]) parts = min((a.q_bblk[i] - 1u) / lim + 1u, a.q_nbin[i]);
-        uint32_t tot;
-        const uint32_t ex = block_excl_scan<1024>(parts, s_w32, &tot);
-        if (i < n_q) a.parts_pref[i] = carry + ex;
-        carry += tot;
-    }
-    if (tid == 0) {
-        a.parts_pref[n_q] = carry;
-        *a.ticket = 0;
-    }
+    __shared__ unsigned long long s64[32];
+    __shared__ uint32_t s32[32];
+    wait_previous();
+    queue_scan_body<1024>(a, a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q, s64, s32);
 }
 
 // Runs of consecutive keys with the same bitmap index, in one CTA: a flattened
@@ -497,6 +572,7 @@ __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
 __global__ void __launch_bounds__(1024) key_runs_kernel(KeyRunsArgs a) {
     __shared__ uint32_t s_warp[32];
     const uint32_t tid = threadIdx.x;
+    wait_previous();
     uint32_t carry = 0;
     for (uint64_t c0 = 0; c0 < a.n_keys; c0 += 4096) {
         uint32_t v[4], heads = 0;
@@ -548,6 +624,7 @@ __device__ __forceinline__ uint32_t term_words(const TermListArgs& a) {
 
 __global__ void __launch_bounds__(kTermThreads) term_count_kernel(TermListArgs a) {
     __shared__ unsigned long long s_red[kTermThreads / 32];
+    wait_previous();
     const uint32_t nw = term_words(a);
     for (uint32_t q = blockIdx.x; q < a.n_q; q += gridDim.x) {
         const uint32_t* bm = a.qbm + uint64_t(q) * a.qbm_stride;
@@ -564,6 +641,7 @@ __global__ void __launch_bounds__(kTermThreads) term_list_kernel(TermListArgs a)
     __shared__ uint32_t s_wcnt[kTermThreads / 32];
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     constexpr uint32_t kNW = kTermThreads / 32u;
+    wait_previous();
     const uint32_t nw = term_words(a);
     const uint32_t per = (nw + kNW * 32u - 1u) / (kNW * 32u) * 32u;  // words of a warp's share, whole warps' worth
     for (uint32_t q = blockIdx.x; q < a.n_q; q += gridDim.x) {
@@ -665,6 +743,7 @@ __device__ __forceinline__ bool full_vec(uint32_t a) { return a == ~0u; }
 constexpr uint32_t kStreamThreads = 256;
 template <typename V, bool ACC>
 __global__ void __launch_bounds__(kStreamThreads) dense_stream_kernel(IndexView ix, DenseStreamArgs a) {
+    wait_previous();
     constexpr uint32_t KT = 8, VW = sizeof(V) / 4u;
     const uint64_t n_v = (a.n_words + VW - 1u) / VW;  // columns (the last may be partial)
     const uint32_t n_cb = uint32_t((n_v + kStreamThreads - 1u) / kStreamThreads);
@@ -729,6 +808,7 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
     __shared__ uint32_t s_pref[NT + 1];
     __shared__ uint32_t s_warp[32];
     const uint32_t tid = threadIdx.x, warp = warp_id();
+    wait_previous();
     const uint32_t n_q = *a.n_tile_list;
     const uint64_t items = uint64_t(n_q) * a.n_tiles;
     uint4* tile4 = reinterpret_cast<uint4*>(tile);
@@ -924,6 +1004,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     uint4* s_lists = reinterpret_cast<uint4*>(base + a.stages * stage_bytes + ((6u * a.n_q + 15u) & ~15u));
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     constexpr uint32_t kNW = kGroupThreads / 32u;
+    wait_previous();
     uint32_t t = blockIdx.x;
     if (t >= a.n_tiles) return;
     const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
@@ -1150,6 +1231,7 @@ __global__ void __launch_bounds__(NW * 32, 6) scatter_kernel(IndexView ix, Scatt
     __shared__ uint32_t s_row[NW][32];             // row of saturation marks
     constexpr uint32_t kMixed = 0x80000000u;       // some of the block's tiles are all ones
     const uint32_t warp = warp_id(), lane = lane_id();
+    wait_previous();
     const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
     if (n_q == 0) return;
     const uint64_t total = a.q_light_pref[n_q];
@@ -1306,6 +1388,12 @@ __global__ void __launch_bounds__(256) plain_ids_kernel(IndexView ix, const uint
     }
 }
 
+// the plan kernel's table: per term {first block, postings, dense bitmap, plain list}
+__global__ void __launch_bounds__(256) term_info_kernel(IndexView ix, uint4* info) {
+    for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < ix.n_terms; t += gridDim.x * 256u)
+        info[t] = make_uint4(ix.term_blk[t], ix.term_len[t], ix.term_dense[t], ix.n_plain ? ix.term_plain[t] : kNone);
+}
+
 // position in the plain ids of each list's first id at or past every tile start
 __global__ void __launch_bounds__(256) plain_dir_kernel(IndexView ix, const uint32_t* plain_term,
                                                         const uint32_t* plain_off, uint32_t* dir) {
@@ -1350,6 +1438,7 @@ __global__ void __launch_bounds__(kBinThreads, kBinCtasPerSm) bin_kernel(IndexVi
     __shared__ uint64_t s_qb[2];                  // of the current and the next item: first slot of the query,
     __shared__ uint32_t s_it[2][6];                // {item left?, tile, query, part, parts, lists of the query}
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
+    wait_previous();
     const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
     if (n_q == 0) return;
     const uint32_t n_parts = a.parts_pref[n_q];
@@ -1518,6 +1607,7 @@ __global__ void __launch_bounds__(NW * 32) probe_kernel(IndexView ix, ProbeArgs 
     __shared__ __align__(16) uint4 stage[NW][32];
     __shared__ __align__(8) uint64_t bar;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = warp_id();
+    wait_previous();
     // the device counter also counts queries demoted past the slot capacity
     uint32_t n_probe = a.n_probe_host;
     if (a.d_n_probe && *a.d_n_probe < n_probe) n_probe = *a.d_n_probe;
@@ -1812,6 +1902,7 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compac
     uint32_t* buf = s_buf[warp];
     const uint64_t n_words = (a.n_bits + 31) / 32;
     const uint64_t items = uint64_t(a.n_q) * a.n_chunks;
+    wait_previous();
     if (warp == 0) prepare_chunk(a, items, n_words, buf, &s_item, &s_prefix, s_wtot);
     if (threadIdx.x == 0) {
         s_src = 0;
@@ -1967,6 +2058,7 @@ IndexView view_of(const abf_index* ix) {
     v.dir = ix->dev.dir;
     v.term_cbytes = ix->dev.term_cbytes;
     v.term_plain = ix->dev.term_plain;
+    v.term_info = reinterpret_cast<const uint4*>(ix->dev.term_info);
     v.plain = ix->dev.plain;
     v.plain_dir = ix->dev.plain_dir;
     v.plain_dir_n = ix->derived.plain_dir_n;
@@ -1980,6 +2072,28 @@ IndexView view_of(const abf_index* ix) {
     return v;
 }
 
+namespace {
+// A launch that may come up while the kernel before it on the stream finishes
+// (see wait_previous). With the counters, marks and look-back words zeroed by
+// the plan kernel instead of memsets, the scan in its last CTA and one upload,
+// a single query has 6 nodes on the stream instead of 13: 56 -> 33 us on c0,
+// 95 -> 68 on c1 with the planner.
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+}  // namespace
+
 uint32_t compact_chunks(uint64_t n_bits) {
     const uint64_t n_words = (n_bits + 31) / 32;
     return uint32_t((n_words + kCompactChunkWords - 1) / kCompactChunkWords);
@@ -1989,31 +2103,25 @@ cudaError_t launch_plan(const IndexView& v, const PlanArgs& a, cudaStream_t s) {
     if (a.n_q == 0) return cudaSuccess;
     // with a device count the bound may be far above it: a few waves of CTAs
     const uint32_t most = a.d_n_q ? 148u * 16u : 65535u * 16u;
-    plan_kernel<<<a.n_q < most ? a.n_q : most, 256, 0, s>>>(v, a);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(plan_kernel, a.n_q < most ? a.n_q : most, 256, 0, s, v, a);
 }
 
 cudaError_t launch_queue_scan(const QueueArgs& a, cudaStream_t s) {
-    queue_scan_kernel<<<1, 1024, 0, s>>>(a);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(queue_scan_kernel, 1, 1024, 0, s, a);
 }
 
 cudaError_t launch_key_runs(const KeyRunsArgs& a, cudaStream_t s) {
-    key_runs_kernel<<<1, 1024, 0, s>>>(a);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(key_runs_kernel, 1, 1024, 0, s, a);
 }
 
 cudaError_t launch_term_lists(const TermListArgs& a, cudaStream_t s) {
     if (a.n_q == 0) return cudaSuccess;
-    term_count_kernel<<<a.n_q, kTermThreads, 0, s>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    term_list_kernel<<<a.n_q, kTermThreads, 0, s>>>(a);
     count_launch(2);
-    return cudaGetLastError();
+    const cudaError_t e = launch_after(term_count_kernel, a.n_q, kTermThreads, 0, s, a);
+    return e != cudaSuccess ? e : launch_after(term_list_kernel, a.n_q, kTermThreads, 0, s, a);
 }
 
 template <int W, int NW, bool ACC>
@@ -2034,8 +2142,7 @@ static cudaError_t tile_launch(const IndexView& v, const TileArgs& a, int grid, 
             done.fetch_or(bit);
         }
     }
-    tile_union_kernel<W, NW, ACC><<<grid, NW * 32, smem, s>>>(v, a);
-    return cudaGetLastError();
+    return launch_after(tile_union_kernel<W, NW, ACC>, uint32_t(grid), NW * 32, smem, s, v, a);
 }
 
 template <int W>
@@ -2050,21 +2157,19 @@ static cudaError_t tile_dispatch_w(const IndexView& v, const TileArgs& a, uint32
 
 namespace {
 template <typename V, bool ACC>
-void stream_launch(const IndexView& v, const DenseStreamArgs& a, int sm_count, cudaStream_t s) {
+cudaError_t stream_launch(const IndexView& v, const DenseStreamArgs& a, int sm_count, cudaStream_t s) {
     const uint64_t cols = (a.n_words + sizeof(V) / 4u - 1u) / (sizeof(V) / 4u);
     const uint64_t items = (cols + kStreamThreads - 1u) / kStreamThreads * a.n_q;
-    dense_stream_kernel<V, ACC><<<grid_for(items, sm_count, 64), kStreamThreads, 0, s>>>(v, a);
+    return launch_after(dense_stream_kernel<V, ACC>, uint32_t(grid_for(items, sm_count, 64)), kStreamThreads, 0, s, v, a);
 }
 }  // namespace
 
 cudaError_t launch_dense_stream(const IndexView& v, const DenseStreamArgs& a, int sm_count, cudaStream_t s) {
     if (a.n_q == 0 || a.n_words == 0) return cudaSuccess;
-    if (a.vec_ok && a.accumulate) stream_launch<uint4, true>(v, a, sm_count, s);
-    else if (a.vec_ok) stream_launch<uint4, false>(v, a, sm_count, s);
-    else if (a.accumulate) stream_launch<uint32_t, true>(v, a, sm_count, s);
-    else stream_launch<uint32_t, false>(v, a, sm_count, s);
     count_launch();
-    return cudaGetLastError();
+    if (a.vec_ok)
+        return a.accumulate ? stream_launch<uint4, true>(v, a, sm_count, s) : stream_launch<uint4, false>(v, a, sm_count, s);
+    return a.accumulate ? stream_launch<uint32_t, true>(v, a, sm_count, s) : stream_launch<uint32_t, false>(v, a, sm_count, s);
 }
 
 cudaError_t launch_tile_union(const IndexView& v, const TileArgs& a, const abf_tuning& t, int sm_count,
@@ -2149,8 +2254,7 @@ cudaError_t launch_group_w(const CUtensorMap (&m)[2], const DenseGroupArgs& a, i
         done.fetch_or(1ull << dev);
     }
     const uint32_t grid = a.n_tiles < uint32_t(sm_count) ? a.n_tiles : uint32_t(sm_count);
-    dense_group_kernel<GW, ACC><<<grid, kGroupThreads, kGroupSmemBytes, s>>>(m[0], m[1], a);
-    return cudaGetLastError();
+    return launch_after(dense_group_kernel<GW, ACC>, grid, kGroupThreads, kGroupSmemBytes, s, m[0], m[1], a);
 }
 }  // namespace
 
@@ -2178,10 +2282,8 @@ cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_t
     if (a.n_q == 0) return cudaSuccess;
     // one wave of resident CTAs (6 of 8 warps per SM) at most
     const int grid = grid_for(~0ull, sm_count, std::min<uint32_t>(t.ctas_per_sm ? t.ctas_per_sm * 2u : 6u, 6u));
-    if (a.key_slot) scatter_kernel<8, true><<<grid, 256, 0, s>>>(v, a);
-    else scatter_kernel<8, false><<<grid, 256, 0, s>>>(v, a);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(a.key_slot ? scatter_kernel<8, true> : scatter_kernel<8, false>, uint32_t(grid), 256, 0, s, v, a);
 }
 
 namespace {
@@ -2196,10 +2298,15 @@ cudaError_t launch_bin_acc(const IndexView& v, const BinArgs& a, int sm_count, c
         if (e != cudaSuccess) return e;
         done.fetch_or(1ull << (dev & 63));
     }
-    bin_kernel<ACC><<<uint32_t(sm_count) * kBinCtasPerSm, kBinThreads, kBinWords * 4u, s>>>(v, a);
-    return cudaGetLastError();
+    return launch_after(bin_kernel<ACC>, uint32_t(sm_count) * kBinCtasPerSm, kBinThreads, kBinWords * 4u, s, v, a);
 }
 }  // namespace
+
+cudaError_t launch_term_info(const IndexView& v, uint4* info, int sm_count, cudaStream_t s) {
+    term_info_kernel<<<sm_count * 8, 256, 0, s>>>(v, info);
+    count_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t launch_plain_ids(const IndexView& v, const uint32_t* plain_term, const uint32_t* plain_off, uint32_t* plain,
                              uint32_t* plain_dir, int sm_count, cudaStream_t s) {
@@ -2223,23 +2330,23 @@ cudaError_t launch_probe(const IndexView& v, const ProbeArgs& a, const abf_tunin
     if (v.n_blocks == 0) return cudaSuccess;
     const uint64_t n_chunks = (v.n_blocks + a.chunk_blocks - 1) / a.chunk_blocks;
     const int grid = grid_for(n_chunks, sm_count, t.ctas_per_sm ? t.ctas_per_sm : 4u);
-    probe_kernel<8><<<grid, 256, 0, s>>>(v, a);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(probe_kernel<8>, uint32_t(grid), 256, 0, s, v, a);
 }
 
 cudaError_t launch_compact(const CompactArgs& a, int sm_count, uint32_t ctas_per_sm, cudaStream_t s) {
     const uint64_t items = uint64_t(a.n_q) * a.n_chunks;
     if (items == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(a.status, 0, items * sizeof(uint64_t), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.ticket, 0, sizeof(unsigned long long), s);
-    if (e == cudaSuccess && a.id_counts) e = cudaMemsetAsync(a.id_counts, 0, uint64_t(a.n_q) * sizeof(uint64_t), s);
-    if (e != cudaSuccess) return e;
+    if (!a.zeroed) {
+        cudaError_t e = cudaMemsetAsync(a.status, 0, items * sizeof(uint64_t), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a.ticket, 0, sizeof(unsigned long long), s);
+        if (e == cudaSuccess && a.id_counts) e = cudaMemsetAsync(a.id_counts, 0, uint64_t(a.n_q) * sizeof(uint64_t), s);
+        if (e != cudaSuccess) return e;
+    }
     // ctas_per_sm counts CTAs of 8 warps: the same resident warps whatever the CTA size
     const uint32_t per_sm = (ctas_per_sm ? ctas_per_sm : 6u) * 8u / kCompactWarps;
-    compact_kernel<<<grid_for(items, sm_count, per_sm), kCompactWarps * 32, 0, s>>>(a);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(compact_kernel, uint32_t(grid_for(items, sm_count, per_sm)), kCompactWarps * 32, 0, s, a);
 }
 
 cudaError_t launch_wait_selftest(uint64_t* status2, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {

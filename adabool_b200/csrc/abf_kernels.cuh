@@ -60,6 +60,24 @@ constexpr uint32_t kErrTermRange = 4u;
 // hardware-defined interval), so the default allows well over a second.
 constexpr uint32_t kDefaultSpinLimit = 1u << 22;
 
+struct QueueArgs {
+    const uint64_t* q_light_cnt;
+    uint64_t* q_light_pref;   // n_q + 1
+    uint32_t n_q;
+    const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
+    // optional (q_bblk): the bin kernel's work split, see BinArgs
+    const uint32_t* q_bblk;
+    const uint32_t* q_nbin;
+    uint32_t* parts_pref;     // out: n_q + 1
+    uint32_t* ticket;         // out: zeroed
+    uint32_t n_tiles;
+    uint32_t slots;           // CTAs of the bin kernel that run at a time
+};
+
+// queries whose scan the plan kernel's last CTA runs: in steps of 256, a step
+// costs it ~0.6 us, a launch of the scan kernel ~3 us
+constexpr uint32_t kScanInPlan = 2048;
+
 struct PlanArgs {
     const uint32_t* terms;
     const uint64_t* q_off;
@@ -105,22 +123,17 @@ struct PlanArgs {
     uint32_t* q_nbin;         // out: per query, such lists
     uint32_t* q_bblk;         // out: per query, their blocks
     uint32_t bin_min_blocks;
+    // optional: what later kernels of the batch find zeroed, per query
+    uint32_t* sat;            // sat_stride words of saturation marks
+    uint32_t sat_stride;
+    uint64_t* status;         // n_chunks compaction look-back words
+    uint32_t n_chunks;
+    uint64_t* id_counts;
+    // optional: the CTA that finishes last runs the scan over the queries
+    uint32_t* done;           // CTAs finished, zeroed before launch
+    QueueArgs queue;
     uint32_t no_dense_from;   // queries from this one on scatter their dense-bitmap lists too
                               // (0: none do; only with dense_in_tile)
-};
-
-struct QueueArgs {
-    const uint64_t* q_light_cnt;
-    uint64_t* q_light_pref;   // n_q + 1
-    uint32_t n_q;
-    const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
-    // optional (q_bblk): the bin kernel's work split, see BinArgs
-    const uint32_t* q_bblk;
-    const uint32_t* q_nbin;
-    uint32_t* parts_pref;     // out: n_q + 1
-    uint32_t* ticket;         // out: zeroed
-    uint32_t n_tiles;
-    uint32_t slots;           // CTAs of the bin kernel that run at a time
 };
 
 // Consecutive keys with the same bitmap index form one run, which the kernels
@@ -280,6 +293,7 @@ struct CompactArgs {
     uint64_t* id_counts;       // optional n_q, accumulated (zeroed before launch)
     uint32_t* err;
     uint32_t spin_limit;       // polls of a look-back wait before it gives up
+    int zeroed;                // status, ticket and id_counts are zero already
 };
 
 IndexView view_of(const abf_index* ix);
@@ -304,6 +318,7 @@ cudaError_t launch_tile_union(const IndexView& v, const TileArgs& a, const abf_t
                               cudaStream_t s);
 cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_tuning& t, int sm_count,
                            cudaStream_t s);
+cudaError_t launch_term_info(const IndexView& v, uint4* info, int sm_count, cudaStream_t s);
 // ids and positions of the plain lists (IndexView::plain, plain_dir) from the blocks
 cudaError_t launch_plain_ids(const IndexView& v, const uint32_t* plain_term, const uint32_t* plain_off, uint32_t* plain,
                              uint32_t* plain_dir, int sm_count, cudaStream_t s);

@@ -58,8 +58,8 @@ __device__ void query_features(const IndexView& ix, const uint32_t* terms, const
     double S = 0, Q = 0, Cb = 0, Lg = 0, Sd = 0, Bnd = 0;
     const double inv_ads = 1.0 / double(ix.n_ads);
     for (uint64_t i0 = qb + threadIdx.x; i0 < qe; i0 += uint64_t(kFeatThreads) * kFeatUnroll) {
-        uint32_t t[kFeatUnroll], len[kFeatUnroll], dn[kFeatUnroll], cb[kFeatUnroll], b0[kFeatUnroll],
-            b1[kFeatUnroll];
+        uint32_t t[kFeatUnroll], cb[kFeatUnroll];
+        uint4 e[kFeatUnroll];  // {first block, postings, dense bitmap, plain list}
 #pragma unroll
         for (int u = 0; u < kFeatUnroll; ++u) {
             const uint64_t i = i0 + uint64_t(u) * kFeatThreads;
@@ -68,27 +68,25 @@ __device__ void query_features(const IndexView& ix, const uint32_t* terms, const
 #pragma unroll
         for (int u = 0; u < kFeatUnroll; ++u) {
             const bool ok = t[u] < ix.n_terms;
-            len[u] = ok ? __ldg(ix.term_len + t[u]) : 0u;
-            dn[u] = ok ? __ldg(ix.term_dense + t[u]) : kNone;
+            e[u] = ok ? __ldg(ix.term_info + t[u]) : make_uint4(0u, 0u, kNone, kNone);
             cb[u] = ok ? __ldg(ix.term_cbytes + t[u]) : 0u;
-            b0[u] = ok ? __ldg(ix.term_blk + t[u]) : 0u;
-            b1[u] = ok ? __ldg(ix.term_blk + t[u] + 1) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < kFeatUnroll; ++u) {
             if (t[u] >= ix.n_terms) continue;
+            const uint32_t len = e[u].y;
             ++n;
-            mx = max(mx, len[u]);
-            S += len[u];
-            Q += double(len[u]) * len[u];
+            mx = max(mx, len);
+            S += len;
+            Q += double(len) * len;
             Cb += cb[u];
-            Lg += log1p(-fmin(double(len[u]) * inv_ads, 0.999999));
-            if (dn[u] != kNone) {
+            Lg += log1p(-fmin(double(len) * inv_ads, 0.999999));
+            if (e[u].z != kNone) {
                 ++nd;
-                Sd += len[u];
+                Sd += len;
             } else {
-                Bnd += b1[u] - b0[u];
-                if (len[u] < c.hybrid_min) ++nl;
+                Bnd += (len + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS;
+                if (len < c.hybrid_min) ++nl;
             }
         }
     }
@@ -174,24 +172,78 @@ __device__ __forceinline__ void mlp_forward_cta(const float* __restrict__ p, con
     __syncthreads();
 }
 
-// The state the planner keeps in shared memory for one query.
+// The state the planner keeps in shared memory: the parameters, copied in once
+// per CTA, and one query's values.
+constexpr int kParamVecs = (kNParams + 3) / 4;
 struct PlannerSmem {
+    float4 p4[kParamVecs];
     float f[F], xs[F], h1[H], h2[H], y[O];
+    __device__ const float* p() const { return reinterpret_cast<const float*>(p4); }
 };
 
-// features -> standardise -> MLP -> cheapest path (an abf_path) of query q,
-// by the whole CTA (kFeatThreads threads); sm.f holds the features and sm.y
-// the predictions afterwards.
-__device__ __forceinline__ uint32_t planner_path(const IndexView& ix, const float* __restrict__ p,
-                                                 const uint32_t* terms, const uint64_t* q_off, uint32_t q,
-                                                 const FeatCtx& c, PlannerSmem& sm) {
-    query_features(ix, terms, q_off, q, c, sm.f);
-    if (threadIdx.x < F) {
-        const float sd = __ldg(p + kSd + threadIdx.x);
-        sm.xs[threadIdx.x] = (sm.f[threadIdx.x] - __ldg(p + kMu + threadIdx.x)) / (sd > 0.0f ? sd : 1.0f);
+// Starts the copy of the parameters (16-byte aligned); planner_path waits for it.
+__device__ __forceinline__ void load_params(const float* __restrict__ p, PlannerSmem& sm) {
+    for (int i = threadIdx.x; i < kNParams / 4; i += kFeatThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(sm.p4 + i))),
+                     "l"(reinterpret_cast<const float4*>(p) + i)
+                     : "memory");
+    for (int i = kNParams / 4 * 4 + threadIdx.x; i < kNParams; i += kFeatThreads)
+        reinterpret_cast<float*>(sm.p4)[i] = __ldg(p + i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// MLP forward on standardised x by the whole CTA: four threads per hidden unit
+// (a quarter of its inputs each, in 16-byte steps whose order turns with the
+// unit, so that a warp's eight units read all banks), a warp per output.
+__device__ __forceinline__ void mlp_forward_smem(PlannerSmem& sm) {
+    const int j = threadIdx.x >> 2, r = threadIdx.x & 3, w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    static_assert(kFeatThreads == 4 * H && F == 16 && H == 64, "four threads per unit");
+    const float* p = sm.p();
+    {
+        const float4 v = *reinterpret_cast<const float4*>(p + kW1 + j * F + 4 * r);
+        float a = fmaf(v.w, sm.xs[4 * r + 3], fmaf(v.z, sm.xs[4 * r + 2], fmaf(v.y, sm.xs[4 * r + 1], v.x * sm.xs[4 * r])));
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        if (r == 0) sm.h1[j] = fmaxf(a + p[kB1 + j], 0.0f);
     }
     __syncthreads();
-    mlp_forward_cta(p, sm.xs, sm.h1, sm.h2, sm.y);
+    {
+        float a = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = 16 * r + 4 * ((i + j) & 3);
+            const float4 v = *reinterpret_cast<const float4*>(p + kW2 + j * H + k);
+            a = fmaf(v.w, sm.h1[k + 3], fmaf(v.z, sm.h1[k + 2], fmaf(v.y, sm.h1[k + 1], fmaf(v.x, sm.h1[k], a))));
+        }
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        if (r == 0) sm.h2[j] = fmaxf(a + p[kB2 + j], 0.0f);
+    }
+    __syncthreads();
+    if (w < O) {
+        const float* q = p + kW3 + w * H;
+        float a = fmaf(q[l + 32], sm.h2[l + 32], q[l] * sm.h2[l]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (l == 0) sm.y[w] = a + p[kB3 + w];
+    }
+    __syncthreads();
+}
+
+// features -> standardise -> MLP -> cheapest path (an abf_path) of query q,
+// by the whole CTA (kFeatThreads threads), after load_params; sm.f holds the
+// features and sm.y the predictions afterwards.
+__device__ __forceinline__ uint32_t planner_path(const IndexView& ix, const uint32_t* terms, const uint64_t* q_off,
+                                                 uint32_t q, const FeatCtx& c, PlannerSmem& sm) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    query_features(ix, terms, q_off, q, c, sm.f);  // ends with a barrier: every thread's copies are there
+    if (threadIdx.x < F) {
+        const float sd = sm.p()[kSd + threadIdx.x];
+        sm.xs[threadIdx.x] = (sm.f[threadIdx.x] - sm.p()[kMu + threadIdx.x]) / (sd > 0.0f ? sd : 1.0f);
+    }
+    __syncthreads();
+    mlp_forward_smem(sm);
     int best = 0;
     for (int o = 1; o < O; ++o)
         if (sm.y[o] < sm.y[best]) best = o;

@@ -464,7 +464,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
         (st = dev_alloc(&w->lcnt, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref_q, uint64_t(max_q) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->probe_list, w->probe_cap)) != ABF_OK ||
         (st = dev_alloc(&w->probe_bm, uint64_t(w->probe_cap) * w->probe_stride)) != ABF_OK ||
-        (st = dev_alloc(&w->scan_status, chunks + 1)) != ABF_OK ||
+        (st = dev_alloc(&w->scan_status, std::max<uint64_t>(chunks, abf::kCompactFewStatus) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->id_off, uint64_t(max_q) + 1)) != ABF_OK ||
         (st = dev_alloc(&w->path_out, max_q)) != ABF_OK || (st = dev_alloc(&w->err, 1)) != ABF_OK ||
         (st = dev_alloc(&w->auto_paths, max_q)) != ABF_OK ||
@@ -669,7 +669,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     const bool ids = b->d_ids || ro.id_counts;
     if (ids) {
         pa.status = ws->scan_status;
-        pa.n_chunks = abf::compact_chunks(ix->n_ads);
+        pa.n_chunks = abf::compact_chunks(ix->n_ads, abf::compact_units(b->n_queries, ix->n_ads));
         pa.id_counts = ro.id_counts;
     }
     if (b->n_queries <= abf::kScanInPlan) {
@@ -790,7 +790,8 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         ca.stride = b->bitmap_stride_words;
         ca.n_q = b->n_queries;
         ca.n_bits = ix->n_ads;
-        ca.n_chunks = abf::compact_chunks(ix->n_ads);
+        ca.units = abf::compact_units(ca.n_q, ca.n_bits);
+        ca.n_chunks = abf::compact_chunks(ca.n_bits, ca.units);
         ca.status = ws->scan_status;
         ca.ticket = ws->ticket;
         ca.ids = b->d_ids;
@@ -1557,7 +1558,8 @@ abf_status abf_collect_ids(abf_index* ix, const uint32_t* d_bitmap, uint64_t n_b
     ca.stride = n_words_of(n_bits);
     ca.n_q = 1;
     ca.n_bits = n_bits;
-    ca.n_chunks = abf::compact_chunks(n_bits);
+    ca.units = abf::compact_units(1, n_bits);
+    ca.n_chunks = abf::compact_chunks(n_bits, ca.units);
     ca.status = ws->scan_status;
     ca.ticket = ws->ticket;
     ca.ids = d_ids;
@@ -1588,7 +1590,8 @@ abf_status abf_batch_collect_ids(abf_index* ix, abf_workspace* ws, const uint32_
     ca.stride = stride_words;
     ca.n_q = n_bitmaps;
     ca.n_bits = ix->n_ads;
-    ca.n_chunks = abf::compact_chunks(ix->n_ads);
+    ca.units = abf::compact_units(ca.n_q, ca.n_bits);
+    ca.n_chunks = abf::compact_chunks(ca.n_bits, ca.units);
     ca.status = ws->scan_status;
     ca.ticket = ws->ticket;
     ca.ids = d_ids;

@@ -1774,9 +1774,11 @@ __device__ bool lookback_prefix(uint64_t* status, uint64_t item, uint32_t agg, u
 // look-back before the CTA starts it, and then every warp expands its units
 // on its own into ascending ids (three expansions by the unit's id count,
 // below). The bitmap is read once: there is no separate counting pass.
-constexpr uint32_t kUnits = kCompactChunkWords / 32;
-constexpr uint32_t kWarpUnits = kUnits / kCompactWarps;
-static_assert(kWarpUnits == 8, "each warp covers 8 units of its CTA's chunk");
+//
+// U: units per warp. 8 where there are chunks for half the CTA slots of a full
+// GPU; else 2 or 1, so that a single bitmap is spread over more SMs: one query
+// on c0 (32 chunks of 8 units per warp, 256 of one) 9.8 -> 5.7 us, on c1 (512,
+// 2,048 of two) 18 -> 16.
 
 // bulk copy shared -> global (TMA engine), completion tracked per thread
 __device__ __forceinline__ void bulk_s2g(void* gdst, const void* ssrc, uint32_t bytes) {
@@ -1788,7 +1790,7 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-constexpr uint32_t kIdBuf = 1024 + 8;  // one unit's ids plus the 16-byte alignment head
+constexpr uint32_t kIdBuf = 1024 + 32;  // one unit's ids plus the part of a 128-byte line before them
 
 // Ids of one unit into dst[0 .. tot): lane l holds word l of the unit in v
 // and the ids of the lower lanes' words in ex; id0 = first id of the unit +
@@ -1805,36 +1807,34 @@ constexpr uint32_t kIdBuf = 1024 + 8;  // one unit's ids plus the 16-byte alignm
 // the non-zero words for the rest, and 2x at 25 % density.
 constexpr uint32_t kPairMin = 384;
 
-template <typename Store>
-__device__ __forceinline__ void expand_pairs(uint32_t v, uint32_t ex, uint32_t id0, Store store) {
+__device__ __forceinline__ void st_shared(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v));
+}
+
+// at: shared address of the first id of this lane's word
+__device__ __forceinline__ void expand_pairs(uint32_t v, uint32_t at, uint32_t id0) {
     const uint32_t lane = lane_id();
     const uint32_t half = lane >> 4, j = lane & 15u;
     const uint32_t below = (1u << (2u * j)) - 1u;               // bits under this lane's pair
-    const uint32_t base = id0 - lane + half * 32u + 2u * j;     // id of bit 2j of word `half`
+    uint32_t id = id0 - lane + half * 32u + 2u * j;             // id of bit 2j of word `half`
 #pragma unroll 4
-    for (uint32_t i = 0; i < 16u; ++i) {
-        const uint32_t w = 2u * i + half;
-        const uint32_t word = __shfl_sync(kFull, v, w);
-        const uint32_t pos = __shfl_sync(kFull, ex, w);
-        const uint32_t b2 = (word >> (2u * j)) & 3u;
-        const uint32_t p = pos + __popc(word & below);
-        const uint32_t id = base + i * 64u;
-        if (b2 & 1u) store(p, id);
-        if (b2 & 2u) store(p + (b2 & 1u), id + 1u);
+    for (uint32_t i = 0; i < 16u; ++i, id += 64u) {
+        const uint32_t word = __shfl_sync(kFull, v, 2u * i + half);
+        const uint32_t a = __shfl_sync(kFull, at, 2u * i + half) + 4u * __popc(word & below);
+        const uint32_t b2 = word >> (2u * j);
+        if (b2 & 1u) st_shared(a, id);
+        if (b2 & 2u) st_shared(a + 4u * (b2 & 1u), id + 1u);
     }
 }
 
-template <typename Store>
-__device__ __forceinline__ void expand_lane_word(uint32_t v, uint32_t ex, uint32_t id0, Store store) {
+__device__ __forceinline__ void expand_lane_word(uint32_t v, uint32_t at, uint32_t id0) {
     const uint32_t lane = lane_id();
     const uint32_t wb = id0 - lane + 32u * lane;  // id of bit 0 of this lane's word
     const uint32_t steps = __reduce_max_sync(kFull, uint32_t(__popc(v)));
-    uint32_t w = v, p = ex;
-    for (uint32_t i = 0; i < steps; ++i) {
-        if (w) {
-            store(p, wb + uint32_t(__ffs(w)) - 1u);
-            ++p;
-            w &= w - 1u;
+    for (uint32_t i = 0; i < steps; ++i, at += 4u) {
+        if (v) {
+            st_shared(at, wb + uint32_t(__ffs(v)) - 1u);
+            v &= v - 1u;
         }
     }
 }
@@ -1844,8 +1844,10 @@ __device__ __forceinline__ void expand_lane_word(uint32_t v, uint32_t ex, uint32
 // into s_wtot, the decoupled look-back's exclusive prefix into *s_prefix.
 // The claim is followed at once by the loads and the count's publication, so
 // later items' look-backs never wait long on it.
+template <uint32_t kWarpUnits>
 __device__ void prepare_chunk(const CompactArgs& a, uint64_t items, uint64_t n_words, uint32_t* buf,
                               unsigned long long* s_item, unsigned long long* s_prefix, uint32_t* s_wtot) {
+    constexpr uint32_t kUnits = kWarpUnits * kCompactWarps;
     const uint32_t lane = lane_id();
     unsigned long long n = 0;
     if (lane == 0) n = atomicAdd(a.ticket, 1ull);
@@ -1855,7 +1857,7 @@ __device__ void prepare_chunk(const CompactArgs& a, uint64_t items, uint64_t n_w
     const uint32_t q = uint32_t(n / a.n_chunks);
     const uint32_t c = uint32_t(n - uint64_t(q) * a.n_chunks);
     const uint32_t* bm = a.bm + uint64_t(q) * a.stride;
-    const uint64_t wbase = uint64_t(c) * kCompactChunkWords;
+    const uint64_t wbase = uint64_t(c) * (kUnits * 32u);
 #pragma unroll 8
     for (uint32_t m = 0; m < kUnits; ++m) {
         const uint64_t wi = wbase + m * 32u + lane;
@@ -1891,6 +1893,7 @@ __device__ void prepare_chunk(const CompactArgs& a, uint64_t items, uint64_t n_w
 // the next one in its own id buffer (claim, loads, count, look-back), so the
 // claim's round trip, the loads and the look-back overlap the other warps'
 // expansion instead of stalling the whole CTA.
+template <uint32_t kWarpUnits>
 __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compact_kernel(CompactArgs a) {
     __shared__ __align__(16) uint32_t s_buf[kCompactWarps][kIdBuf];
     __shared__ uint32_t s_wtot[kCompactWarps];
@@ -1898,12 +1901,12 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compac
     __shared__ uint32_t s_src, s_first;
     static_assert(kCompactChunkWords <= kIdBuf, "a chunk fits one id buffer");
     const uint32_t lane = lane_id(), warp = warp_id();
-    const bool ids16 = (reinterpret_cast<uintptr_t>(a.ids) & 15u) == 0;
     uint32_t* buf = s_buf[warp];
+    const uint32_t buf_addr = smem_addr(buf);
     const uint64_t n_words = (a.n_bits + 31) / 32;
     const uint64_t items = uint64_t(a.n_q) * a.n_chunks;
     wait_previous();
-    if (warp == 0) prepare_chunk(a, items, n_words, buf, &s_item, &s_prefix, s_wtot);
+    if (warp == 0) prepare_chunk<kWarpUnits>(a, items, n_words, buf, &s_item, &s_prefix, s_wtot);
     if (threadIdx.x == 0) {
         s_src = 0;
         s_first = 0;
@@ -1914,7 +1917,7 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compac
         if (item >= items) break;
         const uint32_t q = uint32_t(item / a.n_chunks);
         const uint32_t c = uint32_t(item - uint64_t(q) * a.n_chunks);
-        const uint64_t wbase = uint64_t(c) * kCompactChunkWords + uint64_t(warp) * (kWarpUnits * 32u);
+        const uint64_t wbase = uint64_t(c) * (kWarpUnits * 32u * kCompactWarps) + uint64_t(warp) * (kWarpUnits * 32u);
         const uint32_t* src = s_buf[s_src] + warp * (kWarpUnits * 32u);
         uint32_t v[kWarpUnits], tot[kWarpUnits];
 #pragma unroll
@@ -1923,6 +1926,18 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compac
             tot[k] = __reduce_add_sync(kFull, uint32_t(__popc(v[k])));
         }
         uint64_t o0 = s_prefix + __reduce_add_sync(kFull, lane < warp ? s_wtot[lane] : 0u);
+        // The warp's ids leave by bulk copies of whole 128-byte lines (2 % less
+        // time on c1 than 16-byte ends per unit: 4,638 -> 4,588 us for 512
+        // queries, 26.9 GB; without expanding anything the same copies take
+        // 4,430, without copying the rest takes 3,780): buf holds words of the output from a line's start on, of which the first
+        // `from` are not this slice's; what does not fill a line is carried to
+        // the next unit in a register (lane l: word l).
+        uint32_t slice = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kWarpUnits; ++k) slice += tot[k];
+        const bool fits = o0 + slice <= a.capacity && (reinterpret_cast<uintptr_t>(a.ids) & 3u) == 0;
+        uint32_t fill = (uint32_t(reinterpret_cast<uintptr_t>(a.ids) >> 2) + uint32_t(o0)) & 31u, from = fill, carry = 0;
+        uint32_t* line = a.ids + o0 - fill;
         // every warp holds its words and offset: the chunk's buffer and the
         // next item's slots may be reused
         __syncthreads();
@@ -1947,53 +1962,53 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compac
             }
             const uint32_t ex = x - cnt;
             const uint32_t id0 = uint32_t((wbase + k * 32u) * 32u) + lane;
-            uint32_t* dst = a.ids + o0;
-            if (ids16 && o0 + t <= a.capacity) {
-                // the unit's ids go to the warp's shared buffer at their
-                // 16-byte-aligned output position; the aligned middle leaves
-                // by one bulk copy, the ragged ends by plain stores
-                const uint32_t head = uint32_t(o0 & 3u);
-                uint32_t* sb = buf + head;
+            if (fits) {
                 if (lane == 0) bulk_wait_read_all();  // the previous unit's copy has read the buffer
                 __syncwarp();
-                auto st = [sb](uint32_t i, uint32_t id) { sb[i] = id; };
+                if (lane < fill) buf[lane] = carry;
+                const uint32_t end = fill + t;
                 if (t == 1024u) {
-                    // every bit set: buf[x] = first id of the unit + x - head
-                    const uint32_t b0 = id0 - lane - head;
+                    // every bit set: buf[x] = first id of the unit + x - fill
+                    const uint32_t b0 = id0 - lane - fill, m0 = (fill + 3u) / 4u;
                     uint4* b4 = reinterpret_cast<uint4*>(buf);
-#pragma unroll
-                    for (uint32_t m = lane; m < kIdBuf / 4u; m += 32u) {
-                        const uint32_t x = b0 + 4u * m;
-                        b4[m] = make_uint4(x, x + 1u, x + 2u, x + 3u);
+                    for (uint32_t m = m0 + lane; m < end / 4u; m += 32u) {
+                        const uint32_t y = b0 + 4u * m;
+                        b4[m] = make_uint4(y, y + 1u, y + 2u, y + 3u);
+                    }
+                    if (lane < 3u) {  // the words short of a vector at either end
+                        const uint32_t h = fill + lane, e = (end & ~3u) + lane;
+                        if (h < 4u * m0) buf[h] = b0 + h;
+                        if (e < end) buf[e] = b0 + e;
                     }
                 } else if (t >= kPairMin) {
-                    expand_pairs(vk, ex, id0, st);
+                    expand_pairs(vk, buf_addr + 4u * (fill + ex), id0);
                 } else {
-                    expand_lane_word(vk, ex, id0, st);
+                    expand_lane_word(vk, buf_addr + 4u * (fill + ex), id0);
                 }
                 fence_proxy_async();  // these shared writes before the async-proxy read
                 __syncwarp();
-                const uint32_t end = head + t;
-                const uint32_t mid_hi = end & ~3u;
-                uint32_t* gbase = dst - head;  // 16-byte aligned
-                if (lane == 0 && mid_hi > 4u) {
-                    bulk_s2g(gbase + 4, buf + 4, (mid_hi - 4u) * 4u);
-                    bulk_commit();
+                const uint32_t full = end & ~31u;
+                if (full) {
+                    const uint32_t lo = from ? 32u : 0u;
+                    if (lane == 0 && full > lo) {
+                        bulk_s2g(line + lo, buf + lo, (full - lo) * 4u);
+                        bulk_commit();
+                    }
+                    if (from && lane >= from) line[lane] = buf[lane];  // the slice's first, partial line
+                    from = 0;
+                    line += full;
                 }
-                if (lane >= head && lane < 4u && lane < end) gbase[lane] = buf[lane];
-                if (mid_hi + lane < end && mid_hi + lane >= 4u) gbase[mid_hi + lane] = buf[mid_hi + lane];
-            } else if (o0 + t <= a.capacity) {  // whole unit fits: no per-id check
-                expand_lane_word(vk, ex, id0, [dst](uint32_t i, uint32_t id) { dst[i] = id; });
+                fill = end - full;
+                if (lane < fill) carry = buf[full + lane];
             } else {
-                const uint64_t cap = a.capacity;
-                const uint64_t ob = o0;
-                uint32_t* ids = a.ids;
-                expand_lane_word(vk, ex, id0, [=](uint32_t i, uint32_t id) {
-                    if (ob + i < cap) ids[ob + i] = id;
-                });
+                // an output too short for the slice: every id is checked
+                uint64_t o = o0 + ex;
+                for (uint32_t m = vk; m; m &= m - 1u, ++o)
+                    if (o < a.capacity) a.ids[o] = id0 - lane + 32u * lane + uint32_t(__ffs(m)) - 1u;
             }
             o0 += t;
         }
+        if (fits && lane >= from && lane < fill) line[lane] = carry;  // the last, partial line
         // the first warp done prepares the next item in its own buffer
         uint32_t first = 0;
         if (lane == 0) first = atomicAdd(&s_first, 1u);
@@ -2001,7 +2016,7 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 48 / kCompactWarps) compac
         if (first == 0) {
             if (lane == 0) bulk_wait_read_all();  // its last copy has read the buffer
             __syncwarp();
-            prepare_chunk(a, items, n_words, buf, &s_item, &s_prefix, s_wtot);
+            prepare_chunk<kWarpUnits>(a, items, n_words, buf, &s_item, &s_prefix, s_wtot);
             if (lane == 0) s_src = warp;
         }
         __syncthreads();
@@ -2094,9 +2109,14 @@ cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t threads, 
 }
 }  // namespace
 
-uint32_t compact_chunks(uint64_t n_bits) {
-    const uint64_t n_words = (n_bits + 31) / 32;
-    return uint32_t((n_words + kCompactChunkWords - 1) / kCompactChunkWords);
+uint32_t compact_chunks(uint64_t n_bits, uint32_t units) {
+    const uint64_t n_words = (n_bits + 31) / 32, chunk = units * 32u * kCompactWarps;
+    return uint32_t((n_words + chunk - 1) / chunk);
+}
+
+uint32_t compact_units(uint64_t n_q, uint64_t n_bits) {
+    if (n_q * compact_chunks(n_bits, 8) >= kCompactFew) return 8;
+    return n_q * compact_chunks(n_bits, 2) >= kCompactFew ? 2 : 1;
 }
 
 cudaError_t launch_plan(const IndexView& v, const PlanArgs& a, cudaStream_t s) {
@@ -2346,7 +2366,8 @@ cudaError_t launch_compact(const CompactArgs& a, int sm_count, uint32_t ctas_per
     // ctas_per_sm counts CTAs of 8 warps: the same resident warps whatever the CTA size
     const uint32_t per_sm = (ctas_per_sm ? ctas_per_sm : 6u) * 8u / kCompactWarps;
     count_launch();
-    return launch_after(compact_kernel, uint32_t(grid_for(items, sm_count, per_sm)), kCompactWarps * 32, 0, s, a);
+    const auto kernel = a.units == 8u ? compact_kernel<8> : a.units == 2u ? compact_kernel<2> : compact_kernel<1>;
+    return launch_after(kernel, uint32_t(grid_for(items, sm_count, per_sm)), kCompactWarps * 32, 0, s, a);
 }
 
 cudaError_t launch_wait_selftest(uint64_t* status2, uint32_t* err, uint32_t spin_limit, cudaStream_t s) {

@@ -47,6 +47,10 @@ constexpr uint32_t kDenseOnly = 0xfffffffeu; // heavy_min meaning "merge only th
 // buffer, where the warp that prepares it stages it
 constexpr uint32_t kCompactWarps = 4;
 constexpr uint32_t kCompactChunkWords = kCompactWarps * 256;  // bitmap words per compaction work item
+constexpr uint32_t kCompactFew = 888;  // fewer items than this (6 per SM): shorter chunks
+// look-back words that a batch with shorter chunks can need: less than
+// kCompactFew items turn into at most four times as many, plus one per bitmap
+constexpr uint32_t kCompactFewStatus = 8u * kCompactFew;
 constexpr uint32_t kProbeGroup = 32;          // probe queries tested per pass
 
 // device error codes (workspace flag)
@@ -285,6 +289,7 @@ struct CompactArgs {
     uint32_t n_q;
     uint64_t n_bits;           // ids >= n_bits are dropped
     uint32_t n_chunks;         // per bitmap
+    uint32_t units;            // 32-word units per warp of a chunk (8, 2 or 1; see compact_units)
     uint64_t* status;          // n_q * n_chunks look-back words, zeroed before launch
     unsigned long long* ticket;  // item counter, zeroed before launch
     uint32_t* ids;
@@ -297,7 +302,8 @@ struct CompactArgs {
 };
 
 IndexView view_of(const abf_index* ix);
-uint32_t compact_chunks(uint64_t n_bits);
+uint32_t compact_chunks(uint64_t n_bits, uint32_t units = 8);
+uint32_t compact_units(uint64_t n_q, uint64_t n_bits);
 
 cudaError_t launch_plan(const IndexView& v, const PlanArgs& a, cudaStream_t s);
 // two 2-D TMA descriptors (2 x 128 bytes into out) of the dense bitmaps:

@@ -30,6 +30,7 @@ namespace {
 
 constexpr uint64_t kMaxBits = ABF_NOALLOC_MAX_BITS;
 constexpr uint64_t kMaxChunks = (kMaxBits / 32 + abf::kCompactChunkWords - 1) / abf::kCompactChunkWords;
+static_assert(kMaxChunks >= abf::kCompactFewStatus, "shorter chunks of short bitmaps fit the status words");
 // layout in 8-byte words: status[kMaxChunks] (one look-back word per chunk),
 // the item ticket, the error word (low 4 bytes)
 constexpr uint64_t kStatusAt = 0;
@@ -93,7 +94,8 @@ extern "C" abf_status abf_collect_ids_noalloc(const uint32_t* d_bitmap, uint64_t
         ca.stride = (n_bits + 31) / 32;
         ca.n_q = 1;
         ca.n_bits = n_bits;
-        ca.n_chunks = abf::compact_chunks(n_bits);
+        ca.units = abf::compact_units(1, n_bits);
+        ca.n_chunks = abf::compact_chunks(n_bits, ca.units);
         ca.status = reinterpret_cast<uint64_t*>(b + kStatusAt);
         ca.ticket = b + kTicketAt;
         ca.err = reinterpret_cast<uint32_t*>(b + kErrAt);

@@ -638,6 +638,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.dense_in_tile = 1;
     pa.tile_cls = ws->tile_cls;
     pa.q_dense16 = ws->q_dense16;
+    if (group) pa.dense_shift = gw == 64u ? 6u : 5u;
     pa.q_dstart = ws->q_dstart;
     pa.q_ndense = ws->q_ndense;
     pa.tile_list = ws->tile_list;
@@ -913,7 +914,10 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         pa.q_dense16 = w->d_dense16;
         pa.q_dstart = w->d_dstart;
         pa.q_ndense = w->d_ndense;
-        if (group) pa.no_dense_from = nd_q;
+        if (group) {
+            pa.no_dense_from = nd_q;
+            pa.dense_shift = r.group.gw == 64u ? 6u : 5u;
+        }
         // the plan kernel zeroes the marks of the queries there are; with more
         // runs than rows, all rows (the last one stands for the runs past it)
         if (r.d_n_q && r.n_q > w->q_cap) {

@@ -528,11 +528,11 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
             for (uint32_t w = w0; w < w1; ++w) {
                 uint32_t m = s_mask[w];
                 while (m) {
-                    dst[o++] = uint16_t(w * 32u + uint32_t(__ffs(m)) - 1u);
+                    dst[o++] = uint16_t((w * 32u + uint32_t(__ffs(m)) - 1u) << a.dense_shift);
                     m &= m - 1u;
                 }
             }
-            for (uint32_t i = nd + tid; i < ((nd + 7u) & ~7u); i += 256) dst[i] = uint16_t(ix.n_dense);
+            for (uint32_t i = nd + tid; i < ((nd + 7u) & ~7u); i += 256) dst[i] = uint16_t(ix.n_dense << a.dense_shift);
             if (tid == 0) {
                 a.q_dstart[q] = start;
                 a.q_ndense[q] = nd;
@@ -932,6 +932,10 @@ template <typename T>
 __device__ __forceinline__ T ld_row(const uint8_t* B, uint32_t woff) {
     return *reinterpret_cast<const T*>(B + (woff << 2));
 }
+template <typename T>
+__device__ __forceinline__ T or2w(const uint8_t* B, uint32_t v) {
+    return orw(ld_row<T>(B, v & 0xffffu), ld_row<T>(B, v >> 16));
+}
 // OR of the 8 rows named by the 16-bit word offsets in v
 template <typename T>
 __device__ __forceinline__ T or8w(const uint8_t* B, uint4 v) {
@@ -953,32 +957,32 @@ __device__ __forceinline__ T or_list_words(const uint8_t* B, const uint4* ol, ui
         acc = orw(acc, orw(or8w<T>(B, ol[k >> 3]), or8w<T>(B, ol[(k >> 3) + 1])));
         if (tile_full(acc)) return acc;
     }
-    if (k < nd) acc = orw(acc, or8w<T>(B, ol[k >> 3]));
-    if (k + 8u < nd) acc = orw(acc, or8w<T>(B, ol[(k >> 3) + 1]));
-    return acc;
-}
-// the same over a list of 16-bit row indices read from global memory (used
-// when the batch's lists do not fit in shared memory)
-template <uint32_t GW, typename T>
-__device__ __forceinline__ T or_list_rows(const uint8_t* B, const uint4* dl, uint32_t nd) {
-    T acc = zero_word<T>();
-    for (uint32_t k = 0; k < nd; k += 8u) {
-        const uint4 v = dl[k >> 3];
-        const uint4 wv = make_uint4((v.x & 0xffffu) * GW | ((v.x >> 16) * GW) << 16,
-                                    (v.y & 0xffffu) * GW | ((v.y >> 16) * GW) << 16,
-                                    (v.z & 0xffffu) * GW | ((v.z >> 16) * GW) << 16,
-                                    (v.w & 0xffffu) * GW | ((v.w >> 16) * GW) << 16);
-        acc = orw(acc, or8w<T>(B, wv));
-        if (tile_full(acc)) break;
+    if (k + 8u <= nd) {
+        acc = orw(acc, or8w<T>(B, ol[k >> 3]));
+        k += 8u;
+    }
+    // the last 0 .. 7 rows, without the list's padding
+    const uint32_t r = nd - k;
+    if (r) {
+        uint4 v = ol[k >> 3];
+        if (r & 4u) {
+            acc = orw(acc, orw(or2w<T>(B, v.x), or2w<T>(B, v.y)));
+            v.x = v.z;
+            v.y = v.w;
+        }
+        if (r & 2u) {
+            acc = orw(acc, or2w<T>(B, v.x));
+            v.x = v.y;
+        }
+        if (r & 1u) acc = orw(acc, ld_row<T>(B, v.x & 0xffffu));
     }
     return acc;
 }
-
 // Shared memory (dynamic, 1024-byte aligned base): two stages of n_rows x
 // GW words (rows = dense bitmaps + the zero row), then per such query
 // its list's offset and length, the queue of those queries, and the
-// lists themselves as 16-bit row word offsets (row * GW) when they fit (else
-// the 16-bit row lists are read from global memory). GW = 64 halves the
+// lists themselves when they fit (else they are read from global memory): the
+// plan kernel writes them as 16-bit row word offsets (row * GW). GW = 64 halves the
 // index work per word (each lane ORs two words per row) where two stages of
 // 64-word rows fit.
 // ACC: OR into the output with atomics (bitmaps may be shared, rows need no
@@ -1054,16 +1058,12 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     if (tid == 0) s_ndq = tot_cnt;
     __syncthreads();
     if (in_smem) {
-        constexpr uint32_t kShift = GW == 64u ? 6u : 5u;  // row -> word offset, both halves at once
         for (uint32_t i = warp; i < tot_cnt; i += kNW) {  // a warp per query, 16 bytes per lane
             const uint32_t q = s_qlist[i];
             const uint32_t m = s_meta[q];
             const uint4* src = reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]);
             uint4* dst = s_lists + (m >> 16);
-            for (uint32_t j = lane; j < ((m & 0xffffu) + 7u) / 8u; j += 32u) {
-                const uint4 v = src[j];
-                dst[j] = make_uint4(v.x << kShift, v.y << kShift, v.z << kShift, v.w << kShift);
-            }
+            for (uint32_t j = lane; j < ((m & 0xffffu) + 7u) / 8u; j += 32u) dst[j] = src[j];
         }
     }
     __syncthreads();
@@ -1100,8 +1100,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
             const uint32_t m = s_meta[q];
             const uint32_t nd = m & 0xffffu;
             const T acc = in_smem ? or_list_words<T>(B, s_lists + (m >> 16), nd)
-                                  : or_list_rows<GW, T>(B, reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]),
-                                                        nd);
+                                  : or_list_words<T>(B, reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]), nd);
             if (a.sat && tile_full(acc) && lane == 0)
                 atomicOr(a.sat + uint64_t(q) * a.sat_stride + (t >> 5), 1u << (t & 31u));
             if constexpr (ACC) {

@@ -118,6 +118,7 @@ struct PlanArgs {
     // values from q_dense16 + q_dstart[q] (16-byte aligned), padded to a
     // multiple of 8 with the index n_dense (an all-zero row for the TMA path)
     uint16_t* q_dense16;      // out: max_terms + 8 * n_q + 16 entries
+    uint32_t dense_shift;     // entries are index << this (the group kernel's row word offsets: 6 or 5)
     uint32_t* q_dstart;       // out: per query
     uint32_t* q_ndense;       // out: per query, distinct dense bitmaps
     const uint32_t* d_n_q;    // optional device count of queries (at most n_q)

@@ -119,6 +119,7 @@ struct ProfScope {
 
 struct abf_workspace {
     abf_index* ix = nullptr;
+    void* arena = nullptr;          // the one allocation behind every pointer below
     uint32_t max_q = 0;
     uint64_t max_terms = 0;
     uint32_t probe_cap = 0;
@@ -140,7 +141,6 @@ struct abf_workspace {
     unsigned long long* ticket = nullptr;   // compaction item counter
     uint64_t* id_off = nullptr;
     uint8_t* path_out = nullptr;
-    uint8_t* auto_paths = nullptr;  // planner choices for ABF_PATH_AUTO batches
     uint16_t* q_dense16 = nullptr;  // the queries' dense bitmap lists (see PlanArgs)
     uint32_t* q_dstart = nullptr;   // per query
     uint32_t* q_ndense = nullptr;   // per query
@@ -422,32 +422,51 @@ abf_status need_device(const abf_index* ix) {
     return ABF_OK;
 }
 
+// One allocation for all arrays of a workspace or worker: take() once to size it, once
+// more over the allocation to place them.
+struct Arena {
+    char* base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, uint64_t n) {
+        used = (used + 255) & ~size_t(255);
+        if (base) p = reinterpret_cast<T*>(base + used);
+        used += std::max<uint64_t>(n, 1) * sizeof(T);
+    }
+};
+
 void ws_release(abf_workspace* w) {
-    dev_free(w->slot);
-    dev_free(w->tile_cls);
-    dev_free(w->lcnt);
-    dev_free(w->lpref_q);
-    dev_free(w->probe_list);
-    dev_free(w->probe_bm);
-    dev_free(w->scan_status);
-    dev_free(w->id_off);
-    dev_free(w->path_out);
-    dev_free(w->auto_paths);
-    dev_free(w->q_dense16);
-    dev_free(w->q_dstart);
-    dev_free(w->q_ndense);
-    dev_free(w->err);
-    dev_free(w->bin_list);
-    dev_free(w->q_nbin);
-    dev_free(w->q_bblk);
-    dev_free(w->parts_pref);
-    dev_free(w->bin_ticket);
-    dev_free(w->tile_list);
-    dev_free(w->sat);
-    dev_free(w->ctl);
+    if (w->arena) cudaFree(w->arena);
+    w->arena = nullptr;
 }
 
 constexpr uint32_t kCtlWords = 8;
+
+void ws_take(abf_workspace* w, Arena& a, uint64_t chunks) {
+    const uint32_t max_q = w->max_q;
+    const uint64_t max_terms = w->max_terms;
+    a.take(w->ctl, kCtlWords + 4 + max_terms);
+    a.take(w->slot, max_terms);
+    a.take(w->tile_cls, max_terms);
+    a.take(w->lcnt, max_q);
+    a.take(w->lpref_q, uint64_t(max_q) + 1);
+    a.take(w->probe_list, w->probe_cap);
+    a.take(w->probe_bm, uint64_t(w->probe_cap) * w->probe_stride);
+    a.take(w->scan_status, std::max<uint64_t>(chunks, abf::kCompactFewStatus) + 1);
+    a.take(w->id_off, uint64_t(max_q) + 1);
+    a.take(w->path_out, max_q);
+    a.take(w->err, 1);
+    a.take(w->q_dense16, max_terms + 8ull * max_q + 16);
+    a.take(w->q_dstart, max_q);
+    a.take(w->q_ndense, max_q);
+    a.take(w->tile_list, max_q);
+    a.take(w->bin_list, max_terms);
+    a.take(w->q_nbin, max_q);
+    a.take(w->q_bblk, max_q);
+    a.take(w->parts_pref, uint64_t(max_q) + 1);
+    a.take(w->bin_ticket, 1);
+    a.take(w->sat, uint64_t(max_q) * w->sat_stride);
+}
 
 abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t max_bits, abf_workspace* w) {
     w->ix = ix;
@@ -456,37 +475,26 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     w->probe_cap = ix->tuning.probe_cap;
     w->probe_stride = round4(n_words_of(ix->n_terms));
     w->chunks_per_q = abf::compact_chunks(std::max<uint64_t>(max_bits, ix->n_ads));
-    const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
     w->sat_stride = sat_words(ix);
-    abf_status st;
-    if ((st = dev_alloc(&w->slot, max_terms)) != ABF_OK ||
-        (st = dev_alloc(&w->tile_cls, max_terms)) != ABF_OK ||
-        (st = dev_alloc(&w->lcnt, max_q)) != ABF_OK || (st = dev_alloc(&w->lpref_q, uint64_t(max_q) + 1)) != ABF_OK ||
-        (st = dev_alloc(&w->probe_list, w->probe_cap)) != ABF_OK ||
-        (st = dev_alloc(&w->probe_bm, uint64_t(w->probe_cap) * w->probe_stride)) != ABF_OK ||
-        (st = dev_alloc(&w->scan_status, std::max<uint64_t>(chunks, abf::kCompactFewStatus) + 1)) != ABF_OK ||
-        (st = dev_alloc(&w->id_off, uint64_t(max_q) + 1)) != ABF_OK ||
-        (st = dev_alloc(&w->path_out, max_q)) != ABF_OK || (st = dev_alloc(&w->err, 1)) != ABF_OK ||
-        (st = dev_alloc(&w->auto_paths, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->q_dense16, max_terms + 8ull * max_q + 16)) != ABF_OK ||
-        (st = dev_alloc(&w->q_dstart, max_q)) != ABF_OK || (st = dev_alloc(&w->q_ndense, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->tile_list, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->bin_list, max_terms)) != ABF_OK ||
-        (st = dev_alloc(&w->q_nbin, max_q)) != ABF_OK || (st = dev_alloc(&w->q_bblk, max_q)) != ABF_OK ||
-        (st = dev_alloc(&w->parts_pref, uint64_t(max_q) + 1)) != ABF_OK ||
-        (st = dev_alloc(&w->bin_ticket, 1)) != ABF_OK ||
-        (st = dev_alloc(&w->sat, uint64_t(max_q) * w->sat_stride)) != ABF_OK ||
-        (st = dev_alloc(&w->ctl, kCtlWords + 4 + max_terms)) != ABF_OK) {
-        ws_release(w);
-        return st;
-    }
+    const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
+    Arena a;
+    ws_take(w, a, chunks);
+    char* p = nullptr;
+    ABF_TRY(dev_alloc(&p, a.used));
+    w->arena = p;
+    a = Arena{p, 0};
+    ws_take(w, a, chunks);
     w->n_probe = w->ctl;
     w->n_tile_list = w->ctl + 1;
     w->plan_done = w->ctl + 2;
     w->ticket = reinterpret_cast<unsigned long long*>(w->ctl + 4);
     w->q_off = reinterpret_cast<uint64_t*>(w->ctl + kCtlWords);
     w->q_terms = w->ctl + kCtlWords + 4;
-    CUDA_TRY(cudaMemset(w->err, 0, sizeof(uint32_t)));
+    const cudaError_t e = cudaMemset(w->err, 0, sizeof(uint32_t));
+    if (e != cudaSuccess) {
+        ws_release(w);
+        return fail(ABF_ERR_CUDA, std::string("workspace: ") + cudaGetErrorString(e));
+    }
     return ABF_OK;
 }
 
@@ -811,32 +819,21 @@ constexpr uint32_t kKeyRunCap = 256;    // runs of a keyed batch merged by the g
 constexpr uint32_t kOneQueryKeys = 2048; // keys that one planning CTA takes in a few steps of 256
 constexpr uint32_t kTermWindow = 256;   // query bitmaps extracted and merged at a time
 
-// One allocation for all of a worker's arrays: take() once to size it, once
-// more over the allocation to place them.
-struct Arena {
-    char* base = nullptr;
-    size_t used = 0;
-    template <class T>
-    void take(T*& p, uint64_t n) {
-        used = (used + 255) & ~size_t(255);
-        if (base) p = reinterpret_cast<T*>(base + used);
-        used += std::max<uint64_t>(n, 1) * sizeof(T);
-    }
-};
+constexpr uint32_t kWorkerHead = 8;  // words before the keys: four counters, two 64-bit offsets
 
 // arrays of a worker that plans at most n_q queries over w->term_cap terms
 void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
-    a.take(w->d_off1, 2);  // followed at once by the keys: one upload
-    w->d_keys = reinterpret_cast<uint32_t*>(w->d_off1 + 2);
-    a.used += uint64_t(w->term_cap) * sizeof(uint32_t);
+    // counters, offsets and keys in one piece: one upload
+    a.take(w->d_nprobe, kWorkerHead + w->term_cap);
+    w->d_n_tile_list = w->d_nprobe + 1;
+    w->d_plan_done = w->d_nprobe + 2;
+    w->d_off1 = reinterpret_cast<uint64_t*>(w->d_nprobe + 4);
+    w->d_keys = w->d_nprobe + kWorkerHead;
     a.take(w->d_off, n_q + 1);
     a.take(w->d_tslot, w->term_cap);
     a.take(w->d_tile_cls, w->term_cap);
     a.take(w->d_lcnt, n_q);
     a.take(w->d_lpref_q, n_q + 1);
-    a.take(w->d_nprobe, 4);
-    w->d_n_tile_list = w->d_nprobe + 1;
-    w->d_plan_done = w->d_nprobe + 2;
     a.take(w->d_tile_list, w->q_cap);
     a.take(w->d_n_q, 1);
     a.take(w->d_err, 1);
@@ -863,6 +860,12 @@ abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
     w->arena = p;
     a = Arena{p, 0};
     worker_take(w, a, n_q);
+    const cudaError_t e = cudaMemset(w->d_nprobe, 0, kWorkerHead * 4u);
+    if (e != cudaSuccess) {
+        cudaFree(w->arena);
+        w->arena = nullptr;
+        return fail(ABF_ERR_CUDA, std::string("worker: ") + cudaGetErrorString(e));
+    }
     return ABF_OK;
 }
 
@@ -927,7 +930,8 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
             pa.sat_stride = w->sat_stride;
         }
     }
-    CUDA_TRY(cudaMemsetAsync(w->d_nprobe, 0, 4 * sizeof(uint32_t), s));  // and the other counters
+    // (the count of finished plan CTAs is zero when a run ends)
+    if (merge) CUDA_TRY(cudaMemsetAsync(w->d_n_tile_list, 0, sizeof(uint32_t), s));
     abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, r.n_q, r.d_n_q};
     const bool bins = group && v.n_plain > 0;
     if (bins) {

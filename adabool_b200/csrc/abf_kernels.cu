@@ -553,6 +553,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
     __syncthreads();
     if (s_slot == gridDim.x - 1u) {
         __threadfence();
+        if (tid == 0) *a.done = 0;  // for a next batch that does not zero it
         queue_scan_body<256>(a.queue, n_q, s_red, s_warp);
     }
 }
@@ -731,8 +732,10 @@ __device__ __forceinline__ uint32_t find_slot(const uint32_t* s_pref, uint32_t f
 // warp whose columns are all ones reads no more. Half-warps whose 64 words
 // came out all ones mark them for the scatter kernel.
 // The merge kernel did this with a quarter of its threads at 256-word tiles:
-// seven queries of the serving mix on c1 135 to 186 us, here 74 to 122; one
-// query 17 to 26, here 12 to 18.
+// seven queries of the serving mix on c1 135 to 186 us, one query 17 to 26.
+// Four CTAs per SM leave the registers that keep all eight loads in flight: 70
+// us for seven queries (398 MB of distinct rows: 5.7 TB/s), 92 with the 38
+// registers the compiler takes by itself; 16 rows in flight were no faster.
 // ACC: OR into the output with atomics (other calls may do so at the same
 // time). V: uint4, or uint32_t where rows are not 16-byte aligned.
 __device__ __forceinline__ void or_in(uint4& a, uint4 b) { a.x |= b.x; a.y |= b.y; a.z |= b.z; a.w |= b.w; }
@@ -742,7 +745,7 @@ __device__ __forceinline__ bool full_vec(uint32_t a) { return a == ~0u; }
 
 constexpr uint32_t kStreamThreads = 256;
 template <typename V, bool ACC>
-__global__ void __launch_bounds__(kStreamThreads) dense_stream_kernel(IndexView ix, DenseStreamArgs a) {
+__global__ void __launch_bounds__(kStreamThreads, 4) dense_stream_kernel(IndexView ix, DenseStreamArgs a) {
     wait_previous();
     constexpr uint32_t KT = 8, VW = sizeof(V) / 4u;
     const uint64_t n_v = (a.n_words + VW - 1u) / VW;  // columns (the last may be partial)

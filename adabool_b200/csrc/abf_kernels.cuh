@@ -135,7 +135,7 @@ struct PlanArgs {
     uint32_t n_chunks;
     uint64_t* id_counts;
     // optional: the CTA that finishes last runs the scan over the queries
-    uint32_t* done;           // CTAs finished, zeroed before launch
+    uint32_t* done;           // CTAs finished: zero before the launch, and again when it ends
     QueueArgs queue;
     uint32_t no_dense_from;   // queries from this one on scatter their dense-bitmap lists too
                               // (0: none do; only with dense_in_tile)

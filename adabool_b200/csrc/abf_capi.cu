@@ -530,6 +530,8 @@ abf_status own_ws(abf_index* ix, uint32_t n_q, uint64_t n_terms, uint64_t n_bits
 struct RunOpts {
     uint64_t* id_counts = nullptr;
     bool ctl_zeroed = false;  // the workspace's counters are zero already
+    const uint32_t* inline_terms = nullptr;  // host terms of the one query (n_inline, at most kInlineLarge), to go
+    uint32_t n_inline = 0;                   // with the plan kernel's arguments
 };
 
 abf_status run_compact(abf_index* ix, const abf::CompactArgs& ca, cudaStream_t s) {
@@ -627,6 +629,12 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     const uint32_t gw = gs.gw, stages = gs.stages;
     if (!ro.ctl_zeroed) CUDA_TRY(cudaMemsetAsync(ws->ctl, 0, kCtlWords * 4u, s));
     abf::PlanArgs pa{};
+    if (ro.inline_terms) {
+        pa.inline_terms = ro.inline_terms;
+        pa.n_inline = ro.n_inline;
+        pa.ctl = ws->ctl;
+        pa.ctl_words = kCtlWords;
+    }
     pa.terms = b->d_terms;
     pa.q_off = b->d_offsets;
     pa.n_q = b->n_queries;
@@ -1819,27 +1827,35 @@ abf_status abf_query(abf_index* ix, const uint32_t* terms, uint32_t n_terms, abf
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     abf_workspace* ws = nullptr;
     ABF_TRY(own_ws(ix, 1, n_terms, ix->n_ads, &ws));
-    const size_t need = (kCtlWords + 4 + size_t(n_terms)) * 4;  // zeroed counters, offsets, terms
-    if (!ix->stage_event) {
-        cudaEvent_t ev;
-        CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        ix->stage_event = ev;
+    static const uint32_t none = 0;
+    RunOpts ro;
+    ro.ctl_zeroed = true;
+    if (n_terms <= abf::kInlineLarge) {
+        ro.inline_terms = n_terms ? terms : &none;
+        ro.n_inline = n_terms;
+    } else {
+        const size_t need = (kCtlWords + 4 + size_t(n_terms)) * 4;  // zeroed counters, offsets, terms
+        if (!ix->stage_event) {
+            cudaEvent_t ev;
+            CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+            ix->stage_event = ev;
+        }
+        cudaEvent_t ev = static_cast<cudaEvent_t>(ix->stage_event);
+        CUDA_TRY(cudaEventSynchronize(ev));  // the previous upload has left the staging buffer
+        if (ix->h_stage_bytes < need) {
+            if (ix->h_stage) cudaFreeHost(ix->h_stage);
+            ix->h_stage = nullptr;
+            ix->h_stage_bytes = 0;
+            CUDA_TRY(cudaMallocHost(&ix->h_stage, std::max<size_t>(need, 4096)));
+            ix->h_stage_bytes = std::max<size_t>(need, 4096);
+        }
+        uint32_t* up = static_cast<uint32_t*>(ix->h_stage);
+        std::memset(up, 0, (kCtlWords + 4) * 4);
+        up[kCtlWords + 2] = n_terms;  // {0, n_terms} as 64-bit offsets
+        if (n_terms) std::memcpy(up + kCtlWords + 4, terms, size_t(n_terms) * 4);
+        CUDA_TRY(cudaMemcpyAsync(ws->ctl, up, need, cudaMemcpyHostToDevice, s));
+        CUDA_TRY(cudaEventRecord(ev, s));
     }
-    cudaEvent_t ev = static_cast<cudaEvent_t>(ix->stage_event);
-    CUDA_TRY(cudaEventSynchronize(ev));  // the previous upload has left the staging buffer
-    if (ix->h_stage_bytes < need) {
-        if (ix->h_stage) cudaFreeHost(ix->h_stage);
-        ix->h_stage = nullptr;
-        ix->h_stage_bytes = 0;
-        CUDA_TRY(cudaMallocHost(&ix->h_stage, std::max<size_t>(need, 4096)));
-        ix->h_stage_bytes = std::max<size_t>(need, 4096);
-    }
-    uint32_t* up = static_cast<uint32_t*>(ix->h_stage);
-    std::memset(up, 0, (kCtlWords + 4) * 4);
-    up[kCtlWords + 2] = n_terms;  // {0, n_terms} as 64-bit offsets
-    if (n_terms) std::memcpy(up + kCtlWords + 4, terms, size_t(n_terms) * 4);
-    CUDA_TRY(cudaMemcpyAsync(ws->ctl, up, need, cudaMemcpyHostToDevice, s));
-    CUDA_TRY(cudaEventRecord(ev, s));
     abf_batch b{};
     b.d_terms = ws->q_terms;
     b.d_offsets = ws->q_off;
@@ -1850,9 +1866,7 @@ abf_status abf_query(abf_index* ix, const uint32_t* terms, uint32_t n_terms, abf
     b.d_ids = d_ids;
     b.ids_capacity = d_ids ? ids_capacity : 0;
     b.d_id_offsets = ws->id_off;
-    RunOpts ro;
     ro.id_counts = d_count;
-    ro.ctl_zeroed = true;
     return run_batch(ix, ws, &b, ro, s);
     API_END
 }

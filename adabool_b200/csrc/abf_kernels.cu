@@ -355,7 +355,9 @@ __device__ __forceinline__ void queue_scan_body(const QueueArgs& a, uint32_t n_q
 // last runs the scan over the queries (batches of up to kScanInPlan), which
 // saves that launch.
 constexpr uint32_t kPlanTerms = 4;
-__global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) {
+template <uint32_t kInline>
+__global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
+                                                      const __grid_constant__ InlineTerms<kInline> given) {
     __shared__ uint32_t s_warp[32];
     __shared__ unsigned long long s_red[8];
     __shared__ uint32_t s_path, s_max, s_slot, s_nbin;
@@ -366,6 +368,13 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a) 
     constexpr uint32_t kStep = 256u * kPlanTerms;
     if (a.planner) plan_dev::load_params(a.planner, s_pl);  // not written by any kernel of a batch
     wait_previous();
+    if constexpr (kInline > 0) {
+        uint32_t* terms = const_cast<uint32_t*>(a.terms);
+        for (uint32_t i = tid; i < given.n; i += 256) terms[i] = given.t[i];
+        if (tid < 2) const_cast<uint64_t*>(a.q_off)[tid] = tid ? given.n : 0u;
+        for (uint32_t i = tid; i < a.ctl_words; i += 256) a.ctl[i] = 0u;
+        __syncthreads();
+    }
     const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
     for (uint32_t q = blockIdx.x; q < n_q; q += gridDim.x) {
         uint64_t qb = a.q_off[q], qe = a.q_off[q + 1];
@@ -2126,7 +2135,15 @@ cudaError_t launch_plan(const IndexView& v, const PlanArgs& a, cudaStream_t s) {
     // with a device count the bound may be far above it: a few waves of CTAs
     const uint32_t most = a.d_n_q ? 148u * 16u : 65535u * 16u;
     count_launch();
-    return launch_after(plan_kernel, a.n_q < most ? a.n_q : most, 256, 0, s, v, a);
+    const uint32_t grid = a.n_q < most ? a.n_q : most;
+    auto with = [&](auto given) {
+        if (a.n_inline > sizeof(given.t) / 4u) return cudaErrorInvalidValue;
+        given.n = a.n_inline;
+        std::memcpy(given.t, a.inline_terms, a.n_inline * 4u);
+        return launch_after(plan_kernel<sizeof(given.t) / 4u>, grid, 256, 0, s, v, a, given);
+    };
+    if (!a.inline_terms) return launch_after(plan_kernel<0>, grid, 256, 0, s, v, a, InlineTerms<0>{});
+    return a.n_inline <= kInlineSmall ? with(InlineTerms<kInlineSmall>()) : with(InlineTerms<kInlineLarge>());
 }
 
 cudaError_t launch_queue_scan(const QueueArgs& a, cudaStream_t s) {

@@ -317,6 +317,10 @@ void derive_tables(const HostIndex& h, uint32_t dense_div, int n_threads, Derive
         out->plain_term.push_back(t);
         out->plain_off.push_back(uint32_t(units));
     }
+    out->max_bare_len = 0;
+    for (uint32_t t = 0; t < h.n_terms; ++t)
+        if (out->term_dense[t] == kNone && out->term_plain[t] == kNone)
+            out->max_bare_len = std::max(out->max_bare_len, h.term_len[t]);
     std::vector<uint32_t> dir_terms;
     for (uint32_t t = 0; t < h.n_terms; ++t) {
         if (out->term_dense[t] != kNone) continue;

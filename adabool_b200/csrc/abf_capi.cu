@@ -293,7 +293,7 @@ void free_device(abf_index* ix) {
     dev_free(d.dir);
     dev_free(d.term_info);
     free_plain(ix);
-    dev_free(d.term_cbytes);
+    dev_free(d.term_feat);
     dev_free(d.planner);
     d.bytes = 0;
     ix->on_device = false;
@@ -332,13 +332,21 @@ abf_status make_plain(abf_index* ix, const abf::DerivedHost& h) {
     return ABF_OK;
 }
 
-// The plan kernel's table, from the tables above (synchronises).
+// The plan kernel's tables, from the arrays above (synchronises).
 abf_status make_term_info(abf_index* ix, const abf::DerivedHost& h) {
-    if (!ix->dev.term_info) ABF_TRY(dev_alloc(&ix->dev.term_info, ix->n_terms, &ix->dev.bytes));
+    auto& d = ix->dev;
+    uint32_t* cbytes = nullptr;  // only the first time: a list's blocks do not change
+    if (!d.term_info) ABF_TRY(dev_alloc(&d.term_info, ix->n_terms, &d.bytes));
+    if (!d.term_feat) {
+        ABF_TRY(dev_alloc(&d.term_feat, ix->n_terms, &d.bytes));
+        ABF_TRY(upload_vec(&cbytes, cbytes32(ix), nullptr));
+    }
     abf::IndexView v = abf::view_of(ix);
-    v.n_plain = ix->dev.plain ? h.n_plain() : 0u;
-    CUDA_TRY(abf::launch_term_info(v, ix->dev.term_info, ix->sm_count, nullptr));
-    CUDA_TRY(cudaStreamSynchronize(nullptr));
+    v.n_plain = d.plain ? h.n_plain() : 0u;
+    cudaError_t e = abf::launch_term_info(v, d.term_info, d.term_feat, cbytes, ix->sm_count, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    dev_free(cbytes);
+    CUDA_TRY(e);
     return ABF_OK;
 }
 
@@ -370,7 +378,6 @@ abf_status upload(abf_index* ix, int device) {
         (st = upload_vec(&d.dense, ix->derived.dense, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.term_dir, ix->derived.term_dir, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.dir, ix->derived.dir, &d.bytes)) != ABF_OK ||
-        (st = upload_vec(&d.term_cbytes, cbytes32(ix), &d.bytes)) != ABF_OK ||
         (st = make_plain(ix, ix->derived)) != ABF_OK || (st = make_term_info(ix, ix->derived)) != ABF_OK) {
         free_device(ix);
         return st;
@@ -558,7 +565,16 @@ abf_tuning tile_shape(const abf_index* ix, uint64_t n_q) {
     return t;
 }
 
-// The bin kernel merges plain lists beside the dense group kernel. An item
+// Lists that HYBRID merges: with plain ids by the bin kernel, the others (and
+// TILE's short ones) by the merge kernel.
+bool hybrid_bins(const abf_index* ix) {
+    return ix->dev.plain && ix->derived.max_other_len >= ix->tuning.heavy_min_len;
+}
+bool hybrid_tiles(const abf_index* ix) {
+    return (ix->dev.plain ? ix->derived.max_bare_len : ix->derived.max_other_len) >= ix->tuning.heavy_min_len;
+}
+
+// Beside the dense group kernel the bin kernel merges all plain lists. An item
 // moves a tile's 64 KB in and out at most, the scatter kernel a 32-byte sector
 // in and out per posting once the batch's bitmaps exceed L2: a query's lists
 // are binned from 16 blocks of 128 postings per tile on.
@@ -666,10 +682,11 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.probe_bm = ws->probe_bm;
     pa.probe_stride = ws->probe_stride;
     abf::QueueArgs qa{ws->lcnt, ws->lpref_q, b->n_queries};
-    const bool bins = group && v.n_plain > 0;
+    const bool hybrid = b->d_paths || b->path == ABF_PATH_AUTO || b->path == ABF_PATH_HYBRID || b->path == ABF_PATH_TILE;
+    const bool bins = v.n_plain > 0 && (group || b->path == ABF_PATH_TILE || b->d_paths || (hybrid && hybrid_bins(ix)));
     if (bins) {
         pa.bin_list = ws->bin_list;
-        pa.bin_min_blocks = bin_min_blocks(n_words);
+        pa.bin_min_blocks = group ? bin_min_blocks(n_words) : 0xffffffffu;
         pa.q_nbin = ws->q_nbin;
         pa.q_bblk = ws->q_bblk;
         qa.q_nbin = ws->q_nbin;
@@ -696,10 +713,8 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     TIMED(K_PLAN, abf::launch_plan(v, pa, s));
     if (!pa.done) TIMED(K_QUEUE, abf::launch_queue_scan(qa, s));
     // the merge kernel has work only where a query can merge a list that has
-    // no dense bitmap: never on UNION and PROBE
-    const bool may_merge = b->d_paths || b->path == ABF_PATH_TILE ||
-                           ((b->path == ABF_PATH_AUTO || b->path == ABF_PATH_HYBRID) &&
-                            ix->derived.max_other_len >= t.heavy_min_len);
+    // neither a dense bitmap nor plain ids: never on UNION and PROBE
+    const bool may_merge = b->d_paths || b->path == ABF_PATH_TILE || (hybrid && hybrid_tiles(ix));
     // the probe queries' term bitmaps are written by their plan CTAs
     const bool maybe_probe = ws->probe_cap > 0 && (b->d_paths || b->path == ABF_PATH_PROBE || b->path == ABF_PATH_AUTO);
     abf::TileArgs ta{};
@@ -907,8 +922,8 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     pa.q_off = r.q_off;
     pa.n_q = r.n_q;
     pa.d_n_q = r.d_n_q;
-    const bool merge = r.stream && ix->derived.max_other_len >= t.heavy_min_len;
-    pa.path_uniform = merge ? ABF_PATH_HYBRID : ABF_PATH_UNION;
+    const bool merge = r.stream && hybrid_tiles(ix);
+    pa.path_uniform = r.stream ? ABF_PATH_HYBRID : ABF_PATH_UNION;
     pa.hybrid_min = t.heavy_min_len;
     pa.term_slot = w->d_tslot;
     pa.q_light_cnt = w->d_lcnt;
@@ -941,10 +956,10 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     // (the count of finished plan CTAs is zero when a run ends)
     if (merge) CUDA_TRY(cudaMemsetAsync(w->d_n_tile_list, 0, sizeof(uint32_t), s));
     abf::QueueArgs qa{w->d_lcnt, w->d_lpref_q, r.n_q, r.d_n_q};
-    const bool bins = group && v.n_plain > 0;
+    const bool bins = (group && v.n_plain > 0) || (r.stream && hybrid_bins(ix));
     if (bins) {
         pa.bin_list = w->d_bin_list;
-        pa.bin_min_blocks = bin_min_blocks(n_words);
+        pa.bin_min_blocks = group ? bin_min_blocks(n_words) : 0xffffffffu;
         pa.q_nbin = w->d_nbin;
         pa.q_bblk = w->d_bblk;
         qa.q_nbin = w->d_nbin;

@@ -96,6 +96,7 @@ struct DerivedHost {
     uint32_t dir_n = 0;                 // entries per list: ceil(n_ads / 2^kDirShift) + 1
     uint32_t n_dir = 0;
     uint32_t max_other_len = 0;         // longest list without a dense bitmap
+    uint32_t max_bare_len = 0;          // and without plain ids
     std::vector<uint32_t> term_plain;   // n_terms: plain list index or kNone
     std::vector<uint32_t> plain_term;   // n_plain: its term
     std::vector<uint32_t> plain_off;    // n_plain + 1: first id in the plain ids, in units of 4
@@ -109,6 +110,13 @@ inline uint32_t plain_min_len(uint32_t n_ads) {
     const uint32_t m = n_ads / 32768u;
     return m > 256u ? m : 256u;
 }
+
+// What the planner's features need of a term beside its table entry.
+struct alignas(16) TermFeat {
+    double log_miss;   // log1p(-min(postings / n_ads, 0.999999)): log of the share of ads without it
+    uint32_t cbytes;   // compressed bytes of its list
+    uint32_t pad;
+};
 
 // Device copies of the same arrays.
 struct DeviceIndex {
@@ -129,7 +137,7 @@ struct DeviceIndex {
     uint32_t* plain_off = nullptr;
     uint32_t* plain = nullptr;        // ids
     uint32_t* plain_dir = nullptr;    // n_plain x plain_dir_n positions in `plain`
-    uint32_t* term_cbytes = nullptr;  // compressed bytes per term (planner feature)
+    TermFeat* term_feat = nullptr;    // planner features per term
     float* planner = nullptr;         // planner parameters (ABF_PLANNER_PARAMS) or null
     uint64_t bytes = 0;
 };
@@ -147,7 +155,7 @@ struct IndexView {
     const uint32_t* dense;
     const uint32_t* term_dir;
     const uint32_t* dir;
-    const uint32_t* term_cbytes;
+    const TermFeat* term_feat;
     const abf_u4* term_info;
     const uint32_t* term_plain;
     const uint32_t* plain;

@@ -324,9 +324,9 @@ __device__ __forceinline__ void queue_scan_body(const QueueArgs& a, uint32_t n_q
     if (!a.q_bblk) return;
     // The bin kernel's items: every tile x every part of every query. A query
     // is cut into parts by its lists so that no item has much more than half
-    // an even share of the work (or 128 blocks).
+    // an even share of the work (or 64 blocks).
     sum = block_sum_u64<NT>(sum, s64);
-    const uint64_t lim64 = max(128ull, static_cast<unsigned long long>(sum) / (2ull * a.slots)) * a.n_tiles;
+    const uint64_t lim64 = max(64ull, static_cast<unsigned long long>(sum) / (2ull * a.slots)) * a.n_tiles;
     const uint32_t lim = lim64 < 0xffffffffull ? uint32_t(lim64) : kFull;
     uint32_t pc = 0;
     for (uint32_t c0 = 0; c0 < n_q; c0 += NT) {
@@ -405,7 +405,8 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
         };
         auto blocks_of = [](uint32_t len) { return (len + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS; };
         uint32_t path = a.paths ? a.paths[q] : a.path_uniform;
-        if (path == ABF_PATH_AUTO && a.planner) {
+        const bool planned = path == ABF_PATH_AUTO && a.planner;
+        if (planned) {
             // learned planner: features + MLP of this query, inline
             path = plan_dev::planner_path(ix, a.terms, a.q_off, q, plan_dev::FeatCtx{a.hybrid_min, a.n_postings, a.n_q},
                                           s_pl);
@@ -471,19 +472,34 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
         const uint32_t hm = path == ABF_PATH_TILE ? 0u
                             : path == ABF_PATH_HYBRID ? a.hybrid_min
                             : probe ? kNoHeavy : kDenseOnly;
-        bool bin = false;
+        // shortest plain list that the bin kernel takes: any, where the query
+        // holds enough of them; else those that the path merges
+        uint32_t bin_from = kNone;
         if (a.bin_list) {
-            uint64_t nb = 0;
-            for (uint64_t c0 = qb; c0 < qe && !probe; c0 += kStep) {
-                uint4 e[kPlanTerms];
-                load_step(c0, e);
+            uint64_t nb = 0, nh = 0;  // blocks of the plain lists, and of those the path merges
+            if (planned) {  // added up with the features
+                nb = s_pl.blocks[0];
+                nh = path == ABF_PATH_HYBRID ? s_pl.blocks[1] : 0u;
+            } else {
+                for (uint64_t c0 = qb; c0 < qe; c0 += kStep) {
+                    uint4 e[kPlanTerms];
+                    load_step(c0, e);
 #pragma unroll
-                for (uint32_t k = 0; k < kPlanTerms; ++k)
-                    if (e[k].w != kNone) nb += blocks_of(e[k].y);
+                    for (uint32_t k = 0; k < kPlanTerms; ++k)
+                        if (e[k].w != kNone) {
+                            nb += blocks_of(e[k].y);
+                            if (e[k].y >= hm) nh += blocks_of(e[k].y);
+                        }
+                }
+                nb = block_sum_u64<256>(nb, s_red);
+                nh = block_sum_u64<256>(nh, s_red);
             }
-            nb = block_sum_u64<256>(nb, s_red);
-            bin = nb >= a.bin_min_blocks && nb < 0xffffffffull;
-            if (tid == 0) a.q_bblk[q] = bin ? uint32_t(nb) : 0u;
+            if (probe) nb = nh = 0;
+            if (nb < 0xffffffffull) {
+                if (nb >= a.bin_min_blocks) bin_from = 0;
+                else if (nh) bin_from = hm;
+            }
+            if (tid == 0) a.q_bblk[q] = bin_from == kNone ? 0u : uint32_t(bin_from ? nh : nb);
         }
         uint32_t carry = 0, nmerge = 0;
         for (uint64_t c0 = qb; c0 < qe; c0 += kStep) {
@@ -499,7 +515,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
                 if (i < qe && !probe && e[k].y) {
                     if (d != kNone) {
                         if (want_d) atomicOr(&s_mask[d >> 5], 1u << (d & 31u));
-                    } else if (bin && e[k].w != kNone) {
+                    } else if (e[k].w != kNone && e[k].y >= bin_from) {
                         a.bin_list[qb + atomicAdd(&s_nbin, 1u)] = e[k].w;
                     } else if (e[k].y >= hm) {
                         cls = a.terms[i];
@@ -549,7 +565,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
             }
         }
         if (tid == 0) {
-            if (a.bin_list) a.q_nbin[q] = bin ? s_nbin : 0u;  // the scans' barriers order the last add
+            if (a.bin_list) a.q_nbin[q] = s_nbin;  // the scans' barriers order the last add
             a.q_light_cnt[q] = carry;
             if (a.path_out) a.path_out[q] = uint8_t(path);
         }
@@ -1399,10 +1415,17 @@ __global__ void __launch_bounds__(256) plain_ids_kernel(IndexView ix, const uint
     }
 }
 
-// the plan kernel's table: per term {first block, postings, dense bitmap, plain list}
-__global__ void __launch_bounds__(256) term_info_kernel(IndexView ix, uint4* info) {
-    for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < ix.n_terms; t += gridDim.x * 256u)
-        info[t] = make_uint4(ix.term_blk[t], ix.term_len[t], ix.term_dense[t], ix.n_plain ? ix.term_plain[t] : kNone);
+// The plan kernel's tables: per term {first block, postings, dense bitmap,
+// plain list}, and what the planner's features add up (cbytes: compressed
+// bytes, null: left as they are).
+__global__ void __launch_bounds__(256) term_info_kernel(IndexView ix, uint4* info, TermFeat* feat,
+                                                        const uint32_t* cbytes) {
+    const double inv_ads = 1.0 / double(ix.n_ads);
+    for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < ix.n_terms; t += gridDim.x * 256u) {
+        const uint32_t len = ix.term_len[t];
+        info[t] = make_uint4(ix.term_blk[t], len, ix.term_dense[t], ix.n_plain ? ix.term_plain[t] : kNone);
+        if (cbytes) feat[t] = TermFeat{log1p(-fmin(double(len) * inv_ads, 0.999999)), cbytes[t], 0u};
+    }
 }
 
 // position in the plain ids of each list's first id at or past every tile start
@@ -2082,7 +2105,7 @@ IndexView view_of(const abf_index* ix) {
     v.dense = ix->dev.dense;
     v.term_dir = ix->dev.term_dir;
     v.dir = ix->dev.dir;
-    v.term_cbytes = ix->dev.term_cbytes;
+    v.term_feat = ix->dev.term_feat;
     v.term_plain = ix->dev.term_plain;
     v.term_info = reinterpret_cast<const uint4*>(ix->dev.term_info);
     v.plain = ix->dev.plain;
@@ -2341,8 +2364,9 @@ cudaError_t launch_bin_acc(const IndexView& v, const BinArgs& a, int sm_count, c
 }
 }  // namespace
 
-cudaError_t launch_term_info(const IndexView& v, uint4* info, int sm_count, cudaStream_t s) {
-    term_info_kernel<<<sm_count * 8, 256, 0, s>>>(v, info);
+cudaError_t launch_term_info(const IndexView& v, uint4* info, TermFeat* feat, const uint32_t* cbytes, int sm_count,
+                             cudaStream_t s) {
+    term_info_kernel<<<sm_count * 8, 256, 0, s>>>(v, info, feat, cbytes);
     count_launch();
     return cudaGetLastError();
 }

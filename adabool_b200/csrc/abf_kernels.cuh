@@ -141,7 +141,8 @@ struct PlanArgs {
     uint32_t* q_ndense;       // out: per query, distinct dense bitmaps
     const uint32_t* d_n_q;    // optional device count of queries (at most n_q)
     // optional binning (bin_list set): lists with plain ids go to the bin
-    // kernel, in queries where they hold at least bin_min_blocks blocks in all
+    // kernel in queries where they hold at least bin_min_blocks blocks in all,
+    // and else those that the path merges (HYBRID, TILE)
     uint32_t* bin_list;       // out: from slot q_off[q] on, their plain list indices
     uint32_t* q_nbin;         // out: per query, such lists
     uint32_t* q_bblk;         // out: per query, their blocks
@@ -343,7 +344,8 @@ cudaError_t launch_tile_union(const IndexView& v, const TileArgs& a, const abf_t
                               cudaStream_t s);
 cudaError_t launch_scatter(const IndexView& v, const ScatterArgs& a, const abf_tuning& t, int sm_count,
                            cudaStream_t s);
-cudaError_t launch_term_info(const IndexView& v, uint4* info, int sm_count, cudaStream_t s);
+cudaError_t launch_term_info(const IndexView& v, uint4* info, TermFeat* feat, const uint32_t* cbytes, int sm_count,
+                             cudaStream_t s);
 // ids and positions of the plain lists (IndexView::plain, plain_dir) from the blocks
 cudaError_t launch_plain_ids(const IndexView& v, const uint32_t* plain_term, const uint32_t* plain_off, uint32_t* plain,
                              uint32_t* plain_dir, int sm_count, cudaStream_t s);

@@ -44,22 +44,32 @@ struct FeatCtx {
     uint32_t n_q;
 };
 
-// The 16 features of query q, computed by the whole CTA (kFeatThreads
+__device__ __forceinline__ TermFeat load_feat(const TermFeat* p) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    return TermFeat{__hiloint2double(int(v.y), int(v.x)), v.z, v.w};
+}
+
+// The 16 features of query q (and its plain lists' blocks), computed by the whole CTA (kFeatThreads
 // threads) into f[] in shared memory. Term ids >= n_terms are skipped;
-// repeated terms count once per occurrence. Each thread takes kFeatUnroll
+// repeated terms count once per occurrence. The logarithm that each term adds
+// is in a table (taken here, four per thread and step of 64-bit arithmetic, it
+// was ~1 us a step: 20,000 terms are 20 steps). Each thread takes kFeatUnroll
 // terms per pass and issues all their table loads before using any, so a
 // query of thousands of terms costs a few memory latencies, not one per term.
 __device__ void query_features(const IndexView& ix, const uint32_t* terms, const uint64_t* q_off, uint32_t q,
-                               const FeatCtx& c, float* f) {
+                               const FeatCtx& c, float* f, unsigned long long* blocks = nullptr) {
+    __shared__ unsigned long long s_b[2][kFeatThreads / 32];
     __shared__ double s_d[6][kFeatThreads / 32];
     __shared__ uint32_t s_u[4][kFeatThreads / 32];
     const uint64_t qb = q_off[q], qe = q_off[q + 1];
     uint32_t n = 0, mx = 0, nd = 0, nl = 0;
+    unsigned long long pb = 0, pm = 0;  // blocks of the plain lists, and of those HYBRID merges
     double S = 0, Q = 0, Cb = 0, Lg = 0, Sd = 0, Bnd = 0;
     const double inv_ads = 1.0 / double(ix.n_ads);
     for (uint64_t i0 = qb + threadIdx.x; i0 < qe; i0 += uint64_t(kFeatThreads) * kFeatUnroll) {
-        uint32_t t[kFeatUnroll], cb[kFeatUnroll];
+        uint32_t t[kFeatUnroll];
         uint4 e[kFeatUnroll];  // {first block, postings, dense bitmap, plain list}
+        TermFeat w[kFeatUnroll];
 #pragma unroll
         for (int u = 0; u < kFeatUnroll; ++u) {
             const uint64_t i = i0 + uint64_t(u) * kFeatThreads;
@@ -69,7 +79,7 @@ __device__ void query_features(const IndexView& ix, const uint32_t* terms, const
         for (int u = 0; u < kFeatUnroll; ++u) {
             const bool ok = t[u] < ix.n_terms;
             e[u] = ok ? __ldg(ix.term_info + t[u]) : make_uint4(0u, 0u, kNone, kNone);
-            cb[u] = ok ? __ldg(ix.term_cbytes + t[u]) : 0u;
+            w[u] = ok ? load_feat(ix.term_feat + t[u]) : TermFeat{0.0, 0u, 0u};
         }
 #pragma unroll
         for (int u = 0; u < kFeatUnroll; ++u) {
@@ -79,14 +89,19 @@ __device__ void query_features(const IndexView& ix, const uint32_t* terms, const
             mx = max(mx, len);
             S += len;
             Q += double(len) * len;
-            Cb += cb[u];
-            Lg += log1p(-fmin(double(len) * inv_ads, 0.999999));
+            Cb += w[u].cbytes;
+            Lg += w[u].log_miss;
             if (e[u].z != kNone) {
                 ++nd;
                 Sd += len;
             } else {
-                Bnd += (len + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS;
+                const uint32_t nb = (len + ABF_BLOCK_POSTINGS - 1u) / ABF_BLOCK_POSTINGS;
+                Bnd += nb;
                 if (len < c.hybrid_min) ++nl;
+                if (e[u].w != kNone) {
+                    pb += nb;
+                    if (len >= c.hybrid_min) pm += nb;
+                }
             }
         }
     }
@@ -101,11 +116,21 @@ __device__ void query_features(const IndexView& ix, const uint32_t* terms, const
     Lg = warp_sum(Lg);
     Sd = warp_sum(Sd);
     Bnd = warp_sum(Bnd);
+    if (blocks) {
+        pb = warp_sum(pb);
+        pm = warp_sum(pm);
+    }
     if (lane() == 0) {
+        s_b[0][w] = pb; s_b[1][w] = pm;
         s_u[0][w] = n; s_u[1][w] = nd; s_u[2][w] = nl; s_u[3][w] = mx;
         s_d[0][w] = S; s_d[1][w] = Q; s_d[2][w] = Cb; s_d[3][w] = Lg; s_d[4][w] = Sd; s_d[5][w] = Bnd;
     }
     __syncthreads();
+    if (blocks && threadIdx.x >= 32 && threadIdx.x < 34) {
+        unsigned long long t = 0;
+        for (int k = 0; k < kFeatThreads / 32; ++k) t += s_b[threadIdx.x - 32][k];
+        blocks[threadIdx.x - 32] = t;
+    }
     // each of the first 16 threads sums the warps' partials and computes one
     // feature (the transcendentals run side by side, not one after another)
     if (threadIdx.x < F) {
@@ -183,6 +208,7 @@ constexpr int kParamVecs = (kNParams + 3) / 4;
 struct PlannerSmem {
     float4 p4[kParamVecs];
     float f[F], xs[F], h1[H], h2[H], y[O];
+    unsigned long long blocks[2];  // of the query's plain lists, and of those HYBRID merges
     __device__ const float* p() const { return reinterpret_cast<const float*>(p4); }
 };
 
@@ -242,7 +268,7 @@ __device__ __forceinline__ void mlp_forward_smem(PlannerSmem& sm) {
 __device__ __forceinline__ uint32_t planner_path(const IndexView& ix, const uint32_t* terms, const uint64_t* q_off,
                                                  uint32_t q, const FeatCtx& c, PlannerSmem& sm) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    query_features(ix, terms, q_off, q, c, sm.f);  // ends with a barrier: every thread's copies are there
+    query_features(ix, terms, q_off, q, c, sm.f, sm.blocks);  // ends with a barrier: every thread's copies are there
     if (threadIdx.x < F) {
         const float sd = sm.p()[kSd + threadIdx.x];
         sm.xs[threadIdx.x] = (sm.f[threadIdx.x] - sm.p()[kMu + threadIdx.x]) / (sd > 0.0f ? sd : 1.0f);

@@ -2121,28 +2121,6 @@ IndexView view_of(const abf_index* ix) {
     return v;
 }
 
-namespace {
-// A launch that may come up while the kernel before it on the stream finishes
-// (see wait_previous). With the counters, marks and look-back words zeroed by
-// the plan kernel instead of memsets, the scan in its last CTA and one upload,
-// a single query has 6 nodes on the stream instead of 13: 56 -> 33 us on c0,
-// 95 -> 68 on c1 with the planner.
-template <typename... P, typename... A>
-cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-}  // namespace
-
 uint32_t compact_chunks(uint64_t n_bits, uint32_t units) {
     const uint64_t n_words = (n_bits + 31) / 32, chunk = units * 32u * kCompactWarps;
     return uint32_t((n_words + chunk - 1) / chunk);

@@ -101,11 +101,12 @@ __global__ void mask_sum_kernel(const float* mask, uint64_t n, float* out) {
 // shuffle reduction that leaves one (sample, output) pair per thread.
 // Gradients are accumulated without the 1 / sum(mask) factor, so everything
 // up to the final adds runs before the wait on the kernel that zeroes g and
-// counts the mask.
+// counts the mask. (That kernel lets this one start only after its own wait,
+// so the parameters and the batch are there.)
 // One sample per 64-thread CTA at a time, with every weight read through L1
 // and 5,443 atomics from each of 1,184 CTAs, took 247.8 us for 8,192 samples;
-// this kernel takes 20.2 us (12.9 TFLOP/s with its 128 tiles on 148 SMs), and
-// a whole step (this, the launch before it and Adam) 24.6 us instead of 256.
+// this kernel takes about 18 us with its 128 tiles on 148 SMs, and a whole step (this,
+// the launch before it and Adam, each launched early) 18.3 us instead of 256.
 constexpr int kTS = 64;        // samples per tile
 constexpr int kLd = H + 4;     // row stride: the two rows a warp reads start 16 banks apart
 constexpr int kLdX = F + 4;
@@ -162,12 +163,13 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_kernel(const float* 
     GradSmem& sm = *reinterpret_cast<GradSmem*>(g_smem);
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, wp = tid >> 5;
     const int c0 = tx * 4, s0 = ty * 4;  // this thread's units and samples
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (int i = tid; i < H * F; i += kGradThreads) sm.w1t[i % F][i / F] = p[kW1 + i];
-    {
-        const int i = tid & (H - 1);  // unit of layer 2: consecutive lanes write consecutive words of w2t
-        for (int k = tid / H; k < H; k += kGradThreads / H) sm.w2t[k][i] = p[kW2 + i * H + k];
+    for (int i = tid; i < H * H; i += kGradThreads) {
+        const float v = p[kW2 + i];
+        sm.w2[i / H][i % H] = v;
+        sm.w2t[i % H][i / H] = v;
     }
-    for (int i = tid; i < H * H; i += kGradThreads) sm.w2[i / H][i % H] = p[kW2 + i];
     for (int i = tid; i < O * H; i += kGradThreads) sm.w3[i / H][i % H] = p[kW3 + i];
     if (tid < H) {
         sm.b1[tid] = p[kB1 + tid];
@@ -363,6 +365,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_kernel(const float* 
 
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
                             float c1, float c2) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int i = kW1 + blockIdx.x * blockDim.x + threadIdx.x; i < kNParams; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -411,32 +414,22 @@ cudaError_t launch_mlp_grad(const float* p, const float* x, const float* t, cons
         mask_sum_kernel<<<grid_of(uint32_t((uint64_t(n) * O + 255) / 256), 256u), 256, 0, s>>>(mask, uint64_t(n) * O,
                                                                                                 loss2 + 1);
     } else {
-        grad_init_kernel<<<1, 1024, 0, s>>>(mask, n * O, g, loss2);
+        e = launch_after(grad_init_kernel, 1, 1024, 0, s, mask, n * O, g, loss2);
+        if (e != cudaSuccess) return e;
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(grid_of((n + kTS - 1) / kTS, 148u)));
-    cfg.blockDim = dim3(kGradThreads);
-    cfg.dynamicSmemBytes = sizeof(GradSmem);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, mlp_grad_kernel, p, x, t, mask, n, g, loss2);
     count_launch(2);
-    return e;
+    return launch_after(mlp_grad_kernel, uint32_t(grid_of((n + kTS - 1) / kTS, 148u)), kGradThreads, sizeof(GradSmem), s,
+                        p, x, t, mask, n, g, loss2);
 }
 
 cudaError_t launch_adam(float* p, const float* g, float* m, float* v, uint32_t step, float lr, float b1, float b2,
                         float eps, cudaStream_t s) {
     const float c1 = 1.0f - std::pow(b1, float(step ? step : 1));
     const float c2 = 1.0f - std::pow(b2, float(step ? step : 1));
-    adam_kernel<<<(kNParams + 255) / 256, 256, 0, s>>>(p, g, m, v, lr, b1, b2, eps, c1, c2);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(adam_kernel, (kNParams + 255) / 256, 256, 0, s, p, g, m, v, lr, b1, b2, eps, c1, c2);
 }
 
 }  // namespace abf

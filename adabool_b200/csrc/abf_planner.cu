@@ -105,8 +105,8 @@ __global__ void mask_sum_kernel(const float* mask, uint64_t n, float* out) {
 // so the parameters and the batch are there.)
 // One sample per 64-thread CTA at a time, with every weight read through L1
 // and 5,443 atomics from each of 1,184 CTAs, took 247.8 us for 8,192 samples;
-// this kernel takes about 18 us with its 128 tiles on 148 SMs, and a whole step (this,
-// the launch before it and Adam, each launched early) 18.3 us instead of 256.
+// here a whole step (this kernel with its 128 tiles on 148 SMs, the launch before
+// it and Adam, each launched early) takes 18.3 us instead of 256.
 constexpr int kTS = 64;        // samples per tile
 constexpr int kLd = H + 4;     // row stride: the two rows a warp reads start 16 banks apart
 constexpr int kLdX = F + 4;

@@ -397,12 +397,13 @@ def run_ours(args, rank, world, dev):
     # ---- physical bytes per kernel (roofline numerators) ----
     # every kernel is charged the bytes its design must move once: the dense
     # group kernel reads each dense bitmap once per launch and writes the
-    # bitmaps of the queries it covers; the merge kernel reads the blocks of
-    # the merged lists that have no dense bitmap (and, with the group kernel
-    # on, reads back and rewrites the tiles of the queries that have such
-    # lists); the scatter kernel reads the blocks of the scattered lists and
-    # read-modify-writes one 4-byte word per posting; the compaction reads
-    # each bitmap once and writes 4 bytes per id
+    # bitmaps of the queries it covers; the dense stream kernel reads every
+    # query's dense bitmaps and writes all bitmaps; the bin kernel reads the
+    # plain ids of the lists merged per tile and reads back and rewrites the
+    # bitmaps of the queries that have any; the tile kernel does the same from
+    # blocks for lists without plain ids; the scatter kernel reads the blocks
+    # of the scattered lists and read-modify-writes one 4-byte word per
+    # posting; the compaction reads each bitmap once and writes 4 bytes per id
     bm_bytes = L.n_ads / 8.0
     st = ix.stats()  # after tuning (the dense bitmaps follow dense_div)
     lbytes = ix.list_bytes().astype(np.float64)
@@ -420,22 +421,29 @@ def run_ours(args, rank, world, dev):
         return np.where(empty, 0.0, np.add.reduceat(x.astype(np.float64), seg))
 
     qt_m, qt_d = merged_t[qterms], dense_t[qterms]
-    q_merge_nd = per_query(np.where(qt_m & ~qt_d, lbytes[qterms], 0.0))       # merged from blocks
-    q_merge_nd_n = per_query((qt_m & ~qt_d).astype(np.float64))
-    q_dense_n = per_query((qt_m & qt_d).astype(np.float64))                   # merged dense lists
-    q_scat = per_query(np.where(~qt_m, lbytes[qterms], 0.0))
-    q_scat_post = per_query(np.where(~qt_m, lens[qterms], 0).astype(np.float64))
+    # lists merged from plain ids: those without a dense bitmap of at least
+    # max(256, n_ads / 32768) postings, for a query with 16 of their blocks per
+    # 16,384-word tile beside the group kernel, else only the hybrid path's
+    plain_t = ~dense_t & (lens >= max(256, L.n_ads // 32768)) if "bin_union" in kern else np.zeros_like(dense_t)
     group_on = "dense_group" in kern
+    q_blk = per_query(np.where(plain_t[qterms], (lens[qterms] + 127) // 128, 0))
+    wide = q_blk >= 16 * -(-L.n_ads // (32 * 16384)) if group_on else np.zeros(n_q, bool)
+    bin_e = plain_t[qterms] & (np.repeat(wide, np.diff(qoff).astype(np.int64)) | qt_m)
+    q_bin = per_query(np.where(bin_e, 4.0 * lens[qterms], 0.0))               # merged from plain ids
+    tile_e = qt_m & ~qt_d & ~bin_e
+    q_tile = per_query(np.where(tile_e, lbytes[qterms], 0.0))                 # merged from blocks
+    q_dense_n = per_query((qt_m & qt_d).astype(np.float64))                   # merged dense lists
+    scat_e = ~qt_m & ~bin_e
+    q_scat = per_query(np.where(scat_e, lbytes[qterms], 0.0))
+    q_scat_post = per_query(np.where(scat_e, lens[qterms], 0).astype(np.float64))
     alg = {"scatter_union": float(q_scat.sum() + 8.0 * q_scat_post.sum()),
+           "bin_union": float(q_bin.sum()) + 2.0 * bm_bytes * float((q_bin > 0).sum()),
+           "tile_union": float(q_tile.sum()) + 2.0 * bm_bytes * float((q_tile > 0).sum()),
+           "dense_stream": float(q_dense_n.sum()) * bm_bytes + n_q * bm_bytes,
            "compact": n_q * bm_bytes + 4.0 * float(counts.sum())}
-    dense_only = (q_merge_nd_n == 0) & ~empty
     if group_on:
-        g_launches = kern["dense_group"][0] / args.steps
-        alg["dense_group"] = g_launches * float(st["dense_bytes"]) + float((~empty).sum()) * bm_bytes
-        alg["tile_union"] = float(q_merge_nd[~dense_only & ~empty].sum()) + \
-            2.0 * bm_bytes * float((~dense_only & ~empty).sum()) + bm_bytes * float(empty.sum())
-    else:
-        alg["tile_union"] = float(q_merge_nd.sum() + q_dense_n.sum() * bm_bytes) + n_q * bm_bytes
+        alg["dense_group"] = kern["dense_group"][0] / args.steps * float(st["dense_bytes"]) + n_q * bm_bytes
+    alg = {k: v for k, v in alg.items() if k in kern}
     hbm, peak_kind = peaks()
     cs = clk.summary()
     sm_mhz = (cs or {}).get("sm_mhz") or 1965.0
@@ -470,7 +478,7 @@ def run_ours(args, rank, world, dev):
         sc["postings_per_step"] = float(q_scat_post.sum())
         sc["postings_per_s"] = float(q_scat_post.sum()) * args.steps / (kern["scatter_union"][1] / 1e3)
         sc["bytes_note"] = ("blocks read plus a 4-byte read-modify-write per posting, an upper bound: ORs into "
-                            "tiles the dense group kernel left all ones are skipped")
+                            "tiles left all ones before are skipped")
     dom = max(per_kernel, key=lambda k: per_kernel[k]["ms_per_step"]) if per_kernel else None
     roof = None
     if dom and "achieved_gbs" in per_kernel[dom]:

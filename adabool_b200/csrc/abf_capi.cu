@@ -120,6 +120,7 @@ struct ProfScope {
 struct abf_workspace {
     abf_index* ix = nullptr;
     void* arena = nullptr;          // the one allocation behind every pointer below
+    size_t arena_bytes = 0;
     uint32_t max_q = 0;
     uint64_t max_terms = 0;
     uint32_t probe_cap = 0;
@@ -163,6 +164,8 @@ struct abf_worker {
     abf_index* ix = nullptr;
     int kind = 0;  // 0 sparse, 1 dense (host bitmaps copied), 2 dense (caller device bitmaps)
     void* arena = nullptr;          // the one allocation behind every pointer below but d_ext
+    size_t arena_bytes = 0;
+    bool scan = false;              // dense, no memory for the lists: answered by the scan of the index
     // the lists to merge: sparse, the keys as given; dense, the terms of a
     // window of query bitmaps, extracted when the worker runs
     uint64_t n_keys = 0;            // sparse
@@ -442,8 +445,70 @@ struct Arena {
     }
 };
 
-void ws_release(abf_workspace* w) {
-    if (w->arena) cudaFree(w->arena);
+// Scratch outlives its workspace or worker in a pool of its index: an
+// allocation above 1 MB and its release cost 600 us (a worker for 32 query
+// bitmaps over 2^18 terms needs 1.5 MB and runs for 110); with the pool the
+// whole prepare and free take 5, a workspace of 256 queries 20 instead of 600.
+// At most kPoolBytes are kept; the rest goes back at once, and all of
+// it when the index is freed or memory runs out. Scratch is kept only after a
+// synchronisation of the device, so any stream may use it next.
+constexpr size_t kPoolBytes = size_t(32) << 20;
+
+void pool_drain(abf_index* ix) {
+    std::lock_guard<std::mutex> g(ix->pool_mu);
+    for (auto& e : ix->pool) cudaFree(e.first);
+    ix->pool.clear();
+    ix->pool_bytes = 0;
+}
+
+// the smallest kept allocation that fits without holding more than twice the bytes (and 1 MB)
+abf_status scratch_alloc(abf_index* ix, size_t bytes, void** p, size_t* got) {
+    {
+        std::lock_guard<std::mutex> g(ix->pool_mu);
+        size_t best = ix->pool.size();
+        for (size_t i = 0; i < ix->pool.size(); ++i) {
+            const size_t b = ix->pool[i].second;
+            if (b >= bytes && b <= 2 * bytes + (1u << 20) && (best == ix->pool.size() || b < ix->pool[best].second)) best = i;
+        }
+        if (best < ix->pool.size()) {
+            *p = ix->pool[best].first;
+            *got = ix->pool[best].second;
+            ix->pool_bytes -= *got;
+            ix->pool.erase(ix->pool.begin() + std::ptrdiff_t(best));
+            return ABF_OK;
+        }
+    }
+    char* c = nullptr;
+    abf_status st = dev_alloc(&c, bytes);
+    if (st != ABF_OK) {
+        cudaGetLastError();  // reported here, not by the next launch
+        pool_drain(ix);
+        st = dev_alloc(&c, bytes);
+        if (st != ABF_OK) {
+            cudaGetLastError();
+            return st;
+        }
+    }
+    *p = c;
+    *got = bytes;
+    return ABF_OK;
+}
+
+void scratch_free(abf_index* ix, void* p, size_t bytes, bool idle = true) {
+    if (!p) return;
+    if (idle) {
+        std::lock_guard<std::mutex> g(ix->pool_mu);
+        if (ix->pool_bytes + bytes <= kPoolBytes) {
+            ix->pool.emplace_back(p, bytes);
+            ix->pool_bytes += bytes;
+            return;
+        }
+    }
+    cudaFree(p);
+}
+
+void ws_release(abf_workspace* w, bool idle = true) {
+    scratch_free(w->ix, w->arena, w->arena_bytes, idle);
     w->arena = nullptr;
 }
 
@@ -486,10 +551,8 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
     Arena a;
     ws_take(w, a, chunks);
-    char* p = nullptr;
-    ABF_TRY(dev_alloc(&p, a.used));
-    w->arena = p;
-    a = Arena{p, 0};
+    ABF_TRY(scratch_alloc(ix, a.used, &w->arena, &w->arena_bytes));
+    a = Arena{static_cast<char*>(w->arena), 0};
     ws_take(w, a, chunks);
     w->n_probe = w->ctl;
     w->n_tile_list = w->ctl + 1;
@@ -846,6 +909,8 @@ constexpr uint32_t kWorkerHead = 8;  // words before the keys: four counters, tw
 
 // arrays of a worker that plans at most n_q queries over w->term_cap terms
 void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
+    if (w->kind == 1) a.take(w->d_qbm, std::max<uint64_t>(w->batch, 1) * w->qbm_stride);
+    if (w->scan) return;
     // counters, offsets and keys in one piece: one upload
     a.take(w->d_nprobe, kWorkerHead + w->term_cap);
     w->d_n_tile_list = w->d_nprobe + 1;
@@ -871,29 +936,40 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     a.take(w->d_ticket, 1);
     if (w->kind == 0) a.take(w->d_slot, n_q);
     else a.take(w->d_cnt, n_q);
-    if (w->kind == 1) a.take(w->d_qbm, std::max<uint64_t>(w->batch, 1) * w->qbm_stride);
 }
 
 abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
     w->sat_stride = sat_words(w->ix);
     Arena a;
     worker_take(w, a, n_q);
-    char* p = nullptr;
-    ABF_TRY(dev_alloc(&p, a.used));
-    w->arena = p;
-    a = Arena{p, 0};
+    // (a worker over the caller's device bitmaps may be prepared while a stream is captured)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (w->kind == 2) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    abf_status st = scratch_alloc(w->ix, a.used, &w->arena, &w->arena_bytes);
+    if (w->kind == 2) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    if (st != ABF_OK && w->kind != 0) {
+        // no room for the lists: the scan needs only the bitmaps
+        w->scan = true;
+        if (w->kind == 2) return ABF_OK;
+        a = Arena{};
+        worker_take(w, a, n_q);
+        st = scratch_alloc(w->ix, a.used, &w->arena, &w->arena_bytes);
+    }
+    if (st != ABF_OK) return st;
+    a = Arena{static_cast<char*>(w->arena), 0};
     worker_take(w, a, n_q);
+    if (w->kind != 0) return ABF_OK;  // the term list kernels zero the counters
     const cudaError_t e = cudaMemset(w->d_nprobe, 0, kWorkerHead * 4u);
     if (e != cudaSuccess) {
-        cudaFree(w->arena);
+        scratch_free(w->ix, w->arena, w->arena_bytes);
         w->arena = nullptr;
         return fail(ABF_ERR_CUDA, std::string("worker: ") + cudaGetErrorString(e));
     }
     return ABF_OK;
 }
 
-void worker_release(abf_worker* w) {
-    if (w->arena) cudaFree(w->arena);
+void worker_release(abf_worker* w, bool idle = true) {
+    scratch_free(w->ix, w->arena, w->arena_bytes, idle);
     w->arena = nullptr;
 }
 
@@ -1139,8 +1215,17 @@ abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_w
     }
     pr.out_stride = res_stride_words;
     pr.chunk_blocks = t.probe_chunk_blocks;
-    pr.err = w->d_err;
     pr.spin_limit = abf::kDefaultSpinLimit;
+    if (w->scan) {
+        abf_workspace* ws = nullptr;
+        ABF_TRY(own_ws(ix, 1, 1, ix->n_ads, &ws));
+        pr.err = ws->err;
+        pr.n_probe_host = uint32_t(w->batch);
+        pr.out = d_res;
+        TIMED(K_PROBE, abf::launch_probe(v, pr, t, ix->sm_count, s));
+        return ABF_OK;
+    }
+    pr.err = w->d_err;
     pr.only_if = w->d_n_q;
     const uint32_t* qbm = pr.qbm;
     for (uint64_t q0 = 0; q0 < w->batch; q0 += kTermWindow) {
@@ -1163,6 +1248,8 @@ abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_w
         la.terms = w->d_keys;
         la.off = w->d_off;
         la.overflow = w->d_n_q;
+        la.zero = w->d_nprobe;
+        la.n_zero = kWorkerHead;
         TIMED(K_PROBE, abf::launch_term_lists(la, s));
         if (t.group_min_queries && r.n_q >= t.group_min_queries) r.group = group_shape(ix, v, r.n_q, 64ull * r.n_q, true);
         r.stream = !r.group.on;
@@ -1248,6 +1335,7 @@ abf_status abf_index_free(abf_index* ix) {
         ws_release(ix->own_ws);
         delete ix->own_ws;
     }
+    pool_drain(ix);
     if (ix->h_stage) cudaFreeHost(ix->h_stage);
     if (ix->stage_event) cudaEventDestroy(static_cast<cudaEvent_t>(ix->stage_event));
     delete static_cast<Profiler*>(ix->prof);
@@ -1532,11 +1620,12 @@ abf_status abf_prepare_batch_device(abf_index* ix, uint64_t batch, uint64_t len,
 abf_status abf_worker_free(abf_worker* w) {
     API_BEGIN
     if (!w) return ABF_OK;
+    bool idle = false;
     if (w->ix && w->ix->on_device) {
         cudaSetDevice(w->ix->device);
-        cudaDeviceSynchronize();
+        idle = cudaDeviceSynchronize() == cudaSuccess;
     }
-    worker_release(w);
+    worker_release(w, idle);
     delete w;
     return ABF_OK;
     API_END
@@ -1668,11 +1757,12 @@ extern "C" {
 abf_status abf_workspace_free(abf_workspace* w) {
     API_BEGIN
     if (!w) return ABF_OK;
+    bool idle = false;
     if (w->ix && w->ix->on_device) {
         cudaSetDevice(w->ix->device);
-        cudaDeviceSynchronize();
+        idle = cudaDeviceSynchronize() == cudaSuccess;
     }
-    ws_release(w);
+    ws_release(w, idle);
     delete w;
     return ABF_OK;
     API_END

@@ -26,6 +26,8 @@
 #include <string>
 #include <vector>
 #include <atomic>
+#include <mutex>
+#include <utility>
 
 #include "../../include/adabool.h"
 
@@ -205,6 +207,10 @@ struct abf_index {
     const void* dense_tmap_base = nullptr;
     uint32_t dense_tmap_rows = 0;
     uint32_t dense_tmap_gw = 0;       // tile words of the boxes (32 or 64)
+    // scratch of freed workspaces and workers (pointer, bytes), for the next ones
+    std::mutex pool_mu;
+    std::vector<std::pair<void*, size_t>> pool;
+    size_t pool_bytes = 0;
 };
 
 namespace abf {

@@ -2,9 +2,9 @@
 
 A batch of up to ``max_queries`` queries (``max_terms`` terms in total) is
 answered by one replay of a CUDA graph that holds the whole of
-``abf_batch_run``: planning, merge tiles, scatter, probe and (optionally)
-compaction -- about ten kernel and memset nodes, launched by the host as a
-single graph launch. The graph is captured by the C ABI
+``abf_batch_run``: planning, dense merge, bins, scatter, probe and (optionally)
+compaction -- about six kernel nodes, launched by the host as a single graph
+launch. The graph is captured by the C ABI
 (``abf_batch_graph_create`` / ``abf_batch_graph_replay``), once for a fixed
 batch size on fixed device buffers; each batch copies its terms/offsets (and
 per-query paths) into those buffers on the executor's stream and replays.

@@ -156,8 +156,8 @@ typedef struct abf_tuning {
                                  dense bitmaps of all their queries in one
                                  pass per 64- or 32-word tile (each tile's slice of every
                                  dense bitmap staged once in shared memory by TMA, then
-                                 ORed per query); needs at most 767 dense bitmaps;
-                                 0 = never */
+                                 ORed per query), and their mid-length lists in 16,384-word
+                                 tiles; needs at most 767 dense bitmaps; 0 = never */
     uint32_t fixed_tile_shape;  /* 0: a batch too small to fill the GPU at tile_words x
                                  warps_per_tile runs the merge kernel with 8-warp CTAs
                                  and tiles narrowed down to 1,024 words; 1: always the
@@ -201,6 +201,10 @@ abf_status abf_index_set_dense_div(abf_index* index, uint32_t dense_div);
 abf_status abf_prepare_sparse(abf_index* index, const uint32_t* keys, uint64_t n_keys,
                               abf_worker** out);
 
+/* Dense workers hold scratch for the terms of up to 256 query bitmaps at a
+ * time (2,048 per query on average; a denser window is answered by a scan of
+ * the index). Scratch of freed workers and workspaces stays with the index,
+ * up to 32 MB, for the next ones. */
 /* Dense worker for one query given as a host term bitmap of len bytes
  * (bit t of byte t/8 set = term t in the query). Replaces
  * ivf_list::Prepare(len, bitmap) (src/AdaBool/inverted_list.h:530-543). */

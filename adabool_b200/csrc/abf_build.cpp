@@ -424,18 +424,53 @@ abf_status load_host(const char* path, HostIndex* h) {
     }
     std::fclose(f);
     if (!ok) return fail(ABF_ERR_IO, std::string("not an index file or truncated: ") + path);
-    // structural checks so a corrupt file cannot send a kernel out of bounds
+    // Checks so that a corrupt file cannot send a kernel out of bounds: the
+    // kernels take a list's blocks from its length (all full but the last),
+    // place them by their terms, search their bounds and write the decoded
+    // ids without looking at any of it again.
+    if (hd.n_terms == 0 || hd.n_ads == 0 || hd.n_terms > (1u << 31) || hd.n_ads > (1u << 31))
+        return fail(ABF_ERR_IO, "index file: bad size");
     if (h->term_blk[0] != 0 || h->term_blk[h->n_terms] != hd.n_blocks || h->payload.empty())
         return fail(ABF_ERR_IO, "index file: inconsistent block table");
     for (uint32_t t = 0; t < h->n_terms; ++t)
         if (h->term_blk[t + 1] < h->term_blk[t]) return fail(ABF_ERR_IO, "index file: term table not monotone");
-    for (uint64_t b = 0; b < hd.n_blocks; ++b) {
-        abf_u2 d = h->blk_desc[b];
-        uint32_t bits = desc_bits(d.y), cnt = desc_count(d.y);
-        if (bits > 32 || cnt > kBlock || uint64_t(d.x) + payload_units(cnt, bits) > hd.n_units ||
-            h->blk_first[b] >= h->n_ads || h->blk_last[b] >= h->n_ads || h->blk_term[b] >= h->n_terms)
-            return fail(ABF_ERR_IO, "index file: bad block descriptor");
+    for (uint32_t t = 0; t < h->n_terms; ++t) {
+        uint64_t n = 0;
+        for (uint32_t b = h->term_blk[t]; b < h->term_blk[t + 1]; ++b) {
+            const uint32_t cnt = desc_count(h->blk_desc[b].y);
+            if (h->blk_term[b] != t || cnt > kBlock || (cnt < kBlock && b + 1 < h->term_blk[t + 1]) ||
+                (b > h->term_blk[t] && h->blk_first[b] <= h->blk_last[b - 1]))
+                return fail(ABF_ERR_IO, "index file: inconsistent list");
+            n += cnt;
+        }
+        if (n != h->term_len[t]) return fail(ABF_ERR_IO, "index file: inconsistent list length");
     }
+    // a block's ids start at blk_first and end at blk_last: its gaps add up to
+    // the difference. The payload's last unit is padding: the decoders read up
+    // to two words past a block's own.
+    std::atomic<bool> bad{false};
+    parallel_for(resolve_threads(0), hd.n_blocks, [&](int, uint64_t b0, uint64_t b1) {
+        for (uint64_t b = b0; b < b1 && !bad; ++b) {
+            const abf_u2 d = h->blk_desc[b];
+            const uint32_t bits = desc_bits(d.y), gaps = desc_count(d.y) - 1;
+            if (bits > 32 || uint64_t(d.x) + payload_units(gaps + 1, bits) >= hd.n_units ||
+                h->blk_last[b] >= h->n_ads || h->blk_first[b] > h->blk_last[b]) {
+                bad = true;
+                return;
+            }
+            uint64_t sum = gaps;
+            if (bits) {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(h->payload.data()) + size_t(d.x) * 4;
+                const uint64_t mask = (1ull << bits) - 1;
+                for (uint32_t s = 0, pos = 0; s < gaps; ++s, pos += bits) {
+                    const uint64_t two = uint64_t(w[pos >> 5]) | uint64_t(w[(pos >> 5) + 1]) << 32;
+                    sum += (two >> (pos & 31)) & mask;
+                }
+            }
+            if (sum != h->blk_last[b] - h->blk_first[b]) bad = true;
+        }
+    });
+    if (bad) return fail(ABF_ERR_IO, "index file: bad block");
     return ABF_OK;
 }
 }  // namespace abf

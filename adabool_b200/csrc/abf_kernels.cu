@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
         const bool planned = path == ABF_PATH_AUTO && a.planner;
         if (planned) {
             // learned planner: features + MLP of this query, inline
-            path = plan_dev::planner_path(ix, a.terms, a.q_off, q, plan_dev::FeatCtx{a.hybrid_min, a.n_postings, a.n_q},
+            path = plan_dev::planner_path(ix, a.terms, qb, qe, q, plan_dev::FeatCtx{a.hybrid_min, a.n_postings, a.n_q},
                                           s_pl);
         } else if (path == ABF_PATH_AUTO) {
             // fixed rule: probe when the query's lists cover more than

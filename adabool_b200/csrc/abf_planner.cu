@@ -28,11 +28,11 @@ __global__ void __launch_bounds__(kFeatThreads) planner_kernel(IndexView ix, con
     if (p) load_params(p, sm);
     for (uint32_t q = blockIdx.x; q < c.n_q; q += gridDim.x) {
         if (!p) {
-            query_features(ix, terms, q_off, q, c, sm.f);
+            query_features(ix, terms, q_off[q], q_off[q + 1], q, c, sm.f);
             if (feat_out && threadIdx.x < F) feat_out[uint64_t(q) * F + threadIdx.x] = sm.f[threadIdx.x];
             continue;
         }
-        const uint32_t path = planner_path(ix, terms, q_off, q, c, sm);
+        const uint32_t path = planner_path(ix, terms, q_off[q], q_off[q + 1], q, c, sm);
         if (feat_out && threadIdx.x < F) feat_out[uint64_t(q) * F + threadIdx.x] = sm.f[threadIdx.x];
         if (threadIdx.x == 0) {
             if (pred_out)

@@ -49,19 +49,20 @@ __device__ __forceinline__ TermFeat load_feat(const TermFeat* p) {
     return TermFeat{__hiloint2double(int(v.y), int(v.x)), v.z, v.w};
 }
 
-// The 16 features of query q (and its plain lists' blocks), computed by the whole CTA (kFeatThreads
-// threads) into f[] in shared memory. Term ids >= n_terms are skipped;
+// The 16 features of query q (and its plain lists' blocks), whose terms are
+// terms[qb .. qe), computed by the whole CTA (kFeatThreads threads) into f[] in
+// shared memory. The caller gives the range: inside a batch, offsets past the
+// workspace's terms are an empty query and must not be followed here. Term ids >= n_terms are skipped;
 // repeated terms count once per occurrence. The logarithm that each term adds
 // is in a table (taken here, four per thread and step of 64-bit arithmetic, it
 // was ~1 us a step: 20,000 terms are 20 steps). Each thread takes kFeatUnroll
 // terms per pass and issues all their table loads before using any, so a
 // query of thousands of terms costs a few memory latencies, not one per term.
-__device__ void query_features(const IndexView& ix, const uint32_t* terms, const uint64_t* q_off, uint32_t q,
+__device__ void query_features(const IndexView& ix, const uint32_t* terms, uint64_t qb, uint64_t qe, uint32_t q,
                                const FeatCtx& c, float* f, unsigned long long* blocks = nullptr) {
     __shared__ unsigned long long s_b[2][kFeatThreads / 32];
     __shared__ double s_d[6][kFeatThreads / 32];
     __shared__ uint32_t s_u[4][kFeatThreads / 32];
-    const uint64_t qb = q_off[q], qe = q_off[q + 1];
     uint32_t n = 0, mx = 0, nd = 0, nl = 0;
     unsigned long long pb = 0, pm = 0;  // blocks of the plain lists, and of those HYBRID merges
     double S = 0, Q = 0, Cb = 0, Lg = 0, Sd = 0, Bnd = 0;
@@ -262,13 +263,13 @@ __device__ __forceinline__ void mlp_forward_smem(PlannerSmem& sm) {
     __syncthreads();
 }
 
-// features -> standardise -> MLP -> cheapest path (an abf_path) of query q,
+// features -> standardise -> MLP -> cheapest path (an abf_path) of query q (terms[qb .. qe)),
 // by the whole CTA (kFeatThreads threads), after load_params; sm.f holds the
 // features and sm.y the predictions afterwards.
-__device__ __forceinline__ uint32_t planner_path(const IndexView& ix, const uint32_t* terms, const uint64_t* q_off,
+__device__ __forceinline__ uint32_t planner_path(const IndexView& ix, const uint32_t* terms, uint64_t qb, uint64_t qe,
                                                  uint32_t q, const FeatCtx& c, PlannerSmem& sm) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    query_features(ix, terms, q_off, q, c, sm.f, sm.blocks);  // ends with a barrier: every thread's copies are there
+    query_features(ix, terms, qb, qe, q, c, sm.f, sm.blocks);  // ends with a barrier: every thread's copies are there
     if (threadIdx.x < F) {
         const float sd = sm.p()[kSd + threadIdx.x];
         sm.xs[threadIdx.x] = (sm.f[threadIdx.x] - sm.p()[kMu + threadIdx.x]) / (sd > 0.0f ? sd : 1.0f);

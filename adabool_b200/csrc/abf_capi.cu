@@ -160,11 +160,20 @@ struct abf_workspace {
     uint32_t spin_limit = abf::kDefaultSpinLimit;  // polls of every bounded device wait
 };
 
+// A worker's allocation, shared with the graphs that captured its calls: it is
+// given back when the worker and the last of them are gone.
+struct WorkerScratch {
+    std::shared_ptr<abf::ScratchPool> pool;
+    void* p = nullptr;
+    size_t bytes = 0;
+    bool idle = false;  // no call outside a graph uses it any more
+    ~WorkerScratch();
+};
+
 struct abf_worker {
     abf_index* ix = nullptr;
     int kind = 0;  // 0 sparse, 1 dense (host bitmaps copied), 2 dense (caller device bitmaps)
-    void* arena = nullptr;          // the one allocation behind every pointer below but d_ext
-    size_t arena_bytes = 0;
+    std::shared_ptr<WorkerScratch> scratch;  // the one allocation behind every pointer below but d_ext
     bool scan = false;              // dense, no memory for the lists: answered by the scan of the index
     // the lists to merge: sparse, the keys as given; dense, the terms of a
     // window of query bitmaps, extracted when the worker runs
@@ -451,30 +460,43 @@ struct Arena {
 // whole prepare and free take 5, a workspace of 256 queries 20 instead of 600.
 // At most kPoolBytes are kept; the rest goes back at once, and all of
 // it when the index is freed or memory runs out. Scratch is kept only after a
-// synchronisation of the device, so any stream may use it next.
+// synchronisation of the device, so any stream may use it next, and a worker's
+// only when no graph that captured it is left (see keep_for_graph).
 constexpr size_t kPoolBytes = size_t(32) << 20;
 
-void pool_drain(abf_index* ix) {
-    std::lock_guard<std::mutex> g(ix->pool_mu);
-    for (auto& e : ix->pool) cudaFree(e.first);
-    ix->pool.clear();
-    ix->pool_bytes = 0;
+void pool_drain(abf::ScratchPool& pool) {
+    std::lock_guard<std::mutex> g(pool.mu);
+    for (auto& e : pool.kept) cudaFree(e.first);
+    for (void* p : pool.over) cudaFree(p);
+    pool.kept.clear();
+    pool.over.clear();
+    pool.bytes = 0;
+}
+
+// with the index: what graphs still name goes too, as they name its arrays
+void pool_close(abf::ScratchPool& pool) {
+    pool_drain(pool);
+    std::lock_guard<std::mutex> g(pool.mu);
+    pool.closed = true;
+    for (void* p : pool.held) cudaFree(p);
+    pool.held.clear();
 }
 
 // the smallest kept allocation that fits without holding more than twice the bytes (and 1 MB)
-abf_status scratch_alloc(abf_index* ix, size_t bytes, void** p, size_t* got) {
+abf_status scratch_alloc(abf::ScratchPool& pool, size_t bytes, void** p, size_t* got) {
     {
-        std::lock_guard<std::mutex> g(ix->pool_mu);
-        size_t best = ix->pool.size();
-        for (size_t i = 0; i < ix->pool.size(); ++i) {
-            const size_t b = ix->pool[i].second;
-            if (b >= bytes && b <= 2 * bytes + (1u << 20) && (best == ix->pool.size() || b < ix->pool[best].second)) best = i;
+        std::lock_guard<std::mutex> g(pool.mu);
+        auto& kept = pool.kept;
+        size_t best = kept.size();
+        for (size_t i = 0; i < kept.size(); ++i) {
+            const size_t b = kept[i].second;
+            if (b >= bytes && b <= 2 * bytes + (1u << 20) && (best == kept.size() || b < kept[best].second)) best = i;
         }
-        if (best < ix->pool.size()) {
-            *p = ix->pool[best].first;
-            *got = ix->pool[best].second;
-            ix->pool_bytes -= *got;
-            ix->pool.erase(ix->pool.begin() + std::ptrdiff_t(best));
+        if (best < kept.size()) {
+            *p = kept[best].first;
+            *got = kept[best].second;
+            pool.bytes -= *got;
+            kept.erase(kept.begin() + std::ptrdiff_t(best));
             return ABF_OK;
         }
     }
@@ -482,7 +504,7 @@ abf_status scratch_alloc(abf_index* ix, size_t bytes, void** p, size_t* got) {
     abf_status st = dev_alloc(&c, bytes);
     if (st != ABF_OK) {
         cudaGetLastError();  // reported here, not by the next launch
-        pool_drain(ix);
+        pool_drain(pool);
         st = dev_alloc(&c, bytes);
         if (st != ABF_OK) {
             cudaGetLastError();
@@ -494,21 +516,42 @@ abf_status scratch_alloc(abf_index* ix, size_t bytes, void** p, size_t* got) {
     return ABF_OK;
 }
 
-void scratch_free(abf_index* ix, void* p, size_t bytes, bool idle = true) {
+void scratch_free(abf::ScratchPool& pool, void* p, size_t bytes, bool idle = true) {
     if (!p) return;
     if (idle) {
-        std::lock_guard<std::mutex> g(ix->pool_mu);
-        if (ix->pool_bytes + bytes <= kPoolBytes) {
-            ix->pool.emplace_back(p, bytes);
-            ix->pool_bytes += bytes;
+        std::lock_guard<std::mutex> g(pool.mu);
+        for (void* o : pool.over) cudaFree(o);
+        pool.over.clear();
+        if (!pool.closed && pool.bytes + bytes <= kPoolBytes) {
+            pool.kept.emplace_back(p, bytes);
+            pool.bytes += bytes;
             return;
         }
     }
     cudaFree(p);
 }
 
+}  // namespace
+
+// May run on a thread of the driver's, where CUDA must not be called.
+WorkerScratch::~WorkerScratch() {
+    if (!p) return;
+    std::lock_guard<std::mutex> g(pool->mu);
+    if (pool->closed) return;
+    auto& held = pool->held;
+    held.erase(std::remove(held.begin(), held.end(), p), held.end());
+    if (idle && pool->bytes + bytes <= kPoolBytes) {
+        pool->kept.emplace_back(p, bytes);
+        pool->bytes += bytes;
+    } else {
+        pool->over.push_back(p);
+    }
+}
+
+namespace {
+
 void ws_release(abf_workspace* w, bool idle = true) {
-    scratch_free(w->ix, w->arena, w->arena_bytes, idle);
+    scratch_free(*w->ix->pool, w->arena, w->arena_bytes, idle);
     w->arena = nullptr;
 }
 
@@ -551,7 +594,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     const uint64_t chunks = uint64_t(max_q) * w->chunks_per_q;
     Arena a;
     ws_take(w, a, chunks);
-    ABF_TRY(scratch_alloc(ix, a.used, &w->arena, &w->arena_bytes));
+    ABF_TRY(scratch_alloc(*ix->pool, a.used, &w->arena, &w->arena_bytes));
     a = Arena{static_cast<char*>(w->arena), 0};
     ws_take(w, a, chunks);
     w->n_probe = w->ctl;
@@ -938,14 +981,37 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     else a.take(w->d_cnt, n_q);
 }
 
+void worker_release(abf_worker* w, bool idle = true) {
+    const std::shared_ptr<WorkerScratch> sc = std::move(w->scratch);
+    if (!sc) return;
+    abf::ScratchPool& pool = *sc->pool;
+    if (sc.use_count() == 1) {  // no graph has it, and none can get it any more
+        void* p = sc->p;
+        sc->p = nullptr;
+        scratch_free(pool, p, sc->bytes, idle);
+        return;
+    }
+    std::lock_guard<std::mutex> g(pool.mu);
+    sc->idle = idle;
+    if (pool.closed) {
+        cudaFree(sc->p);
+        sc->p = nullptr;
+    } else {
+        pool.held.push_back(sc->p);
+    }
+}
+
 abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
     w->sat_stride = sat_words(w->ix);
+    w->scratch = std::make_shared<WorkerScratch>();
+    WorkerScratch& sc = *w->scratch;
+    sc.pool = w->ix->pool;
     Arena a;
     worker_take(w, a, n_q);
     // (a worker over the caller's device bitmaps may be prepared while a stream is captured)
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     if (w->kind == 2) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-    abf_status st = scratch_alloc(w->ix, a.used, &w->arena, &w->arena_bytes);
+    abf_status st = scratch_alloc(*sc.pool, a.used, &sc.p, &sc.bytes);
     if (w->kind == 2) CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
     if (st != ABF_OK && w->kind != 0) {
         // no room for the lists: the scan needs only the bitmaps
@@ -953,24 +1019,44 @@ abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
         if (w->kind == 2) return ABF_OK;
         a = Arena{};
         worker_take(w, a, n_q);
-        st = scratch_alloc(w->ix, a.used, &w->arena, &w->arena_bytes);
+        st = scratch_alloc(*sc.pool, a.used, &sc.p, &sc.bytes);
     }
     if (st != ABF_OK) return st;
-    a = Arena{static_cast<char*>(w->arena), 0};
+    a = Arena{static_cast<char*>(sc.p), 0};
     worker_take(w, a, n_q);
     if (w->kind != 0) return ABF_OK;  // the term list kernels zero the counters
     const cudaError_t e = cudaMemset(w->d_nprobe, 0, kWorkerHead * 4u);
     if (e != cudaSuccess) {
-        scratch_free(w->ix, w->arena, w->arena_bytes);
-        w->arena = nullptr;
+        worker_release(w);
         return fail(ABF_ERR_CUDA, std::string("worker: ") + cudaGetErrorString(e));
     }
     return ABF_OK;
 }
 
-void worker_release(abf_worker* w, bool idle = true) {
-    scratch_free(w->ix, w->arena, w->arena_bytes, idle);
-    w->arena = nullptr;
+// A call that is captured: the graph, and every executable one made of it,
+// shares the worker's scratch from here on, so that it may be replayed after
+// the worker is gone (its kernels name nothing else of the worker's).
+abf_status keep_for_graph(const abf_worker* w, cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo_v2(s, &st, nullptr, &graph, nullptr, nullptr) != cudaSuccess) {
+        cudaGetLastError();  // the launches will say so
+        return ABF_OK;
+    }
+    if (st != cudaStreamCaptureStatusActive || !w->scratch->p) return ABF_OK;
+    auto* share = new std::shared_ptr<WorkerScratch>(w->scratch);
+    cudaUserObject_t obj = nullptr;
+    cudaError_t e = cudaUserObjectCreate(
+        &obj, share, [](void* p) { delete static_cast<std::shared_ptr<WorkerScratch>*>(p); }, 1,
+        cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        delete share;
+        CUDA_TRY(e);
+    }
+    e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);
+    CUDA_TRY(e);
+    return ABF_OK;
 }
 
 // Plan, merge and scatter of a worker's lists, ORed into d_res: n_q queries
@@ -1156,6 +1242,7 @@ abf_status run_sparse(const abf_worker* w, uint32_t* d_res, bool keyed, const ui
     if (!d_res) return fail(ABF_ERR_INVALID, "null d_res");
     if (w->n_keys == 0) return ABF_OK;
     CUDA_TRY(cudaSetDevice(ix->device));
+    ABF_TRY(keep_for_graph(w, s));
     const abf::IndexView v = abf::view_of(ix);
     WorkerRun r{};
     r.out = d_res;
@@ -1199,6 +1286,7 @@ abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_w
     if (!d_res) return fail(ABF_ERR_INVALID, "null d_res");
     if (w->batch == 0) return ABF_OK;
     CUDA_TRY(cudaSetDevice(ix->device));
+    ABF_TRY(keep_for_graph(w, s));
     const abf::IndexView v = abf::view_of(ix);
     const abf_tuning& t = ix->tuning;
     abf::ProbeArgs pr{};
@@ -1335,7 +1423,7 @@ abf_status abf_index_free(abf_index* ix) {
         ws_release(ix->own_ws);
         delete ix->own_ws;
     }
-    pool_drain(ix);
+    pool_close(*ix->pool);
     if (ix->h_stage) cudaFreeHost(ix->h_stage);
     if (ix->stage_event) cudaEventDestroy(static_cast<cudaEvent_t>(ix->stage_event));
     delete static_cast<Profiler*>(ix->prof);
@@ -1620,8 +1708,12 @@ abf_status abf_prepare_batch_device(abf_index* ix, uint64_t batch, uint64_t len,
 abf_status abf_worker_free(abf_worker* w) {
     API_BEGIN
     if (!w) return ABF_OK;
-    bool idle = false;
-    if (w->ix && w->ix->on_device) {
+    bool idle = false, closed = false;
+    if (w->scratch) {
+        std::lock_guard<std::mutex> g(w->scratch->pool->mu);
+        closed = w->scratch->pool->closed;  // the index went first: it must not be looked at
+    }
+    if (!closed && w->ix && w->ix->on_device) {
         cudaSetDevice(w->ix->device);
         idle = cudaDeviceSynchronize() == cudaSuccess;
     }

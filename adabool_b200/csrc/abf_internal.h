@@ -26,6 +26,7 @@
 #include <string>
 #include <vector>
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <utility>
 
@@ -176,6 +177,22 @@ struct IndexView {
 
 struct abf_workspace;
 
+namespace abf {
+
+// Scratch of freed workspaces and workers (pointer, bytes), for an index's
+// next ones. The index and its workers share it: a graph may let go of a
+// worker's scratch after both are gone.
+struct ScratchPool {
+    std::mutex mu;
+    std::vector<std::pair<void*, size_t>> kept;
+    size_t bytes = 0;            // of `kept`
+    std::vector<void*> held;     // of freed workers, still named by graphs
+    std::vector<void*> over;     // let go by a graph and not kept: for the next call that may free memory
+    bool closed = false;         // the index is gone, and all of these allocations with it
+};
+
+}  // namespace abf
+
 struct abf_index {
     abf::HostIndex host;          // emptied after upload unless kept
     abf::DerivedHost derived;     // dense bitmaps + directory (host copy until uploaded)
@@ -207,10 +224,7 @@ struct abf_index {
     const void* dense_tmap_base = nullptr;
     uint32_t dense_tmap_rows = 0;
     uint32_t dense_tmap_gw = 0;       // tile words of the boxes (32 or 64)
-    // scratch of freed workspaces and workers (pointer, bytes), for the next ones
-    std::mutex pool_mu;
-    std::vector<std::pair<void*, size_t>> pool;
-    size_t pool_bytes = 0;
+    std::shared_ptr<abf::ScratchPool> pool = std::make_shared<abf::ScratchPool>();
 };
 
 namespace abf {

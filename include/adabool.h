@@ -201,10 +201,6 @@ abf_status abf_index_set_dense_div(abf_index* index, uint32_t dense_div);
 abf_status abf_prepare_sparse(abf_index* index, const uint32_t* keys, uint64_t n_keys,
                               abf_worker** out);
 
-/* Dense workers hold scratch for the terms of up to 256 query bitmaps at a
- * time (2,048 per query on average; a denser window is answered by a scan of
- * the index). Scratch of freed workers and workspaces stays with the index,
- * up to 32 MB, for the next ones. */
 /* Dense worker for one query given as a host term bitmap of len bytes
  * (bit t of byte t/8 set = term t in the query). Replaces
  * ivf_list::Prepare(len, bitmap) (src/AdaBool/inverted_list.h:530-543). */
@@ -221,6 +217,15 @@ abf_status abf_prepare_batch(abf_index* index, uint64_t batch_size, uint64_t len
 abf_status abf_prepare_batch_device(abf_index* index, uint64_t batch_size, uint64_t len,
                                     const uint8_t* d_query_bitmap, abf_worker** out);
 
+/* Frees a worker (synchronises the device). Workers hold scratch -- a dense
+ * one for the terms of up to 256 query bitmaps at a time, 2,048 per query on
+ * average; a denser window is answered by a scan of the index. Scratch of
+ * freed workers and workspaces stays with the index, up to 32 MB, for the next
+ * ones. A graph that captured a worker's calls keeps that worker's scratch for
+ * itself, so it may be replayed after the worker is freed (the index and the
+ * caller's arrays must still be there); its replays and the worker's other
+ * calls must not overlap. A workspace must outlive the graphs that captured
+ * it. */
 abf_status abf_worker_free(abf_worker* worker);
 
 /* Union of the sparse worker's lists ORed into d_res. Replaces

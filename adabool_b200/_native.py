@@ -147,6 +147,8 @@ PROTOTYPES = {
     "abf_batch_collect_ids": [vp, vp, vp, C.c_uint64, C.c_uint32, vp, C.c_uint64, vp, vp],
     "abf_collect_ids_noalloc": [vp, C.c_uint64, vp, C.c_uint64, vp, vp],
     "abf_collect_ids_noalloc_check": [vp],
+    "abf_worker_check": [vp, vp],
+    "abf_worker_selftest_waits": [vp, C.c_uint32, vp],
     "abf_workspace_create": [vp, C.c_uint32, C.c_uint64, C.POINTER(vp)],
     "abf_workspace_free": [vp],
     "abf_workspace_check": [vp, vp],

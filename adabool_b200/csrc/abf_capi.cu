@@ -206,7 +206,11 @@ struct abf_worker {
     uint32_t* d_bblk = nullptr;
     uint32_t* d_parts = nullptr;
     uint32_t* d_ticket = nullptr;
+    // error flag of the kernels' bounded waits, below the worker's own mark: a
+    // word without the mark is some other scratch's (a dense worker's is
+    // written when it runs: preparing one makes no stream work)
     uint32_t* d_err = nullptr;
+    uint32_t mark = 0;
     uint64_t dense_keys = 0;        // sparse: keys whose lists have dense bitmaps, and their postings
     uint64_t dense_postings = 0;
     // dense
@@ -948,7 +952,13 @@ constexpr uint32_t kKeyRunCap = 256;    // runs of a keyed batch merged by the g
 constexpr uint32_t kOneQueryKeys = 2048; // keys that one planning CTA takes in a few steps of 256
 constexpr uint32_t kTermWindow = 256;   // query bitmaps extracted and merged at a time
 
-constexpr uint32_t kWorkerHead = 8;  // words before the keys: four counters, two 64-bit offsets
+constexpr uint32_t kWorkerHead = 8;  // words before the keys: three counters, the error flag, two 64-bit offsets
+constexpr uint32_t kErrBits = 0xffu; // of an error flag; the rest is the worker's mark
+
+uint32_t next_mark() {
+    static std::atomic<uint32_t> n{0};
+    return (n.fetch_add(1u, std::memory_order_relaxed) + 1u) << 8;
+}
 
 // arrays of a worker that plans at most n_q queries over w->term_cap terms
 void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
@@ -958,6 +968,7 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     a.take(w->d_nprobe, kWorkerHead + w->term_cap);
     w->d_n_tile_list = w->d_nprobe + 1;
     w->d_plan_done = w->d_nprobe + 2;
+    w->d_err = w->d_nprobe + 3;
     w->d_off1 = reinterpret_cast<uint64_t*>(w->d_nprobe + 4);
     w->d_keys = w->d_nprobe + kWorkerHead;
     a.take(w->d_off, n_q + 1);
@@ -967,7 +978,6 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     a.take(w->d_lpref_q, n_q + 1);
     a.take(w->d_tile_list, w->q_cap);
     a.take(w->d_n_q, 1);
-    a.take(w->d_err, 1);
     a.take(w->d_dense16, w->term_cap + 8ull * w->q_cap + 16);
     a.take(w->d_dstart, w->q_cap);
     a.take(w->d_ndense, w->q_cap);
@@ -1003,6 +1013,7 @@ void worker_release(abf_worker* w, bool idle = true) {
 
 abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
     w->sat_stride = sat_words(w->ix);
+    w->mark = next_mark();
     w->scratch = std::make_shared<WorkerScratch>();
     WorkerScratch& sc = *w->scratch;
     sc.pool = w->ix->pool;
@@ -1024,13 +1035,7 @@ abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
     if (st != ABF_OK) return st;
     a = Arena{static_cast<char*>(sc.p), 0};
     worker_take(w, a, n_q);
-    if (w->kind != 0) return ABF_OK;  // the term list kernels zero the counters
-    const cudaError_t e = cudaMemset(w->d_nprobe, 0, kWorkerHead * 4u);
-    if (e != cudaSuccess) {
-        worker_release(w);
-        return fail(ABF_ERR_CUDA, std::string("worker: ") + cudaGetErrorString(e));
-    }
-    return ABF_OK;
+    return ABF_OK;  // the head is uploaded with the keys, or written by the term list kernels
 }
 
 // A call that is captured: the graph, and every executable one made of it,
@@ -1337,7 +1342,11 @@ abf_status run_dense(const abf_worker* w, uint32_t* d_res, uint64_t res_stride_w
         la.off = w->d_off;
         la.overflow = w->d_n_q;
         la.zero = w->d_nprobe;
-        la.n_zero = kWorkerHead;
+        la.n_zero = 3;
+        if (q0 == 0) {
+            la.err = w->d_err;
+            la.err_value = w->mark;
+        }
         TIMED(K_PROBE, abf::launch_term_lists(la, s));
         if (t.group_min_queries && r.n_q >= t.group_min_queries) r.group = group_shape(ix, v, r.n_q, 64ull * r.n_q, true);
         r.stream = !r.group.on;
@@ -1626,15 +1635,16 @@ abf_status abf_prepare_sparse(abf_index* ix, const uint32_t* keys, uint64_t n_ke
         ++w->dense_keys;
         w->dense_postings += ix->h_term_len[keys[i]];
     }
-    std::vector<uint32_t> up(4 + n_keys);  // {0, n_keys} as 64-bit offsets, then the keys
-    up[2] = uint32_t(n_keys);
-    if (n_keys) std::memcpy(up.data() + 4, keys, n_keys * 4);
+    std::vector<uint32_t> up(kWorkerHead + n_keys);  // three zeros, the mark, {0, n_keys} as 64-bit offsets, the keys
+    up[6] = uint32_t(n_keys);
+    if (n_keys) std::memcpy(up.data() + kWorkerHead, keys, n_keys * 4);
     abf_status st = worker_alloc(w, w->term_cap);
     if (st != ABF_OK) {
         delete w;
         return st;
     }
-    const cudaError_t e = cudaMemcpy(w->d_off1, up.data(), up.size() * 4, cudaMemcpyHostToDevice);
+    up[3] = w->mark;
+    const cudaError_t e = cudaMemcpy(w->d_nprobe, up.data(), up.size() * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         worker_release(w);
         delete w;
@@ -1719,6 +1729,38 @@ abf_status abf_worker_free(abf_worker* w) {
     }
     worker_release(w, idle);
     delete w;
+    return ABF_OK;
+    API_END
+}
+
+abf_status abf_worker_check(abf_worker* w, void* stream) {
+    API_BEGIN
+    if (!w) return fail(ABF_ERR_INVALID, "null worker");
+    CUDA_TRY(cudaSetDevice(w->ix->device));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // the scan of a worker without scratch marks the index's own workspace
+    uint32_t* flag = !w->scan ? w->d_err : w->ix->own_ws ? w->ix->own_ws->err : nullptr;
+    if (!flag) return ABF_OK;
+    const uint32_t clear = w->scan ? 0u : w->mark;
+    uint32_t err = 0;
+    CUDA_TRY(cudaMemcpyAsync(&err, flag, 4, cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if ((err & ~kErrBits) != clear || err == clear) return ABF_OK;  // no call yet, or none that gave up
+    CUDA_TRY(cudaMemcpyAsync(flag, &clear, 4, cudaMemcpyHostToDevice, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    return fail(ABF_ERR_TIMEOUT, "a bounded device wait gave up (code " + std::to_string(err & kErrBits) + ")");
+    API_END
+}
+
+abf_status abf_worker_selftest_waits(abf_worker* w, uint32_t polls, void* stream) {
+    API_BEGIN
+    if (!w || polls == 0) return fail(ABF_ERR_INVALID, "abf_worker_selftest_waits: null worker or zero polls");
+    if (w->scan) return fail(ABF_ERR_STATE, "abf_worker_selftest_waits: the worker has no scratch");
+    CUDA_TRY(cudaSetDevice(w->ix->device));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    CUDA_TRY(cudaMemcpyAsync(w->d_err, &w->mark, 4, cudaMemcpyHostToDevice, s));
+    // the first two block prefixes: every call writes them before it reads them
+    CUDA_TRY(abf::launch_wait_selftest(w->d_lpref_q, w->d_err, polls, s));
     return ABF_OK;
     API_END
 }

@@ -650,6 +650,7 @@ __global__ void __launch_bounds__(kTermThreads) term_count_kernel(TermListArgs a
     __shared__ unsigned long long s_red[kTermThreads / 32];
     wait_previous();
     if (blockIdx.x == 0 && threadIdx.x < a.n_zero) a.zero[threadIdx.x] = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == a.n_zero && a.err) *a.err = a.err_value;
     const uint32_t nw = term_words(a);
     for (uint32_t q = blockIdx.x; q < a.n_q; q += gridDim.x) {
         const uint32_t* bm = a.qbm + uint64_t(q) * a.qbm_stride;

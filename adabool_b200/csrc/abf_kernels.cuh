@@ -182,8 +182,10 @@ struct TermListArgs {
     uint32_t* terms;          // out
     uint64_t* off;            // out: n_q + 1
     uint32_t* overflow;       // out: 0 or 1
-    uint32_t* zero;           // n_zero (<= 512) counters that the next kernels find zeroed
+    uint32_t* zero;           // n_zero (< 512) counters that the next kernels find zeroed
     uint32_t n_zero;
+    uint32_t* err;            // optional error flag, set to err_value
+    uint32_t err_value;
 };
 
 struct TileArgs {

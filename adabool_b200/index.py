@@ -46,6 +46,14 @@ class Worker:
     def handle(self):
         return self._h
 
+    def check(self, stream=None):
+        """Raises ABF_ERR_TIMEOUT when a bounded device wait of the worker's calls gave up (abf_worker_check)."""
+        check(lib().abf_worker_check(self._h, stream_ptr(stream)))
+
+    def selftest_waits(self, polls: int, stream=None):
+        """Makes two such waits run out (abf_worker_selftest_waits); check() then raises."""
+        check(lib().abf_worker_selftest_waits(self._h, int(polls), stream_ptr(stream)))
+
     def free(self):
         if self._h:
             lib().abf_worker_free(self._h)

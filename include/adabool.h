@@ -228,6 +228,15 @@ abf_status abf_prepare_batch_device(abf_index* index, uint64_t batch_size, uint6
  * it. */
 abf_status abf_worker_free(abf_worker* worker);
 
+/* Reads and clears the worker's error flag (synchronises the stream):
+ * ABF_ERR_TIMEOUT when a bounded device wait of one of its calls gave up, so
+ * that the bitmaps may miss bits. A dense worker's next call clears the flag
+ * too. abf_worker_selftest_waits makes two such waits run out (see
+ * abf_workspace_selftest_waits; not concurrently with a call of the worker).
+ * No reference counterpart. */
+abf_status abf_worker_check(abf_worker* worker, void* stream);
+abf_status abf_worker_selftest_waits(abf_worker* worker, uint32_t polls, void* stream);
+
 /* Union of the sparse worker's lists ORed into d_res. Replaces
  * ListUnion_sparse (test/adsfilter_q_all.cu:64-105). */
 abf_status abf_list_union_sparse(const abf_worker* worker, uint32_t* d_res, void* stream);

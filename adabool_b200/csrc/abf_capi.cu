@@ -394,7 +394,10 @@ abf_status upload(abf_index* ix, int device) {
         (st = upload_vec(&d.dense, ix->derived.dense, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.term_dir, ix->derived.term_dir, &d.bytes)) != ABF_OK ||
         (st = upload_vec(&d.dir, ix->derived.dir, &d.bytes)) != ABF_OK ||
-        (st = make_plain(ix, ix->derived)) != ABF_OK || (st = make_term_info(ix, ix->derived)) != ABF_OK) {
+        // what the index cannot do without comes first: the plain ids take what
+        // is left, and the term tables then learn of them
+        (st = make_term_info(ix, ix->derived)) != ABF_OK || (st = make_plain(ix, ix->derived)) != ABF_OK ||
+        (d.plain && (st = make_term_info(ix, ix->derived)) != ABF_OK)) {
         free_device(ix);
         return st;
     }

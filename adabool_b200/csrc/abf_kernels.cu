@@ -35,7 +35,11 @@ constexpr uint64_t kValMask = (1ull << 62) - 1;
 // Programmatic launch order: the kernels of a batch are launched so that each
 // may come up while the one before it finishes. Every kernel begins with this
 // wait, before it reads or writes any global memory, and on every CTA (a
-// kernel is complete only when the ones before it are).
+// kernel is complete only when the ones before it are). What the kernel before
+// it, or the caller, writes is read by plain loads: __ldg promises data that
+// nobody writes while this kernel runs, which it does from before the wait, and
+// the compiler may move it across the wait. It is for the index's arrays, and
+// for what a kernel further back wrote (complete when this one comes up).
 __device__ __forceinline__ void wait_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -638,7 +642,7 @@ __global__ void __launch_bounds__(1024) key_runs_kernel(KeyRunsArgs a) {
 // query on 2^16 x 2^20 138 -> 47 us.
 constexpr uint32_t kTermThreads = 512;
 __device__ __forceinline__ uint32_t term_word(const uint32_t* bm, uint32_t w, uint32_t n_terms) {
-    const uint32_t v = __ldg(bm + w), left = n_terms - w * 32u;
+    const uint32_t v = bm[w], left = n_terms - w * 32u;
     return left < 32u ? v & ((1u << left) - 1u) : v;
 }
 __device__ __forceinline__ uint32_t term_words(const TermListArgs& a) {
@@ -787,7 +791,7 @@ __global__ void __launch_bounds__(kStreamThreads, 4) dense_stream_kernel(IndexVi
         const uint4* dl = reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]);  // eight rows each
         const V* base = reinterpret_cast<const V*>(ix.dense) + (in ? j : 0u);
         for (uint32_t k = 0; k < nd; k += KT) {
-            const uint4 r = __ldg(dl + k / KT);
+            const uint4 r = dl[k / KT];
             const uint32_t row[KT] = {r.x & 0xffffu, r.x >> 16, r.y & 0xffffu, r.y >> 16,
                                       r.z & 0xffffu, r.z >> 16, r.w & 0xffffu, r.w >> 16};
             V x[KT];
@@ -860,7 +864,7 @@ __global__ void __launch_bounds__(NW * 32) tile_union_kernel(IndexView ix, TileA
         for (uint64_t c0 = qb; c0 < qe; c0 += NT) {
             const uint64_t i = c0 + tid;
             uint32_t lo = 0, cnt = 0;
-            const uint32_t cls = i < qe ? __ldg(a.tile_cls + i) : kNone;
+            const uint32_t cls = i < qe ? __ldg(a.tile_cls + i) : kNone;  // two kernels back
             if (cls != kNone) tile_block_range(ix, cls, lo_id, hi_id, dj0, dj1, lo, cnt);
             uint32_t total;
             const uint32_t ex = block_excl_scan<NT>(cnt, s_warp, &total);
@@ -1323,7 +1327,7 @@ __global__ void __launch_bounds__(NW * 32, 6) scatter_kernel(IndexView ix, Scatt
                     uint32_t m = kFull;
                     if (w == w0) m &= kFull << (t0 & 31u);
                     if (w == w1) m &= kFull >> (31u - (t1 & 31u));
-                    const uint32_t v = __ldg(sat + w) & m;
+                    const uint32_t v = sat[w] & m;
                     all &= v == m;
                     some |= v != 0u;
                 }
@@ -1372,7 +1376,7 @@ __global__ void __launch_bounds__(NW * 32, 6) scatter_kernel(IndexView ix, Scatt
 #pragma unroll
                 for (uint32_t e = 0; e < 4u; ++e) {
                     const uint32_t t = id[e] >> tshift;
-                    if (m[e] && (__ldg(sat + (t >> 5)) >> (t & 31u) & 1u)) m[e] = 0u;
+                    if (m[e] && (sat[t >> 5] >> (t & 31u) & 1u)) m[e] = 0u;
                 }
             }
             // ids of one word become one atomic
@@ -1712,7 +1716,7 @@ __global__ void __launch_bounds__(NW * 32) probe_kernel(IndexView ix, ProbeArgs 
                     if (wd < a.qbm_words) {
                         for (uint32_t g = 0; g < G; ++g) {
                             const uint32_t word = staged ? sbm[g * span + (wd - w0)]
-                                                         : __ldg(a.qbm + uint64_t(g0 + g) * a.qbm_stride + wd);
+                                                         : a.qbm[uint64_t(g0 + g) * a.qbm_stride + wd];
                             hit |= ((word >> bit) & 1u) << g;
                         }
                     }

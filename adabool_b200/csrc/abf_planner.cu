@@ -60,8 +60,7 @@ __global__ void __launch_bounds__(64) mlp_forward_kernel(const float* __restrict
 // loads in flight per thread), so that a training step has one launch here
 // instead of two memsets and a counting kernel.
 constexpr uint32_t kInitSamples = 16384;
-__global__ void __launch_bounds__(1024) grad_init_kernel(const float* __restrict__ mask, uint32_t n, float* g,
-                                                         float* loss2) {
+__global__ void __launch_bounds__(1024) grad_init_kernel(const float* mask, uint32_t n, float* g, float* loss2) {
     __shared__ float s_part[32];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

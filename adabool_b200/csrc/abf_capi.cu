@@ -880,7 +880,6 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     }
     if (may_merge) TIMED(K_TILE, abf::launch_tile_union(v, ta, tt, ix->sm_count, s));
     abf::ScatterArgs sa{};
-    sa.terms = b->d_terms;
     sa.q_off = b->d_offsets;
     sa.term_slot = ws->slot;
     sa.q_light_pref = ws->lpref_q;
@@ -952,7 +951,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
 
 // ---- workers ----
 constexpr uint32_t kKeyRunCap = 256;    // runs of a keyed batch merged by the group kernel; later ones are scattered
-constexpr uint32_t kOneQueryKeys = 2048; // keys that one planning CTA takes in a few steps of 256
+constexpr uint32_t kOneQueryKeys = 2048; // keys that one planning CTA takes in two steps
 constexpr uint32_t kTermWindow = 256;   // query bitmaps extracted and merged at a time
 
 constexpr uint32_t kWorkerHead = 8;  // words before the keys: three counters, the error flag, two 64-bit offsets
@@ -1200,7 +1199,6 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
         TIMED(K_TILE, abf::launch_tile_union(v, ta, tt, ix->sm_count, s));
     }
     abf::ScatterArgs sa{};
-    sa.terms = w->d_keys;
     sa.q_off = r.q_off;
     sa.term_slot = w->d_tslot;
     sa.q_light_pref = w->d_lpref_q;

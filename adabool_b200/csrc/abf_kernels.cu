@@ -139,30 +139,18 @@ __device__ __forceinline__ void or_tile(uint32_t* tile, uint32_t lo, uint32_t sp
     if (cur != kFull) atomicOr(tile + cur, m);
 }
 
-// OR decoded ids (< n_ads) into a global bitmap, same lane-local combining.
-// true when word wd lies in a tile whose bits are all set already
-__device__ __forceinline__ bool in_full_tile(const uint32_t* sat, uint32_t sat_shift, uint32_t wd) {
-    const uint32_t t = wd >> sat_shift;
-    return (__ldg(sat + (t >> 5)) >> (t & 31u)) & 1u;
-}
-
-// OR of this lane's four ids into the bitmap, one atomic per distinct word;
-// with sat (the dense group kernel's saturated-tile bits of this bitmap),
-// words inside an all-ones tile are skipped: the OR cannot change them
-__device__ __forceinline__ void or_global(uint32_t* bm, uint32_t n_ads, const uint32_t (&id)[4], uint32_t cnt,
-                                          const uint32_t* sat = nullptr, uint32_t sat_shift = 0) {
+// OR of this lane's four ids (those below n_ads) into the bitmap, one atomic
+// per distinct word
+__device__ __forceinline__ void or_global(uint32_t* bm, uint32_t n_ads, const uint32_t (&id)[4], uint32_t cnt) {
     const uint32_t lane = lane_id();
     uint32_t cur = kFull, m = 0;
-    auto flush = [&]() {
-        if (!sat || !in_full_tile(sat, sat_shift, cur)) atomicOr(bm + cur, m);
-    };
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const uint32_t i = lane * 4u + k;
         if (i < cnt && id[k] < n_ads) {
             const uint32_t wd = id[k] >> 5, bit = 1u << (id[k] & 31u);
             if (wd != cur) {
-                if (cur != kFull) flush();
+                if (cur != kFull) atomicOr(bm + cur, m);
                 cur = wd;
                 m = bit;
             } else {
@@ -170,7 +158,7 @@ __device__ __forceinline__ void or_global(uint32_t* bm, uint32_t n_ads, const ui
             }
         }
     }
-    if (cur != kFull) flush();
+    if (cur != kFull) atomicOr(bm + cur, m);
 }
 
 template <int NT>

@@ -49,7 +49,7 @@ constexpr uint32_t kCompactWarps = 4;
 constexpr uint32_t kCompactChunkWords = kCompactWarps * 256;  // bitmap words per compaction work item
 constexpr uint32_t kCompactFew = 888;  // fewer items than this (6 per SM): shorter chunks
 // look-back words that a batch with shorter chunks can need: less than
-// kCompactFew items turn into at most four times as many, plus one per bitmap
+// kCompactFew items turn into at most eight times as many
 constexpr uint32_t kCompactFewStatus = 8u * kCompactFew;
 constexpr uint32_t kProbeGroup = 32;          // probe queries tested per pass
 
@@ -270,7 +270,6 @@ struct BinArgs {
 };
 
 struct ScatterArgs {
-    const uint32_t* terms;
     const uint64_t* q_off;
     const uint2* term_slot;
     const uint64_t* q_light_pref; // n_q + 1

@@ -111,8 +111,8 @@ def planner_experiment(n_train: int = 66_667, batch_config: str = "c2", reps: in
     n = qoff.size - 1
     tau_info = {"source": "this library's timing labels", "tau": tau_labels}
     if callable(fixed_tau):
-        tau_info = dict(fixed_tau(ix, qoff, qt, P.touched_fraction(ix, qoff, qt)),
-                        source="crossover of the reference's kernels")
+        tau_info = {"source": "crossover of the reference's kernels",
+                    **fixed_tau(ix, qoff, qt, P.touched_fraction(ix, qoff, qt))}
     elif fixed_tau is not None:
         tau_info = {"source": "given", "tau": float(fixed_tau)}
     tau = float(tau_info.get("tau", tau_labels))

@@ -796,7 +796,13 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.probe_stride = ws->probe_stride;
     abf::QueueArgs qa{ws->lcnt, ws->lpref_q, b->n_queries};
     const bool hybrid = b->d_paths || b->path == ABF_PATH_AUTO || b->path == ABF_PATH_HYBRID || b->path == ABF_PATH_TILE;
-    const bool bins = v.n_plain > 0 && (group || b->path == ABF_PATH_TILE || b->d_paths || (hybrid && hybrid_bins(ix)));
+    // A small batch on TILE has the merge kernel run in any case, for the short
+    // lists; up to 32 tiles in all it takes the plain ones too. 4 to 64 terms
+    // each, us without / with the bin kernel: one query on 2^20 ads (2 tiles)
+    // 20.3 / 27.4, 8 (16) 34.3 / 38.6, 31 (62) 47.0 / 45.6; 4 on 2^22 (32) 38.7 /
+    // 38.4, 8 (64) 51.9 / 43.8.
+    const bool binned = b->path == ABF_PATH_TILE ? uint64_t(b->n_queries) * n_tiles_bin > 32 : hybrid && hybrid_bins(ix);
+    const bool bins = v.n_plain > 0 && (group || b->d_paths || binned);
     if (bins) {
         pa.bin_list = ws->bin_list;
         pa.bin_min_blocks = group ? bin_min_blocks(n_words) : 0xffffffffu;
@@ -910,7 +916,8 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
         ba.sat_last = sa.sat_last;
         TIMED(K_BIN, abf::launch_bin(v, ba, ix->sm_count, s));
     }
-    TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
+    // a batch on TILE merges every list: nothing is left to scatter
+    if (b->d_paths || b->path != ABF_PATH_TILE) TIMED(K_SCATTER, abf::launch_scatter(v, sa, t, ix->sm_count, s));
     if (maybe_probe) {
         abf::ProbeArgs pr{};
         pr.qbm = ws->probe_bm;

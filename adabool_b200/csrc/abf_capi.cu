@@ -137,7 +137,8 @@ struct abf_workspace {
     uint32_t* ctl = nullptr;
     uint32_t* n_probe = nullptr;
     uint32_t* probe_bm = nullptr;
-    uint64_t* scan_status = nullptr;         // compaction look-back words, one per chunk (+1)
+    uint64_t* scan_status = nullptr;         // compaction look-back words, one per chunk (+1), behind a
+                                             // ticket for compactions that are no part of a batch
     uint32_t* plan_done = nullptr;
     unsigned long long* ticket = nullptr;   // compaction item counter
     uint64_t* id_off = nullptr;
@@ -574,7 +575,7 @@ void ws_take(abf_workspace* w, Arena& a, uint64_t chunks) {
     a.take(w->lpref_q, uint64_t(max_q) + 1);
     a.take(w->probe_list, w->probe_cap);
     a.take(w->probe_bm, uint64_t(w->probe_cap) * w->probe_stride);
-    a.take(w->scan_status, std::max<uint64_t>(chunks, abf::kCompactFewStatus) + 1);
+    a.take(w->scan_status, std::max<uint64_t>(chunks, abf::kCompactFewStatus) + 2);
     a.take(w->id_off, uint64_t(max_q) + 1);
     a.take(w->path_out, max_q);
     a.take(w->err, 1);
@@ -607,6 +608,7 @@ abf_status ws_alloc(abf_index* ix, uint32_t max_q, uint64_t max_terms, uint64_t 
     w->n_probe = w->ctl;
     w->n_tile_list = w->ctl + 1;
     w->plan_done = w->ctl + 2;
+    ++w->scan_status;
     w->ticket = reinterpret_cast<unsigned long long*>(w->ctl + 4);
     w->q_off = reinterpret_cast<uint64_t*>(w->ctl + kCtlWords);
     w->q_terms = w->ctl + kCtlWords + 4;
@@ -1823,7 +1825,7 @@ abf_status abf_collect_ids(abf_index* ix, const uint32_t* d_bitmap, uint64_t n_b
     ca.units = abf::compact_units(1, n_bits);
     ca.n_chunks = abf::compact_chunks(n_bits, ca.units);
     ca.status = ws->scan_status;
-    ca.ticket = ws->ticket;
+    ca.ticket = reinterpret_cast<unsigned long long*>(ws->scan_status - 1);
     ca.ids = d_ids;
     ca.capacity = ids_capacity;
     ca.id_offsets = ws->id_off;
@@ -1855,7 +1857,7 @@ abf_status abf_batch_collect_ids(abf_index* ix, abf_workspace* ws, const uint32_
     ca.units = abf::compact_units(ca.n_q, ca.n_bits);
     ca.n_chunks = abf::compact_chunks(ca.n_bits, ca.units);
     ca.status = ws->scan_status;
-    ca.ticket = ws->ticket;
+    ca.ticket = reinterpret_cast<unsigned long long*>(ws->scan_status - 1);
     ca.ids = d_ids;
     ca.capacity = d_ids ? ids_capacity : 0;
     ca.id_offsets = d_id_offsets;

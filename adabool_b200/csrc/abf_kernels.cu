@@ -2367,8 +2367,10 @@ cudaError_t launch_compact(const CompactArgs& a, int sm_count, uint32_t ctas_per
     const uint64_t items = uint64_t(a.n_q) * a.n_chunks;
     if (items == 0) return cudaSuccess;
     if (!a.zeroed) {
-        cudaError_t e = cudaMemsetAsync(a.status, 0, items * sizeof(uint64_t), s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(a.ticket, 0, sizeof(unsigned long long), s);
+        // the ticket beside the look-back words saves a memset
+        const bool both = static_cast<void*>(a.ticket + 1) == static_cast<void*>(a.status);
+        cudaError_t e = cudaMemsetAsync(both ? static_cast<void*>(a.ticket) : a.status, 0, (items + both) * sizeof(uint64_t), s);
+        if (e == cudaSuccess && !both) e = cudaMemsetAsync(a.ticket, 0, sizeof(unsigned long long), s);
         if (e == cudaSuccess && a.id_counts) e = cudaMemsetAsync(a.id_counts, 0, uint64_t(a.n_q) * sizeof(uint64_t), s);
         if (e != cudaSuccess) return e;
     }

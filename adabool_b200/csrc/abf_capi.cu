@@ -182,9 +182,10 @@ struct abf_worker {
     uint32_t term_cap = 0;          // room in d_keys
     uint32_t* d_keys = nullptr;
     uint64_t* d_off1 = nullptr;     // sparse: {0, n_keys}, the keys as one query
+    uint64_t* d_offc = nullptr;     // sparse: the keys kKeyChunk at a time
     uint64_t* d_off = nullptr;      // offsets of the queries (sparse: runs of keys with one bitmap index)
     uint32_t* d_slot = nullptr;     // sparse: bitmap index of each run
-    uint32_t* d_n_q = nullptr;      // sparse: number of runs; dense: overflow word of the term lists
+    uint32_t* d_n_q = nullptr;      // sparse: number of runs, first mixed one; dense: overflow word of the term lists
     uint32_t* d_cnt = nullptr;      // dense: terms per query
     // planning scratch (see PlanArgs); the dense-bitmap lists and saturation
     // marks cover the first q_cap queries or runs
@@ -963,7 +964,10 @@ constexpr uint32_t kKeyRunCap = 256;    // runs of a keyed batch merged by the g
 constexpr uint32_t kOneQueryKeys = 2048; // keys that one planning CTA takes in two steps
 constexpr uint32_t kTermWindow = 256;   // query bitmaps extracted and merged at a time
 
-constexpr uint32_t kWorkerHead = 8;  // words before the keys: three counters, the error flag, two 64-bit offsets
+constexpr uint32_t kWorkerHead = 8;  // words before the keys: three counters, the error flag, two 64-bit offsets;
+                                     // between them and the keys, the chunks' offsets
+uint64_t key_chunks(uint64_t n_keys) { return (n_keys + abf::kKeyChunk - 1) / abf::kKeyChunk; }
+uint64_t head_words(const abf_worker* w) { return kWorkerHead + (w->kind == 0 ? 2 * (key_chunks(w->n_keys) + 1) : 0); }
 constexpr uint32_t kErrBits = 0xffu; // of an error flag; the rest is the worker's mark
 
 uint32_t next_mark() {
@@ -976,19 +980,20 @@ void worker_take(abf_worker* w, Arena& a, uint64_t n_q) {
     if (w->kind == 1) a.take(w->d_qbm, std::max<uint64_t>(w->batch, 1) * w->qbm_stride);
     if (w->scan) return;
     // counters, offsets and keys in one piece: one upload
-    a.take(w->d_nprobe, kWorkerHead + w->term_cap);
+    a.take(w->d_nprobe, head_words(w) + w->term_cap);
     w->d_n_tile_list = w->d_nprobe + 1;
     w->d_plan_done = w->d_nprobe + 2;
     w->d_err = w->d_nprobe + 3;
     w->d_off1 = reinterpret_cast<uint64_t*>(w->d_nprobe + 4);
-    w->d_keys = w->d_nprobe + kWorkerHead;
+    w->d_offc = reinterpret_cast<uint64_t*>(w->d_nprobe + kWorkerHead);
+    w->d_keys = w->d_nprobe + head_words(w);
     a.take(w->d_off, n_q + 1);
     a.take(w->d_tslot, w->term_cap);
     a.take(w->d_tile_cls, w->term_cap);
     a.take(w->d_lcnt, n_q);
     a.take(w->d_lpref_q, n_q + 1);
     a.take(w->d_tile_list, w->q_cap);
-    a.take(w->d_n_q, 1);
+    a.take(w->d_n_q, 2);
     a.take(w->d_dense16, w->term_cap + 8ull * w->q_cap + 16);
     a.take(w->d_dstart, w->q_cap);
     a.take(w->d_ndense, w->q_cap);
@@ -1082,7 +1087,8 @@ struct WorkerRun {
     uint32_t n_q;
     const uint32_t* d_n_q = nullptr;
     const uint32_t* out_slot = nullptr;
-    const uint32_t* key_slot = nullptr;
+    const uint32_t* key_slot = nullptr;    // instead, for the scatter: output bitmap of each key
+    const uint32_t* mixed_from = nullptr;  // first query whose keys have several (see PlanArgs)
     uint32_t* out;
     uint64_t out_stride;
     bool stream;       // dense bitmaps by the stream kernel, other long lists by the merge kernel
@@ -1100,6 +1106,7 @@ abf_status run_worker_lists(const abf_worker* w, const abf::IndexView& v, const 
     pa.q_off = r.q_off;
     pa.n_q = r.n_q;
     pa.d_n_q = r.d_n_q;
+    pa.mixed_from = r.mixed_from;
     const bool merge = r.stream && hybrid_tiles(ix);
     pa.path_uniform = r.stream ? ABF_PATH_HYBRID : ABF_PATH_UNION;
     pa.hybrid_min = t.heavy_min_len;
@@ -1275,19 +1282,22 @@ abf_status run_sparse(const abf_worker* w, uint32_t* d_res, bool keyed, const ui
     // n_dense * n_ads / 64 + 2^23 postings on.
     if (ix->tuning.group_min_queries && w->dense_postings >= uint64_t(v.n_dense) * v.n_ads / 64u + (1u << 23))
         r.group = group_shape(ix, v, w->q_cap, w->dense_keys + 8ull * w->q_cap, true);
-    if (!r.group.on && w->n_keys <= kOneQueryKeys) {
-        // scattered whole: one query, a bitmap index per key
-        r.q_off = w->d_off1;
-        r.n_q = 1;
-        r.key_slot = d_qidx;
+    r.key_slot = d_qidx;  // several runs of keys may name one bitmap: every kernel ORs with atomics
+    if (!r.group.on) {
+        // scattered whole, a bitmap index per key: one query, or chunks of the
+        // keys as queries, whatever their bitmaps. (As runs of one bitmap each,
+        // 300,000 short lists in no order on 2^20 ads took 1,827 us, here 141.)
+        const bool one = w->n_keys <= kOneQueryKeys;
+        r.q_off = one ? w->d_off1 : w->d_offc;
+        r.n_q = one ? 1u : uint32_t(key_chunks(w->n_keys));
         return run_worker_lists(w, v, r, s);
     }
-    // several runs of keys may name one bitmap: every kernel ORs with atomics
-    abf::KeyRunsArgs ka{d_qidx, uint32_t(w->n_keys), w->d_off, w->d_slot, w->d_n_q};
+    abf::KeyRunsArgs ka{d_qidx, uint32_t(w->n_keys), w->q_cap, w->d_off, w->d_slot, w->d_n_q};
     TIMED(K_QUEUE, abf::launch_key_runs(ka, s));
     r.q_off = w->d_off;
     r.n_q = uint32_t(w->n_keys);
     r.d_n_q = w->d_n_q;
+    r.mixed_from = w->d_n_q + 1;
     r.out_slot = w->d_slot;
     return run_worker_lists(w, v, r, s);
 }
@@ -1645,9 +1655,13 @@ abf_status abf_prepare_sparse(abf_index* ix, const uint32_t* keys, uint64_t n_ke
         ++w->dense_keys;
         w->dense_postings += ix->h_term_len[keys[i]];
     }
-    std::vector<uint32_t> up(kWorkerHead + n_keys);  // three zeros, the mark, {0, n_keys} as 64-bit offsets, the keys
+    // three zeros, the mark, {0, n_keys} and the chunks as 64-bit offsets, the keys
+    const uint64_t head = head_words(w);
+    std::vector<uint32_t> up(head + n_keys);
     up[6] = uint32_t(n_keys);
-    if (n_keys) std::memcpy(up.data() + kWorkerHead, keys, n_keys * 4);
+    for (uint64_t c = 0; c <= key_chunks(n_keys); ++c)
+        up[kWorkerHead + 2 * c] = uint32_t(std::min<uint64_t>(c * abf::kKeyChunk, n_keys));
+    if (n_keys) std::memcpy(up.data() + head, keys, n_keys * 4);
     abf_status st = worker_alloc(w, w->term_cap);
     if (st != ABF_OK) {
         delete w;

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
                 nb = block_sum_u64<256>(nb, s_red);
                 nh = block_sum_u64<256>(nh, s_red);
             }
-            if (probe) nb = nh = 0;
+            if (probe || (a.mixed_from && q >= *a.mixed_from)) nb = nh = 0;
             if (nb < 0xffffffffull) {
                 if (nb >= a.bin_min_blocks) bin_from = 0;
                 else if (nh) bin_from = hm;
@@ -582,8 +582,10 @@ __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
 
 // Runs of consecutive keys with the same bitmap index, in one CTA: a flattened
 // batch of queries has a run per query. (A bitmap index may come back in a
-// later run: the kernels that follow OR with atomics.) Merged run by run, the
-// keys of 32 queries on 2^18 terms x 2^22 ads take 131 us; scattered key by
+// later run: the kernels that follow OR with atomics.) Keys in no order would
+// give a planning CTA a key each: 300,000 on 2^16 terms x 2^20 ads 2,669 us,
+// as chunks 525.
+// Merged run by run, the keys of 32 queries on 2^18 terms x 2^22 ads take 131 us; scattered key by
 // key, one atomic per posting of every list, they took 1,234.
 __global__ void __launch_bounds__(1024) key_runs_kernel(KeyRunsArgs a) {
     __shared__ uint32_t s_warp[32];
@@ -612,9 +614,21 @@ __global__ void __launch_bounds__(1024) key_runs_kernel(KeyRunsArgs a) {
         }
         carry += total;
     }
+    uint32_t n = carry, mixed = kNone;
+    if (tid == 0) a.off[carry] = a.n_keys;
+    if (carry > a.cap && carry > a.n_keys / 8u) {
+        __syncthreads();  // the runs' first keys are written
+        const uint64_t k0 = a.off[a.cap];
+        const uint32_t chunks = uint32_t((a.n_keys - k0 + kKeyChunk - 1u) / kKeyChunk);
+        __syncthreads();  // and read
+        for (uint32_t c = tid; c <= chunks; c += 1024u)
+            a.off[a.cap + c] = min(static_cast<unsigned long long>(k0 + uint64_t(c) * kKeyChunk), static_cast<unsigned long long>(a.n_keys));
+        mixed = a.cap;
+        n = a.cap + chunks;
+    }
     if (tid == 0) {
-        a.off[carry] = a.n_keys;
-        *a.n_runs = carry;
+        a.n_runs[0] = n;
+        a.n_runs[1] = mixed;
     }
 }
 
@@ -1243,7 +1257,7 @@ __device__ __forceinline__ uint32_t warp_last_le(At at, uint32_t n, Key key) {
 // staged in shared memory) took about 300 instructions per block of 128 ids
 // and a chain of ~20 loads per chunk: one query's few hundred blocks 16.5 us
 // where they now take 4 (c0), 32 queries' 94 thousand 49 instead of 55.
-// KEYED: one query whose term slots each have an output bitmap of their own.
+// KEYED: every term slot has an output bitmap of its own.
 template <int NW, bool KEYED>
 __global__ void __launch_bounds__(NW * 32, 6) scatter_kernel(IndexView ix, ScatterArgs a) {
     __shared__ __align__(16) uint4 s_blk[NW][32];  // {payload unit, first id, meta | kMixed, output bitmap}

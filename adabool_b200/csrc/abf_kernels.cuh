@@ -156,18 +156,24 @@ struct PlanArgs {
     // optional: the CTA that finishes last runs the scan over the queries
     uint32_t* done;           // CTAs finished: zero before the launch, and again when it ends
     QueueArgs queue;
+    const uint32_t* mixed_from;  // optional device word: queries from this one on have keys of several
+                              // output bitmaps, and bin none
     uint32_t no_dense_from;   // queries from this one on scatter their dense-bitmap lists too
                               // (0: none do; only with dense_in_tile)
 };
 
 // Consecutive keys with the same bitmap index form one run, which the kernels
-// above then treat as a query.
+// above then treat as a query. Of keys in no order (fewer than eight per run),
+// those past the first `cap` runs are cut into chunks of kKeyChunk instead,
+// whatever their bitmaps.
+constexpr uint32_t kKeyChunk = 1024;  // keys that a planning CTA takes in one step
 struct KeyRunsArgs {
     const uint32_t* qidx;
     uint32_t n_keys;
-    uint64_t* off;            // out: first key of each run, then n_keys (n_keys + 1 entries)
+    uint32_t cap;
+    uint64_t* off;            // out: first key of each run or chunk, then n_keys (n_keys + 1 entries)
     uint32_t* slot;           // out: the run's bitmap index
-    uint32_t* n_runs;         // out
+    uint32_t* n_runs;         // out: runs and chunks, and the first chunk (kNone: none)
 };
 
 // Term bitmaps -> term lists (ascending), one list per bitmap, packed.
@@ -275,7 +281,7 @@ struct ScatterArgs {
     const uint64_t* q_light_pref; // n_q + 1
     uint32_t n_q;
     const uint32_t* out_slot;  // query -> output bitmap index (null: identity)
-    const uint32_t* key_slot;  // instead, with n_q 1: term slot -> output bitmap index
+    const uint32_t* key_slot;  // instead: term slot -> output bitmap index
     uint32_t* out;
     uint64_t out_stride;
     uint32_t chunk_blocks;     // consecutive blocks a warp takes at a time (at most 32)

@@ -108,7 +108,10 @@ struct DerivedHost {
 };
 
 // Shortest list that gets plain ids: below it a list's few postings per tile
-// cost less as atomics than the look-up of the tile's range.
+// cost less as atomics than the look-up of the tile's range, and their plain
+// ids take memory. 2^18 terms x 2^22 ads, from 64 / 256 / 1,024 / 4,096 postings
+// on: 256 queries 319 / 321 / 332 / 376 us, 1,024 (more uneven ones) 1,578 /
+// 1,535 / 1,535 / 1,678, the index 0.65 / 0.60 / 0.54 / 0.49 GB.
 inline uint32_t plain_min_len(uint32_t n_ads) {
     const uint32_t m = n_ads / 32768u;
     return m > 256u ? m : 256u;

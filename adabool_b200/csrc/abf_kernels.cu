@@ -1815,6 +1815,14 @@ __device__ bool lookback_prefix(uint64_t* status, uint64_t item, uint32_t agg, u
 // GPU; else 2 or 1, so that a single bitmap is spread over more SMs: one query
 // on c0 (32 chunks of 8 units per warp, 256 of one) 9.8 -> 5.7 us, on c1 (512,
 // 2,048 of two) 18 -> 16.
+//
+// What bounds it depends on the density. 64 bitmaps of 2^22 ads, memset and
+// launch included, us and TB/s: empty 53; one bit in 64 85, 0.6; in 8 112, 1.5;
+// in 4 130, 2.3; half 146, 3.9; three in four 157, 5.3; 15 in 16 189, 5.5; full
+// 201, 5.5. From three in four on it is the copies' way out (5.5 TB/s at this
+// size, 5.9 in the 26.9 GB of 512 queries on c1); below, the chunks' own way
+// through claim, load, count and look-back (53 us for 8,192) and the expansion,
+// which takes longer the fuller the words are.
 
 // bulk copy shared -> global (TMA engine), completion tracked per thread
 __device__ __forceinline__ void bulk_s2g(void* gdst, const void* ssrc, uint32_t bytes) {

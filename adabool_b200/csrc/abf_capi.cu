@@ -132,7 +132,7 @@ struct abf_workspace {
     uint64_t* lpref_q = nullptr;
     uint32_t* probe_list = nullptr;
     // counters of one batch, zeroed together: probe slots taken, merge list
-    // length, plan CTAs finished, compaction ticket (8 bytes); before the
+    // length, plan CTAs finished, overlapping queries, compaction ticket (8 bytes); before the
     // single-query staging, so that abf_query uploads the zeros with its terms
     uint32_t* ctl = nullptr;
     uint32_t* n_probe = nullptr;
@@ -787,6 +787,7 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.path_out = ws->path_out;
     pa.max_terms = ws->max_terms;
     pa.err = ws->err;
+    pa.overlap = ws->ctl + 3;
     pa.dense_in_tile = 1;
     pa.tile_cls = ws->tile_cls;
     pa.q_dense16 = ws->q_dense16;
@@ -802,6 +803,9 @@ abf_status run_batch(abf_index* ix, abf_workspace* ws, const abf_batch* b, const
     pa.probe_bm = ws->probe_bm;
     pa.probe_stride = ws->probe_stride;
     abf::QueueArgs qa{ws->lcnt, ws->lpref_q, b->n_queries};
+    qa.overlap = pa.overlap;
+    qa.n_tile_list = ws->n_tile_list;
+    qa.q_ndense = ws->q_ndense;
     const bool hybrid = b->d_paths || b->path == ABF_PATH_AUTO || b->path == ABF_PATH_HYBRID || b->path == ABF_PATH_TILE;
     // A small batch on TILE has the merge kernel run in any case, for the short
     // lists; up to 32 tiles in all it takes the plain ones too. 4 to 64 terms

@@ -334,6 +334,17 @@ __device__ __forceinline__ void queue_scan_body(const QueueArgs& a, uint32_t n_q
     }
 }
 
+// No work for any query of a batch whose term slots overlap; after the scan.
+__device__ __forceinline__ void drop_batch(const QueueArgs& a, uint32_t n_q) {
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n_q; i += blockDim.x) a.q_ndense[i] = 0u;
+    if (threadIdx.x == 0) {
+        a.q_light_pref[n_q] = 0ull;
+        if (a.q_bblk) a.parts_pref[n_q] = 0u;
+        *a.n_tile_list = 0u;
+    }
+}
+
 // A CTA per query at a time, four terms per thread and step (one 16-byte load
 // of a term's table entry each): a step's latency, not its work, is what the
 // longest queries' CTAs wait for, and they end last (one term per step from
@@ -342,6 +353,10 @@ __device__ __forceinline__ void queue_scan_body(const QueueArgs& a, uint32_t n_q
 // last runs the scan over the queries (batches of up to kScanInPlan), which
 // saves that launch.
 constexpr uint32_t kPlanTerms = 4;
+// added to the count of finished CTAs by a query whose followers overlap
+// earlier ones (no load of a word of its own: it cost the scan 1.5 us)
+constexpr uint32_t kOverlap = 1u << 16;
+static_assert(kScanInPlan < kOverlap, "the count stays below it");
 template <uint32_t kInline>
 __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
                                                       const __grid_constant__ InlineTerms<kInline> given) {
@@ -368,6 +383,12 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
         if (qe < qb || qe > a.max_terms) {
             // offsets outside the scratch arrays: the query gets no work
             if (tid == 0 && a.err) atomicOr(a.err, kErrTermRange);
+            if constexpr (kInline == 0) {
+                if (tid == 0 && qe < qb && q + 1u < n_q) {
+                    if (a.done) atomicAdd(a.done, kOverlap);
+                    else if (a.overlap) *a.overlap = 1u;
+                }
+            }
             qe = qb = 0;
         }
         // what the later kernels find zeroed: the query's saturation marks,
@@ -566,18 +587,23 @@ __global__ void __launch_bounds__(256, 4) plan_kernel(IndexView ix, PlanArgs a,
         __syncthreads();
         if (tid == 0) s_slot = atomicAdd(a.done, 1u);
         __syncthreads();
-        if (s_slot != gridDim.x - 1u) return;
+        if ((s_slot & (kOverlap - 1u)) != gridDim.x - 1u) return;
         __threadfence();
         if (tid == 0) *a.done = 0;  // for a next batch that does not zero it
     }
     queue_scan_body<256>(a.queue, n_q, s_red, s_warp);
+    if constexpr (kInline == 0) {
+        if (gridDim.x > 1 && s_slot >= kOverlap) drop_batch(a.queue, n_q);
+    }
 }
 
 __global__ void __launch_bounds__(1024) queue_scan_kernel(QueueArgs a) {
     __shared__ unsigned long long s64[32];
     __shared__ uint32_t s32[32];
     wait_previous();
-    queue_scan_body<1024>(a, a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q, s64, s32);
+    const uint32_t n_q = a.d_n_q ? min(*a.d_n_q, a.n_q) : a.n_q;
+    queue_scan_body<1024>(a, n_q, s64, s32);
+    if (a.overlap && *a.overlap) drop_batch(a, n_q);
 }
 
 // Runs of consecutive keys with the same bitmap index, in one CTA: a flattened

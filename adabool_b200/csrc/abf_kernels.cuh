@@ -76,6 +76,12 @@ struct QueueArgs {
     uint32_t* ticket;         // out: zeroed
     uint32_t n_tiles;
     uint32_t slots;           // CTAs of the bin kernel that run at a time
+    // optional: where this word is set (or the plan kernel says so), the
+    // queries' term slots overlap and nothing of them may be followed: no
+    // blocks, parts, listed or dense lists
+    const uint32_t* overlap;
+    uint32_t* n_tile_list;
+    uint32_t* q_ndense;
 };
 
 // Terms of a single query given to the plan kernel with its arguments: no
@@ -124,6 +130,8 @@ struct PlanArgs {
     uint8_t* path_out;        // out (optional): resolved path per query
     uint64_t max_terms;       // term slots of the scratch arrays; queries past it get no work
     uint32_t* err;            // device error flag (optional)
+    uint32_t* overlap;        // out (optional, without `done`, zeroed before launch): set when a query ends before
+                              // it begins and others follow, so that theirs may be slots of earlier ones
     // optional: queries that (also) merge lists without dense bitmaps, in any
     // order; n_tile_list is zeroed before launch
     uint32_t* tile_list;

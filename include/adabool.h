@@ -346,7 +346,11 @@ abf_status abf_workspace_selftest_waits(abf_workspace* ws, uint32_t polls, void*
 
 typedef struct abf_batch {
     const uint32_t* d_terms;     /* flat query terms (device) */
-    const uint64_t* d_offsets;   /* n_queries + 1 offsets into d_terms (device) */
+    const uint64_t* d_offsets;   /* n_queries + 1 ascending offsets into d_terms (device). A query that
+                                    ends past the workspace's max_terms or before it begins gets no
+                                    work; one that ends before it begins, with others after it, ends
+                                    the union paths' work for the whole batch (abf_workspace_check:
+                                    ABF_ERR_CAPACITY) */
     uint32_t n_queries;
     const uint8_t* d_paths;      /* per-query abf_path (device) or NULL */
     abf_path path;               /* used when d_paths is NULL; AUTO = fixed rule per query */

@@ -76,3 +76,35 @@ def test_offsets_past_the_terms(env, n, what):
     finally:
         if what == "planner":
             P.uninstall(ix)
+
+
+@pytest.mark.parametrize("n", [3, 40, 2100])
+@pytest.mark.parametrize("path", [ab.PATH_UNION, ab.PATH_HYBRID, ab.PATH_TILE])
+def test_queries_over_one_another(env, n, path):
+    """A query that ends before it begins gives those after it slots of those before: the batch gets no work, an
+    error to read, and the next batch is answered as ever."""
+    import torch
+    ix = env["ix"]
+    qoff, qt = W.gen_queries(W.QueriesSpec(n, "uniform", 0.0, 0.0, 4, 30, seed=63), env["lens"])
+    terms = torch.from_numpy(qt.view(np.int32)).cuda()
+    nw = (N_ADS + 31) // 32
+    stride = (nw + 3) // 4 * 4
+    ws = ix.workspace(n, qt.size)
+    back = qoff.copy()
+    back[n // 2], back[n // 2 + 1] = qoff[n // 2 + 1], qoff[n // 2]
+    for offs, good in ((back, False), (qoff, True)):
+        bm = torch.full((n, stride), -1, dtype=torch.int32, device="cuda")
+        idoff = torch.full((n + 1,), -1, dtype=torch.int64, device="cuda")
+        ids = torch.zeros(n * 4096 if not good else n * N_ADS, dtype=torch.int32, device="cuda")
+        ix.batch_run(ws, terms, torch.from_numpy(offs.view(np.int64)).cuda(), n, bm, stride, path=path, d_ids=ids,
+                     d_id_offsets=idoff)
+        if not good:
+            with pytest.raises(ab.AbfError) as e:
+                ws.check()
+            assert e.value.status == ABF_ERR_CAPACITY
+            assert not bm[:, :nw].any() and not idoff.any()
+            continue
+        ws.check()
+        got = bm.cpu().numpy().view(np.uint32)
+        for i in sorted({0, n // 2, n - 1}):
+            assert np.array_equal(got[i, :nw], O.ids_to_bitmap(O.kway_union(env["off"], env["ads"], qt[qoff[i]:qoff[i + 1]]), nw)), i

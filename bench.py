@@ -58,9 +58,9 @@ METRIC = "batched queries/s & postings GB/s vs HBM peak; learned vs fixed path p
 # same workload at 1/4 scale (profiles/)
 TRAFFIC_PER_ALGORITHMIC_BYTE: dict = {"compact": 1.000}
 TRAFFIC_SOURCE: dict = {
-    "compact": "ncu --set full of compact_kernel, config c1 at 1/4 scale, sub-batch 64: "
-               "34.2 MB read + 752.3 MB written per launch = 1.000 x its algorithmic bytes "
-               "(profiles/compact_kernel_c1x0.25.md)",
+    "compact": "ncu of compact_kernel, config c1 at 1/4 scale, sub-batch 64: 34.3 MB read + 791.7 MB written "
+               "of 883.7 MB algorithmic, the other 57.7 MB still in L2 (126 MB) when the kernel ends: 1.000 x "
+               "for a launch far larger than L2 (profiles/compact_kernel_c1x0.25.md)",
 }
 UNIT = "queries/s"
 

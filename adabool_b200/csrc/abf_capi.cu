@@ -473,8 +473,7 @@ struct Arena {
 // only when no graph that captured it is left (see keep_for_graph).
 constexpr size_t kPoolBytes = size_t(32) << 20;
 
-void pool_drain(abf::ScratchPool& pool) {
-    std::lock_guard<std::mutex> g(pool.mu);
+void pool_drain_locked(abf::ScratchPool& pool) {
     for (auto& e : pool.kept) cudaFree(e.first);
     for (void* p : pool.over) cudaFree(p);
     pool.kept.clear();
@@ -482,10 +481,15 @@ void pool_drain(abf::ScratchPool& pool) {
     pool.bytes = 0;
 }
 
+void pool_drain(abf::ScratchPool& pool) {
+    std::lock_guard<std::mutex> g(pool.mu);
+    pool_drain_locked(pool);
+}
+
 // with the index: what graphs still name goes too, as they name its arrays
 void pool_close(abf::ScratchPool& pool) {
-    pool_drain(pool);
     std::lock_guard<std::mutex> g(pool.mu);
+    pool_drain_locked(pool);
     pool.closed = true;
     for (void* p : pool.held) cudaFree(p);
     pool.held.clear();

@@ -1070,6 +1070,7 @@ abf_status worker_alloc(abf_worker* w, uint64_t n_q) {
 // shares the worker's scratch from here on, so that it may be replayed after
 // the worker is gone (its kernels name nothing else of the worker's).
 abf_status keep_for_graph(const abf_worker* w, cudaStream_t s) {
+    if (s == nullptr || s == cudaStreamLegacy) return ABF_OK;  // cannot be captured; asking takes 0.5 us
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
     if (cudaStreamGetCaptureInfo_v2(s, &st, nullptr, &graph, nullptr, nullptr) != cudaSuccess) {

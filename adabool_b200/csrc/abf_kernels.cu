@@ -818,8 +818,12 @@ __global__ void __launch_bounds__(kStreamThreads, 4) dense_stream_kernel(IndexVi
         V acc = V();
         const uint4* dl = reinterpret_cast<const uint4*>(a.q_dense16 + a.q_dstart[q]);  // eight rows each
         const V* base = reinterpret_cast<const V*>(ix.dense) + (in ? j : 0u);
+        // the list is read eight rows ahead (a single query of c1's kind on 2^22
+        // ads 39.6 -> 37.6 us, the marks' words at once in the scatter with it)
+        uint4 nr = nd ? dl[0] : make_uint4(0u, 0u, 0u, 0u);
         for (uint32_t k = 0; k < nd; k += KT) {
-            const uint4 r = dl[k / KT];
+            const uint4 r = nr;
+            if (k + KT < nd) nr = dl[k / KT + 1u];
             const uint32_t row[KT] = {r.x & 0xffffu, r.x >> 16, r.y & 0xffffu, r.y >> 16,
                                       r.z & 0xffffu, r.z >> 16, r.w & 0xffffu, r.w >> 16};
             V x[KT];
@@ -1350,13 +1354,16 @@ __global__ void __launch_bounds__(NW * 32, 6) scatter_kernel(IndexView ix, Scatt
             const uint32_t t0 = first >> tshift, t1 = __ldg(ix.blk_last + b) >> tshift;
             const uint32_t w0 = t0 >> 5, w1 = t1 >> 5;
             bool all = true, some = false;
+            // the first and the last word of marks at once: most blocks have no other
+            const uint32_t va = sat[w0], vb = sat[w1];
             if (w1 - w0 < 32u) {
-                for (uint32_t w = w0; w <= w1; ++w) {
-                    uint32_t m = kFull;
-                    if (w == w0) m &= kFull << (t0 & 31u);
-                    if (w == w1) m &= kFull >> (31u - (t1 & 31u));
-                    const uint32_t v = sat[w] & m;
-                    all &= v == m;
+                uint32_t ma = kFull << (t0 & 31u), mb = kFull >> (31u - (t1 & 31u));
+                if (w0 == w1) ma = mb = ma & mb;
+                all = (va & ma) == ma && (vb & mb) == mb;
+                some = ((va & ma) | (vb & mb)) != 0u;
+                for (uint32_t w = w0 + 1u; w < w1; ++w) {
+                    const uint32_t v = sat[w];
+                    all &= v == kFull;
                     some |= v != 0u;
                 }
             } else {  // a wide range is not checked as a whole
